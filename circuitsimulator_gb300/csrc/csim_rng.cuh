@@ -53,19 +53,15 @@ struct DevRng {
 
     __device__ __forceinline__ uint32_t next(int& err) { return at(cur++, err); }
 
-    // ceil(n/8) bytes rand() % 256, bit j of byte b (MSB first) -> bit 8b+j
+    // ceil(n/8) bytes rand() % 256, bit j of byte b (MSB first) -> bit 8b+j.  Lane b
+    // draws byte b, so the warp waits for one draw instead of eight.
     __device__ __forceinline__ uint64_t bits(int n, int& err) {
+        const int bytes = (n + 7) / 8, b = threadIdx.x & 31;
         uint64_t w = 0ull;
-        const int bytes = (n + 7) / 8;
-        for (int b = 0; b < bytes; b++) {
-            const uint32_t byte = next(err) % 256u;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int loc = 8 * b + j;
-                if (loc < n && (byte & (0x80u >> j))) w |= bit1(loc);
-            }
-        }
-        return w;
+        if (b < bytes) w = (uint64_t)(__brev(at(cur + b, err) & 255u) >> 24) << (8 * b);
+        if (mode == 1 && __any_sync(kFull, (err & kErrReplay) != 0)) err |= kErrReplay;  // seen by every lane
+        cur += bytes;
+        return warp_or64(w) & lowmask(n);
     }
 };
 
@@ -96,21 +92,58 @@ __device__ void random_state(WS<NR>& s, int n, DevRng& rng, const double* cum, i
     s.h = rng.bits(n, err);
     s.D1 = rng.bits(n, err);
     s.D2 = rng.bits(n, err);
+    // J: word base + x (x - 1) / 2 + c holds J[x][c], c < x, in its low bit, so the lower
+    // triangle is a string of bits with row x at bit x (x - 1) / 2.  The warp draws it
+    // into shared memory (each word once; a Philox block's four words by one lane),
+    // lanes take their rows, and ballots give the columns (1024 states of 40 qubits: 34 us
+    // when every lane drew the words of its own row, 11 us now; latency-bound).
     const int k = s.k;
     const int64_t base = rng.cur;
+    const int nbits = k * (k - 1) / 2, lane = lane_id();
+    __shared__ uint32_t tri_s[8][68];  // blocks have at most 8 warps; 2016 bits, up to 3 in front, a word beyond
+    uint32_t* const tri = tri_s[threadIdx.x >> 5];
+    const int lead = rng.mode == 1 ? 0 : (int)(base & 3);
+    __syncwarp();
+    if (rng.mode == 1) {
+        for (int w = 0; 32 * w < nbits; w++) {
+            const int i = 32 * w + lane;
+            const uint32_t v = __ballot_sync(kFull, i < nbits && (rng.at(base + i, err) & 1u));
+            if (lane == 0) tri[w] = v;
+        }
+    } else {
+        for (int w = 0; 32 * w < nbits + lead; w += 4) {
+            const int64_t q = (base >> 2) + 8 * w + lane;  // lane's block: words 4 q .. 4 q + 3
+            const uint4 r = philox4x32_10(make_uint4((uint32_t)q, rng.id0, rng.id1, (uint32_t)(q >> 32)), rng.k0, rng.k1);
+            uint32_t v = ((r.x >> 1) & 1u) | (r.y & 2u) | ((r.z & 2u) << 1) | ((r.w & 2u) << 2);
+            v |= __shfl_down_sync(kFull, v, 1) << 4;
+            v |= __shfl_down_sync(kFull, v, 2) << 8;
+            v |= __shfl_down_sync(kFull, v, 4) << 16;
+            if ((lane & 7) == 0) tri[w + (lane >> 3)] = v;
+        }
+    }
+    __syncwarp();
+    uint64_t low[NR];  // J[x][c], c < x
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        uint64_t row = 0ull;
-        if (x < k) {
-            row = (uint64_t)getbit(s.D1, x) << x;  // J[x][x] = ((2 D[x]) mod 8) / 4
-            for (int c = 0; c < k; c++) {
-                if (c == x) continue;
-                const int64_t idx = x > c ? base + (int64_t)x * (x - 1) / 2 + c : base + (int64_t)c * (c - 1) / 2 + x;
-                row |= (uint64_t)(rng.at(idx, err) & 1u) << c;
-            }
+        low[sl] = 0ull;
+        if (x >= 1 && x < k) {
+            const int at = lead + x * (x - 1) / 2, w = at >> 5, sh = at & 31;
+            const uint64_t v = (uint64_t)tri[w] | ((uint64_t)tri[w + 1] << 32);
+            low[sl] = ((v >> sh) | (sh ? (uint64_t)tri[w + 2] << (64 - sh) : 0ull)) & lowmask(x);
         }
-        s.J[sl] = row;
+    }
+#pragma unroll
+    for (int sl = 0; sl < NR; sl++) {
+        const int x = row_of<NR>(sl);
+        s.J[sl] = x < k ? low[sl] | ((uint64_t)getbit(s.D1, x) << x) : 0ull;  // J[x][x] = ((2 D[x]) mod 8) / 4
+    }
+    for (int x = 0; x < k; x++) {
+        const uint64_t col = ballot_bit<NR>(low, x);  // rows c > x with J[c][x] = 1
+        if (lane == (x & 31)) {
+            if (NR == 2 && x >= 32) s.J[NR - 1] |= col;
+            else s.J[0] |= col;
+        }
     }
     rng.cur = base + (int64_t)k * (k - 1) / 2;
     // every lane may have seen a different replay overrun

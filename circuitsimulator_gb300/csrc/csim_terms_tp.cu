@@ -162,20 +162,8 @@ __global__ void __launch_bounds__(kTP) k_terms_tp(const uint64_t* codewords, con
 using pc::CanonG;
 
 namespace {
-__device__ __forceinline__ uint64_t shfl_xor_u64(uint64_t v, int m) {
-    const uint32_t lo = __shfl_xor_sync(kFull, (uint32_t)v, m), hi = __shfl_xor_sync(kFull, (uint32_t)(v >> 32), m);
-    return ((uint64_t)hi << 32) | lo;
-}
 __device__ __forceinline__ uint64_t ballot64(bool lo, bool hi) {
     return (uint64_t)__ballot_sync(kFull, lo) | ((uint64_t)__ballot_sync(kFull, hi) << 32);
-}
-__device__ __forceinline__ uint64_t xor_reduce64(uint64_t v) {
-    for (int o = 16; o > 0; o >>= 1) v ^= shfl_xor_u64(v, o);
-    return v;
-}
-__device__ __forceinline__ uint64_t or_reduce64(uint64_t v) {
-    for (int o = 16; o > 0; o >>= 1) v |= shfl_xor_u64(v, o);
-    return v;
 }
 // coordinate-indexed mask of a variable-indexed one (variable a -> its pivot coordinate)
 __device__ __forceinline__ uint64_t to_coords(uint64_t v, const unsigned char* piv) {
@@ -246,13 +234,13 @@ __global__ void __launch_bounds__(64) k_canon(const GState* theta, const int* co
     if (w1) dq += 2 * (2 * (int)(((D2 >> r1) ^ (uint64_t)__popcll(j1 & wv & pc::lowmask(r1))) & 1ull) +
                        (int)((D1 >> r1) & 1ull));
     dq = (int)__reduce_add_sync(kFull, (unsigned)dq);
-    const uint64_t flips = xor_reduce64((w0 ? j0 & ~(1ull << r0) : 0ull) ^ (w1 ? j1 & ~(1ull << r1) : 0ull));
+    const uint64_t flips = warp_xor64((w0 ? j0 & ~(1ull << r0) : 0ull) ^ (w1 ? j1 & ~(1ull << r1) : 0ull));
     D2 ^= (D1 & wv) ^ (flips & km);
     // to coordinate indexing
     piv[r0] = (unsigned char)(r0 < k ? p0 : 0);
     piv[r1] = (unsigned char)(r1 < k ? p1 : 0);
     __syncwarp();
-    const uint64_t P = or_reduce64((r0 < k ? 1ull << p0 : 0ull) | (r1 < k ? 1ull << p1 : 0ull));
+    const uint64_t P = warp_or64((r0 < k ? 1ull << p0 : 0ull) | (r1 < k ? 1ull << p1 : 0ull));
     o.Jc[r0] = 0ull;
     o.Jc[r1] = 0ull;
     o.acol[r0] = 0ull;

@@ -55,10 +55,14 @@ __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
     return ((uint64_t)hi << 32) | lo;
 }
 
-__device__ __forceinline__ int warp_sum(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    return v;
+// Reductions of the warp in one instruction per 32 bits instead of five shuffles:
+// a warp's steps are one serial chain, so their latency is what a state costs.
+__device__ __forceinline__ int warp_sum(int v) { return (int)__reduce_add_sync(kFull, (unsigned)v); }
+__device__ __forceinline__ uint64_t warp_xor64(uint64_t v) {
+    return (uint64_t)__reduce_xor_sync(kFull, (uint32_t)v) | ((uint64_t)__reduce_xor_sync(kFull, (uint32_t)(v >> 32)) << 32);
+}
+__device__ __forceinline__ uint64_t warp_or64(uint64_t v) {
+    return (uint64_t)__reduce_or_sync(kFull, (uint32_t)v) | ((uint64_t)__reduce_or_sync(kFull, (uint32_t)(v >> 32)) << 32);
 }
 
 // ------------------------------------------------------------------ state
@@ -124,9 +128,7 @@ __device__ __forceinline__ uint64_t xor_rows(const uint64_t (&m)[NR], uint64_t m
     const int l = lane_id();
     uint64_t acc = getbit(mask, l) ? m[0] : 0ull;
     if constexpr (NR == 2) acc ^= getbit(mask, l + 32) ? m[1] : 0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc ^= shfl_xor64(acc, o);
-    return acc;
+    return warp_xor64(acc);
 }
 
 template <int NR>
