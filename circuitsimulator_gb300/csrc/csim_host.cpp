@@ -64,8 +64,9 @@ extern "C" void csim_ctx_destroy(csim_ctx* ctx) {
     for (int i = 0; i < kNumBufs + 32; i++)
         if (ctx->buf[i]) cudaFree(ctx->buf[i]);
     if (ctx->d_err) cudaFree(ctx->d_err);
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < 4; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
+    for (int i = 0; i < 6; i++) {
         if (ctx->pin_ev[i]) cudaEventDestroy(ctx->pin_ev[i]);
         if (ctx->pin[i]) cudaFreeHost(ctx->pin[i]);
     }
@@ -524,6 +525,26 @@ extern "C" int csim_term_products(csim_ctx* ctx, int32_t t, int32_t exact, const
 namespace {
 
 
+// The tree plan of code L on this context for `count` states, with its arrays in kBufTreePlan
+int tree_plan_for(csim_ctx* ctx, const uint64_t* L, int k, int t, int64_t count) {
+    std::vector<uint64_t> key(L, L + k);
+    key.push_back((uint64_t)k);
+    key.push_back((uint64_t)t);
+    if (key == ctx->tree_key && ctx->buf[kBufTreePlan]) {  // the device arrays do not depend on the levels
+        csim::tree::choose_levels(ctx->tree_plan, count);
+        return 0;
+    }
+    ctx->tree_key.clear();
+    ctx->tree_plan = csim::tree::Plan();
+    csim::tree::make_plan(L, k, t, count, ctx->tree_plan);
+    unsigned char image[kTreePlanBytes];
+    tree_plan_image(ctx->tree_plan, image);
+    unsigned char* d;
+    CKR(dput(ctx, kBufTreePlan, image, sizeof(image), &d));
+    ctx->tree_key = key;
+    return 0;
+}
+
 // Draws `count` states, projects them onto P, sums their terms on the GPU, and
 // returns singleProjectorSample's value for each (innerprod.c:88-144).
 int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, int exact, int64_t count,
@@ -531,7 +552,9 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int t = P->nqubits;
     CKR(check_code(ctx, t, exact, L, k));
     if (rng != CSIM_RNG_LIBC && rng != CSIM_RNG_PHILOX) return fail(ctx, CSIM_ERR_ARG, "unknown rng %d", rng);
-    const bool tp = !exact && ctx->pair_kernel != 1;
+    // |L> terms: the tree sum (csim_tree.cuh), unless a pair kernel is asked for
+    const bool tree = !exact && ctx->pair_kernel == 0 && !ctx->tuning && k <= kTreeMaxRows;
+    const bool tp = !exact && !tree && ctx->pair_kernel != 1;
     TpTune tn = default_tune(t);
     if (tp && count > 0) CKR(tune_for(ctx, t, &tn, P, L, k));  // before any draw: tuning leaves the streams as they are
     // the run kernel takes whole blocks of 64 runs
@@ -548,7 +571,11 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int P2 = 2 * t;
     const int64_t chunk = chunk_for(chi);
     const int pt = tn.per_thread;
-    const int64_t nchunks = tp ? csim::terms_tp_blocks(chi, pt) : (chi + chunk - 1) / chunk;
+    const int64_t batch = 1 << 14;
+    const int64_t shape_count = std::min(count, batch);
+    if (tree) CKR(tree_plan_for(ctx, L, k, t, shape_count));
+    const int64_t nchunks = tree ? tree_leaf_shape(ctx->tree_plan, shape_count).parts_per_state
+                                 : (tp ? csim::terms_tp_blocks(chi, pt) : (chi + chunk - 1) / chunk);
 
     std::vector<int> hm(P->nstabs);
     for (int r = 0; r < P->nstabs; r++) hm[r] = phase_m(P->phase[r]);
@@ -561,9 +588,9 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     CKR(upload_cum(ctx, t, &dcum));
     double hcum[CSIM_MAX_QUBITS + 1];
     cum_table(t, hcum);
-    uint64_t* dcw;
-    csim_state* dphis;
-    CKR(stage_terms(ctx, t, exact, L, k, 0, chi, &dcw, &dphis, /*ordered=*/true, &tn));
+    uint64_t* dcw = nullptr;
+    csim_state* dphis = nullptr;
+    if (!tree) CKR(stage_terms(ctx, t, exact, L, k, 0, chi, &dcw, &dphis, /*ordered=*/true, &tn));
     const int dsl = ctx->direct_slots > 0 ? std::min(t, ctx->direct_slots) : direct_slots(t);
     unsigned char* dscr = nullptr;
     size_t scr_bytes = 0;
@@ -575,7 +602,8 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         dscr = (unsigned char*)sv;
     }
 
-    const int64_t batch = 1 << 14;
+    TreeRun run;
+    std::vector<unsigned char> jobs;
     std::vector<uint32_t> words;
     std::vector<int64_t> offs;
     std::vector<int> code;
@@ -583,8 +611,11 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     for (int64_t o = 0; o < count; o += batch) {
         const int64_t c = std::min(batch, count - o);
         void* v;
-        CKR(dbuf(ctx, kBufA, c * sizeof(csim_state), &v));
-        csim::GState* dth = (csim::GState*)v;
+        csim::GState* dth = nullptr;  // the tree's states stay in registers
+        if (!tree) {
+            CKR(dbuf(ctx, kBufA, c * sizeof(csim_state), &v));
+            dth = (csim::GState*)v;
+        }
         CKR(dbuf(ctx, kBufCode, c * 4, &v));
         int* dcode = (int*)v;
         void* dcanon = nullptr;
@@ -602,7 +633,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         CKR(dbuf(ctx, kBufParts, nparts * sizeof(__int128), &v));
         __int128* dpart = (__int128*)v;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-        CK(cudaMemsetAsync(dpart, 0, nparts * sizeof(__int128), ctx->stream));
+        if (!tree) CK(cudaMemsetAsync(dpart, 0, nparts * sizeof(__int128), ctx->stream));
         // With the C library's draws the host makes every state's rand() words.
         // The batch goes in sub-batches: the host draws sub-batch s+1 while the
         // GPU works on sub-batch s, all launches queued on the stream.  The
@@ -613,8 +644,9 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         for (int64_t s0 = 0, sb = 0; s0 < c; sb++) {
             const int64_t cs = std::min(ramp, c - s0);
             ramp = std::min<int64_t>(4 * ramp, rng == CSIM_RNG_LIBC ? 1024 : c);
-            csim::GState* sth = (csim::GState*)((csim_state*)dth + s0);
+            csim::GState* sth = tree ? nullptr : (csim::GState*)((csim_state*)dth + s0);
             int* scode = dcode + s0;
+            csim::TreeDraw draw{};
             if (rng == CSIM_RNG_LIBC) {
                 words.clear();
                 offs.assign(1, 0);
@@ -628,15 +660,18 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
                 int64_t* doff;
                 CKR(staged_put(ctx, 2 * (sb & 1), kBufWords, words.data(), words.size(), &dw));
                 CKR(staged_put(ctx, 2 * (sb & 1) + 1, kBufOffsets, offs.data(), offs.size(), &doff));
-                if (csim::launch_random_states(launch_of(ctx), t, cs, 1, 0, 0, dw, doff, dcum, sth, nullptr))
+                draw = csim::TreeDraw{1, P->nstabs, 0, 0, dw, doff, dcum, dpm, dpz, dpx, scode};
+                if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 1, 0, 0, dw, doff, dcum, sth, nullptr))
                     return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
             } else {
-                if (csim::launch_random_states(launch_of(ctx), t, cs, 0, ctx->philox_seed, ctx->philox_next, nullptr,
-                                               nullptr, dcum, sth, nullptr))
+                draw = csim::TreeDraw{0, P->nstabs, ctx->philox_seed, ctx->philox_next, nullptr, nullptr, dcum, dpm, dpz,
+                                      dpx, scode};
+                if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 0, ctx->philox_seed, ctx->philox_next,
+                                                        nullptr, nullptr, dcum, sth, nullptr))
                     return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
                 ctx->philox_next += cs;
             }
-            if (csim::launch_project(launch_of(ctx), nr, sth, cs, P->nstabs, dpm, dpz, dpx, scode))
+            if (!tree && csim::launch_project(launch_of(ctx), nr, sth, cs, P->nstabs, dpm, dpz, dpx, scode))
                 return fail(ctx, CSIM_ERR_CUDA, "projection launch failed");
             if (tp && tn.kernel == 3) {
                 CK(cudaMemsetAsync(drest, 0, 4, ctx->stream));
@@ -645,11 +680,26 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
                                        dcode_rest + s0, drest))
                     return fail(ctx, CSIM_ERR_CUDA, "pivot-form launch failed");
             }
-            if (first) CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+            if (first && !tree) CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+            const bool first_sub = first;
             first = false;
             __int128* spart = dpart + (size_t)s0 * nchunks * 4;
             int rc = 0;
-            if (tp && tn.kernel == 2) {
+            if (tree) {
+                TreeGroup g;
+                g.plan = &ctx->tree_plan;
+                g.dplan = (const unsigned char*)ctx->buf[kBufTreePlan];
+                g.count = cs;
+                g.shape_count = shape_count;
+                g.part = spart;
+                void* scratch;
+                unsigned char* djobs;
+                CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
+                run.build((unsigned char*)scratch, jobs);
+                CKR(staged_put(ctx, 4 + (sb & 1), kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+                // the event that starts the pair kernels' time is recorded behind the first roots
+                rc = run.launch(launch_of(ctx), djobs, nullptr, nullptr, &draw, first_sub ? ctx->ev[1] : nullptr);
+            } else if (tp && tn.kernel == 2) {
                 // one launch per occupancy class; class c's launch starts at its first whole item
                 const int64_t span = 64 * (int64_t)pt;
                 const int nc = (int)ctx->cw_bounds.size();

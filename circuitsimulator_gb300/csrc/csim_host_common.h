@@ -18,6 +18,7 @@
 
 #include "../../include/csim.h"
 #include "csim_internal.h"
+#include "csim_tree_host.h"
 
 namespace csim_host {
 
@@ -371,7 +372,7 @@ enum BufId {
     kBufA, kBufB, kBufEps, kBufP, kBufM, kBufXi, kBufZeta, kBufAlpha, kBufCode, kBufWords, kBufOffsets,
     kBufCum, kBufCodewords, kBufAcc, kBufAccDiag, kBufPhis, kBufIdx, kBufConsumed, kBufPm, kBufPz, kBufPx,
     kBufL, kBufParts, kBufPartsDiag, kBufCwOrdered, kBufRunScratch, kBufCanon, kBufCodeDirect, kBufCodeRest,
-    kBufRestCount, kNumBufs
+    kBufRestCount, kBufTreePlan, kBufTreeJobs, kBufTreeScratch, kNumBufs
 };
 
 class Engine;                     // csim_engine.cpp: the batched query engine
@@ -394,15 +395,17 @@ struct csim_ctx {
     int pair_kernel = 0;  // CSIM_OPT_PAIR_KERNEL
     int per_thread = 0;  // CSIM_OPT_PER_THREAD; 0 = auto_per_thread(t)
     cudaEvent_t ev[4] = {};
-    // pinned staging of host-made uploads (staged_put): four slots, each with the event of its last copy
-    void* pin[4] = {};
-    size_t pin_cap[4] = {};
-    cudaEvent_t pin_ev[4] = {};
+    // pinned staging of host-made uploads (staged_put): six slots, each with the event of its last copy
+    void* pin[6] = {};
+    size_t pin_cap[6] = {};
+    cudaEvent_t pin_ev[6] = {};
     Engine* engine = nullptr;  // created by the first batched csim_run_queries
     std::vector<uint64_t> cw_key;  // (k, rows of L, t, light bound) of the ordered codeword table in kBufCwOrdered
     int64_t cw_split = 0;          // first index of that table whose codewords have <= the light bound's zeros
     std::vector<int> cw_bounds;        // occupancy-class order: the launches' zero bounds
     std::vector<int64_t> cw_starts;    // and the first index of each class
+    std::vector<uint64_t> tree_key;    // (rows of L, k, t) of tree_plan, whose device arrays are in kBufTreePlan
+    csim::tree::Plan tree_plan;
     // autotuner (CSIM_OPT_AUTOTUNE): the tuned launch parameters live in a
     // process-wide table per device (csim_host.cpp), filled a t bucket at a time
     int direct_slots = 0;  // CSIM_OPT_DIRECT_SLOTS; 0 = direct_slots(t)

@@ -27,6 +27,7 @@
 
 #include "csim_internal.h"
 #include "csim_block_prefix.cuh"
+#include "csim_canon_warp.cuh"
 #include "csim_pair_core.cuh"
 #include "csim_warp.cuh"
 
@@ -153,29 +154,10 @@ __global__ void __launch_bounds__(kTP) k_terms_tp(const uint64_t* codewords, con
 }
 
 // ---------------------------------------------------------------- direct restriction
-// k_canon: one warp per state, theta in pivot coordinates: pc::canon_theta's
-// steps with lane l holding variables l and l + 32 (rows of G and J), the
-// pivot step's row set B a ballot and its rank-two update done by every lane
-// on its own rows; states whose d = n - k exceeds `dslots` are left to the
-// block-prefix kernel (code_direct < 0), the others to the direct kernel
-// (code_rest < 0).
+// k_canon: one warp per state, theta in pivot coordinates (canon_warp); states
+// whose d = n - k exceeds `dslots` are left to the block-prefix kernel
+// (code_direct < 0), the others to the direct kernel (code_rest < 0).
 using pc::CanonG;
-
-namespace {
-__device__ __forceinline__ uint64_t ballot64(bool lo, bool hi) {
-    return (uint64_t)__ballot_sync(kFull, lo) | ((uint64_t)__ballot_sync(kFull, hi) << 32);
-}
-// coordinate-indexed mask of a variable-indexed one (variable a -> its pivot coordinate)
-__device__ __forceinline__ uint64_t to_coords(uint64_t v, const unsigned char* piv) {
-    uint64_t r = 0ull;
-    while (v) {
-        const int a = __ffsll((long long)v) - 1;
-        v &= v - 1ull;
-        r |= 1ull << piv[a];
-    }
-    return r;
-}
-}  // namespace
 
 __global__ void __launch_bounds__(64) k_canon(const GState* theta, const int* code, int64_t ntheta, int dslots,
                                                CanonG* out, int* code_direct, int* code_rest, int* rest_count) {
@@ -197,73 +179,42 @@ __global__ void __launch_bounds__(64) k_canon(const GState* theta, const int* co
     CanonG& o = out[a0];
     const uint64_t nm = pc::lowmask(n), km = pc::lowmask(k);
     const int r0 = lane, r1 = lane + 32;  // this lane's variables
-    uint64_t g0 = r0 < k ? g->G[r0] & nm : 0ull, g1 = r1 < k ? g->G[r1] & nm : 0ull;
-    uint64_t j0 = r0 < k ? g->J[r0] & km : 0ull, j1 = r1 < k ? g->J[r1] & km : 0ull;
-    uint64_t D1 = g->D1 & km, D2 = g->D2 & km;
-    int p0 = 0, p1 = 0;
-    // Gauss-Jordan on the rows of G: rows b of B += row a (u_a = u'_a + u'_b), J <- R J R^T with
-    // rows in B getting J_a and rows in C getting B, D_b += D_a + 4 J_ab (pc::canon_theta)
-    for (int a = 0; a < k; a++) {
-        const int src = a & 31;
-        const bool up = a >= 32;
-        const uint64_t ga = shfl64(up ? g1 : g0, src);
-        const int pcol = ga ? __ffsll((long long)ga) - 1 : 0;
-        if (lane == src) {
-            if (up) p1 = pcol;
-            else p0 = pcol;
-        }
-        const bool in0 = r0 < k && r0 != a && ((g0 >> pcol) & 1ull), in1 = r1 < k && r1 != a && ((g1 >> pcol) & 1ull);
-        const uint64_t B = ballot64(in0, in1);
-        if (!B) continue;  // warp-uniform
-        if (in0) g0 ^= ga;
-        if (in1) g1 ^= ga;
-        const uint64_t Ja = shfl64(up ? j1 : j0, src);
-        const uint64_t C = Ja ^ (((Ja >> a) & 1ull) ? B : 0ull);
-        j0 ^= (((B >> r0) & 1ull) ? Ja : 0ull) ^ (((C >> r0) & 1ull) ? B : 0ull);
-        j1 ^= (((B >> r1) & 1ull) ? Ja : 0ull) ^ (((C >> r1) & 1ull) ? B : 0ull);
-        pc::add_D64(D1, D2, B, (int)((D1 >> a) & 1ull), (int)((D2 >> a) & 1ull));
-        D2 ^= B & Ja;
-    }
-    // shift v = u + w, w_a = h at a's pivot: in order of a, Q += D_a and D_a -> -D_a, D_b += 4 J_ab;
-    // D_a as read at step a carries the earlier steps' flips J_{a'a}, a' < a in w
-    const bool w0 = r0 < k && ((g->h >> p0) & 1ull), w1 = r1 < k && ((g->h >> p1) & 1ull);
-    const uint64_t wv = ballot64(w0, w1);
-    int dq = 0;
-    if (w0) dq += 2 * (2 * (int)(((D2 >> r0) ^ (uint64_t)__popcll(j0 & wv & pc::lowmask(r0))) & 1ull) +
-                       (int)((D1 >> r0) & 1ull));
-    if (w1) dq += 2 * (2 * (int)(((D2 >> r1) ^ (uint64_t)__popcll(j1 & wv & pc::lowmask(r1))) & 1ull) +
-                       (int)((D1 >> r1) & 1ull));
-    dq = (int)__reduce_add_sync(kFull, (unsigned)dq);
-    const uint64_t flips = warp_xor64((w0 ? j0 & ~(1ull << r0) : 0ull) ^ (w1 ? j1 & ~(1ull << r1) : 0ull));
-    D2 ^= (D1 & wv) ^ (flips & km);
+    CanonWarp w;
+    w.g0 = r0 < k ? g->G[r0] & nm : 0ull;
+    w.g1 = r1 < k ? g->G[r1] & nm : 0ull;
+    w.j0 = r0 < k ? g->J[r0] & km : 0ull;
+    w.j1 = r1 < k ? g->J[r1] & km : 0ull;
+    w.D1 = g->D1 & km;
+    w.D2 = g->D2 & km;
+    canon_warp(w, k, g->h);
     // to coordinate indexing
-    piv[r0] = (unsigned char)(r0 < k ? p0 : 0);
-    piv[r1] = (unsigned char)(r1 < k ? p1 : 0);
+    piv[r0] = (unsigned char)(r0 < k ? w.p0 : 0);
+    piv[r1] = (unsigned char)(r1 < k ? w.p1 : 0);
     __syncwarp();
-    const uint64_t P = warp_or64((r0 < k ? 1ull << p0 : 0ull) | (r1 < k ? 1ull << p1 : 0ull));
+    const uint64_t P = w.P;
     o.Jc[r0] = 0ull;
     o.Jc[r1] = 0ull;
     o.acol[r0] = 0ull;
     o.acol[r1] = 0ull;
     __syncwarp();
-    if (r0 < k) o.Jc[p0] = to_coords(j0, piv);
-    if (r1 < k) o.Jc[p1] = to_coords(j1, piv);
+    if (r0 < k) o.Jc[w.p0] = to_coords(w.j0, piv);
+    if (r1 < k) o.Jc[w.p1] = to_coords(w.j1, piv);
     // each non-pivot coordinate: the variables its coordinate depends on, and the constraint's bit
     uint64_t bm = 0ull;
     for (uint64_t np = ~P & nm; np;) {
         const int cc = __ffsll((long long)np) - 1;
         np &= np - 1ull;
-        const uint64_t av = ballot64(r0 < k && ((g0 >> cc) & 1ull), r1 < k && ((g1 >> cc) & 1ull));
+        const uint64_t av = ballot64(r0 < k && ((w.g0 >> cc) & 1ull), r1 < k && ((w.g1 >> cc) & 1ull));
         if (lane == (cc & 31)) o.acol[cc] = to_coords(av, piv);
-        if ((((g->h >> cc) & 1ull) ^ (uint64_t)(__popcll(wv & av) & 1)) != 0ull) bm |= 1ull << cc;
+        if ((((g->h >> cc) & 1ull) ^ (uint64_t)(__popcll(w.wv & av) & 1)) != 0ull) bm |= 1ull << cc;
     }
     if (lane == 0) {
         pc::Canon cs;
         cs.P = P;
-        cs.D1 = to_coords(D1, piv);
-        cs.D2 = to_coords(D2, piv);
+        cs.D1 = to_coords(w.D1, piv);
+        cs.D2 = to_coords(w.D2, piv);
         cs.bm = bm;
-        cs.Q = (g->Q + dq) & 7;
+        cs.Q = (g->Q + w.dq) & 7;
         cs.k = k;
         cs.n = n;
         cs.pad = 0;

@@ -1,0 +1,245 @@
+// csim_tree_host.h — the launches of a tree sum (csim_tree.cu) over groups of
+// states, each group with its own decomposition: chunks that fit the scratch
+// memory, the job tables and their order.  Used by the single-query sampler
+// (csim_host.cpp) and the query engine (csim_engine.cpp).
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+#include <cstring>
+#include <vector>
+
+#include "csim_tree.cuh"
+#include "csim_tree.h"
+#include "csim_tree_plan.h"
+
+namespace csim_host {
+
+// A plan's arrays on the device: gen (64 words), then perm (64 bytes)
+constexpr size_t kTreePlanBytes = 64 * 8 + 64;
+
+struct TreeGroup {
+    const csim::tree::Plan* plan = nullptr;
+    const unsigned char* dplan = nullptr;  // the plan's device arrays (kTreePlanBytes)
+    const int32_t* index = nullptr;        // device: states of the group (null: first, first + 1, ...)
+    int64_t first = 0, count = 0;
+    int64_t shape_count = 0;               // states that tree_leaf_shape is asked for (0: count)
+    __int128* part = nullptr;              // device: parts_per_state partial sums for each state
+};
+
+// How the leaf kernel covers the states of a group.  Small groups split a
+// node's leaves over several threads until the GPU has enough of them; large
+// ones give each thread several nodes, so its reduction at the end is shared.
+struct TreeLeafShape {
+    int split = 0, reps = 1, group = 1;
+    int64_t threads_per_state = 1, parts_per_state = 1;
+};
+inline TreeLeafShape tree_leaf_shape(const csim::tree::Plan& p, int64_t count) {
+    TreeLeafShape s;
+    const int je = p.level.back();
+    const int64_t nodes = (int64_t)1 << (p.r - je);
+    while (s.split < je && ((count * nodes) << s.split) < (1 << 17)) s.split++;
+    const int64_t parts = nodes << s.split;
+    while (s.reps < 8 && parts >= 2 * 128 * s.reps && count * parts / (2 * s.reps) >= (1 << 19)) s.reps *= 2;
+    s.threads_per_state = parts / s.reps;
+    s.group = (int)std::min<int64_t>(s.threads_per_state, csim::kTreeLeafThreads);
+    s.parts_per_state = std::max<int64_t>(1, s.threads_per_state / csim::kTreeLeafThreads);
+    return s;
+}
+
+// Bytes of node planes per state in the two scratch halves (written levels
+// alternate between them)
+inline void tree_scratch_per_state(const csim::tree::Plan& p, int64_t (&half)[2]) {
+    half[0] = half[1] = 0;
+    for (size_t i = 0; i < p.level.size(); i++) {
+        const int64_t b = ((int64_t)csim::tree::node_words(p.vert[i]) * 4) << (p.r - p.level[i]);
+        half[i & 1] = std::max(half[i & 1], b);
+    }
+}
+
+constexpr size_t kTreeScratchMax = (size_t)1 << 30;
+// codes of more rows run on the pair kernels (node indices are 32 bits)
+constexpr int kTreeMaxRows = 30;
+
+class TreeRun {
+  public:
+    // Splits the groups into chunks whose node planes fit `budget` bytes (one
+    // state at least).  Returns the scratch bytes needed.
+    size_t layout(const std::vector<TreeGroup>& groups, size_t budget) {
+        chunks_.clear();
+        scratch_ = 0;
+        size_t used = 0;
+        Chunk cur;
+        for (const TreeGroup& g : groups) {
+            int64_t half[2];
+            tree_scratch_per_state(*g.plan, half);
+            const int64_t per = half[0] + half[1];
+            for (int64_t f = 0; f < g.count;) {
+                const int64_t room = (int64_t)((budget > used ? budget - used : 0)) / std::max<int64_t>(1, per);
+                int64_t c = std::min(g.count - f, room);
+                if (c <= 0) {
+                    if (!cur.pieces.empty()) {
+                        chunks_.push_back(cur);
+                        scratch_ = std::max(scratch_, used);
+                        cur.pieces.clear();
+                        used = 0;
+                        continue;
+                    }
+                    c = 1;
+                }
+                // equal chunks of a large group
+                if (cur.pieces.empty() && c < g.count - f) {
+                    const int64_t n = (g.count - f + c - 1) / c;
+                    c = (g.count - f + n - 1) / n;
+                }
+                Piece pc{g, f, c, {used, 0}};
+                used += align((size_t)(half[0] * c));
+                pc.off[1] = used;
+                used += align((size_t)(half[1] * c));
+                cur.pieces.push_back(pc);
+                f += c;
+                if (f < g.count) {  // the group's next states start a chunk of their own
+                    chunks_.push_back(cur);
+                    scratch_ = std::max(scratch_, used);
+                    cur.pieces.clear();
+                    used = 0;
+                }
+            }
+        }
+        if (!cur.pieces.empty()) {
+            chunks_.push_back(cur);
+            scratch_ = std::max(scratch_, used);
+        }
+        return scratch_;
+    }
+
+    // The job tables, to be copied to the device (`scratch`: the device scratch)
+    void build(unsigned char* scratch, std::vector<unsigned char>& blob) {
+        blob.clear();
+        steps_.clear();
+        for (const Chunk& ch : chunks_) {
+            std::vector<csim::TreeRootJob> roots;
+            std::vector<csim::TreeLeafJob> leaves[4];  // by table words 1, 2, 4, 8
+            int64_t rb = 0, lb[4] = {0, 0, 0, 0};
+            size_t depth = 0;
+            for (const Piece& p : ch.pieces) {
+                const csim::tree::Plan& pl = *p.g.plan;
+                csim::TreeRootJob r{};
+                r.index = p.g.index ? p.g.index + p.first : nullptr;
+                r.first = p.g.first + p.first;
+                r.perm = p.g.dplan + 64 * 8;
+                r.out = (uint32_t*)(scratch + p.off[0]);
+                r.count = p.count;
+                r.block0 = rb;
+                r.t = pl.t;
+                rb += (p.count + csim::kTreeRootWarps - 1) / csim::kTreeRootWarps;
+                roots.push_back(r);
+                depth = std::max(depth, pl.level.size());
+                const TreeLeafShape s = tree_leaf_shape(pl, p.g.shape_count ? p.g.shape_count : p.g.count);
+                csim::TreeLeafJob l{};
+                const int je = pl.level.back();
+                l.in = (const uint32_t*)(scratch + p.off[(pl.level.size() - 1) & 1]);
+                l.part = p.g.part + 4 * p.first * s.parts_per_state;
+                l.in_count = p.count << (pl.r - je);
+                l.threads = p.count * s.threads_per_state;
+                const int wc = std::max(0, pl.tv - 5);
+                l.block0 = lb[wc];
+                l.m = pl.vert.back();
+                l.je = je;
+                l.tv = pl.tv;
+                l.tj = pl.tj;
+                l.split = s.split;
+                l.reps = s.reps;
+                l.group = s.group;
+                l.shift = pl.t - pl.tv + 2 * (pl.k - pl.r);  // each codeword 2^{k - r} times
+                for (int j = 0; j < je; j++) l.gen[j] = (uint16_t)pl.gen[j];
+                lb[wc] += (l.threads + csim::kTreeLeafThreads - 1) / csim::kTreeLeafThreads;
+                leaves[wc].push_back(l);
+            }
+            add(blob, Step{0, false, ch.pieces[0].g.plan->t, (int)roots.size(), rb, 0}, roots);
+            for (size_t d = 1; d < depth; d++)
+                for (int wide = 1; wide >= 0; wide--) {
+                    std::vector<csim::TreeStageJob> st;
+                    int64_t sb = 0;
+                    int mmax = 0;
+                    for (const Piece& p : ch.pieces) {
+                        const csim::tree::Plan& pl = *p.g.plan;
+                        if (pl.level.size() <= d || (pl.vert[d - 1] > 32) != (wide != 0)) continue;
+                        csim::TreeStageJob j{};
+                        j.in = (const uint32_t*)(scratch + p.off[(d - 1) & 1]);
+                        j.out = (uint32_t*)(scratch + p.off[d & 1]);
+                        j.gen = (const uint64_t*)p.g.dplan + pl.level[d];
+                        j.in_count = p.count << (pl.r - pl.level[d - 1]);
+                        j.count = p.count << (pl.r - pl.level[d]);
+                        j.block0 = sb;
+                        j.mp = pl.vert[d - 1];
+                        j.mc = pl.vert[d];
+                        j.sub = pl.level[d - 1] - pl.level[d];
+                        const int64_t threads = j.sub > 0 ? j.count / 2 : j.count;  // a pair of siblings each
+                        sb += (threads + csim::kTreeStageThreads - 1) / csim::kTreeStageThreads;
+                        mmax = std::max(mmax, j.mp);
+                        st.push_back(j);
+                    }
+                    if (!st.empty()) add(blob, Step{1, wide != 0, mmax, (int)st.size(), sb, 0}, st);
+                }
+            for (int wc = 0; wc < 4; wc++)
+                if (!leaves[wc].empty()) add(blob, Step{2, false, 1 << wc, (int)leaves[wc].size(), lb[wc], 0}, leaves[wc]);
+        }
+    }
+
+    // Queues the launches; `djobs`: build()'s tables on the device.  The states are in
+    // memory (states, code), or with `draw` made by the root launches (one group).
+    // after_first (optional) is recorded behind the first launch.
+    int launch(const csim::Launch& L, const unsigned char* djobs, const csim::GState* states, const int* code,
+               const csim::TreeDraw* draw = nullptr, cudaEvent_t after_first = nullptr) const {
+        for (size_t i = 0; i < steps_.size(); i++) {
+            const Step& s = steps_[i];
+            const void* j = djobs + s.off;
+            if (i == 1 && after_first && cudaEventRecord(after_first, L.stream) != cudaSuccess) return -1;
+            const int rc =
+                s.kind == 0 && draw ? csim::launch_tree_draw(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, s.size, *draw)
+                : s.kind == 0 ? csim::launch_tree_root(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, states, code)
+                : s.kind == 1 ? csim::launch_tree_stage(L, (const csim::TreeStageJob*)j, s.njobs, s.blocks, s.wide, s.size)
+                              : csim::launch_tree_leaf(L, (const csim::TreeLeafJob*)j, s.njobs, s.blocks, s.size);
+            if (rc) return rc;
+        }
+        return 0;
+    }
+
+  private:
+    struct Piece {
+        TreeGroup g;
+        int64_t first, count;
+        size_t off[2];
+    };
+    struct Chunk {
+        std::vector<Piece> pieces;
+    };
+    struct Step {
+        int kind;  // 0 roots, 1 a stage, 2 leaves
+        bool wide;
+        int size;  // roots: the first group's qubits; a stage's largest parent; the leaves' table words
+        int njobs;
+        int64_t blocks;
+        size_t off;
+    };
+    static size_t align(size_t x) { return (x + 255) & ~(size_t)255; }
+    template <class J>
+    void add(std::vector<unsigned char>& blob, Step s, const std::vector<J>& jobs) {
+        s.off = align(blob.size());
+        blob.resize(s.off + jobs.size() * sizeof(J));
+        memcpy(blob.data() + s.off, jobs.data(), jobs.size() * sizeof(J));
+        steps_.push_back(s);
+    }
+    std::vector<Chunk> chunks_;
+    std::vector<Step> steps_;
+    size_t scratch_ = 0;
+};
+
+// A plan's device image (kTreePlanBytes)
+inline void tree_plan_image(const csim::tree::Plan& p, unsigned char* out) {
+    memcpy(out, p.gen, 64 * 8);
+    memcpy(out + 64 * 8, p.perm, 64);
+}
+
+}  // namespace csim_host

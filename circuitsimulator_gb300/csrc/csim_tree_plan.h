@@ -1,0 +1,156 @@
+// csim_tree_plan.h — host side of the tree sum (csim_tree.cuh): the chain of
+// subcodes, the order of the coordinates, and the levels at which nodes are
+// written out.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+#include <vector>
+
+namespace csim {
+namespace tree {
+
+struct Plan {
+    int t = 0, k = 0, r = 0;      // qubits, rows of L, its rank
+    int m[65] = {0};              // m[j]: vertices of a node of level j (m[r] = t)
+    uint8_t perm[64] = {0};       // position -> coordinate; C_j lives on positions < m[j]
+    uint64_t gen[64] = {0};       // gen[j]: generator of C_{j+1} over C_j, in positions
+    // levels of the written nodes, root (r) first; the last one is the leaf kernel's
+    // entry.  vert: their vertices
+    std::vector<int> level, vert;
+    int tj = 0, tv = 0;           // the table level, largest j with m[j] <= 8, and the table's vertices:
+                                  // m[tj], or for tj = 0 the first (up to) 8 positions
+};
+
+// Chooses C_1 < C_2 < ...: each step adds the codeword with the fewest ones
+// outside the support so far (all 2^d words of the remaining quotient code
+// while d <= 16; beyond that the span of its first 16 rows).
+inline void build_chain(const uint64_t* L, int k, int t, Plan& p) {
+    p.t = t;
+    p.k = k;
+    std::vector<uint64_t> rows(L, L + k);
+    uint64_t supp = 0;
+    uint64_t picked[64];
+    p.r = 0;
+    for (;;) {
+        // a basis of the quotient code, reduced outside supp
+        std::vector<uint64_t> e;
+        for (uint64_t v : rows) {
+            for (uint64_t b : e) {
+                const int c = __builtin_ctzll(b & ~supp);
+                if ((v >> c) & 1) v ^= b;
+            }
+            if (!(v & ~supp)) continue;
+            const int c = __builtin_ctzll(v & ~supp);
+            for (uint64_t& b : e)
+                if ((b >> c) & 1) b ^= v;
+            e.push_back(v);
+        }
+        if (e.empty()) break;
+        const int d = std::min((int)e.size(), 16);
+        uint64_t x = 0, best = e[0];
+        int bw = 65;
+        for (uint64_t i = 1; i < (1ull << d); i++) {
+            x ^= e[(size_t)__builtin_ctzll(i)];
+            const int w = __builtin_popcountll(x & ~supp);
+            if (w < bw) {
+                bw = w;
+                best = x;
+            }
+        }
+        picked[p.r++] = best;
+        const uint64_t add = best & ~supp;
+        const int m0 = p.m[p.r - 1];
+        int m = m0;
+        for (uint64_t a = add; a; a &= a - 1) p.perm[m++] = (uint8_t)__builtin_ctzll(a);
+        p.m[p.r] = m;
+        supp |= best;
+        rows = e;
+    }
+    // coordinates that are 0 in every codeword: contracted with the root's block
+    int m = p.m[p.r];
+    for (int c = 0; c < t; c++)
+        if (!((supp >> c) & 1)) p.perm[m++] = (uint8_t)c;
+    if (p.r > 0) p.m[p.r] = t;
+    for (int j = 0; j < p.r; j++) {
+        uint64_t g = 0;
+        for (int i = 0; i < t; i++) g |= ((picked[j] >> p.perm[i]) & 1ull) << i;
+        p.gen[j] = g;
+    }
+    p.tj = 0;
+    // tables of up to 8 vertices: 6 at most is 34% slower at t = 40 (2^16 terms), where m[1] is often 7
+    // or 8, 7 at most 27% slower at t = 24 (2^14)
+    while (p.tj < p.r && p.m[p.tj + 1] <= 8) p.tj++;
+    p.tv = p.tj > 0 ? p.m[p.tj] : std::min(t, 8);
+}
+
+// Levels of the written nodes by dynamic programming on the time for `count`
+// states.  A stage from vp to vc vertices runs about 0.31 steps per vertex and
+// node (pairs of siblings share a lane), each a pass over the rows still live, and
+// every node pays for its loads and stores; a launch costs its latency, which
+// decides when the states are few.
+inline double stage_steps(int vp, int vc) { return 0.31 * (vp - vc) + 0.5; }
+inline double stage_ops(int vp, int vc) {  // ALU operations per node
+    const double w = vp > 32 ? (vc > 32 ? 2 : 1 + (vp - 32.0) / (vp - vc)) : 1;
+    return stage_steps(vp, vc) * (80 + 2.6 * w * (vp + vc) / 2) + 2 * w * vp + 3 * vc + 50;
+}
+constexpr double kTreeOpsPerSecond = 1.6e13;  // 152 SMs, 64 lanes per cycle, 90% busy
+inline double stage_seconds(int vp, int vc, double nodes) {
+    const double latency = 4e-6 + 2 * stage_steps(vp, vc) * (0.35e-6 + 0.012e-6 * vp);
+    return latency + nodes * stage_ops(vp, vc) / kTreeOpsPerSecond;
+}
+inline void choose_levels(Plan& p, int64_t count) {
+    const int r = p.r;
+    // candidates: index 0 the root (r, t), then (j, m[j]) for j = r - 1 .. tj, with the table's
+    // vertices alone at level tj
+    std::vector<int> lv{r}, vt{p.t};
+    for (int j = r - 1; j > p.tj; j--) {
+        lv.push_back(j);
+        vt.push_back(p.m[j]);
+    }
+    if (p.t > p.tv) {
+        lv.push_back(p.tj);
+        vt.push_back(p.tv);
+    }
+    const int n = (int)lv.size();
+    std::vector<double> cost((size_t)n, 1e300);
+    std::vector<int> from((size_t)n, -1);
+    cost[0] = 0;
+    double best = 1e300;
+    int end = 0;
+    for (int i = 0; i < n; i++) {
+        for (int h = 0; h < i; h++) {
+            if (cost[(size_t)h] >= 1e300) continue;
+            const double nodes = (double)count * (double)(1ull << (r - lv[(size_t)i]));
+            const double c = cost[(size_t)h] + stage_seconds(vt[(size_t)h], vt[(size_t)i], nodes);
+            if (c < cost[(size_t)i]) {
+                cost[(size_t)i] = c;
+                from[(size_t)i] = h;
+            }
+        }
+        if (vt[(size_t)i] <= 16) {  // the leaf kernel may start here
+            const double tables = (double)count * (double)(1ull << (r - p.tj));
+            const double leaf = vt[(size_t)i] > p.tv ? stage_seconds(vt[(size_t)i], p.tv, tables) : 0;
+            const double c = cost[(size_t)i] + leaf +
+                             (double)count * (double)(1ull << (r - lv[(size_t)i])) * 60 / kTreeOpsPerSecond;
+            if (c < best) {
+                best = c;
+                end = i;
+            }
+        }
+    }
+    p.level.clear();
+    p.vert.clear();
+    for (int i = end; i >= 0; i = from[(size_t)i]) {
+        p.level.insert(p.level.begin(), lv[(size_t)i]);
+        p.vert.insert(p.vert.begin(), vt[(size_t)i]);
+    }
+}
+
+inline void make_plan(const uint64_t* L, int k, int t, int64_t count, Plan& p) {
+    build_chain(L, k, t, p);
+    choose_levels(p, count);
+}
+
+}  // namespace tree
+}  // namespace csim

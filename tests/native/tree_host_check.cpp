@@ -1,0 +1,189 @@
+// Host build of the tree sum (circuitsimulator_gb300/csrc/csim_tree.cuh and
+// csim_tree_plan.h), for CPU tests only: the plan the host code makes and the
+// node steps the kernels run, in the kernels' order, without a GPU.
+#include <cstdint>
+#include <cstring>
+#include <vector>
+
+#include "../../circuitsimulator_gb300/csrc/csim_tree.cuh"
+#include "../../circuitsimulator_gb300/csrc/csim_tree_plan.h"
+#include "../../include/csim.h"
+
+using namespace csim::tree;
+
+namespace {
+
+struct HostNode {
+    uint64_t row[64];
+    uint64_t d1, d2, h, x;
+    int q, iso, dead;
+};
+
+template <class W>
+Work<W> work_of(const HostNode& n, int mp, int mc) {
+    const W pm = wlow<W>(mp), cm = wlow<W>(mc);
+    Work<W> w{{(W)n.d1, (W)n.d2, (W)n.h, n.q, n.iso, 0}, 0, 0};
+    w.sum = ((W)n.x ^ w.s.h) & pm & ~cm;
+    w.live = cm | w.sum;
+    return w;
+}
+template <class W, class R>
+void take(HostNode& n, const Work<W>& w, const R& rows, int mc) {
+    const W cm = wlow<W>(mc);
+    n.d1 = (uint64_t)(w.s.d1 & cm);
+    n.d2 = (uint64_t)(w.s.d2 & cm);
+    n.h = (uint64_t)(w.s.h & cm);
+    n.x &= (uint64_t)cm;
+    n.q = w.s.q & 7;
+    n.iso = w.s.iso;
+    n.dead |= w.s.dead;
+    for (int i = 0; i < mc; i++) n.row[i] = (uint64_t)((W)rows.get(i) & cm);
+}
+
+// contracts positions [mc, mp) of two siblings with the row type that the
+// kernels use for mp vertices (`leaf`: the leaf kernel's 16-bit rows)
+void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf) {
+    alignas(16) uint32_t w[256] = {0};
+    const HostNode* n[2] = {&a, &b};
+    if (leaf) {
+        const Rows16 r0{w, 1}, r1{w + 8, 1};
+        for (int e = 0; e < 2; e++)
+            for (int i = 0; i < mp; i++) reinterpret_cast<uint16_t*>(w + 8 * e)[i] = (uint16_t)n[e]->row[i];
+        auto wa = work_of<uint32_t>(a, mp, mc), wb = work_of<uint32_t>(b, mp, mc);
+        sum_out_pair<uint32_t>(r0, 8, wa, wb, ~0u);
+        take(a, wa, r0, mc);
+        take(b, wb, r1, mc);
+    } else if (mp > 32) {
+        const Rows64 r0{w, w + 64, 1}, r1{w + 128, w + 192, 1};
+        for (int e = 0; e < 2; e++)
+            for (int i = 0; i < mp; i++) {
+                w[128 * e + i] = (uint32_t)n[e]->row[i];
+                w[128 * e + 64 + i] = (uint32_t)(n[e]->row[i] >> 32);
+            }
+        auto wa = work_of<uint64_t>(a, mp, mc), wb = work_of<uint64_t>(b, mp, mc);
+        contract_pair(r0, 128, wa, wb, mc);
+        take(a, wa, r0, mc);
+        take(b, wb, r1, mc);
+    } else {
+        const Rows32 r0{w, 1}, r1{w + 32, 1};
+        for (int e = 0; e < 2; e++)
+            for (int i = 0; i < mp; i++) w[32 * e + i] = (uint32_t)n[e]->row[i];
+        auto wa = work_of<uint32_t>(a, mp, mc), wb = work_of<uint32_t>(b, mp, mc);
+        contract_pair(r0, 32, wa, wb, mc);
+        take(a, wa, r0, mc);
+        take(b, wb, r1, mc);
+    }
+}
+
+HostNode root_of(const csim_state& th, const Plan& p) {
+    csim::pc::Canon cs;
+    uint64_t G[64], Jc[64], acol[64], h = 0;
+    auto perm = [&](uint64_t v) {
+        uint64_t r = 0;
+        for (int i = 0; i < p.t; i++) r |= ((v >> p.perm[i]) & 1ull) << i;
+        return r;
+    };
+    for (int a = 0; a < 64; a++) G[a] = a < th.k ? perm(th.G[a]) : 0;
+    h = perm(th.h);
+    csim::pc::canon_theta(th.n, th.k, th.Q, h, th.D1, th.D2, G, th.J, Jc, acol, cs);
+    HostNode n{};
+    const uint64_t nm = csim::pc::lowmask(th.n);
+    for (int c = 0; c < th.n; c++) {
+        n.row[c] |= Jc[c] | acol[c];
+        for (int y = 0; y < th.n; y++)
+            if ((acol[c] >> y) & 1) n.row[y] |= 1ull << c;
+    }
+    n.h = ~cs.P & nm;
+    n.d1 = cs.D1;
+    n.d2 = cs.D2 | (cs.bm & n.h);
+    n.q = cs.Q;
+    return n;
+}
+
+}  // namespace
+
+// Sums of all 2^k terms for each theta, as the kernels' exact coordinates
+// scaled by 2^t: out[8 a + 2 q] low and out[8 a + 2 q + 1] high word of
+// coordinate q.  info (optional): r, table vertices, written levels.
+extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_t* L, int k, int t, int64_t count,
+                              uint64_t* out, int* info) {
+    Plan p;
+    make_plan(L, k, t, count, p);  // the levels for `count` states
+    if (info) {
+        info[0] = p.r;
+        info[1] = p.tv;
+        info[2] = (int)p.level.size();
+        for (size_t i = 0; i < p.level.size(); i++) info[3 + i] = p.vert[i];
+    }
+    uint32_t lin[32], sub[32];
+    for (uint32_t i = 0; i < 32; i++) {
+        lin[i] = linear_word(i);
+        sub[i] = subset_word(i);
+    }
+    const int words = table_words(p.tv);
+    for (int a = 0; a < ntheta; a++) {
+        std::vector<HostNode> cur{root_of(theta[a], p)};
+        for (size_t s = 1; s < p.level.size(); s++) {
+            const int sb = p.level[s - 1] - p.level[s];
+            std::vector<HostNode> next;
+            for (const HostNode& par : cur)
+                for (int c = 0; c < (1 << sb); c += 2) {
+                    HostNode n = par;
+                    for (int b = 1; b < sb; b++)
+                        if ((c >> b) & 1) n.x ^= p.gen[p.level[s] + b];
+                    HostNode o = n;
+                    if (sb) o.x ^= p.gen[p.level[s]];
+                    if (!par.dead) stage(n, o, p.vert[s - 1], p.vert[s], false);
+                    next.push_back(n);
+                    if (sb) next.push_back(o);
+                }
+            cur.swap(next);
+        }
+        const int je = p.level.back(), m = p.vert.back();
+        __int128 z[4] = {0, 0, 0, 0};
+        for (const HostNode& entry : cur) {
+            if (entry.dead) continue;
+            uint64_t x = entry.x;
+            for (int s = 0; s < (1 << (je - p.tj)); s++) {
+                if (s) x ^= p.gen[p.tj + __builtin_ctz((unsigned)s)];
+                HostNode n = entry;
+                n.x = x;
+                n.iso = 0;
+                HostNode o = n;
+                if (m > p.tv) stage(n, o, m, p.tv, true);
+                uint32_t r[kTableVars] = {0};
+                for (int i = 0; i < kTableVars && i < m; i++) r[i] = (uint32_t)n.row[i];
+                const uint32_t vm = wlow<uint32_t>(p.tv), d1 = (uint32_t)n.d1 & vm;
+                int e0 = 0, e1 = 0, o0 = 0, o1 = 0;
+                uint32_t S = ((uint32_t)(x ^ n.h)) & vm;
+                auto leaves = [&](auto tb) {
+                    build_table(r, d1, (uint32_t)n.d2 & vm, lin, tb);
+                    for (int l = 0; l < (1 << p.tj); l++) {
+                        if (l) S ^= (uint32_t)p.gen[__builtin_ctz((unsigned)l)] & vm;
+                        table_leaf(tb, S, d1, p.tv, sub, e0, e1, o0, o1);
+                    }
+                };
+                if (words == 1) leaves(Table<1>());
+                else if (words == 2) leaves(Table<2>());
+                else if (words == 4) leaves(Table<4>());
+                else leaves(Table<8>());
+                if (n.dead) continue;
+                int v[4] = {e0, o0 + o1, e1, o1 - o0};
+                times_omega(v, n.q);
+                if (n.iso & 1) times_sqrt2(v);
+                __int128 y[4];
+                for (int q = 0; q < 4; q++) y[q] = (__int128)v[q] << (n.iso >> 1);
+                if (entry.iso & 1) times_sqrt2(y);
+                for (int q = 0; q < 4; q++) z[q] += y[q] << (entry.iso >> 1);
+            }
+        }
+        const int shift = t - p.tv;
+        if (shift & 1) times_sqrt2(z);
+        for (int q = 0; q < 4; q++) {
+            const unsigned __int128 w = (unsigned __int128)z[q] << ((shift >> 1) + (k - p.r));
+            out[8 * a + 2 * q] = (uint64_t)w;
+            out[8 * a + 2 * q + 1] = (uint64_t)(w >> 64);
+        }
+    }
+    return 0;
+}

@@ -1,0 +1,132 @@
+"""The tree sum over all terms of |L> (csim_tree.cuh, csim_tree_plan.h),
+compiled for the host, against the oracle: the exact Z[w] coordinates of
+sum_j <theta|phi_j> are whole numbers, so they are equal, not close."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from helpers import phase_m, rand_word, random_projector_rows
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SRC = os.path.join(HERE, "native", "tree_host_check.cpp")
+SO = os.path.join(HERE, "native", "_build", "libtreehost.so")
+CSRC = os.path.join(os.path.dirname(HERE), "circuitsimulator_gb300", "csrc")
+DEPS = [SRC] + [os.path.join(CSRC, f) for f in ("csim_tree.cuh", "csim_tree_plan.h", "csim_pair_core.cuh")]
+
+
+@pytest.fixture(scope="module")
+def tree_sums():
+    os.makedirs(os.path.dirname(SO), exist_ok=True)
+    if not os.path.exists(SO) or os.path.getmtime(SO) < max(os.path.getmtime(f) for f in DEPS):
+        subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", SRC, "-o", SO])
+    lib = C.CDLL(SO)
+    lib.tree_host_sums.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_int64, C.c_void_p, C.c_void_p]
+
+    def run(thetas, L, t, count):
+        thetas = np.ascontiguousarray(thetas)
+        Lw = np.array([int(x) for x in L] or [0], dtype=np.uint64)
+        out = np.zeros((len(thetas), 4, 2), dtype=np.uint64)
+        info = np.zeros(80, dtype=np.int32)
+        assert lib.tree_host_sums(thetas.ctypes.data, len(thetas), Lw.ctypes.data, len(L), t, count, out.ctypes.data,
+                                  info.ctypes.data) == 0
+        vals = [[(int(w[0]) | (int(w[1]) << 64)) - ((1 << 128) if int(w[1]) >> 63 else 0) for w in row] for row in out]
+        return vals, info
+
+    return run
+
+
+def _exact_sum(eps, p, m, P):
+    """sum of eps 2^{p/2} w^m as Z[w] coordinates scaled by 2^{P/2}."""
+    z = [0, 0, 0, 0]
+    for e, pp, mm in zip(eps.tolist(), p.tolist(), m.tolist()):
+        if not e:
+            continue
+        q, mm = pp + P, mm % 8
+        terms = [(mm, 1 << (q // 2))] if q % 2 == 0 else [((mm + 1) % 8, 1 << (q // 2)), ((mm + 7) % 8, 1 << (q // 2))]
+        for k, c in terms:
+            z[k & 3] += -c if k >= 4 else c
+    return z
+
+
+def _thetas(oracle, rs, t, rows, count):
+    r = oracle.rng(1000 + t)
+    out = []
+    for _ in range(20 * count):
+        s = oracle.random_state(t, r)
+        pf = 1.0
+        for q in range(len(rows[0])):
+            pf *= oracle.measure_pauli(s, phase_m(rows[0][q]), rows[2][q], rows[1][q])
+            if pf == 0:
+                break
+        if pf:
+            out.append(s[0])
+        if len(out) == count:
+            break
+    return np.array(out)
+
+
+def _check(tree_sums, oracle, t, L, thetas):
+    k = len(L)
+    got, info = tree_sums(thetas, L, t, 4096)
+    assert tree_sums(thetas, L, t, 1)[0] == got  # fewer levels for a single state
+    Lw = np.array([int(x) for x in L] or [0], dtype=np.uint64)
+    for a in range(len(thetas)):
+        e, p, m = oracle.term_products(t, 0, Lw, k, thetas[a:a + 1], 0, 2 ** k, threads=4)
+        assert got[a] == _exact_sum(e, p, m, 2 * t), (t, k, a)
+    return info
+
+
+@pytest.mark.parametrize("t,k", [(1, 0), (1, 1), (2, 2), (5, 2), (7, 5), (8, 8), (15, 4), (16, 7), (17, 6), (24, 10),
+                                 (31, 8), (32, 7), (33, 8), (40, 9), (48, 8), (57, 7), (63, 6), (64, 7)])
+@pytest.mark.parametrize("frac", [0.0, 0.3, 0.8])
+def test_tree_sum_equals_oracle(tree_sums, oracle, t, k, frac):
+    """Random codes and projected states (few to many non-pivot coordinates)."""
+    rs = np.random.RandomState(100 * t + k)
+    L = [rand_word(rs, t) for _ in range(k)]
+    rows = random_projector_rows(rs, t, int(frac * t))
+    thetas = _thetas(oracle, rs, t, rows, 3)
+    assert len(thetas)
+    _check(tree_sums, oracle, t, L, thetas)
+
+
+@pytest.mark.parametrize("t", [6, 16, 20, 33, 64])
+def test_tree_sum_of_unusual_codes(tree_sums, oracle, t):
+    """No rows; a zero row; repeated rows (each codeword several times); rows
+    that leave coordinates 0 in every codeword; unit vectors; the all-ones word."""
+    rs = np.random.RandomState(t)
+    full = (1 << t) - 1
+    a, b = rand_word(rs, t), rand_word(rs, t)
+    low = full >> (t // 2)
+    codes = [[], [0], [full], [a, a, b, a ^ b, 0], [a & low, b & low, rand_word(rs, t) & low],
+             [1 << i for i in range(0, t, max(1, t // 6))], [full, 1 << (t - 1), 3 & full]]
+    thetas = _thetas(oracle, rs, t, random_projector_rows(rs, t, t // 3), 4)
+    ranks = [int(_check(tree_sums, oracle, t, L, thetas)[0]) for L in codes]
+    assert ranks[:4] == [0, 0, 1, 2]
+
+
+def test_tree_sum_on_extreme_states(tree_sums, oracle):
+    """States of every dimension k = 0..n of the affine space, and D, J of one kind only."""
+    rs = np.random.RandomState(8)
+    for t in (12, 20, 40):
+        r = oracle.rng(t)
+        base = oracle.random_state(t, r)
+        while int(base[0]["k"]) < t - 1:
+            base = oracle.random_state(t, r)
+        L = [rand_word(rs, t) for _ in range(7)]
+        states = [base[0].copy()]
+        s = base.copy()
+        for q in range(t):
+            oracle.shrink(s, 1 << q, int(rs.randint(2)))
+            states.append(s[0].copy())
+        for zero in ("D1", "D2", "J"):
+            w = base[0].copy()
+            w[zero] = 0
+            if zero in ("D1", "J"):  # J's diagonal is D1
+                w["D1"] = 0
+                for x in range(int(w["k"])):
+                    w["J"][x] = int(w["J"][x]) & ~(1 << x)
+            states.append(w)
+        _check(tree_sums, oracle, t, L, np.array(states))

@@ -1,0 +1,63 @@
+"""The tree sum's kernels (csim_tree.cu) against the pair kernels on the same
+draws: every sampled value is an exact sum in Z[w], so they are equal."""
+import numpy as np
+import pytest
+
+from circuitsimulator_gb300 import backend
+from helpers import rand_word, random_projector_rows
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    g = backend.Backend(0)
+    g.set_option(backend.OPT_AUTOTUNE, 0)
+    yield g
+    g.close()
+
+
+def _values(gpu, kernel, *args):
+    try:
+        gpu.set_option(backend.OPT_PAIR_KERNEL, kernel)
+        return gpu.singleProjectorSample(*args)
+    finally:
+        gpu.set_option(backend.OPT_PAIR_KERNEL, 0)
+
+
+def _code(kind, t, k, rs):
+    L = [rand_word(rs, t) for _ in range(k)]
+    if kind == "repeated":  # rank below k: each codeword several times
+        L[1::2] = L[0::2][:len(L[1::2])]
+    if kind == "low":  # coordinates that are 0 in every codeword
+        L = [v & ((1 << (t // 2)) - 1) for v in L]
+    return L
+
+
+@pytest.mark.parametrize("t,k,count,kind", [
+    (1, 0, 3, "random"), (1, 1, 5, "random"), (7, 5, 64, "random"), (8, 8, 33, "random"), (9, 3, 300, "random"),
+    (16, 6, 129, "random"), (17, 6, 128, "low"), (23, 11, 500, "random"), (27, 9, 70, "repeated"),
+    (32, 12, 40, "random"), (33, 12, 40, "random"), (40, 14, 300, "random"), (47, 8, 31, "low"),
+    (56, 13, 20, "random"), (64, 11, 65, "random"), (64, 2, 200, "random"), (64, 0, 9, "random")])
+def test_tree_sampler_equals_pair_kernel(gpu, t, k, count, kind):
+    rs = np.random.RandomState(17 * t + k)
+    L = _code(kind, t, k, rs)
+    rows = random_projector_rows(rs, t, max(1, t // 3))
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    for rng in (backend.RNG_PHILOX, backend.RNG_LIBC):
+        a = _values(gpu, 0, P, L, False, count, rng, 91)
+        b = _values(gpu, 2, P, L, False, count, rng, 91)
+        assert (a == b).all(), np.nonzero(a != b)[0][:8]
+
+
+def test_tree_sampler_in_chunks(gpu):
+    """More states than the scratch memory takes at once, more than one batch of
+    states, and a code change between calls."""
+    rs = np.random.RandomState(3)
+    rows = random_projector_rows(rs, 40, 12)
+    P = backend.projector(rows[0], rows[1], rows[2], 40)
+    L = [rand_word(rs, 40) for _ in range(16)]
+    a = _values(gpu, 0, P, L, False, 2100, backend.RNG_LIBC, 5)
+    b = _values(gpu, 0, P, L[:4], False, 17000, backend.RNG_PHILOX, 5)
+    assert (a == _values(gpu, 5, P, L, False, 2100, backend.RNG_LIBC, 5)).all()
+    assert (b == _values(gpu, 5, P, L[:4], False, 17000, backend.RNG_PHILOX, 5)).all()
