@@ -12,8 +12,9 @@ namespace csim {
 
 struct GState;
 
-// one state to prepare: draw it (mode 0 Philox, 1 replayed rand() words) or copy
-// `src` (mode 2, a term state of the exact projector), then project it onto the
+// one state to prepare: draw it (mode 0 Philox, 1 replayed rand() values, 3 raw
+// words of its generator) or copy `src` (mode 2, a term state of the exact
+// projector), then project it onto the
 // query's projector (nstabs rows pm/pz/px)
 struct DrawDesc {
     int32_t n, mode, nstabs, pad;

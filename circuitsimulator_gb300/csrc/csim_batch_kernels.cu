@@ -40,16 +40,7 @@ __device__ void draw_project(const DrawDesc& d, GState* out, int* code, int& e) 
     if (d.mode == 2) {
         load_state<NR>(d.src, st);
     } else {
-        DevRng rng;
-        rng.mode = d.mode;
-        rng.k0 = (uint32_t)d.seed;
-        rng.k1 = (uint32_t)(d.seed >> 32);
-        rng.id0 = (uint32_t)d.id;
-        rng.id1 = (uint32_t)(d.id >> 32);
-        rng.words = d.words;
-        rng.base = d.wbegin;
-        rng.end = d.wend;
-        rng.cur = 0;
+        DevRng rng = make_rng(d.mode == 3 ? 2 : d.mode, d.seed, d.id, d.words, d.wbegin, d.wend);
         random_state<NR>(st, d.n, rng, d.cum, e);
     }
     int c = 0;

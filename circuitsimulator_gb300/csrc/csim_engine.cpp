@@ -574,7 +574,8 @@ int Engine::launch_round() {
         QueryRec* q;
         int t;
         std::vector<int64_t> slots;
-        std::vector<uint32_t> words;
+        std::vector<uint32_t> words;  // raw words, history first
+        size_t nwords;                // without the history
         std::vector<int64_t> ends;
     };
     std::vector<WordJob> jobs;
@@ -586,7 +587,7 @@ int Engine::launch_round() {
             auto it = jix.find(e->q);
             if (it == jix.end()) {
                 it = jix.emplace(e->q, jobs.size()).first;
-                jobs.push_back(WordJob{e->q, e->t, {}, {}, {}});
+                jobs.push_back(WordJob{e->q, e->t, {}, {}, 0, {}});
             }
             jobs[it->second].slots.push_back(i);
         }
@@ -594,10 +595,21 @@ int Engine::launch_round() {
             double cum[CSIM_MAX_QUBITS + 1];
             cum_table(j.t, cum);
             j.ends.reserve(j.slots.size());
+            j.words.resize(kRawHistory + j.slots.size() * state_words(j.t));
+            RawWords w{j.words.data(), kRawHistory, j.words.size()};
+            j.q->lr.history(w.p);
+            auto grow = [&](size_t more) {
+                j.words.resize(w.cap + w.cap / 2 + more);
+                w.p = j.words.data();
+                w.cap = j.words.size();
+                return true;
+            };
             for (size_t k = 0; k < j.slots.size(); k++) {
-                draw_state_words(j.q->lr, j.t, cum, j.words);
-                j.ends.push_back((int64_t)j.words.size());
+                draw_state_words(w, j.t, cum, grow);
+                j.ends.push_back((int64_t)(w.n - kRawHistory));
             }
+            j.nwords = w.n - kRawHistory;
+            j.q->lr.set_history(w.p + w.n - kRawHistory);
         };
         const int nthreads = (int)std::min<size_t>(jobs.size(), std::max(1u, std::thread::hardware_concurrency()));
         if (nthreads <= 1) {
@@ -616,7 +628,7 @@ int Engine::launch_round() {
     for (auto& j : jobs) {
         for (size_t k = 0; k < j.slots.size(); k++)
             wr[j.slots[k]] = {nwords + (k ? j.ends[k - 1] : 0), nwords + j.ends[k]};
-        nwords += (int64_t)j.words.size();
+        nwords += (int64_t)j.nwords;
     }
     std::map<Eval*, int> evix;  // evaluations in this round -> projector block
     // thread-per-pair items are grouped by t bucket: each bucket's launch sizes
@@ -702,8 +714,8 @@ int Engine::launch_round() {
     {
         size_t o = 0;
         for (auto& j : jobs) {
-            if (!j.words.empty()) memcpy(hb + o_words + 4 * o, j.words.data(), j.words.size() * 4);
-            o += j.words.size();
+            if (j.nwords) memcpy(hb + o_words + 4 * o, j.words.data() + kRawHistory, j.nwords * 4);
+            o += j.nwords;
         }
     }
     const uint64_t* dproj = (const uint64_t*)(db + o_proj);
@@ -733,7 +745,7 @@ int Engine::launch_round() {
             d.mode = 2;
             d.src = (const csim::GState*)(r->dec->phis + s);
         } else if (r->q.rng == CSIM_RNG_LIBC) {
-            d.mode = 1;
+            d.mode = 3;
             d.words = dwords;
             d.wbegin = wr[i].first;
             d.wend = wr[i].second;

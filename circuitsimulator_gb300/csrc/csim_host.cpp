@@ -66,7 +66,7 @@ extern "C" void csim_ctx_destroy(csim_ctx* ctx) {
     if (ctx->d_err) cudaFree(ctx->d_err);
     for (int i = 0; i < 4; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
-    for (int i = 0; i < 6; i++) {
+    for (int i = 0; i < kPinSlots; i++) {
         if (ctx->pin_ev[i]) cudaEventDestroy(ctx->pin_ev[i]);
         if (ctx->pin[i]) cudaFreeHost(ctx->pin[i]);
     }
@@ -525,23 +525,80 @@ extern "C" int csim_term_products(csim_ctx* ctx, int32_t t, int32_t exact, const
 namespace {
 
 
-// The tree plan of code L on this context for `count` states, with its arrays in kBufTreePlan
-int tree_plan_for(csim_ctx* ctx, const uint64_t* L, int k, int t, int64_t count) {
+// The tree plan of code L for `count` states, kept from call to call while L is the same
+void tree_plan_for(csim_ctx* ctx, const uint64_t* L, int k, int t, int64_t count) {
     std::vector<uint64_t> key(L, L + k);
     key.push_back((uint64_t)k);
     key.push_back((uint64_t)t);
-    if (key == ctx->tree_key && ctx->buf[kBufTreePlan]) {  // the device arrays do not depend on the levels
-        csim::tree::choose_levels(ctx->tree_plan, count);
-        return 0;
+    if (key != ctx->tree_key) {
+        ctx->tree_key.clear();
+        ctx->tree_plan = csim::tree::Plan();
+        csim::tree::build_chain(L, k, t, ctx->tree_plan);
+        ctx->tree_key = key;
     }
-    ctx->tree_key.clear();
-    ctx->tree_plan = csim::tree::Plan();
-    csim::tree::make_plan(L, k, t, count, ctx->tree_plan);
-    unsigned char image[kTreePlanBytes];
-    tree_plan_image(ctx->tree_plan, image);
-    unsigned char* d;
-    CKR(dput(ctx, kBufTreePlan, image, sizeof(image), &d));
-    ctx->tree_key = key;
+    csim::tree::choose_levels(ctx->tree_plan, count);
+}
+
+// A sampler call's inputs on the device, one upload: the projector's rows, the
+// d-distribution of randomStabilizerState, the projection factors, the tree plan
+struct CallInputs {
+    const int* pm;
+    const uint64_t *pz, *px;
+    const double *cum, *factor;
+    const unsigned char* plan;
+};
+int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Plan* plan, CallInputs* in) {
+    const size_t n = (size_t)P->nstabs;
+    const size_t o_px = 8 * n, o_cum = 16 * n, o_factor = o_cum + 8 * (CSIM_MAX_QUBITS + 1),
+                 o_plan = o_factor + 8 * (n + 1), o_pm = o_plan + kTreePlanBytes, bytes = o_pm + 4 * n;
+    void* v;
+    CKR(staged_room(ctx, 6, bytes, &v));
+    unsigned char* const h = (unsigned char*)v;
+    if (n) memcpy(h, P->zs, 8 * n);
+    if (n) memcpy(h + o_px, P->xs, 8 * n);
+    cum_table(P->nqubits, (double*)(h + o_cum));
+    for (size_t c = 0; c <= n; c++) ((double*)(h + o_factor))[c] = sqrt_half_power((int)c);
+    if (plan) tree_plan_image(*plan, h + o_plan);
+    else memset(h + o_plan, 0, kTreePlanBytes);
+    for (size_t r = 0; r < n; r++) ((int32_t*)(h + o_pm))[r] = phase_m(P->phase[r]);
+    CKR(staged_send(ctx, 6, kBufCall, bytes, &v));
+    const unsigned char* const d = (const unsigned char*)v;
+    in->pz = (const uint64_t*)d;
+    in->px = (const uint64_t*)(d + o_px);
+    in->cum = (const double*)(d + o_cum);
+    in->factor = (const double*)(d + o_factor);
+    in->plan = d + o_plan;
+    in->pm = (const int*)(d + o_pm);
+    return 0;
+}
+
+// The raw words of the next `count` states in pinned slots `slot` (words) and
+// slot + 1 (offsets), and their upload
+int put_state_words(csim_ctx* ctx, int slot, int t, const double* cum, int64_t count, const uint32_t** dwords,
+                    const int64_t** doffs) {
+    void *v, *o;
+    CKR(staged_room(ctx, slot, (kRawHistory + (size_t)count * state_words(t)) * 4, &v));
+    CKR(staged_room(ctx, slot + 1, (size_t)(count + 1) * 8, &o));
+    RawWords w{(uint32_t*)v, kRawHistory, ctx->pin_cap[slot] / 4};
+    int64_t* const offs = (int64_t*)o;
+    ctx->lr.history(w.p);
+    auto grow = [&](size_t more) {
+        const size_t cap = w.cap + w.cap / 2 + more;
+        if (staged_grow(ctx, slot, cap * 4, w.n * 4, &v)) return false;
+        w.p = (uint32_t*)v;
+        w.cap = cap;
+        return true;
+    };
+    for (int64_t i = 0; i < count; i++) {
+        offs[i] = (int64_t)w.n;
+        if (!draw_state_words(w, t, cum, grow)) return CSIM_ERR_NOMEM;
+    }
+    offs[count] = (int64_t)w.n;
+    ctx->lr.set_history(w.p + w.n - kRawHistory);
+    CKR(staged_send(ctx, slot, kBufWords, w.n * 4, &v));
+    *dwords = (const uint32_t*)v;
+    CKR(staged_send(ctx, slot + 1, kBufOffsets, (size_t)(count + 1) * 8, &v));
+    *doffs = (const int64_t*)v;
     return 0;
 }
 
@@ -573,19 +630,12 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int pt = tn.per_thread;
     const int64_t batch = 1 << 14;
     const int64_t shape_count = std::min(count, batch);
-    if (tree) CKR(tree_plan_for(ctx, L, k, t, shape_count));
+    if (tree) tree_plan_for(ctx, L, k, t, shape_count);
     const int64_t nchunks = tree ? tree_leaf_shape(ctx->tree_plan, shape_count).parts_per_state
                                  : (tp ? csim::terms_tp_blocks(chi, pt) : (chi + chunk - 1) / chunk);
 
-    std::vector<int> hm(P->nstabs);
-    for (int r = 0; r < P->nstabs; r++) hm[r] = phase_m(P->phase[r]);
-    int* dpm;
-    uint64_t *dpz, *dpx;
-    CKR(dput(ctx, kBufPm, hm.data(), hm.size(), &dpm));
-    CKR(dput(ctx, kBufPz, P->zs, (size_t)P->nstabs, &dpz));
-    CKR(dput(ctx, kBufPx, P->xs, (size_t)P->nstabs, &dpx));
-    double* dcum;
-    CKR(upload_cum(ctx, t, &dcum));
+    CallInputs in;
+    CKR(put_call_inputs(ctx, P, tree ? &ctx->tree_plan : nullptr, &in));
     double hcum[CSIM_MAX_QUBITS + 1];
     cum_table(t, hcum);
     uint64_t* dcw = nullptr;
@@ -604,8 +654,6 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
 
     TreeRun run;
     std::vector<unsigned char> jobs;
-    std::vector<uint32_t> words;
-    std::vector<int64_t> offs;
     std::vector<int> code;
     std::vector<__int128> acc;
     for (int64_t o = 0; o < count; o += batch) {
@@ -634,44 +682,37 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         __int128* dpart = (__int128*)v;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
         if (!tree) CK(cudaMemsetAsync(dpart, 0, nparts * sizeof(__int128), ctx->stream));
-        // With the C library's draws the host makes every state's rand() words.
-        // The batch goes in sub-batches: the host draws sub-batch s+1 while the
-        // GPU works on sub-batch s, all launches queued on the stream.  The
-        // sub-batches grow 64, 256, 1024 states, so the GPU starts after a short
-        // draw and each draw stays shorter than the GPU's work on the one before.
-        int64_t ramp = rng == CSIM_RNG_LIBC ? 64 : c;
+        // With the C library's draws the host makes every state's words.  The batch
+        // goes in sub-batches: the host draws sub-batch s+1 while the GPU works on
+        // sub-batch s, all launches queued on the stream.  The sub-batches grow 128,
+        // 512, 2048 states, so the GPU starts after a short draw and each draw stays
+        // shorter than the GPU's work on the one before.
+        int64_t ramp = rng == CSIM_RNG_LIBC ? 128 : c;
         bool first = true;
         for (int64_t s0 = 0, sb = 0; s0 < c; sb++) {
             const int64_t cs = std::min(ramp, c - s0);
-            ramp = std::min<int64_t>(4 * ramp, rng == CSIM_RNG_LIBC ? 1024 : c);
+            ramp = std::min<int64_t>(4 * ramp, rng == CSIM_RNG_LIBC ? 2048 : c);
             csim::GState* sth = tree ? nullptr : (csim::GState*)((csim_state*)dth + s0);
             int* scode = dcode + s0;
             csim::TreeDraw draw{};
             if (rng == CSIM_RNG_LIBC) {
-                words.clear();
-                offs.assign(1, 0);
-                for (int64_t i = 0; i < cs; i++) {
-                    draw_state_words(ctx->lr, t, hcum, words);
-                    offs.push_back((int64_t)words.size());
-                }
-                // pinned staging, alternating slot pairs: the upload does not wait for the sub-batch
-                // before it, so the host goes on to draw the next one
-                uint32_t* dw;
-                int64_t* doff;
-                CKR(staged_put(ctx, 2 * (sb & 1), kBufWords, words.data(), words.size(), &dw));
-                CKR(staged_put(ctx, 2 * (sb & 1) + 1, kBufOffsets, offs.data(), offs.size(), &doff));
-                draw = csim::TreeDraw{1, P->nstabs, 0, 0, dw, doff, dcum, dpm, dpz, dpx, scode};
-                if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 1, 0, 0, dw, doff, dcum, sth, nullptr))
+                // alternating pinned slots: the upload does not wait for the sub-batch before it, so
+                // the host goes on to draw the next one
+                const uint32_t* dw;
+                const int64_t* doff;
+                CKR(put_state_words(ctx, 2 * (sb & 1), t, hcum, cs, &dw, &doff));
+                draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, scode};
+                if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 2, 0, 0, dw, doff, in.cum, sth, nullptr))
                     return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
             } else {
-                draw = csim::TreeDraw{0, P->nstabs, ctx->philox_seed, ctx->philox_next, nullptr, nullptr, dcum, dpm, dpz,
-                                      dpx, scode};
+                draw = csim::TreeDraw{0, P->nstabs, ctx->philox_seed, ctx->philox_next, nullptr, nullptr, in.cum, in.pm,
+                                      in.pz, in.px, scode};
                 if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 0, ctx->philox_seed, ctx->philox_next,
-                                                        nullptr, nullptr, dcum, sth, nullptr))
+                                                        nullptr, nullptr, in.cum, sth, nullptr))
                     return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
                 ctx->philox_next += cs;
             }
-            if (!tree && csim::launch_project(launch_of(ctx), nr, sth, cs, P->nstabs, dpm, dpz, dpx, scode))
+            if (!tree && csim::launch_project(launch_of(ctx), nr, sth, cs, P->nstabs, in.pm, in.pz, in.px, scode))
                 return fail(ctx, CSIM_ERR_CUDA, "projection launch failed");
             if (tp && tn.kernel == 3) {
                 CK(cudaMemsetAsync(drest, 0, 4, ctx->stream));
@@ -688,7 +729,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             if (tree) {
                 TreeGroup g;
                 g.plan = &ctx->tree_plan;
-                g.dplan = (const unsigned char*)ctx->buf[kBufTreePlan];
+                g.dplan = in.plan;
                 g.count = cs;
                 g.shape_count = shape_count;
                 g.part = spart;
@@ -760,6 +801,28 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             s0 += cs;
         }
         CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+        if (tree) {  // results: the live states' count, the error word, the values
+            CKR(dbuf(ctx, kBufResults, 16 + (size_t)c * 8, &v));
+            unsigned char* const dres = (unsigned char*)v;
+            CK(cudaMemsetAsync(dres, 0, 16, ctx->stream));
+            if (csim::launch_tree_values(launch_of(ctx), dpart, c, nchunks, t, dcode, in.factor, (double*)(dres + 16),
+                                         (unsigned long long*)dres))
+                return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
+            CK(cudaMemcpyAsync(dres + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
+            CK(cudaEventRecord(ctx->ev[3], ctx->stream));
+            CKR(staged_room(ctx, 7, 16 + (size_t)c * 8, &v));
+            CKR(dget(ctx, (unsigned char*)v, dres, 16 + (size_t)c * 8));
+            CK(cudaStreamSynchronize(ctx->stream));
+            CK(cudaGetLastError());
+            CKR(error_status(ctx, ((const int*)v)[2]));
+            CKR(stats_batch(ctx));
+            const int64_t live = *(const int64_t*)v;
+            memcpy(values + o, (const unsigned char*)v + 16, (size_t)c * 8);
+            ctx->stats.states += c;
+            ctx->stats.states_live += live;
+            ctx->stats.pairs += live * chi;
+            continue;
+        }
         CKR(dbuf(ctx, kBufAcc, (size_t)c * 4 * sizeof(__int128), &v));
         __int128* dacc = (__int128*)v;
         if (csim::launch_reduce_parts(launch_of(ctx), dpart, c, nchunks, dacc))

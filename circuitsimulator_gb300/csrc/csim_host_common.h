@@ -57,7 +57,37 @@ struct LibcRand {
         for (int i = 34; i < 344; i++) step();
     }
     int32_t next() { return (int32_t)(step() >> 1); }
+    // the last 34 raw words, oldest first, and back
+    void history(uint32_t* h) const {
+        for (int i = 0; i < 34; i++) h[i] = ring[(idx + i) % 34];
+    }
+    void set_history(const uint32_t* h) {
+        for (int i = 0; i < 34; i++) ring[i] = h[i];
+        idx = 0;
+    }
 };
+
+// The generator's raw words (rand() returns their upper 31 bits) appended to a
+// buffer that starts with 34 words of history.  Memory that holds the sequence
+// itself needs no ring: one add per word, three chains at once (0.4 ns a word;
+// word by word through the ring it was 4 ns, 13 ms for 4096 states of 40 qubits).
+struct RawWords {
+    uint32_t* p = nullptr;
+    size_t n = 0, cap = 0;  // words in the buffer (history included), and room
+    void extend(size_t count) {
+        uint32_t* e = p + n;
+        uint32_t* const end = e + count;
+        n += count;
+        uint32_t a = e[-3], b = e[-2], c = e[-1];
+        for (; end - e >= 3; e += 3) {
+            e[0] = a += e[-31];
+            e[1] = b += e[-30];
+            e[2] = c += e[-29];
+        }
+        for (; e < end; e++) *e = e[-3] + e[-31];
+    }
+};
+constexpr size_t kRawHistory = 34;
 
 // ---------------------------------------------------------------- helpers
 inline int popc(uint64_t x) { return __builtin_popcountll(x); }
@@ -98,15 +128,25 @@ inline uint64_t codeword(int64_t j, const uint64_t* L, int k) {
     return x;
 }
 
-// The rand() words randomStabilizerState consumes for one n-qubit state, drawn
-// from `lr` in the reference's order.  The lazy shrink loop is simulated on G
-// alone to know how many random vectors are drawn (stabilizer.c:736-740).
-inline void draw_state_words(LibcRand& lr, int n, const double* cum, std::vector<uint32_t>& words) {
+// Room for one state's words besides the vectors its lazy shrinks draw again
+inline size_t state_words(int n) { return (size_t)(64 + 8 * 16 + n * (n - 1) / 2); }
+
+// The words randomStabilizerState consumes for one n-qubit state, appended in the
+// reference's order.  The lazy shrink loop is simulated on G alone to know how
+// many random vectors are drawn (stabilizer.c:736-740).  grow(words): makes room
+// for that many more; returns false when there is none.
+template <class Grow>
+bool draw_state_words(RawWords& w, int n, const double* cum, Grow grow) {
+    auto room = [&](size_t c) { return w.n + c <= w.cap || grow(c); };
+    if (!room(state_words(n))) return false;
+    auto rand31 = [&]() {
+        w.extend(1);
+        return (int32_t)(w.p[w.n - 1] >> 1);
+    };
     double sample;
     do {
-        const int32_t w = lr.next();
-        words.push_back((uint32_t)w);
-        sample = 0. + (w / (2147483647 / 1.0));
+        if (!room(1)) return false;
+        sample = 0. + (rand31() / (2147483647 / 1.0));
     } while (sample == 0.);
     int d = 0;
     for (; d <= n; d++)
@@ -117,11 +157,10 @@ inline void draw_state_words(LibcRand& lr, int n, const double* cum, std::vector
     int k = n;
     const int bytes = (n + 7) / 8;
     while (k > kt) {
+        if (!room((size_t)bytes)) return false;
         uint64_t xi = 0;
         for (int b = 0; b < bytes; b++) {
-            const int32_t w = lr.next();
-            words.push_back((uint32_t)w);
-            const int byte = w % 256;
+            const int byte = rand31() % 256;
             for (int j = 0; j < 8; j++) {
                 const int loc = 8 * b + j;
                 if (loc < n && (byte & (0x80 >> j))) xi |= 1ull << loc;
@@ -140,10 +179,10 @@ inline void draw_state_words(LibcRand& lr, int n, const double* cum, std::vector
         std::swap(G[last], G[k - 1]);
         k--;
     }
-    const int64_t rest = 3 * bytes + (int64_t)k * (k - 1) / 2;
-    const size_t w0 = words.size();
-    words.resize(w0 + (size_t)rest);
-    for (int64_t i = 0; i < rest; i++) words[w0 + (size_t)i] = (uint32_t)lr.next();
+    const size_t rest = (size_t)(3 * bytes + k * (k - 1) / 2);
+    if (!room(rest)) return false;
+    w.extend(rest);
+    return true;
 }
 
 // Zero bound of the "light" part of an ordered codeword table: codewords with
@@ -372,8 +411,10 @@ enum BufId {
     kBufA, kBufB, kBufEps, kBufP, kBufM, kBufXi, kBufZeta, kBufAlpha, kBufCode, kBufWords, kBufOffsets,
     kBufCum, kBufCodewords, kBufAcc, kBufAccDiag, kBufPhis, kBufIdx, kBufConsumed, kBufPm, kBufPz, kBufPx,
     kBufL, kBufParts, kBufPartsDiag, kBufCwOrdered, kBufRunScratch, kBufCanon, kBufCodeDirect, kBufCodeRest,
-    kBufRestCount, kBufTreePlan, kBufTreeJobs, kBufTreeScratch, kNumBufs
+    kBufRestCount, kBufTreeJobs, kBufTreeScratch, kBufCall, kBufResults, kNumBufs
 };
+
+constexpr int kPinSlots = 8;      // words and offsets twice, jobs twice, a call's inputs, its results
 
 class Engine;                     // csim_engine.cpp: the batched query engine
 void engine_free(Engine* engine);  // releases it and its device memory
@@ -395,16 +436,16 @@ struct csim_ctx {
     int pair_kernel = 0;  // CSIM_OPT_PAIR_KERNEL
     int per_thread = 0;  // CSIM_OPT_PER_THREAD; 0 = auto_per_thread(t)
     cudaEvent_t ev[4] = {};
-    // pinned staging of host-made uploads (staged_put): six slots, each with the event of its last copy
-    void* pin[6] = {};
-    size_t pin_cap[6] = {};
-    cudaEvent_t pin_ev[6] = {};
+    // pinned staging of host-made uploads (staged_put): kPinSlots of them, each with the event of its last copy
+    void* pin[kPinSlots] = {};
+    size_t pin_cap[kPinSlots] = {};
+    cudaEvent_t pin_ev[kPinSlots] = {};
     Engine* engine = nullptr;  // created by the first batched csim_run_queries
     std::vector<uint64_t> cw_key;  // (k, rows of L, t, light bound) of the ordered codeword table in kBufCwOrdered
     int64_t cw_split = 0;          // first index of that table whose codewords have <= the light bound's zeros
     std::vector<int> cw_bounds;        // occupancy-class order: the launches' zero bounds
     std::vector<int64_t> cw_starts;    // and the first index of each class
-    std::vector<uint64_t> tree_key;    // (rows of L, k, t) of tree_plan, whose device arrays are in kBufTreePlan
+    std::vector<uint64_t> tree_key;    // (rows of L, k, t) of tree_plan
     csim::tree::Plan tree_plan;
     // autotuner (CSIM_OPT_AUTOTUNE): the tuned launch parameters live in a
     // process-wide table per device (csim_host.cpp), filled a t bucket at a time
@@ -477,15 +518,9 @@ inline int dput(csim_ctx* ctx, int id, const T* src, size_t count, T** out) {
     return 0;
 }
 
-// dput through pinned staging slot `slot`: an upload from pageable memory first waits for the
-// stream, one from pinned memory returns at once, so the host can prepare the next upload
-// while the GPU works.  The slot's previous copy must have run before the slot is rewritten;
-// alternating slots makes that wait rare.
-template <class T>
-inline int staged_put(csim_ctx* ctx, int slot, int id, const T* src, size_t count, T** out) {
-    void* p;
-    const size_t bytes = count * sizeof(T);
-    CKR(dbuf(ctx, id, bytes, &p));
+// Pinned staging slot `slot` with room for `bytes`, free for the host to write once
+// its last copy has run; staged_send queues the copy of its first `bytes`.
+inline int staged_room(csim_ctx* ctx, int slot, size_t bytes, void** out) {
     if (ctx->pin_ev[slot]) CK(cudaEventSynchronize(ctx->pin_ev[slot]));
     else CK(cudaEventCreateWithFlags(&ctx->pin_ev[slot], cudaEventDisableTiming));
     if (ctx->pin_cap[slot] < bytes) {
@@ -499,12 +534,38 @@ inline int staged_put(csim_ctx* ctx, int slot, int id, const T* src, size_t coun
         }
         ctx->pin_cap[slot] = c;
     }
-    if (count) {
-        memcpy(ctx->pin[slot], src, bytes);
-        CK(cudaMemcpyAsync(p, ctx->pin[slot], bytes, cudaMemcpyHostToDevice, ctx->stream));
-    }
+    *out = ctx->pin[slot];
+    return 0;
+}
+// a larger slot with the first `keep` bytes of the old one (no copy of it is in flight)
+inline int staged_grow(csim_ctx* ctx, int slot, size_t bytes, size_t keep, void** out) {
+    void* p;
+    if (cudaMallocHost(&p, bytes) != cudaSuccess)
+        return fail(ctx, CSIM_ERR_NOMEM, "cudaMallocHost of %zu bytes failed", bytes);
+    memcpy(p, ctx->pin[slot], keep);
+    cudaFreeHost(ctx->pin[slot]);
+    ctx->pin[slot] = *out = p;
+    ctx->pin_cap[slot] = bytes;
+    return 0;
+}
+inline int staged_send(csim_ctx* ctx, int slot, int id, size_t bytes, void** out) {
+    CKR(dbuf(ctx, id, bytes, out));
+    if (bytes) CK(cudaMemcpyAsync(*out, ctx->pin[slot], bytes, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaEventRecord(ctx->pin_ev[slot], ctx->stream));
     ctx->stats.h2d_bytes += (int64_t)bytes;
+    return 0;
+}
+
+// dput through a pinned staging slot: an upload from pageable memory first waits for the
+// stream, one from pinned memory returns at once, so the host can prepare the next upload
+// while the GPU works.  The slot's previous copy must have run before the slot is rewritten;
+// alternating slots makes that wait rare.
+template <class T>
+inline int staged_put(csim_ctx* ctx, int slot, int id, const T* src, size_t count, T** out) {
+    void* p;
+    CKR(staged_room(ctx, slot, count * sizeof(T), &p));
+    if (count) memcpy(p, src, count * sizeof(T));
+    CKR(staged_send(ctx, slot, id, count * sizeof(T), &p));
     *out = (T*)p;
     return 0;
 }
@@ -535,12 +596,8 @@ inline void stats_end(csim_ctx* ctx) { ctx->stats.kernels = ctx->launches - ctx-
 
 inline csim::Launch launch_of(csim_ctx* ctx) { return csim::Launch{ctx->stream, ctx->d_err, &ctx->launches, ctx->num_sms}; }
 
-// waits for the stream, then turns device error flags into a status
-inline int finish(csim_ctx* ctx) {
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    CK(cudaGetLastError());
+// device error flags `h` as a status, and the flags cleared (the stream is idle)
+inline int error_status(csim_ctx* ctx, int h) {
     if (h) {
         CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
@@ -548,6 +605,14 @@ inline int finish(csim_ctx* ctx) {
                     h);
     }
     return 0;
+}
+// waits for the stream, then turns device error flags into a status
+inline int finish(csim_ctx* ctx) {
+    int h = 0;
+    CK(cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaGetLastError());
+    return error_status(ctx, h);
 }
 
 inline int check_states(csim_ctx* ctx, const csim_state* s, int64_t count, int* nr_out, int n_expect = -1) {

@@ -26,6 +26,7 @@ int launch_shrink(const Launch& L, int nr, GState* s, const uint64_t* xi, const 
 int launch_measure(const Launch& L, int nr, GState* s, const int* m, const uint64_t* zeta, const uint64_t* xi,
                    int64_t count, int* code);
 int launch_extend(const Launch& L, int nr, GState* s, const uint64_t* xi, int64_t count);
+// mode: 0 Philox, 1 replay of rand() values, 2 replay of the generator's raw words (csim_rng.cuh)
 int launch_random_states(const Launch& L, int n, int64_t count, int mode, uint64_t seed, uint64_t first,
                          const uint32_t* words, const int64_t* offsets, const double* cum, GState* out,
                          int64_t* consumed);

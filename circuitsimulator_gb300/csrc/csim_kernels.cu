@@ -120,16 +120,7 @@ __global__ void __launch_bounds__(256) k_random_states(int n, int64_t count, int
                                                        const double* cum, GState* out, int64_t* consumed, int* err) {
     int e = 0;
     for (int64_t i = warp_global(); i < count; i += warp_count()) {
-        DevRng rng;
-        rng.mode = mode;
-        rng.k0 = (uint32_t)seed;
-        rng.k1 = (uint32_t)(seed >> 32);
-        rng.id0 = (uint32_t)(first + i);
-        rng.id1 = (uint32_t)((first + i) >> 32);
-        rng.words = words;
-        rng.base = mode == 1 ? offsets[i] : 0;
-        rng.end = mode == 1 ? offsets[i + 1] : 0;
-        rng.cur = 0;
+        DevRng rng = make_rng(mode, seed, first + i, words, mode ? offsets[i] : 0, mode ? offsets[i + 1] : 0);
         WS<NR> st;
         random_state<NR>(st, n, rng, cum, e);
         store_state<NR>(out + i, st);

@@ -6,8 +6,9 @@
 // sequence, from one of two sources:
 //   * Philox-4x32-10 (Salmon et al., SC'11), counter (c/4, id, id_hi, c>>34),
 //     key = seed: an independent stream per state, 31-bit outputs like rand();
-//   * replay: words[base + c], the exact values rand() returned to the
-//     reference, recorded or regenerated on the host.
+//   * replay: words[base + c] >> shift, the exact values rand() returned to the
+//     reference (shift 0), or its generator's raw words, whose upper 31 bits those
+//     are (shift 1).
 #pragma once
 
 #include <cstdint>
@@ -30,6 +31,7 @@ __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, uint32_t k1
 
 struct DevRng {
     int mode;                // 0 = Philox, 1 = replay
+    int shift;               // replay: 1 for raw words
     uint32_t k0, k1;         // Philox key
     uint32_t id0, id1;       // Philox stream (state index)
     const uint32_t* words;   // replay words
@@ -43,7 +45,7 @@ struct DevRng {
                 err |= kErrReplay;
                 return 0u;
             }
-            return words[q];
+            return words[q] >> shift;
         }
         const uint4 r = philox4x32_10(make_uint4((uint32_t)(c >> 2), id0, id1, (uint32_t)(c >> 34)), k0, k1);
         const int j = (int)(c & 3);
@@ -64,6 +66,24 @@ struct DevRng {
         return warp_or64(w) & lowmask(n);
     }
 };
+
+// The generator of one state: Philox stream (seed, id) (mode 0), or words
+// [begin, end) as rand() values (mode 1) or raw words (mode 2)
+__device__ __forceinline__ DevRng make_rng(int mode, uint64_t seed, uint64_t id, const uint32_t* words, int64_t begin,
+                                           int64_t end) {
+    DevRng r;
+    r.mode = mode == 0 ? 0 : 1;
+    r.shift = mode == 2 ? 1 : 0;
+    r.k0 = (uint32_t)seed;
+    r.k1 = (uint32_t)(seed >> 32);
+    r.id0 = (uint32_t)id;
+    r.id1 = (uint32_t)(id >> 32);
+    r.words = words;
+    r.base = begin;
+    r.end = end;
+    r.cur = 0;
+    return r;
+}
 
 // randomStabilizerState (stabilizer.c:689-756).  cum[0..n] is the
 // normalized cumulative distribution of eq. 79 computed on the host with the

@@ -8,6 +8,7 @@
 //   k_tree_leaf   one thread per node of the last written level (or a part of
 //                 one): the remaining levels, then the leaves' values from truth
 //                 tables, summed exactly
+//   k_tree_values one warp per state: its sum, as the sampler's value
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -181,16 +182,7 @@ __global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRoo
     if (i >= J.count) return;  // warp-uniform
     const int64_t a = J.first + i;
     int e = 0;
-    DevRng rng;
-    rng.mode = d.mode;
-    rng.k0 = (uint32_t)d.seed;
-    rng.k1 = (uint32_t)(d.seed >> 32);
-    rng.id0 = (uint32_t)(d.id + a);
-    rng.id1 = (uint32_t)((d.id + a) >> 32);
-    rng.words = d.words;
-    rng.base = d.mode == 1 ? d.offsets[a] : 0;
-    rng.end = d.mode == 1 ? d.offsets[a + 1] : 0;
-    rng.cur = 0;
+    DevRng rng = make_rng(d.mode, d.seed, d.id + a, d.words, d.mode ? d.offsets[a] : 0, d.mode ? d.offsets[a + 1] : 0);
     WS<NR> st;
     random_state<NR>(st, J.t, rng, d.cum, e);
     int c = 0;  // the number of 2^{-1/2} factors, -1 once a measurement annihilates the state
@@ -498,6 +490,63 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
     }
 }
 
+// ---------------------------------------------------------------- values
+// z to double, to nearest even as the host's conversion: the top 64 bits with the
+// rest folded into the lowest one convert with a single rounding
+__device__ __forceinline__ double int128_to_double(__int128 z) {
+    const bool neg = z < 0;
+    const unsigned __int128 a = neg ? -(unsigned __int128)z : (unsigned __int128)z;
+    const uint64_t hi = (uint64_t)(a >> 64), lo = (uint64_t)a;
+    double d;
+    if (hi == 0ull) {
+        d = __ull2double_rn(lo);
+    } else {
+        const int s = 64 - __clzll((long long)hi);  // 1..64
+        const uint64_t top = s == 64 ? hi : ((hi << (64 - s)) | (lo >> s));
+        const uint64_t rest = s == 64 ? lo : lo << (64 - s);
+        d = __dmul_rn(__ull2double_rn(top | (rest != 0ull ? 1ull : 0ull)), __hiloint2double((1023 + s) << 20, 0));
+    }
+    return neg ? -d : d;
+}
+
+// One warp per state: the sum of its partial sums, and singleProjectorSample's
+// value 2^t |projfactor sum|^2 (innerprod.c:142) with the host's own roundings
+// (csim_host::zomega_to_complex: no fused multiply-adds).  factor[c]: the
+// projection factor of c measurements that halved the norm.  *live counts the
+// states that the projector left alive (0 for the others).
+__global__ void __launch_bounds__(128) k_tree_values(const __int128* part, int64_t count, int64_t parts, int t,
+                                                     const int* code, const double* factor, double* values,
+                                                     unsigned long long* live) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= count) return;  // warp-uniform
+    const int lane = lane_id(), q = lane & 3;
+    __int128 z = 0;
+    for (int64_t p = lane >> 2; p < parts; p += 8) z += part[4 * (i * parts + p) + q];
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+        const uint64_t lo = shfl_xor64((uint64_t)z, o), hi = shfl_xor64((uint64_t)((unsigned __int128)z >> 64), o);
+        z += (__int128)(((unsigned __int128)hi << 64) | lo);
+    }
+    // lanes 0..3 hold coordinates 0..3; lane 1 takes z1 - z3, lane 3 z1 + z3
+    const uint64_t lo = shfl_xor64((uint64_t)z, 2), hi = shfl_xor64((uint64_t)((unsigned __int128)z >> 64), 2);
+    const __int128 other = (__int128)(((unsigned __int128)hi << 64) | lo);
+    const double d = int128_to_double(q == 1 ? z - other : (q == 3 ? other + z : z));
+    const double s = 0.70710678118654752440;
+    const double x0 = __shfl_sync(kFull, d, 0), x1 = __shfl_sync(kFull, d, 1), x2 = __shfl_sync(kFull, d, 2),
+                 x3 = __shfl_sync(kFull, d, 3);
+    if (lane != 0) return;
+    const int c = code[i];
+    double v = 0;
+    if (c >= 0) {
+        const double unit = __hiloint2double((1023 - t) << 20, 0);  // 2^-t
+        const double re = __dmul_rn(__dadd_rn(x0, __dmul_rn(x1, s)), unit), im = __dmul_rn(__dadd_rn(x2, __dmul_rn(x3, s)), unit);
+        const double a = __dmul_rn(re, factor[c]), b = __dmul_rn(im, factor[c]);
+        v = __dmul_rn(__hiloint2double((1023 + t) << 20, 0), __dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)));
+        atomicAdd(live, 1ull);
+    }
+    values[i] = v;
+}
+
 // ---------------------------------------------------------------- launchers
 int launch_tree_root(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, const GState* states,
                      const int* code) {
@@ -527,6 +576,14 @@ int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int6
         return -1;
     if (wide) k_tree_stage<uint64_t><<<(unsigned)blocks, kTreeStageThreads, smem, L.stream>>>(jobs, njobs);
     else k_tree_stage<uint32_t><<<(unsigned)blocks, kTreeStageThreads, smem, L.stream>>>(jobs, njobs);
+    (*L.launches)++;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_tree_values(const Launch& L, const __int128* part, int64_t count, int64_t parts, int t, const int* code,
+                       const double* factor, double* values, unsigned long long* live) {
+    if (count <= 0) return 0;
+    k_tree_values<<<(unsigned)((count + 3) / 4), 128, 0, L.stream>>>(part, count, parts, t, code, factor, values, live);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

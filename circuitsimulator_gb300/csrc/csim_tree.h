@@ -49,7 +49,7 @@ struct TreeLeafJob {
 // call is state id + a of Philox stream `seed` (mode 0) or replays words
 // [offsets[a], offsets[a + 1]) (mode 1); code[a] as k_project writes it
 struct TreeDraw {
-    int32_t mode, nstabs;
+    int32_t mode, nstabs;  // mode 2: the words are raw (csim_rng.cuh)
     uint64_t seed, id;
     const uint32_t* words;
     const int64_t* offsets;
@@ -70,5 +70,9 @@ int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_
 int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax);
 // words: the jobs' table words (tree::table_words(tv))
 int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words);
+
+// values[i] of `count` states from `parts` partial sums each; factor: 65 doubles; *live is added to
+int launch_tree_values(const Launch& L, const __int128* part, int64_t count, int64_t parts, int t, const int* code,
+                       const double* factor, double* values, unsigned long long* live);
 
 }  // namespace csim
