@@ -13,6 +13,8 @@
 //   k_items_tp      (state, |L> term range) items, thread per pair
 //   k_items_direct  the same items by direct restriction, thread per pair
 //   k_items_warp    (state, prepH term range) items, warp per pair
+//   k_tree_*        sampled terms of |L> as trees of shared contractions, one group
+//                   of states per decomposition
 //   k_reduce_slots  exact Z[w] sums per state
 // Two round buffers alternate.  The host builds round r+1 and queues it behind
 // round r, then reads round r's results.
@@ -119,6 +121,8 @@ struct Decomp {
     int kern = 0;                // the tuner's kernel: 3 = direct restriction, else the block-prefix kernel
     csim_state* phis = nullptr;  // term states: prepH (exact == 1), prepL (exact projector on |L>)
     uint64_t* dL = nullptr;
+    csim::tree::Plan plan;             // the tree sum's chain of subcodes (exact == 0, sampled estimators)
+    unsigned char* dplan = nullptr;    // and its device arrays
     size_t bytes = 0;
     int refs = 0;
     int64_t last_use = 0;
@@ -127,10 +131,12 @@ struct Decomp {
         if (cws) cudaFree(cws);
         if (phis) cudaFree(phis);
         if (dL) cudaFree(dL);
+        if (dplan) cudaFree(dplan);
         cw = nullptr;
         cws = nullptr;
         phis = nullptr;
         dL = nullptr;
+        dplan = nullptr;
     }
 };
 
@@ -142,6 +148,7 @@ struct Eval {
     int which = 0;  // 0 G', 1 H'
     int kind = 1;   // 1 sampled (multiSampledProjector), 2 exactProjector
     int t = 0;
+    bool tree = false;  // summed by the tree kernels (sampled, terms of |L>)
     int64_t chi = 0, ns = 0;
     int samples = 0, bins = 1;
     int64_t next = 0, done = 0;
@@ -219,6 +226,7 @@ class Engine {
         for (auto& kv : decomps_) kv.second->release();
         cum_.release();
         iota_.release();
+        tree_scratch_.release();
     }
 
     int init() {
@@ -281,13 +289,15 @@ class Engine {
     int next_set_ = 0;
     std::deque<RoundSet*> inflight_;
     DevBuf cum_, iota_;
+    DevBuf tree_scratch_;  // node planes; rounds on the stream take turns
+    TreeRun tree_run_;
     int64_t iota_n_ = 0;
     int bucket_of_[CSIM_MAX_QUBITS + 1] = {0};
     int bucket_hi_[kBuckets] = {0};
     int nbuckets_ = 0;
 
     csim::Launch launch_on(int* d_err) { return csim::Launch{ctx_->stream, d_err, &ctx_->launches, ctx_->num_sms}; }
-    int ensure_decomp(QueryRec* r, bool need_phis, bool force, Decomp** out);
+    int ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp** out);
     void finish_eval(Eval* e);
     void finish_query(QueryRec* r);
     void fail_query(QueryRec* r, int status);
@@ -358,7 +368,9 @@ static bool plan_query(csim_ctx* ctx, QueryRec* r) {
     return true;
 }
 
-int Engine::ensure_decomp(QueryRec* r, bool need_phis, bool force, Decomp** out) {
+// rows: the exactProjector's evaluations (term order, term states); otherwise the
+// sampled estimators', as a tree or with a pair kernel
+int Engine::ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp** out) {
     csim_ctx* const ctx = ctx_;  // for CK
     *out = nullptr;
     std::vector<uint64_t> key = {(uint64_t)r->q.t, (uint64_t)r->exact, (uint64_t)(r->exact ? 0 : r->k)};
@@ -366,9 +378,13 @@ int Engine::ensure_decomp(QueryRec* r, bool need_phis, bool force, Decomp** out)
     auto it = decomps_.find(key);
     Decomp* d = it == decomps_.end() ? nullptr : it->second.get();
     const int64_t chi = r->chi;
-    const bool want_cw = !r->exact, want_phis = r->exact || need_phis;
+    const bool want_cw = !r->exact && rows, want_cws = !r->exact && !rows && !tree, want_plan = !r->exact && tree,
+               want_phis = r->exact || rows;
+    const size_t table = align_up((size_t)chi * 8);
     size_t add = 0;
-    if (!d && want_cw) add += 2 * align_up((size_t)chi * 8) + kAlign;
+    if (want_cw && !(d && d->cw)) add += table + kAlign;
+    if (want_cws && !(d && d->cws)) add += table;
+    if (want_plan && !(d && d->dplan)) add += align_up(kTreePlanBytes);
     if (want_phis && !(d && d->phis)) add += align_up((size_t)chi * sizeof(csim_state));
     if (add && resident_ + (int64_t)add > budget_) {  // evict unused decompositions, least recently used first
         std::vector<std::pair<int64_t, std::vector<uint64_t>>> lru;
@@ -394,37 +410,48 @@ int Engine::ensure_decomp(QueryRec* r, bool need_phis, bool force, Decomp** out)
         nd->L.assign(r->L, r->L + (r->exact ? 0 : r->k));
         d = nd.get();
         decomps_[key] = std::move(nd);
-        if (want_cw) {
-            if (cudaMalloc(&d->cw, (size_t)chi * 8) != cudaSuccess ||
-                cudaMalloc(&d->cws, (size_t)chi * 8) != cudaSuccess ||
-                cudaMalloc(&d->dL, 8 * (size_t)CSIM_MAX_QUBITS) != cudaSuccess) {
-                d->release();
-                decomps_.erase(key);
-                return fail(ctx_, CSIM_ERR_NOMEM, "codeword table of 2^%d terms", r->k);
-            }
-            d->bytes += 2 * align_up((size_t)chi * 8) + kAlign;
-            TpTune tn;
-            const csim_projector* Pw = r->q.G.nstabs > 0 ? &r->q.G : (r->q.H.nstabs > 0 ? &r->q.H : nullptr);
-            if (const int rc = tune_for(ctx_, d->t, &tn, Pw, d->L.data(), d->k)) {
-                d->release();
-                decomps_.erase(key);
-                return rc;
-            }
-            d->pt = tn.per_thread;
-            d->kern = tn.kernel;
-            // the items kernel shares top bits per block; the direct kernel's bound splits narrow from wide
-            d->lz = (tn.kernel == 0 || tn.kernel == 3) ? tn.light : light_zeros(d->t);
-            std::vector<uint64_t> ordered;
-            ordered_codewords(d->L.data(), d->k, d->t, d->lz, ordered);
-            d->light = light_split(ordered, d->t, d->lz);
-            CK(cudaMemcpy(d->cws, ordered.data(), (size_t)chi * 8, cudaMemcpyHostToDevice));
-            uint64_t rows[CSIM_MAX_QUBITS] = {0};
-            for (int i = 0; i < d->k; i++) rows[i] = d->L[i];
-            CK(cudaMemcpy(d->dL, rows, sizeof(rows), cudaMemcpyHostToDevice));
-            if (csim::launch_codewords(launch_of(ctx_), d->dL, d->k, 0, chi, d->cw))
-                return fail(ctx_, CSIM_ERR_CUDA, "codeword launch failed");
+    }
+    // device memory of this decomposition; what one call cannot make is made by the next
+    auto grow = [&](void** p, size_t bytes) {
+        if (cudaMalloc(p, bytes) != cudaSuccess) {
+            *p = nullptr;
+            return fail(ctx_, CSIM_ERR_NOMEM, "decomposition of 2^%d terms on t = %d", r->k, r->q.t);
         }
-        resident_ += (int64_t)d->bytes;
+        d->bytes += align_up(bytes);
+        resident_ += (int64_t)align_up(bytes);
+        return 0;
+    };
+    if (want_plan && !d->dplan) {
+        csim::tree::build_chain(d->L.data(), d->k, d->t, d->plan);
+        unsigned char image[kTreePlanBytes];
+        tree_plan_image(d->plan, image);
+        CKR(grow((void**)&d->dplan, kTreePlanBytes));
+        CK(cudaMemcpyAsync(d->dplan, image, sizeof(image), cudaMemcpyHostToDevice, ctx_->stream));
+    }
+    if ((want_cw || want_cws) && !d->pt) {
+        TpTune tn;
+        const csim_projector* Pw = r->q.G.nstabs > 0 ? &r->q.G : (r->q.H.nstabs > 0 ? &r->q.H : nullptr);
+        CKR(tune_for(ctx_, d->t, &tn, Pw, d->L.data(), d->k));
+        d->pt = tn.per_thread;
+        d->kern = tn.kernel;
+        // the items kernel shares top bits per block; the direct kernel's bound splits narrow from wide
+        d->lz = (tn.kernel == 0 || tn.kernel == 3) ? tn.light : light_zeros(d->t);
+    }
+    if (want_cws && !d->cws) {
+        std::vector<uint64_t> ordered;
+        ordered_codewords(d->L.data(), d->k, d->t, d->lz, ordered);
+        d->light = light_split(ordered, d->t, d->lz);
+        CKR(grow((void**)&d->cws, (size_t)chi * 8));
+        CK(cudaMemcpy(d->cws, ordered.data(), (size_t)chi * 8, cudaMemcpyHostToDevice));
+    }
+    if (want_cw && !d->cw) {
+        uint64_t code_rows[CSIM_MAX_QUBITS] = {0};
+        for (int i = 0; i < d->k; i++) code_rows[i] = d->L[i];
+        if (!d->dL) CKR(grow((void**)&d->dL, sizeof(code_rows)));
+        CK(cudaMemcpy(d->dL, code_rows, sizeof(code_rows), cudaMemcpyHostToDevice));
+        CKR(grow((void**)&d->cw, (size_t)chi * 8));
+        if (csim::launch_codewords(launch_of(ctx_), d->dL, d->k, 0, chi, d->cw))
+            return fail(ctx_, CSIM_ERR_CUDA, "codeword launch failed");
     }
     if (want_phis && !d->phis) {
         if (cudaMalloc(&d->phis, (size_t)chi * sizeof(csim_state)) != cudaSuccess) {
@@ -461,7 +488,9 @@ int Engine::admit(QueryRec* r, bool force, bool* admitted) {
         return 0;
     }
     Decomp* d = nullptr;
-    const int rc = ensure_decomp(r, r->noapprox != 0, force, &d);
+    // sampled terms of |L>: the tree sum, unless a pair kernel is asked for
+    const bool tree = !r->exact && !r->noapprox && ctx_->pair_kernel == 0 && r->k <= kTreeMaxRows;
+    const int rc = ensure_decomp(r, r->noapprox != 0, tree, force, &d);
     if (rc) {
         fail_query(r, rc);
         *admitted = true;
@@ -483,6 +512,7 @@ int Engine::admit(QueryRec* r, bool force, bool* admitted) {
         e->which = w;
         e->kind = r->noapprox ? 2 : 1;
         e->t = Q.t;
+        e->tree = tree;
         e->chi = r->chi;
         e->samples = Q.samples;
         e->bins = Q.bins;
@@ -639,6 +669,7 @@ int Engine::launch_round() {
     // a launch runs as many rows per thread as its longest items need
     auto span_tp_of = [this](const Eval* e) { return 64 * (int64_t)(per_thread_ > 0 ? per_thread_ : e->q->dec->pt); };
     const int launch_pt = per_thread_ > 0 ? per_thread_ : 32;  // the largest item any t is tuned to
+    std::map<Decomp*, std::vector<int32_t>> tree_slots;  // slots of the tree sums, by decomposition
     int lzmax[kBuckets] = {0};  // per light launch: the largest light bound of its items
     const int64_t span_w = 64;
     for (int64_t i = 0; i < ns; i++) {
@@ -646,6 +677,10 @@ int Engine::launch_round() {
         if (!evix.count(e)) {
             const int ix = (int)evix.size();
             evix[e] = ix;
+        }
+        if (e->tree) {
+            tree_slots[e->q->dec].push_back((int32_t)i);
+            continue;
         }
         const int64_t jb = e->kind == 2 ? rs.slots[i].s : 0;
         const int64_t nj = e->chi - jb;
@@ -672,20 +707,43 @@ int Engine::launch_round() {
     for (int b = 0; b < kBuckets; b++) bstart[b + 1] = bstart[b] + nbucket[b];
     const int64_t nitp = bstart[kBuckets];
     const int64_t nitems = nitp + niw;
-    // upload block: desc | proj | words | items | ranges
+    // tree sums: a group of states per decomposition, its partial sums behind the items'
+    std::vector<TreeGroup> groups;
+    std::vector<int64_t> group_parts;  // each group's partial sums per state
+    int64_t ntree = 0, nparts = nitems;
+    for (auto& kv : tree_slots) {
+        Decomp* d = kv.first;
+        const int64_t c = (int64_t)kv.second.size();
+        csim::tree::choose_levels(d->plan, c);
+        TreeGroup g;
+        g.plan = &d->plan;
+        g.dplan = d->dplan;
+        g.count = c;
+        groups.push_back(g);
+        group_parts.push_back(tree_leaf_shape(d->plan, c).parts_per_state);
+        ntree += c;
+        nparts += c * group_parts.back();
+    }
+    const size_t scratch_bytes = tree_run_.layout(groups, kTreeScratchMax);
+    std::vector<unsigned char> tree_jobs;
+    tree_run_.build(nullptr, tree_jobs);  // for its size
+    // upload block: desc | proj | words | items | ranges | tree slots | tree jobs
     const size_t o_desc = 0;
     const size_t o_proj = align_up(o_desc + (size_t)ns * sizeof(csim::DrawDesc));
     const size_t o_words = align_up(o_proj + evix.size() * 192 * 8);
     const size_t o_items = align_up(o_words + (size_t)nwords * 4);
     const size_t o_range = align_up(o_items + (size_t)nitems * sizeof(csim::PairItem));
     const size_t o_range2 = align_up(o_range + (size_t)ns * 16);
-    const size_t up_bytes = align_up(o_range2 + (size_t)ns * 16);
+    const size_t o_ranged = align_up(o_range2 + (size_t)ns * 16);
+    const size_t o_tslots = align_up(o_ranged + (size_t)ns * 16);
+    const size_t o_tjobs = align_up(o_tslots + (size_t)ntree * 4);
+    const size_t up_bytes = align_up(o_tjobs + tree_jobs.size());
     bool any_direct = false;
     for (int b = 0; b < kBuckets; b++) any_direct |= b % 4 >= 2 && nbucket[b] > 0;
     // work block: states | parts | parts diag | pivot forms | direct and rest codes (direct launches)
     const size_t w_states = 0;
     const size_t w_part = align_up((size_t)ns * sizeof(csim_state));
-    const size_t w_partd = align_up(w_part + (size_t)std::max<int64_t>(nitems, 1) * 64);
+    const size_t w_partd = align_up(w_part + (size_t)std::max<int64_t>(nparts, 1) * 64);
     const size_t w_canon = align_up(w_partd + (size_t)std::max<int64_t>(nitems, 1) * 64);
     const size_t w_cdir = align_up(w_canon + (any_direct ? (size_t)ns * csim::canon_bytes() : 0));
     const size_t w_crest = align_up(w_cdir + (any_direct ? (size_t)ns * 4 : 0));
@@ -695,7 +753,7 @@ int Engine::launch_round() {
     rs.off_sum = align_up(rs.off_codes + (size_t)ns * 4);
     rs.off_sumd = align_up(rs.off_sum + (size_t)ns * 64);
     const size_t down_bytes = align_up(rs.off_sumd + (size_t)ns * 64);
-    if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) || rs.down.ensure(down_bytes) ||
+    if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) || tree_scratch_.ensure(scratch_bytes) || rs.down.ensure(down_bytes) ||
         rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes))
         return fail(ctx_, CSIM_ERR_NOMEM, "round buffers (%lld states, %lld items)", (long long)ns,
                     (long long)nitems);
@@ -724,6 +782,7 @@ int Engine::launch_round() {
     csim::PairItem* hitems = (csim::PairItem*)(hb + o_items);
     int64_t* hrange = (int64_t*)(hb + o_range);    // a slot's items in its heavy or warp launch
     int64_t* hrange2 = (int64_t*)(hb + o_range2);  // and in its light launch
+    int64_t* hranged = (int64_t*)(hb + o_ranged);  // items with a diagonal term (exactProjector rows)
     const double* dcum = (const double*)cum_.p;
     const csim::GState* dstates = (const csim::GState*)(wb + w_states);
     int64_t cur[kBuckets];
@@ -755,6 +814,8 @@ int Engine::launch_round() {
             d.id = e->id0 + (uint64_t)s;
         }
         hdesc[i] = d;
+        hranged[2 * i] = hranged[2 * i + 1] = 0;
+        if (e->tree) continue;  // ranges below, by group
         const int64_t jb = e->kind == 2 ? s : 0;
         const int64_t diag = e->kind == 2 ? s : -1;
         if (!r->exact && r->dec->kern == 3) {
@@ -773,6 +834,10 @@ int Engine::launch_round() {
             for (int64_t j = jn; j < e->chi; j += span_tp)
                 hitems[cd++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, cw, nullptr};
             hrange2[2 * i + 1] = cd;
+            if (e->kind == 2) {  // no narrow items
+                hranged[2 * i] = hrange2[2 * i];
+                hranged[2 * i + 1] = cd;
+            }
         } else if (!r->exact) {
             // heavy items first, then light ones; a slot's items may sit in two
             // launches, so its range is kept per slot in each (see below)
@@ -790,6 +855,10 @@ int Engine::launch_round() {
             for (int64_t j = std::max(jl, jb); j < e->chi; j += span_tp)
                 hitems[cl++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, r->dec->cws, nullptr};
             hrange2[2 * i + 1] = cl;
+            if (e->kind == 2) {  // no light items
+                hranged[2 * i] = hrange[2 * i];
+                hranged[2 * i + 1] = hrange[2 * i + 1];
+            }
         } else {
             hrange2[2 * i] = hrange2[2 * i + 1] = 0;
             hrange[2 * i] = iw;
@@ -797,7 +866,31 @@ int Engine::launch_round() {
                 hitems[iw++] = csim::PairItem{i, j, std::min(span_w, e->chi - j), diag, nullptr,
                                               (const csim::GState*)r->dec->phis};
             hrange[2 * i + 1] = iw;
+            if (e->kind == 2) {
+                hranged[2 * i] = hrange[2 * i];
+                hranged[2 * i + 1] = iw;
+            }
         }
+    }
+    {
+        int32_t* hslots = (int32_t*)(hb + o_tslots);
+        int64_t at = 0, p0 = nitems;
+        size_t gi = 0;
+        for (auto& kv : tree_slots) {
+            groups[gi].index = (const int32_t*)(db + o_tslots) + at;
+            groups[gi].part = (__int128*)(wb + w_part) + 4 * p0;
+            const int64_t pp = group_parts[gi];
+            for (int32_t i : kv.second) {
+                hslots[at++] = i;
+                hrange[2 * i] = p0;
+                hrange[2 * i + 1] = p0 += pp;
+                hrange2[2 * i] = hrange2[2 * i + 1] = 0;
+            }
+            gi++;
+        }
+        tree_run_.layout(groups, kTreeScratchMax);
+        tree_run_.build((unsigned char*)tree_scratch_.p, tree_jobs);
+        if (!tree_jobs.empty()) memcpy(hb + o_tjobs, tree_jobs.data(), tree_jobs.size());
     }
     int* derr = (int*)dd;
     const csim::Launch L = launch_on(derr);
@@ -847,13 +940,15 @@ int Engine::launch_round() {
         }
         if (rc) return fail(ctx_, CSIM_ERR_CUDA, "pair launch failed");
     }
+    if (!groups.empty() && tree_run_.launch(L, db + o_tjobs, dstates, dcode))
+        return fail(ctx_, CSIM_ERR_CUDA, "tree launch failed");
     if (csim::launch_items_warp(L, ditems + nitp, niw, dstates, dcode, part + 4 * nitp, partd + 4 * nitp))
         return fail(ctx_, CSIM_ERR_CUDA, "pair launch failed");
     CK(cudaEventRecord(rs.ev[2], ctx_->stream));
     const int64_t* drange = (const int64_t*)(db + o_range);
     const int64_t* drange2 = (const int64_t*)(db + o_range2);
     if (csim::launch_reduce_slots(L, part, drange, drange2, ns, (__int128*)(dd + rs.off_sum)) ||
-        csim::launch_reduce_slots(L, partd, drange, drange2, ns, (__int128*)(dd + rs.off_sumd)))
+        csim::launch_reduce_slots(L, partd, (const int64_t*)(db + o_ranged), nullptr, ns, (__int128*)(dd + rs.off_sumd)))
         return fail(ctx_, CSIM_ERR_CUDA, "reduce launch failed");
     CK(cudaMemcpyAsync(rs.hdown.p, dd, down_bytes, cudaMemcpyDeviceToHost, ctx_->stream));
     CK(cudaEventRecord(rs.ev[3], ctx_->stream));
