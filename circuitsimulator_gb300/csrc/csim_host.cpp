@@ -525,32 +525,43 @@ extern "C" int csim_term_products(csim_ctx* ctx, int32_t t, int32_t exact, const
 namespace {
 
 
-// The tree plan of code L for `count` states, kept from call to call while L is the same
-void tree_plan_for(csim_ctx* ctx, const uint64_t* L, int k, int t, int64_t count) {
-    std::vector<uint64_t> key(L, L + k);
-    key.push_back((uint64_t)k);
+// The tree plan of a decomposition (|H^t> if exact, code L otherwise) for `count`
+// states, kept from call to call while the decomposition is the same
+void tree_plan_for(csim_ctx* ctx, int exact, const uint64_t* L, int k, int t, int64_t count) {
+    std::vector<uint64_t> key;
+    if (!exact) key.assign(L, L + k);
+    key.push_back(exact ? ~0ull : (uint64_t)k);
     key.push_back((uint64_t)t);
     if (key != ctx->tree_key) {
         ctx->tree_key.clear();
         ctx->tree_plan = csim::tree::Plan();
-        csim::tree::build_chain(L, k, t, ctx->tree_plan);
+        if (exact) csim::tree::build_pairs(t, ctx->tree_plan);
+        else csim::tree::build_chain(L, k, t, ctx->tree_plan);
         ctx->tree_key = key;
     }
     csim::tree::choose_levels(ctx->tree_plan, count);
 }
 
+// whether a decomposition's terms are summed as a tree: unless a pair kernel is asked for
+bool use_tree(const csim_ctx* ctx, int t, int exact, int k) {
+    return ctx->pair_kernel == 0 && !ctx->tuning && (exact ? (t + 1) / 2 : k) <= kTreeMaxRows;
+}
+
 // A sampler call's inputs on the device, one upload: the projector's rows, the
-// d-distribution of randomStabilizerState, the projection factors, the tree plan
+// d-distribution of randomStabilizerState, the projection factors, the tree plan, the code
 struct CallInputs {
     const int* pm;
     const uint64_t *pz, *px;
     const double *cum, *factor;
     const unsigned char* plan;
+    const uint64_t* L;
 };
-int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Plan* plan, CallInputs* in) {
+int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Plan* plan, CallInputs* in,
+                    const uint64_t* L = nullptr, int k = 0) {
     const size_t n = (size_t)P->nstabs;
     const size_t o_px = 8 * n, o_cum = 16 * n, o_factor = o_cum + 8 * (CSIM_MAX_QUBITS + 1),
-                 o_plan = o_factor + 8 * (n + 1), o_pm = o_plan + kTreePlanBytes, bytes = o_pm + 4 * n;
+                 o_plan = o_factor + 8 * (n + 1), o_L = o_plan + kTreePlanBytes, o_pm = o_L + 8 * (size_t)k,
+                 bytes = o_pm + 4 * n;
     void* v;
     CKR(staged_room(ctx, 6, bytes, &v));
     unsigned char* const h = (unsigned char*)v;
@@ -560,6 +571,7 @@ int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Pl
     for (size_t c = 0; c <= n; c++) ((double*)(h + o_factor))[c] = sqrt_half_power((int)c);
     if (plan) tree_plan_image(*plan, h + o_plan);
     else memset(h + o_plan, 0, kTreePlanBytes);
+    if (k) memcpy(h + o_L, L, 8 * (size_t)k);
     for (size_t r = 0; r < n; r++) ((int32_t*)(h + o_pm))[r] = phase_m(P->phase[r]);
     CKR(staged_send(ctx, 6, kBufCall, bytes, &v));
     const unsigned char* const d = (const unsigned char*)v;
@@ -568,6 +580,7 @@ int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Pl
     in->cum = (const double*)(d + o_cum);
     in->factor = (const double*)(d + o_factor);
     in->plan = d + o_plan;
+    in->L = (const uint64_t*)(d + o_L);
     in->pm = (const int*)(d + o_pm);
     return 0;
 }
@@ -609,8 +622,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int t = P->nqubits;
     CKR(check_code(ctx, t, exact, L, k));
     if (rng != CSIM_RNG_LIBC && rng != CSIM_RNG_PHILOX) return fail(ctx, CSIM_ERR_ARG, "unknown rng %d", rng);
-    // |L> terms: the tree sum (csim_tree.cuh), unless a pair kernel is asked for
-    const bool tree = !exact && ctx->pair_kernel == 0 && !ctx->tuning && k <= kTreeMaxRows;
+    const bool tree = use_tree(ctx, t, exact, k);
     const bool tp = !exact && !tree && ctx->pair_kernel != 1;
     TpTune tn = default_tune(t);
     if (tp && count > 0) CKR(tune_for(ctx, t, &tn, P, L, k));  // before any draw: tuning leaves the streams as they are
@@ -630,7 +642,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int pt = tn.per_thread;
     const int64_t batch = 1 << 14;
     const int64_t shape_count = std::min(count, batch);
-    if (tree) tree_plan_for(ctx, L, k, t, shape_count);
+    if (tree) tree_plan_for(ctx, exact, L, k, t, shape_count);
     const int64_t nchunks = tree ? tree_leaf_shape(ctx->tree_plan, shape_count).parts_per_state
                                  : (tp ? csim::terms_tp_blocks(chi, pt) : (chi + chunk - 1) / chunk);
 
@@ -701,12 +713,12 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
                 const uint32_t* dw;
                 const int64_t* doff;
                 CKR(put_state_words(ctx, 2 * (sb & 1), t, hcum, cs, &dw, &doff));
-                draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, scode};
+                draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, scode, nullptr, 0, 0};
                 if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 2, 0, 0, dw, doff, in.cum, sth, nullptr))
                     return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
             } else {
                 draw = csim::TreeDraw{0, P->nstabs, ctx->philox_seed, ctx->philox_next, nullptr, nullptr, in.cum, in.pm,
-                                      in.pz, in.px, scode};
+                                      in.pz, in.px, scode, nullptr, 0, 0};
                 if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 0, ctx->philox_seed, ctx->philox_next,
                                                         nullptr, nullptr, in.cum, sth, nullptr))
                     return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
@@ -1084,6 +1096,70 @@ extern "C" int csim_median_of_means(const double* values, int32_t samples, int32
 
 namespace {
 
+// exact_rows through the tree sum: each row's state is a term, made, projected and
+// put into graph form by one warp; the tree runs over all terms of the row, and the
+// leaves j <= i are left out of its sum (the diagonal j = i is kept apart).
+int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, int exact, int64_t i0, int64_t nrow,
+              double* re_out, double* im_out) {
+    const int t = P->nqubits;
+    const csim::tree::Plan& plan = ctx->tree_plan;
+    const int64_t chi = (int64_t)1 << plan.r, parts = tree_leaf_shape(plan, nrow).parts_per_state;
+    void* v;
+    CallInputs in;
+    CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+    CKR(put_call_inputs(ctx, P, &plan, &in, exact ? nullptr : L, exact ? 0 : k));
+    CKR(dbuf(ctx, kBufCode, (size_t)nrow * 4, &v));
+    int* const dcode = (int*)v;
+    CKR(dbuf(ctx, kBufParts, (size_t)nrow * parts * 64, &v));
+    __int128* const dpart = (__int128*)v;
+    CKR(dbuf(ctx, kBufPartsDiag, (size_t)nrow * 64, &v));
+    __int128* const ddiag = (__int128*)v;
+    CK(cudaMemsetAsync(ddiag, 0, (size_t)nrow * 64, ctx->stream));
+    TreeGroup g;
+    g.plan = &plan;
+    g.dplan = in.plan;
+    g.count = nrow;
+    g.part = dpart;
+    g.rows = true;
+    g.row0 = i0;
+    g.diag = ddiag;
+    TreeRun run;
+    std::vector<unsigned char> jobs;
+    void* scratch;
+    unsigned char* djobs;
+    CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
+    run.build((unsigned char*)scratch, jobs);
+    CKR(staged_put(ctx, 4, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+    const csim::TreeDraw draw{3,       P->nstabs, 0,     (uint64_t)i0, nullptr, nullptr,        nullptr, in.pm,
+                              in.pz,   in.px,     dcode, in.L,         exact ? -1 : k, 0};
+    if (run.launch(launch_of(ctx), djobs, nullptr, nullptr, &draw, ctx->ev[1]))
+        return fail(ctx, CSIM_ERR_CUDA, "tree launch failed");
+    CK(cudaEventRecord(ctx->ev[2], ctx->stream));
+    // results: the live rows' count, the error word, the live rows' terms, re, im
+    const size_t head = 32, bytes = head + (size_t)nrow * 16;
+    CKR(dbuf(ctx, kBufResults, bytes, &v));
+    unsigned char* const dres = (unsigned char*)v;
+    CK(cudaMemsetAsync(dres, 0, head, ctx->stream));
+    if (csim::launch_tree_rows(launch_of(ctx), dpart, ddiag, nrow, parts, t, dcode, in.factor, (double*)(dres + head),
+                               (double*)(dres + head) + nrow, (unsigned long long*)dres, chi - i0))
+        return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
+    CK(cudaMemcpyAsync(dres + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(cudaEventRecord(ctx->ev[3], ctx->stream));
+    CKR(staged_room(ctx, 7, bytes, &v));
+    CKR(dget(ctx, (unsigned char*)v, dres, bytes));
+    CK(cudaStreamSynchronize(ctx->stream));
+    CK(cudaGetLastError());
+    CKR(error_status(ctx, ((const int*)v)[2]));
+    CKR(stats_batch(ctx));
+    const double* const res = (const double*)((const unsigned char*)v + head);
+    memcpy(re_out, res, (size_t)nrow * 8);
+    memcpy(im_out, res + nrow, (size_t)nrow * 8);
+    ctx->stats.states = nrow;
+    ctx->stats.states_live = ((const int64_t*)v)[0];
+    ctx->stats.pairs += ((const int64_t*)v)[2];
+    return CSIM_OK;
+}
+
 // Rows [i0, i1) of exactProjector (innerprod.c:148-261): row i adds
 // 2^{-c_i/2} (diag_i + 2 Re off_i), where off_i = sum_{j>i} <Pi phi_i|phi_j> and
 // c_i counts the 2^{-1/2} factors of the projection.  Each row's sum is exact
@@ -1099,6 +1175,11 @@ int exact_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k,
     if (i0 < 0 || i1 < i0 || i1 > chi) return fail(ctx, CSIM_ERR_ARG, "row range [%lld, %lld) outside [0, chi)",
                                                   (long long)i0, (long long)i1);
     if (i0 == i1) return CSIM_OK;
+    const int64_t nrow = i1 - i0;
+    if (use_tree(ctx, t, exact, k)) {
+        tree_plan_for(ctx, exact, L, k, t, nrow);
+        if (tree_rows_ok(ctx->tree_plan)) return tree_rows(ctx, P, L, k, exact, i0, nrow, re_out, im_out);
+    }
     const int nr = t > 32 ? 2 : 1;
     const int P2 = 2 * t;
     void* v;
@@ -1158,7 +1239,6 @@ int exact_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k,
         csim::launch_reduce_parts(launch_of(ctx), dpartd, chi, nchunks, daccd))
         return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-    const int64_t nrow = i1 - i0;
     std::vector<int> code(nrow);
     std::vector<__int128> acc(nrow * 4), accd(nrow * 4);
     CKR(dget(ctx, code.data(), dcode + i0, nrow));

@@ -159,38 +159,6 @@ __global__ void __launch_bounds__(256) k_project(GState* s, int64_t count, int n
 }
 
 // ------------------------------------------------------------ decomposition terms
-// prepH (stateprep.c:36-81): bit j of the ceil(t/2)-bit index, MSB first
-template <int NR>
-__device__ void prep_h(WS<NR>& s, int t, int64_t idx) {
-    const int size = (t + 1) / 2;
-    init_identity<NR>(s, t);
-#pragma unroll
-    for (int sl = 0; sl < NR; sl++) {
-        const int x = row_of<NR>(sl);
-        if (x < t) {
-            const int j = x / 2;
-            const int bit = (int)((idx >> (size - 1 - j)) & 1);
-            if (bit == 0 && !((t % 2) && j == size - 1)) s.J[sl] |= bit1(x ^ 1);
-        }
-    }
-    for (int j = 0; j < size; j++) {
-        const int bit = (int)((idx >> (size - 1 - j)) & 1);
-        if ((t % 2) && j == size - 1) {
-            if (bit == 1) shrink<NR, false, true>(s, bit1(t - 1), 0);
-            continue;
-        }
-        if (bit == 1) shrink<NR, false, true>(s, bit1(2 * j + 1) | bit1(2 * j), 0);
-    }
-}
-
-// prepL (stateprep.c:85-120) from the codeword x of the term
-template <int NR>
-__device__ void prep_l(WS<NR>& s, int t, uint64_t x) {
-    init_identity<NR>(s, t);
-    for (int idx = 0; idx < t; idx++)
-        if (!getbit(x, idx)) shrink_unit<NR, true>(s, idx);
-}
-
 // codeword of term j: rows r of L with bit (k-1-r) of j set (binrep, stateprep.c:5-32)
 __global__ void k_codewords(const uint64_t* L, int k, int64_t j0, int64_t count, uint64_t* out) {
     __shared__ uint64_t sL[64];

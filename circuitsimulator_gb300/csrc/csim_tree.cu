@@ -1,5 +1,5 @@
-// csim_tree.cu — kernels of the tree sum (csim_tree.cuh): all terms of a |L>
-// decomposition for many states.
+// csim_tree.cu — kernels of the tree sum (csim_tree.cuh): all terms of a
+// decomposition, |L> or |H^t>, for many states.
 //   k_tree_root   one warp per state: its graph form (csim_canon_warp.cuh) on
 //                 coordinates in the plan's order, as a root node
 //   k_tree_draw   the same for states that the warp draws and projects itself
@@ -8,7 +8,8 @@
 //   k_tree_leaf   one thread per node of the last written level (or a part of
 //                 one): the remaining levels, then the leaves' values from truth
 //                 tables, summed exactly
-//   k_tree_values one warp per state: its sum, as the sampler's value
+//   k_tree_values one warp per state: its sum, as the sampler's value or as a row
+//                 of exactProjector
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -133,7 +134,7 @@ __device__ void store_root(const TreeRootJob& J, int64_t i, const WS<NR>& st, Ro
     if (r0 < k) store_row(J.out, J.count, i, t, w.p0, row0);
     if (r1 < k) store_row(J.out, J.count, i, t, w.p1, row1);
     if (r0 == 0)
-        store_scalars(J.out, J.count, i, t, to_coords(w.D1, piv), to_coords(w.D2, piv) | bm, ~w.P & nm, 0ull,
+        store_scalars(J.out, J.count, i, t, to_coords(w.D1, piv), to_coords(w.D2, piv) | bm, ~w.P & nm, J.x0,
                       pack_status(st.Q + w.dq, 0, 0));
 }
 
@@ -182,9 +183,23 @@ __global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRoo
     if (i >= J.count) return;  // warp-uniform
     const int64_t a = J.first + i;
     int e = 0;
-    DevRng rng = make_rng(d.mode, d.seed, d.id + a, d.words, d.mode ? d.offsets[a] : 0, d.mode ? d.offsets[a + 1] : 0);
+    const bool replay = d.mode == 1 || d.mode == 2;
+    DevRng rng = make_rng(replay ? d.mode : 0, d.seed, d.id + a, d.words, replay ? d.offsets[a] : 0,
+                          replay ? d.offsets[a + 1] : 0);
     WS<NR> st;
-    random_state<NR>(st, J.t, rng, d.cum, e);
+    if (d.mode == 3) {  // uniform
+        const int64_t j = (int64_t)d.id + a;
+        if (d.k < 0) {
+            prep_h<NR>(st, J.t, j);
+        } else {
+            uint64_t x = 0ull;
+            for (int r = 0; r < d.k; r++)
+                if ((j >> (d.k - 1 - r)) & 1) x ^= d.words64[r];
+            prep_l<NR>(st, J.t, x);
+        }
+    } else {
+        random_state<NR>(st, J.t, rng, d.cum, e);
+    }
     int c = 0;  // the number of 2^{-1/2} factors, -1 once a measurement annihilates the state
     for (int r = 0; r < d.nstabs; r++) {
         const int res = measure_pauli<NR>(st, d.pm[r], d.pz[r], d.px[r]);
@@ -231,7 +246,7 @@ __device__ __forceinline__ void store_two(uint32_t* plane, uint32_t at, uint32_t
 // twice, so a lane moves on from one sibling to the other without a load: a stage
 // from 28 to 15 vertices took 985 us for 14.3e6 nodes with a node per thread, 576
 // with a pair.
-template <class W>
+template <class W, bool PAIRS>
 __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStageJob* jobs, int njobs) {
     extern __shared__ __align__(16) uint32_t smem[];
     const TreeStageJob& J = job_of(jobs, njobs, blockIdx.x);
@@ -310,8 +325,21 @@ __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStag
     const W xc = both ? x ^ (W)J.gen[0] : x;
     a.sum = alive ? (x ^ a.s.h) & block : (W)0;  // the others of the block are set to 0
     c.sum = (alive && both) ? (xc ^ c.s.h) & block : (W)0;
-    a.live = cm | a.sum;
-    c.live = cm | c.sum;
+    auto two = rows;
+    two.shift(copy);
+    if constexpr (PAIRS) {
+        const int hi = J.paired < mp ? J.paired : mp;
+        const W pm2 = wlow<W>(hi) & block;  // the block's paired positions
+        a.sum &= ~pm2;
+        c.sum &= ~pm2;
+        a.live = cm | a.sum | pm2;
+        c.live = cm | c.sum | pm2;
+        join_pairs<W>(rows, a, x, mc, hi, alive);
+        join_pairs<W>(two, c, xc, mc, hi, alive && both);
+    } else {
+        a.live = cm | a.sum;
+        c.live = cm | c.sum;
+    }
     contract_pair(rows, copy, a, c, mc);
     if (!valid) return;
     const uint32_t sa = pack_status(a.s.q, a.s.iso, a.s.dead), sc = pack_status(c.s.q, c.s.iso, c.s.dead);
@@ -324,8 +352,6 @@ __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStag
         return;
     }
     const uint32_t at = 2u * i;
-    auto two = rows;
-    two.shift(copy);
     if (!(a.s.dead && c.s.dead)) {
         if (mc > 32) {
             for (int r = 0; r < mc; r++) {
@@ -376,8 +402,9 @@ __device__ __forceinline__ int64_t shfl_xor_i64(int64_t v, int m) { return (int6
 // ALU-bound (80% of the pipe; the counts run on the XU pipe).  Six blocks per SM:
 // 80 registers without spills; with 128 registers (four blocks) t = 40 is 1.5%
 // slower and t = 48 3.5%, with 72 (seven) within 0.4%.
-template <int WORDS>
-__global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLeafJob* jobs, int njobs) {
+// ROWS: exactProjector rows, PAIRS: terms of |H^t> (TreeLeafJob).
+template <int WORDS, bool ROWS, bool PAIRS>
+__global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(const TreeLeafJob* jobs, int njobs) {
     __shared__ uint32_t lin[32], sub[32];
     __shared__ __align__(16) uint32_t wrows[2 * 8 * kTreeLeafThreads];
     __shared__ int64_t red[kTreeLeafThreads / 32][4];
@@ -413,10 +440,21 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
         uint32_t x = hx >> 16;
         for (int b = 0; b < J.split; b++)
             if ((part >> b) & 1) x ^= J.gen[J.je - J.split + b];
+        int64_t state = 0, row = 0, term = 0;  // ROWS: the state, its row, and the term index so far
+        if constexpr (ROWS) {
+            state = node >> J.nodes_log2;
+            row = J.row ? J.row[state] : J.row0 + state;
+            for (int b = 0; b < J.nodes_log2; b++)
+                if ((node >> b) & 1) term ^= (int64_t)J.term[J.je + b];
+            for (int b = 0; b < J.split; b++)
+                if ((part >> b) & 1) term ^= (int64_t)J.term[J.je - J.split + b];
+        }
         int y[4] = {0, 0, 0, 0};  // this part's sum, relative to 2^{iso0 / 2}
         // table nodes two at a time, in Gray code order
         for (int s = 0; s < nsub; s += 2) {
             if (s) x ^= J.gen[tj + __ffs(s) - 1];
+            if constexpr (ROWS)
+                if (s) term ^= (int64_t)J.term[tj + __ffs(s) - 1];
             const uint32_t x2 = nsub > 1 ? x ^ J.gen[tj] : x;
             Work<uint32_t> wa, wb;
             wa.s = Node<uint32_t>{dd & 0xFFFFu, dd >> 16, hx & 0xFFFFu, (int)(status & 7u), 0, 0};
@@ -424,10 +462,20 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
             if (m > tv) {
                 *rows.unit(0) = *rows2.unit(0) = U32x4{w[0], w[1], w[2], w[3]};
                 if (m > 8) *rows.unit(1) = *rows2.unit(1) = U32x4{w[4], w[5], w[6], w[7]};
-                wa.sum = alive ? (x ^ wa.s.h) & mm & ~vm : 0u;
-                wb.sum = alive && nsub > 1 ? (x2 ^ wb.s.h) & mm & ~vm : 0u;
-                wa.live = vm | wa.sum;
-                wb.live = vm | wb.sum;
+                if constexpr (PAIRS) {  // every position below paired is a pair's, a single qubit above them
+                    const uint32_t pm = wlow<uint32_t>(m & ~1);
+                    wa.sum = alive ? (x ^ wa.s.h) & mm & ~pm : 0u;
+                    wb.sum = alive && nsub > 1 ? (x2 ^ wb.s.h) & mm & ~pm : 0u;
+                    wa.live = pm | wa.sum;
+                    wb.live = pm | wb.sum;
+                    join_pairs<uint32_t>(rows, wa, x, 0, m & ~1, alive);
+                    join_pairs<uint32_t>(rows2, wb, x2, 0, m & ~1, alive && nsub > 1);
+                } else {
+                    wa.sum = alive ? (x ^ wa.s.h) & mm & ~vm : 0u;
+                    wb.sum = alive && nsub > 1 ? (x2 ^ wb.s.h) & mm & ~vm : 0u;
+                    wa.live = vm | wa.sum;
+                    wb.live = vm | wb.sum;
+                }
                 sum_out_pair<uint32_t>(rows, copy, wa, wb, ~0u);
             }
 #pragma unroll 1
@@ -448,20 +496,58 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
                 build_table<WORDS>(r, d1, nd.d2 & vm, lin, tb);
                 int evr = 0, evi = 0, odr = 0, odi = 0;
                 uint32_t S = ((e ? x2 : x) ^ nd.h) & vm;
-                for (int l = 0; l < (1 << tj); l++) {
-                    if (l) S ^= J.gen[__ffs(l) - 1] & vm;
-                    table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
-                }
-                if (alive && !nd.dead) {
-                    // (evr + i evi) + sqrt2 (odr + i odi), times w^q 2^{iso / 2}
-                    int v[4] = {evr, odr + odi, evi, odi - odr};
+                // (evr + i evi) + sqrt2 (odr + i odi), times w^q 2^{iso / 2}
+                auto node_sum = [&](int (&v)[4]) {
+                    v[0] = evr;
+                    v[1] = odr + odi;
+                    v[2] = evi;
+                    v[3] = odi - odr;
                     times_omega(v, nd.q);
                     if (nd.iso & 1) times_sqrt2(v);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) y[q] += v[q] << (nd.iso >> 1);
+                    for (int q = 0; q < 4; q++) v[q] <<= nd.iso >> 1;
+                };
+                int v[4];
+                if constexpr (ROWS) {
+                    int64_t j = e ? term ^ (int64_t)J.term[tj] : term;
+                    for (int l = 0; l < (1 << tj); l++) {
+                        if (l) {
+                            S ^= J.gen[__ffs(l) - 1] & vm;
+                            j ^= (int64_t)J.term[__ffs(l) - 1];
+                        }
+                        if (j > row) table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
+                        if (j == row && alive) {  // one leaf of a state
+                            const int keep[4] = {evr, evi, odr, odi};
+                            evr = evi = odr = odi = 0;
+                            if (!nd.dead) table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
+                            node_sum(v);
+                            int64_t dz[4];
+                            if (iso0 & 1) times_sqrt2(v);
+                            for (int q = 0; q < 4; q++) dz[q] = (int64_t)v[q] << (iso0 >> 1);
+                            if (J.shift & 1) times_sqrt2(dz);
+                            for (int q = 0; q < 4; q++) J.diag[4 * state + q] = (__int128)dz[q] << (J.shift >> 1);
+                            evr = keep[0];
+                            evi = keep[1];
+                            odr = keep[2];
+                            odi = keep[3];
+                        }
+                    }
+                } else {
+                    for (int l = 0; l < (1 << tj); l++) {
+                        if (l) S ^= J.gen[__ffs(l) - 1] & vm;
+                        table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
+                    }
+                }
+                if (alive && !nd.dead) {
+                    node_sum(v);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) y[q] += v[q];
                 }
             }
-            if (nsub > 1) x = x2;
+            if (nsub > 1) {
+                x = x2;
+                if constexpr (ROWS) term ^= (int64_t)J.term[tj];
+            }
         }
         if (iso0 & 1) times_sqrt2(y);
 #pragma unroll
@@ -509,42 +595,56 @@ __device__ __forceinline__ double int128_to_double(__int128 z) {
     return neg ? -d : d;
 }
 
-// One warp per state: the sum of its partial sums, and singleProjectorSample's
-// value 2^t |projfactor sum|^2 (innerprod.c:142) with the host's own roundings
-// (csim_host::zomega_to_complex: no fused multiply-adds).  factor[c]: the
+__device__ __forceinline__ __int128 shfl_xor_i128(__int128 v, int m) {
+    const uint64_t lo = shfl_xor64((uint64_t)v, m), hi = shfl_xor64((uint64_t)((unsigned __int128)v >> 64), m);
+    return (__int128)(((unsigned __int128)hi << 64) | lo);
+}
+
+// One warp per state: the sum of its partial sums as a double, with the host's own
+// roundings (csim_host::zomega_to_complex: no fused multiply-adds).  factor[c]: the
 // projection factor of c measurements that halved the norm.  *live counts the
-// states that the projector left alive (0 for the others).
-__global__ void __launch_bounds__(128) k_tree_values(const __int128* part, int64_t count, int64_t parts, int t,
-                                                     const int* code, const double* factor, double* values,
-                                                     unsigned long long* live) {
+// states that the projector left alive (0 for the others).  Without diag: out is
+// singleProjectorSample's value 2^t |projfactor sum|^2 (innerprod.c:142); with it
+// out and im are exactProjector's row, diag + 2 Re sum (innerprod.c:187-195), and
+// live[2] counts the live rows' terms, row_terms - i for row i.
+__global__ void __launch_bounds__(128) k_tree_values(const __int128* part, const __int128* diag, int64_t count,
+                                                     int64_t parts, int t, const int* code, const double* factor,
+                                                     double* out, double* im_out, unsigned long long* live,
+                                                     int64_t row_terms) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= count) return;  // warp-uniform
     const int lane = lane_id(), q = lane & 3;
+    const int c = code[i];
     __int128 z = 0;
     for (int64_t p = lane >> 2; p < parts; p += 8) z += part[4 * (i * parts + p) + q];
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-        const uint64_t lo = shfl_xor64((uint64_t)z, o), hi = shfl_xor64((uint64_t)((unsigned __int128)z >> 64), o);
-        z += (__int128)(((unsigned __int128)hi << 64) | lo);
+    for (int o = 4; o < 32; o <<= 1) z += shfl_xor_i128(z, o);
+    // lanes 0..3 hold coordinates 0..3 and need z0, z1 - z3, z2, z1 + z3
+    const __int128 other = shfl_xor_i128(z, 2);
+    __int128 v = q == 1 ? z - other : (q == 3 ? other + z : z);
+    if (diag) {  // 2 Re(o) = 2 o0 + (o1 - o3) (w - w^3)
+        const __int128 d = c >= 0 ? diag[4 * i + q] : 0, dother = shfl_xor_i128(d, 2);
+        v = q == 0 ? d + 2 * z : (q == 1 ? d - dother + 2 * v : (q == 2 ? d : dother + d));
     }
-    // lanes 0..3 hold coordinates 0..3; lane 1 takes z1 - z3, lane 3 z1 + z3
-    const uint64_t lo = shfl_xor64((uint64_t)z, 2), hi = shfl_xor64((uint64_t)((unsigned __int128)z >> 64), 2);
-    const __int128 other = (__int128)(((unsigned __int128)hi << 64) | lo);
-    const double d = int128_to_double(q == 1 ? z - other : (q == 3 ? other + z : z));
+    const double x = int128_to_double(v);
     const double s = 0.70710678118654752440;
-    const double x0 = __shfl_sync(kFull, d, 0), x1 = __shfl_sync(kFull, d, 1), x2 = __shfl_sync(kFull, d, 2),
-                 x3 = __shfl_sync(kFull, d, 3);
+    const double x0 = __shfl_sync(kFull, x, 0), x1 = __shfl_sync(kFull, x, 1), x2 = __shfl_sync(kFull, x, 2),
+                 x3 = __shfl_sync(kFull, x, 3);
     if (lane != 0) return;
-    const int c = code[i];
-    double v = 0;
+    double a = 0, b = 0;
     if (c >= 0) {
         const double unit = __hiloint2double((1023 - t) << 20, 0);  // 2^-t
-        const double re = __dmul_rn(__dadd_rn(x0, __dmul_rn(x1, s)), unit), im = __dmul_rn(__dadd_rn(x2, __dmul_rn(x3, s)), unit);
-        const double a = __dmul_rn(re, factor[c]), b = __dmul_rn(im, factor[c]);
-        v = __dmul_rn(__hiloint2double((1023 + t) << 20, 0), __dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)));
+        a = __dmul_rn(__dmul_rn(__dadd_rn(x0, __dmul_rn(x1, s)), unit), factor[c]);
+        b = __dmul_rn(__dmul_rn(__dadd_rn(x2, __dmul_rn(x3, s)), unit), factor[c]);
         atomicAdd(live, 1ull);
+        if (diag) atomicAdd(live + 2, (unsigned long long)(row_terms - i));
     }
-    values[i] = v;
+    if (im_out) {
+        out[i] = a;
+        im_out[i] = b;
+    } else {
+        out[i] = __dmul_rn(__hiloint2double((1023 + t) << 20, 0), __dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)));
+    }
 }
 
 // ---------------------------------------------------------------- launchers
@@ -566,16 +666,18 @@ int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax) {
+int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax,
+                      bool pairs) {
     if (njobs <= 0 || blocks <= 0) return 0;
     if (blocks > 0x7fffffff || mmax < 1 || mmax > (wide ? 64 : 32)) return -1;
     // two copies of every lane's rows: at most 64 KB
     const size_t smem = 2 * (size_t)((mmax + 3) / 4) * 16 * kTreeStageThreads * (wide ? 2 : 1);
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(k_tree_stage<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 64 * 1024) != cudaSuccess)
+    const auto kernel = wide ? (pairs ? k_tree_stage<uint64_t, true> : k_tree_stage<uint64_t, false>)
+                             : (pairs ? k_tree_stage<uint32_t, true> : k_tree_stage<uint32_t, false>);
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess)
         return -1;
-    if (wide) k_tree_stage<uint64_t><<<(unsigned)blocks, kTreeStageThreads, smem, L.stream>>>(jobs, njobs);
-    else k_tree_stage<uint32_t><<<(unsigned)blocks, kTreeStageThreads, smem, L.stream>>>(jobs, njobs);
+    kernel<<<(unsigned)blocks, kTreeStageThreads, smem, L.stream>>>(jobs, njobs);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -583,20 +685,39 @@ int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int6
 int launch_tree_values(const Launch& L, const __int128* part, int64_t count, int64_t parts, int t, const int* code,
                        const double* factor, double* values, unsigned long long* live) {
     if (count <= 0) return 0;
-    k_tree_values<<<(unsigned)((count + 3) / 4), 128, 0, L.stream>>>(part, count, parts, t, code, factor, values, live);
+    k_tree_values<<<(unsigned)((count + 3) / 4), 128, 0, L.stream>>>(part, nullptr, count, parts, t, code, factor, values,
+                                                                     nullptr, live, 0);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words) {
+int launch_tree_rows(const Launch& L, const __int128* part, const __int128* diag, int64_t count, int64_t parts, int t,
+                     const int* code, const double* factor, double* re, double* im, unsigned long long* live,
+                     int64_t row_terms) {
+    if (count <= 0) return 0;
+    k_tree_values<<<(unsigned)((count + 3) / 4), 128, 0, L.stream>>>(part, diag, count, parts, t, code, factor, re, im,
+                                                                     live, row_terms);
+    (*L.launches)++;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+namespace {
+template <bool ROWS>
+void (*leaf_kernel(int words, bool pairs))(const TreeLeafJob*, int) {
+    if (pairs) return words == 1 ? k_tree_leaf<1, ROWS, true> : nullptr;
+    return words == 1 ? k_tree_leaf<1, ROWS, false>
+                      : (words == 2 ? k_tree_leaf<2, ROWS, false>
+                                    : (words == 4 ? k_tree_leaf<4, ROWS, false>
+                                                  : (words == 8 ? k_tree_leaf<8, ROWS, false> : nullptr)));
+}
+}  // namespace
+
+int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words, bool rows,
+                     bool pairs) {
     if (njobs <= 0 || blocks <= 0) return 0;
-    if (blocks > 0x7fffffff) return -1;
-    const unsigned g = (unsigned)blocks;
-    if (words == 1) k_tree_leaf<1><<<g, kTreeLeafThreads, 0, L.stream>>>(jobs, njobs);
-    else if (words == 2) k_tree_leaf<2><<<g, kTreeLeafThreads, 0, L.stream>>>(jobs, njobs);
-    else if (words == 4) k_tree_leaf<4><<<g, kTreeLeafThreads, 0, L.stream>>>(jobs, njobs);
-    else if (words == 8) k_tree_leaf<8><<<g, kTreeLeafThreads, 0, L.stream>>>(jobs, njobs);
-    else return -1;
+    const auto kernel = rows ? leaf_kernel<true>(words, pairs) : leaf_kernel<false>(words, pairs);
+    if (blocks > 0x7fffffff || !kernel) return -1;
+    kernel<<<(unsigned)blocks, kTreeLeafThreads, 0, L.stream>>>(jobs, njobs);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -277,6 +277,34 @@ CSIM_HD_INLINE void sum_out_pair(R rows, size_t words, Work<W>& a, Work<W>& b, W
     else a = w;
 }
 
+// Terms of |H^t> (libcirc/stateprep.c:36-81) are products of two-qubit states on the
+// vertices 2 i, 2 i + 1: for a term bit 0 CZ|++>, for 1 (|00> + |11>) / sqrt2.  With
+// an odd number of Hadamards on the two vertices they change places, with two each is
+// its own image.  Contracting with the first is an edge between the vertices and a
+// sum over both; with the second z_a = z_b: vertex a joins b and b is summed.
+// Brings the pairs in positions [lo, hi) into that form (x: the term bits, one on
+// each of a pair's positions); they are all in w.live before, in w.sum after.
+template <class W, class R>
+CSIM_HD_INLINE void join_pairs(const R& rows, Work<W>& w, W x, int lo, int hi, bool act) {
+    using T = WordTraits<W>;
+    Node<W>& s = w.s;
+    for (int a = lo; a < hi; a += 2) {  // uniform
+        const W ma = act ? wbit<W>(a) : (W)0, mb = act ? wbit<W>(a + 1) : (W)0;
+        const bool bell = (((x >> a) ^ (s.h >> a) ^ (s.h >> (a + 1))) & (W)1) != (W)0;
+        const W row = (W)rows.get(a) & w.live & ~ma;
+        const W N = (bell && act) ? row & ~mb : ma;  // U; the other kind: the edge a b
+        const bool jab = (row & mb) != (W)0;
+        if (bell) {
+            const bool a1 = (s.d1 & ma) != (W)0, a2 = (s.d2 & ma) != (W)0, b1 = (s.d1 & mb) != (W)0;
+            s.d2 ^= (a2 != (a1 && b1)) != jab ? mb : (W)0;  // D_b += D_a + 4 J_ab
+            s.d1 ^= a1 ? mb : (W)0;
+            w.live &= ~ma;
+        }
+        w.sum |= bell ? mb : ma | mb;
+        rows.rank2(uniform_max(T::bits - T::clz(w.live)), N, mb, mb, N);
+    }
+}
+
 // Sums two sibling nodes down to their first mc vertices.  With rows of two words
 // and mc <= 32 the second words are needed only until the vertices from 32 up are gone.
 CSIM_HD_INLINE void contract_pair(const Rows32& rows, size_t words, Work<uint32_t>& a, Work<uint32_t>& b, int) {

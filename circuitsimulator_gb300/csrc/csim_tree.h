@@ -20,6 +20,7 @@ struct TreeRootJob {
     const uint8_t* perm;  // position -> coordinate (t of them)
     uint32_t* out;        // node planes, one node per state
     int64_t count, block0;
+    uint64_t x0;          // the roots' X
     int32_t t, pad;
 };
 
@@ -29,7 +30,8 @@ struct TreeStageJob {
     uint32_t* out;
     const uint64_t* gen;  // generators of the levels jc .. jp - 1, sub of them
     int64_t count, in_count, block0;
-    int32_t mp, mc, sub, pad;
+    int32_t mp, mc, sub;
+    int32_t paired;       // terms of |H^t>: positions below this are pairs (join_pairs)
 };
 
 // sums below the nodes of level je (m <= 16 vertices).  A part is 2^-split of a
@@ -43,11 +45,20 @@ struct TreeLeafJob {
     int32_t m, je, tv, tj;
     int32_t split, reps, group, shift;  // sums are scaled by 2^{shift / 2}
     uint16_t gen[16];     // generators of the levels below je, positions < m
+    // exactProjector rows: state a is row row[a] (or row0 + a); only its terms j > row are
+    // summed, term j == row is written to diag + 4 a
+    const int32_t* row;
+    const uint64_t* term; // the generators' parts of the term index, all levels
+    __int128* diag;
+    int64_t row0;
+    int32_t nodes_log2, pad;  // log2 of the nodes per state
 };
 
 // How k_tree_draw makes its states (k_random_states, k_project): state a of the
 // call is state id + a of Philox stream `seed` (mode 0) or replays words
-// [offsets[a], offsets[a + 1]) (mode 1); code[a] as k_project writes it
+// [offsets[a], offsets[a + 1]) (mode 1).  Mode 3: exactProjector's term states,
+// state a is term id + a of the k-row code `words64` or (k < 0) of |H^t>.  code[a]
+// as k_project writes it.
 struct TreeDraw {
     int32_t mode, nstabs;  // mode 2: the words are raw (csim_rng.cuh)
     uint64_t seed, id;
@@ -57,6 +68,8 @@ struct TreeDraw {
     const int* pm;
     const uint64_t *pz, *px;
     int* code;
+    const uint64_t* words64;
+    int32_t k, pad;
 };
 
 constexpr int kTreeRootWarps = 4;      // states per root block
@@ -67,12 +80,19 @@ int launch_tree_root(const Launch& L, const TreeRootJob* jobs, int njobs, int64_
                      const int* code);
 int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, int t, const TreeDraw& d);
 // wide: the jobs' parents have more than 32 vertices (two words per row); mmax: the largest mp
-int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax);
-// words: the jobs' table words (tree::table_words(tv))
-int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words);
+int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax,
+                      bool pairs);
+// words: the jobs' table words (tree::table_words(tv)); rows: exactProjector rows; pairs: terms of |H^t> (one word)
+int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words, bool rows,
+                     bool pairs);
 
 // values[i] of `count` states from `parts` partial sums each; factor: 65 doubles; *live is added to
 int launch_tree_values(const Launch& L, const __int128* part, int64_t count, int64_t parts, int t, const int* code,
                        const double* factor, double* values, unsigned long long* live);
+// the rows' values of exactProjector: re[i] + i im[i] = factor (diag + 2 Re sum of the parts);
+// row_terms - i of each live row i is added to live[2]
+int launch_tree_rows(const Launch& L, const __int128* part, const __int128* diag, int64_t count, int64_t parts, int t,
+                     const int* code, const double* factor, double* re, double* im, unsigned long long* live,
+                     int64_t row_terms);
 
 }  // namespace csim

@@ -15,8 +15,8 @@
 
 namespace csim_host {
 
-// A plan's arrays on the device: gen (64 words), then perm (64 bytes)
-constexpr size_t kTreePlanBytes = 64 * 8 + 64;
+// A plan's arrays on the device: gen, term (64 words each), then perm (64 bytes)
+constexpr size_t kTreePlanBytes = 2 * 64 * 8 + 64;
 
 struct TreeGroup {
     const csim::tree::Plan* plan = nullptr;
@@ -25,7 +25,15 @@ struct TreeGroup {
     int64_t first = 0, count = 0;
     int64_t shape_count = 0;               // states that tree_leaf_shape is asked for (0: count)
     __int128* part = nullptr;              // device: parts_per_state partial sums for each state
+    // exactProjector rows (TreeLeafJob): the states' rows (device; null: row0, row0 + 1, ...), and 4
+    // int128 per state that are zero before the launches
+    bool rows = false;
+    const int32_t* row = nullptr;
+    int64_t row0 = 0;
+    __int128* diag = nullptr;
 };
+// whether the tree sums exactProjector rows of a plan: a term index for each leaf
+inline bool tree_rows_ok(const csim::tree::Plan& p) { return p.r == p.k; }
 
 // How the leaf kernel covers the states of a group.  Small groups split a
 // node's leaves over several threads until the GPU has enough of them; large
@@ -58,7 +66,7 @@ inline void tree_scratch_per_state(const csim::tree::Plan& p, int64_t (&half)[2]
 }
 
 constexpr size_t kTreeScratchMax = (size_t)1 << 30;
-// codes of more rows run on the pair kernels (node indices are 32 bits)
+// decompositions of more than 2^30 terms run on the pair kernels (node indices are 32 bits)
 constexpr int kTreeMaxRows = 30;
 
 class TreeRun {
@@ -119,15 +127,16 @@ class TreeRun {
         steps_.clear();
         for (const Chunk& ch : chunks_) {
             std::vector<csim::TreeRootJob> roots;
-            std::vector<csim::TreeLeafJob> leaves[4];  // by table words 1, 2, 4, 8
-            int64_t rb = 0, lb[4] = {0, 0, 0, 0};
+            std::vector<csim::TreeLeafJob> leaves[16];  // by table words (1, 2, 4, 8), rows, pairs
+            int64_t rb = 0, lb[16] = {};
             size_t depth = 0;
             for (const Piece& p : ch.pieces) {
                 const csim::tree::Plan& pl = *p.g.plan;
                 csim::TreeRootJob r{};
                 r.index = p.g.index ? p.g.index + p.first : nullptr;
                 r.first = p.g.first + p.first;
-                r.perm = p.g.dplan + 64 * 8;
+                r.perm = p.g.dplan + 2 * 64 * 8;
+                r.x0 = pl.x0;
                 r.out = (uint32_t*)(scratch + p.off[0]);
                 r.count = p.count;
                 r.block0 = rb;
@@ -142,7 +151,7 @@ class TreeRun {
                 l.part = p.g.part + 4 * p.first * s.parts_per_state;
                 l.in_count = p.count << (pl.r - je);
                 l.threads = p.count * s.threads_per_state;
-                const int wc = std::max(0, pl.tv - 5);
+                const int wc = std::max(0, pl.tv - 5) + (p.g.rows ? 4 : 0) + (pl.pairs ? 8 : 0);
                 l.block0 = lb[wc];
                 l.m = pl.vert.back();
                 l.je = je;
@@ -153,18 +162,25 @@ class TreeRun {
                 l.group = s.group;
                 l.shift = pl.t - pl.tv + 2 * (pl.k - pl.r);  // each codeword 2^{k - r} times
                 for (int j = 0; j < je; j++) l.gen[j] = (uint16_t)pl.gen[j];
+                if (p.g.rows) {
+                    l.row = p.g.row ? p.g.row + p.first : nullptr;
+                    l.row0 = p.g.row0 + p.first;
+                    l.term = (const uint64_t*)p.g.dplan + 64;
+                    l.diag = p.g.diag + 4 * p.first;
+                    l.nodes_log2 = pl.r - je;
+                }
                 lb[wc] += (l.threads + csim::kTreeLeafThreads - 1) / csim::kTreeLeafThreads;
                 leaves[wc].push_back(l);
             }
-            add(blob, Step{0, false, ch.pieces[0].g.plan->t, (int)roots.size(), rb, 0}, roots);
+            add(blob, Step{0, 0, ch.pieces[0].g.plan->t, (int)roots.size(), rb, 0}, roots);
             for (size_t d = 1; d < depth; d++)
-                for (int wide = 1; wide >= 0; wide--) {
+                for (int kind = 0; kind < 4; kind++) {  // bit 0 wide, bit 1 pairs
                     std::vector<csim::TreeStageJob> st;
                     int64_t sb = 0;
                     int mmax = 0;
                     for (const Piece& p : ch.pieces) {
                         const csim::tree::Plan& pl = *p.g.plan;
-                        if (pl.level.size() <= d || (pl.vert[d - 1] > 32) != (wide != 0)) continue;
+                        if (pl.level.size() <= d || (pl.vert[d - 1] > 32) + 2 * pl.pairs != kind) continue;
                         csim::TreeStageJob j{};
                         j.in = (const uint32_t*)(scratch + p.off[(d - 1) & 1]);
                         j.out = (uint32_t*)(scratch + p.off[d & 1]);
@@ -175,15 +191,16 @@ class TreeRun {
                         j.mp = pl.vert[d - 1];
                         j.mc = pl.vert[d];
                         j.sub = pl.level[d - 1] - pl.level[d];
+                        j.paired = pl.pairs ? 2 * (pl.t / 2) : 0;
                         const int64_t threads = j.sub > 0 ? j.count / 2 : j.count;  // a pair of siblings each
                         sb += (threads + csim::kTreeStageThreads - 1) / csim::kTreeStageThreads;
                         mmax = std::max(mmax, j.mp);
                         st.push_back(j);
                     }
-                    if (!st.empty()) add(blob, Step{1, wide != 0, mmax, (int)st.size(), sb, 0}, st);
+                    if (!st.empty()) add(blob, Step{1, kind, mmax, (int)st.size(), sb, 0}, st);
                 }
-            for (int wc = 0; wc < 4; wc++)
-                if (!leaves[wc].empty()) add(blob, Step{2, false, 1 << wc, (int)leaves[wc].size(), lb[wc], 0}, leaves[wc]);
+            for (int wc = 0; wc < 16; wc++)
+                if (!leaves[wc].empty()) add(blob, Step{2, wc >> 2, 1 << (wc & 3), (int)leaves[wc].size(), lb[wc], 0}, leaves[wc]);
         }
     }
 
@@ -199,8 +216,10 @@ class TreeRun {
             const int rc =
                 s.kind == 0 && draw ? csim::launch_tree_draw(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, s.size, *draw)
                 : s.kind == 0 ? csim::launch_tree_root(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, states, code)
-                : s.kind == 1 ? csim::launch_tree_stage(L, (const csim::TreeStageJob*)j, s.njobs, s.blocks, s.wide, s.size)
-                              : csim::launch_tree_leaf(L, (const csim::TreeLeafJob*)j, s.njobs, s.blocks, s.size);
+                : s.kind == 1 ? csim::launch_tree_stage(L, (const csim::TreeStageJob*)j, s.njobs, s.blocks, s.flags & 1, s.size,
+                                                          s.flags & 2)
+                              : csim::launch_tree_leaf(L, (const csim::TreeLeafJob*)j, s.njobs, s.blocks, s.size,
+                                                         s.flags & 1, s.flags & 2);
             if (rc) return rc;
         }
         return 0;
@@ -217,7 +236,7 @@ class TreeRun {
     };
     struct Step {
         int kind;  // 0 roots, 1 a stage, 2 leaves
-        bool wide;
+        int flags;  // stages: bit 0 wide, bit 1 pairs; leaves: bit 0 rows, bit 1 pairs
         int size;  // roots: the first group's qubits; a stage's largest parent; the leaves' table words
         int njobs;
         int64_t blocks;
@@ -239,7 +258,8 @@ class TreeRun {
 // A plan's device image (kTreePlanBytes)
 inline void tree_plan_image(const csim::tree::Plan& p, unsigned char* out) {
     memcpy(out, p.gen, 64 * 8);
-    memcpy(out + 64 * 8, p.perm, 64);
+    memcpy(out + 64 * 8, p.term, 64 * 8);
+    memcpy(out + 2 * 64 * 8, p.perm, 64);
 }
 
 }  // namespace csim_host

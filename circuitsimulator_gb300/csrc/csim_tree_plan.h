@@ -15,6 +15,10 @@ struct Plan {
     int m[65] = {0};              // m[j]: vertices of a node of level j (m[r] = t)
     uint8_t perm[64] = {0};       // position -> coordinate; C_j lives on positions < m[j]
     uint64_t gen[64] = {0};       // gen[j]: generator of C_{j+1} over C_j, in positions
+    uint64_t term[64] = {0};      // gen[j]'s part of the term index (bits of j in codeword(j) = sum of L's rows);
+                                  // the index of a sum of generators is their sum's if r = k
+    uint64_t x0 = 0;              // a root's X
+    bool pairs = false;           // terms of |H^t>: products over vertex pairs (join_pairs) instead of codewords
     // levels of the written nodes, root (r) first; the last one is the leaf kernel's
     // entry.  vert: their vertices
     std::vector<int> level, vert;
@@ -28,36 +32,47 @@ struct Plan {
 inline void build_chain(const uint64_t* L, int k, int t, Plan& p) {
     p.t = t;
     p.k = k;
-    std::vector<uint64_t> rows(L, L + k);
+    struct Word {
+        uint64_t v, term;
+        void add(const Word& o) {
+            v ^= o.v;
+            term ^= o.term;
+        }
+    };
+    std::vector<Word> rows((size_t)k);
+    for (int r = 0; r < k; r++) rows[(size_t)r] = Word{L[r], 1ull << (k - 1 - r)};
     uint64_t supp = 0;
     uint64_t picked[64];
     p.r = 0;
     for (;;) {
         // a basis of the quotient code, reduced outside supp
-        std::vector<uint64_t> e;
-        for (uint64_t v : rows) {
-            for (uint64_t b : e) {
-                const int c = __builtin_ctzll(b & ~supp);
-                if ((v >> c) & 1) v ^= b;
+        std::vector<Word> e;
+        for (Word v : rows) {
+            for (const Word& b : e) {
+                const int c = __builtin_ctzll(b.v & ~supp);
+                if ((v.v >> c) & 1) v.add(b);
             }
-            if (!(v & ~supp)) continue;
-            const int c = __builtin_ctzll(v & ~supp);
-            for (uint64_t& b : e)
-                if ((b >> c) & 1) b ^= v;
+            if (!(v.v & ~supp)) continue;
+            const int c = __builtin_ctzll(v.v & ~supp);
+            for (Word& b : e)
+                if ((b.v >> c) & 1) b.add(v);
             e.push_back(v);
         }
         if (e.empty()) break;
         const int d = std::min((int)e.size(), 16);
-        uint64_t x = 0, best = e[0];
+        Word x{0, 0};
+        Word pick = e[0];
         int bw = 65;
         for (uint64_t i = 1; i < (1ull << d); i++) {
-            x ^= e[(size_t)__builtin_ctzll(i)];
-            const int w = __builtin_popcountll(x & ~supp);
+            x.add(e[(size_t)__builtin_ctzll(i)]);
+            const int w = __builtin_popcountll(x.v & ~supp);
             if (w < bw) {
                 bw = w;
-                best = x;
+                pick = x;
             }
         }
+        const uint64_t best = pick.v;
+        p.term[p.r] = pick.term;
         picked[p.r++] = best;
         const uint64_t add = best & ~supp;
         const int m0 = p.m[p.r - 1];
@@ -84,6 +99,32 @@ inline void build_chain(const uint64_t* L, int k, int t, Plan& p) {
     p.tv = p.tj > 0 ? p.m[p.tj] : std::min(t, 8);
 }
 
+// The terms of |H^t>: bit i of a term's index (LSB first) is the kind of the qubit
+// pair ceil(t/2) - 1 - i; with odd t bit 0 is the last qubit alone, |+> for 0 and |0>
+// for 1.  Pair i is at positions 2 i and 2 i + 1, the single qubit above them.
+inline void build_pairs(int t, Plan& p) {
+    p.t = t;
+    p.pairs = true;
+    const int n = t / 2, odd = t & 1;
+    p.k = p.r = n + odd;
+    for (int i = 0; i < n; i++) {
+        const int q = 2 * (n - 1 - i);
+        p.perm[2 * i] = (uint8_t)q;
+        p.perm[2 * i + 1] = (uint8_t)(q + 1);
+        p.gen[i] = 3ull << (2 * i);
+        p.term[i] = 1ull << (i + odd);
+        p.m[i] = 2 * i;
+    }
+    if (odd) {
+        p.perm[t - 1] = (uint8_t)(t - 1);
+        p.x0 = p.gen[n] = 1ull << (t - 1);  // codeword bit 1 is |+>, the term bit 0
+        p.term[n] = 1;
+        p.m[n] = 2 * n;
+    }
+    p.m[p.r] = t;
+    p.tj = p.tv = 0;
+}
+
 // Levels of the written nodes by dynamic programming on the time for `count`
 // states.  A stage from vp to vc vertices runs about 0.31 steps per vertex and
 // node (pairs of siblings share a lane), each a pass over the rows still live, and
@@ -108,7 +149,7 @@ inline void choose_levels(Plan& p, int64_t count) {
         lv.push_back(j);
         vt.push_back(p.m[j]);
     }
-    if (p.t > p.tv) {
+    if (p.t > p.tv && !p.pairs) {  // pairs: the leaf kernel takes the last ones
         lv.push_back(p.tj);
         vt.push_back(p.tv);
     }

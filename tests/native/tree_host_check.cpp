@@ -40,9 +40,19 @@ void take(HostNode& n, const Work<W>& w, const R& rows, int mc) {
     for (int i = 0; i < mc; i++) n.row[i] = (uint64_t)((W)rows.get(i) & cm);
 }
 
+// terms of |H^t> (paired > 0): the pairs among the positions [mc, mp) joined
+template <class W, class R>
+void join(const R& rows, Work<W>& w, const HostNode& n, int mp, int mc, int paired) {
+    const int hi = paired < mp ? paired : mp;
+    if (hi <= mc) return;
+    const W pm = wlow<W>(hi) & ~wlow<W>(mc);
+    w.sum &= ~pm;
+    w.live = wlow<W>(mc) | w.sum | pm;
+    join_pairs<W>(rows, w, (W)n.x, mc, hi, true);
+}
 // contracts positions [mc, mp) of two siblings with the row type that the
 // kernels use for mp vertices (`leaf`: the leaf kernel's 16-bit rows)
-void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf) {
+void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf, int paired) {
     alignas(16) uint32_t w[256] = {0};
     const HostNode* n[2] = {&a, &b};
     if (leaf) {
@@ -50,6 +60,8 @@ void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf) {
         for (int e = 0; e < 2; e++)
             for (int i = 0; i < mp; i++) reinterpret_cast<uint16_t*>(w + 8 * e)[i] = (uint16_t)n[e]->row[i];
         auto wa = work_of<uint32_t>(a, mp, mc), wb = work_of<uint32_t>(b, mp, mc);
+        join(r0, wa, a, mp, mc, paired);
+        join(r1, wb, b, mp, mc, paired);
         sum_out_pair<uint32_t>(r0, 8, wa, wb, ~0u);
         take(a, wa, r0, mc);
         take(b, wb, r1, mc);
@@ -61,6 +73,8 @@ void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf) {
                 w[128 * e + 64 + i] = (uint32_t)(n[e]->row[i] >> 32);
             }
         auto wa = work_of<uint64_t>(a, mp, mc), wb = work_of<uint64_t>(b, mp, mc);
+        join(r0, wa, a, mp, mc, paired);
+        join(r1, wb, b, mp, mc, paired);
         contract_pair(r0, 128, wa, wb, mc);
         take(a, wa, r0, mc);
         take(b, wb, r1, mc);
@@ -69,6 +83,8 @@ void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf) {
         for (int e = 0; e < 2; e++)
             for (int i = 0; i < mp; i++) w[32 * e + i] = (uint32_t)n[e]->row[i];
         auto wa = work_of<uint32_t>(a, mp, mc), wb = work_of<uint32_t>(b, mp, mc);
+        join(r0, wa, a, mp, mc, paired);
+        join(r1, wb, b, mp, mc, paired);
         contract_pair(r0, 32, wa, wb, mc);
         take(a, wa, r0, mc);
         take(b, wb, r1, mc);
@@ -97,18 +113,24 @@ HostNode root_of(const csim_state& th, const Plan& p) {
     n.d1 = cs.D1;
     n.d2 = cs.D2 | (cs.bm & n.h);
     n.q = cs.Q;
+    n.x = p.x0;
     return n;
 }
 
 }  // namespace
 
-// Sums of all 2^k terms for each theta, as the kernels' exact coordinates
+// Sums of all terms (2^k of code L; of |H^t> if L is null) for each theta, as the kernels' exact coordinates
 // scaled by 2^t: out[8 a + 2 q] low and out[8 a + 2 q + 1] high word of
 // coordinate q.  info (optional): r, table vertices, written levels.
 extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_t* L, int k, int t, int64_t count,
                               uint64_t* out, int* info) {
     Plan p;
-    make_plan(L, k, t, count, p);  // the levels for `count` states
+    if (L) make_plan(L, k, t, count, p);  // the levels for `count` states
+    else {
+        build_pairs(t, p);
+        choose_levels(p, count);
+    }
+    const int paired = p.pairs ? 2 * (t / 2) : 0;
     if (info) {
         info[0] = p.r;
         info[1] = p.tv;
@@ -133,7 +155,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
                         if ((c >> b) & 1) n.x ^= p.gen[p.level[s] + b];
                     HostNode o = n;
                     if (sb) o.x ^= p.gen[p.level[s]];
-                    if (!par.dead) stage(n, o, p.vert[s - 1], p.vert[s], false);
+                    if (!par.dead) stage(n, o, p.vert[s - 1], p.vert[s], false, paired);
                     next.push_back(n);
                     if (sb) next.push_back(o);
                 }
@@ -150,7 +172,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
                 n.x = x;
                 n.iso = 0;
                 HostNode o = n;
-                if (m > p.tv) stage(n, o, m, p.tv, true);
+                if (m > p.tv) stage(n, o, m, p.tv, true, paired);
                 uint32_t r[kTableVars] = {0};
                 for (int i = 0; i < kTableVars && i < m; i++) r[i] = (uint32_t)n.row[i];
                 const uint32_t vm = wlow<uint32_t>(p.tv), d1 = (uint32_t)n.d1 & vm;
@@ -180,7 +202,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
         const int shift = t - p.tv;
         if (shift & 1) times_sqrt2(z);
         for (int q = 0; q < 4; q++) {
-            const unsigned __int128 w = (unsigned __int128)z[q] << ((shift >> 1) + (k - p.r));
+            const unsigned __int128 w = (unsigned __int128)z[q] << ((shift >> 1) + (p.k - p.r));
             out[8 * a + 2 * q] = (uint64_t)w;
             out[8 * a + 2 * q + 1] = (uint64_t)(w >> 64);
         }

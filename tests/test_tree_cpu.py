@@ -27,10 +27,12 @@ def tree_sums():
 
     def run(thetas, L, t, count):
         thetas = np.ascontiguousarray(thetas)
-        Lw = np.array([int(x) for x in L] or [0], dtype=np.uint64)
+        k = 0 if L is None else len(L)
+        Lw = None if L is None else np.array([int(x) for x in L] or [0], dtype=np.uint64)
         out = np.zeros((len(thetas), 4, 2), dtype=np.uint64)
         info = np.zeros(80, dtype=np.int32)
-        assert lib.tree_host_sums(thetas.ctypes.data, len(thetas), Lw.ctypes.data, len(L), t, count, out.ctypes.data,
+        assert lib.tree_host_sums(thetas.ctypes.data, len(thetas), None if L is None else Lw.ctypes.data, k, t, count,
+                                  out.ctypes.data,
                                   info.ctypes.data) == 0
         vals = [[(int(w[0]) | (int(w[1]) << 64)) - ((1 << 128) if int(w[1]) >> 63 else 0) for w in row] for row in out]
         return vals, info
@@ -69,12 +71,13 @@ def _thetas(oracle, rs, t, rows, count):
 
 
 def _check(tree_sums, oracle, t, L, thetas):
-    k = len(L)
+    k = 0 if L is None else len(L)
     got, info = tree_sums(thetas, L, t, 4096)
     assert tree_sums(thetas, L, t, 1)[0] == got  # fewer levels for a single state
-    Lw = np.array([int(x) for x in L] or [0], dtype=np.uint64)
+    Lw = np.array([int(x) for x in L or [0]] or [0], dtype=np.uint64)
+    chi = 2 ** ((t + 1) // 2) if L is None else 2 ** k
     for a in range(len(thetas)):
-        e, p, m = oracle.term_products(t, 0, Lw, k, thetas[a:a + 1], 0, 2 ** k, threads=4)
+        e, p, m = oracle.term_products(t, int(L is None), Lw, k, thetas[a:a + 1], 0, chi, threads=4)
         assert got[a] == _exact_sum(e, p, m, 2 * t), (t, k, a)
     return info
 
@@ -90,6 +93,35 @@ def test_tree_sum_equals_oracle(tree_sums, oracle, t, k, frac):
     thetas = _thetas(oracle, rs, t, rows, 3)
     assert len(thetas)
     _check(tree_sums, oracle, t, L, thetas)
+
+
+@pytest.mark.parametrize("t", [1, 2, 3, 4, 7, 8, 12, 15, 16, 17, 18, 21])
+@pytest.mark.parametrize("frac", [0.0, 0.5])
+def test_tree_sum_of_magic_state_terms(tree_sums, oracle, t, frac):
+    """Terms of |H^t>, products of two-qubit states (a single qubit left over for odd t)."""
+    rs = np.random.RandomState(t)
+    thetas = _thetas(oracle, rs, t, random_projector_rows(rs, t, int(frac * t)), 6)
+    _check(tree_sums, oracle, t, None, thetas)
+
+
+@pytest.mark.parametrize("t", [36])
+def test_tree_sum_of_many_pairs(tree_sums, oracle, t):
+    """Wide rows: 2^18 terms of |H^36> sum to <theta|H^36> for theta a product state,
+    known in closed form: theta = |0>^36 meets the first kind in 1/2 and the second
+    in 1/sqrt2 per pair, |+>^36 both kinds in 1/2 and 1/sqrt2 as well."""
+    s = oracle.state(t)
+    for plus in (True, False):
+        st = s.copy()
+        if not plus:
+            for q in range(t):
+                oracle.shrink(st, 1 << q, 0)
+        got, _ = tree_sums(st, None, t, 1)
+        # <0|a> = 1/2, <0|b> = 1/sqrt2 and <++|a> = 1/2, <++|b> = 1/sqrt2: (1/2 + 1/sqrt2)^18, scaled by 2^36
+        z = [1, 0, 0, 0]
+        for _ in range(t // 2):  # times 4 (1/2 + 1/sqrt2) = 2 + 2 sqrt2, sqrt2 = w - w^3
+            r = [z[1] - z[3], z[0] + z[2], z[1] + z[3], z[2] - z[0]]
+            z = [2 * a + 2 * b for a, b in zip(z, r)]
+        assert got[0] == z
 
 
 @pytest.mark.parametrize("t", [6, 16, 20, 33, 64])

@@ -61,3 +61,43 @@ def test_tree_sampler_in_chunks(gpu):
     b = _values(gpu, 0, P, L[:4], False, 17000, backend.RNG_PHILOX, 5)
     assert (a == _values(gpu, 5, P, L, False, 2100, backend.RNG_LIBC, 5)).all()
     assert (b == _values(gpu, 5, P, L[:4], False, 17000, backend.RNG_PHILOX, 5)).all()
+
+
+@pytest.mark.parametrize("t,count", [(1, 40), (2, 33), (3, 64), (8, 70), (9, 300), (15, 40), (16, 129), (17, 20), (24, 5)])
+def test_tree_sampler_of_magic_state_terms(gpu, t, count):
+    rs = np.random.RandomState(40 + t)
+    rows = random_projector_rows(rs, t, max(1, t // 3))
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    for rng in (backend.RNG_PHILOX, backend.RNG_LIBC):
+        a = _values(gpu, 0, P, None, True, count, rng, 12)
+        assert (a == _values(gpu, 1, P, None, True, count, rng, 12)).all()
+
+
+@pytest.mark.parametrize("t,k,kind", [(1, -1, ""), (2, -1, ""), (3, -1, ""), (8, -1, ""), (13, -1, ""), (16, -1, ""),
+                                      (1, 1, "random"), (6, 4, "random"), (9, 9, "random"), (17, 6, "random"),
+                                      (21, 8, "random"), (33, 7, "random"), (40, 9, "low"), (64, 5, "random"),
+                                      (20, 6, "repeated"), (12, 0, "random")])
+def test_tree_rows_equal_pair_kernel(gpu, t, k, kind):
+    """exactProjector's rows (one term per row left out of the sum, the diagonal apart),
+    whole and in ranges."""
+    rs = np.random.RandomState(t + 50 * (k + 1))
+    L = None if k < 0 else _code(kind, t, k, rs)
+    chi = 1 << ((t + 1) // 2 if k < 0 else k)
+    rows = random_projector_rows(rs, t, max(1, t // 2))
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    out = []
+    for kernel in (0, 1):
+        try:
+            gpu.set_option(backend.OPT_PAIR_KERNEL, kernel)
+            re, im = gpu.exactProjectorRows(P, L, k < 0, 0, chi)
+            cut = chi // 3
+            parts = [gpu.exactProjectorRows(P, L, k < 0, a, b) for a, b in ((0, cut), (cut, chi))]
+            st = gpu.last_stats()
+            out.append((re, im, gpu.exactProjector(P, L, k < 0, 1.0), st.pairs, st.states_live))
+        finally:
+            gpu.set_option(backend.OPT_PAIR_KERNEL, 0)
+        assert (np.concatenate([p[0] for p in parts]) == re).all()
+        assert (np.concatenate([p[1] for p in parts]) == im).all()
+    (re0, im0, v0, n0, l0), (re1, im1, v1, n1, l1) = out
+    assert (re0 == re1).all() and (im0 == im1).all() and v0 == v1
+    assert (n0, l0) == (n1, l1)
