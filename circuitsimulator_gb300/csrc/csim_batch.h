@@ -56,9 +56,16 @@ int launch_items_direct(const Launch& L, const PairItem* items, int64_t nitems, 
                         __int128* part, __int128* part_diag, unsigned long long* queue);
 int launch_items_warp(const Launch& L, const PairItem* items, int64_t nitems, const GState* states, const int* codes,
                       __int128* part, __int128* part_diag);
-// per-slot sums of item partials; slot s owns items [range[2s], range[2s+1]) and,
-// if range2 is not null, [range2[2s], range2[2s+1])
-int launch_reduce_slots(const Launch& L, const __int128* part, const int64_t* range, const int64_t* range2,
-                        int64_t nslots, __int128* out);
+// Values of a round's slots.  Segment: slots slot0 .. (up to the next segment's) of one
+// evaluation on t qubits; with parts > 0 slot i sums partial sums part0 + parts (i - slot0) ..
+// and takes diagonal diag0 + (i - slot0), else it sums items [range[2i], range[2i+1]) and
+// [range2[2i], range2[2i+1]) and the diagonals of [ranged[2i], ranged[2i+1]).
+struct ValueSeg {
+    int64_t slot0, part0, parts, diag0;
+    int32_t t, row;  // row: exactProjector row (out: re, im), else a sample (out: value, 0)
+};
+int launch_seg_values(const Launch& L, const ValueSeg* segs, int nsegs, int64_t nslots, const __int128* part,
+                      const __int128* partd, const int64_t* range, const int64_t* range2, const int64_t* ranged,
+                      const int* code, const double* factor, double* out);
 
 }  // namespace csim

@@ -10,7 +10,7 @@
 //   k_items_direct  the same items by direct restriction of each state's
 //                   pivot form (launch_canon), one thread per pair
 //   k_items_warp    the warp-per-pair kernel over (state, range of term states)
-//   k_reduce_slots  per-slot sums of the items' partial sums
+//   k_seg_values    the slots' values from the items' and the trees' partial sums
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -20,6 +20,7 @@
 #include "csim_block_prefix.cuh"
 #include "csim_pair_core.cuh"
 #include "csim_rng.cuh"
+#include "csim_values.cuh"
 #include "csim_warp.cuh"
 
 namespace csim {
@@ -342,17 +343,47 @@ __global__ void __launch_bounds__(256) k_items_warp(const PairItem* items, int64
     flush(e, err);
 }
 
-// slot s sums the items [range[2s], range[2s+1]) and [range2[2s], range2[2s+1])
-__global__ void k_reduce_slots(const __int128* part, const int64_t* range, const int64_t* range2, int64_t nslots,
-                               __int128* out) {
-    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nslots * 4;
-         w += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s = w / 4, q = w % 4;
-        __int128 acc = 0;
-        for (int64_t i = range[2 * s]; i < range[2 * s + 1]; i++) acc += part[4 * i + q];
-        if (range2)
-            for (int64_t i = range2[2 * s]; i < range2[2 * s + 1]; i++) acc += part[4 * i + q];
-        out[w] = acc;
+// one warp per slot: the sum of its partial sums, as its value (csim_values.cuh)
+__global__ void __launch_bounds__(128) k_seg_values(const ValueSeg* segs, int nsegs, int64_t nslots, const __int128* part,
+                                                    const __int128* partd, const int64_t* range, const int64_t* range2,
+                                                    const int64_t* ranged, const int* code, const double* factor,
+                                                    double* out) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (i >= nslots) return;  // warp-uniform
+    int lo = 0, hi = nsegs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (segs[mid].slot0 <= i) lo = mid;
+        else hi = mid - 1;
+    }
+    const ValueSeg& s = segs[lo];
+    const int lane = lane_id(), q = lane & 3, c = code[i];
+    __int128 z = 0, d = 0;
+    auto add = [&](__int128& acc, const __int128* from, int64_t b, int64_t e) {
+        for (int64_t p = b + (lane >> 2); p < e; p += 8) acc += from[4 * p + q];
+    };
+    if (c >= 0) {
+        if (s.parts > 0) {
+            const int64_t b = s.part0 + s.parts * (i - s.slot0);
+            add(z, part, b, b + s.parts);
+            if (s.row) add(d, partd, s.diag0 + (i - s.slot0), s.diag0 + (i - s.slot0) + 1);
+        } else {
+            add(z, part, range[2 * i], range[2 * i + 1]);
+            add(z, part, range2[2 * i], range2[2 * i + 1]);
+            if (s.row) add(d, partd, ranged[2 * i], ranged[2 * i + 1]);
+        }
+    }
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+        z += shfl_xor_i128(z, o);
+        d += shfl_xor_i128(d, o);
+    }
+    double a, b;
+    warp_value(z, s.row != 0, d, s.t, factor[c >= 0 ? c : 0], a, b);
+    if (lane == 0) {
+        const bool live = c >= 0;
+        out[2 * i] = !live ? 0.0 : (s.row ? a : sample_value(a, b, s.t));
+        out[2 * i + 1] = live && s.row ? b : 0.0;
     }
 }
 
@@ -444,12 +475,12 @@ int launch_items_warp(const Launch& L, const PairItem* items, int64_t nitems, co
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_reduce_slots(const Launch& L, const __int128* part, const int64_t* range, const int64_t* range2,
-                        int64_t nslots, __int128* out) {
+int launch_seg_values(const Launch& L, const ValueSeg* segs, int nsegs, int64_t nslots, const __int128* part,
+                      const __int128* partd, const int64_t* range, const int64_t* range2, const int64_t* ranged,
+                      const int* code, const double* factor, double* out) {
     if (nslots <= 0) return 0;
-    int64_t blocks = (nslots * 4 + 255) / 256;
-    if (blocks > (int64_t)L.num_sms * 16) blocks = (int64_t)L.num_sms * 16;
-    k_reduce_slots<<<(int)blocks, 256, 0, L.stream>>>(part, range, range2, nslots, out);
+    k_seg_values<<<(unsigned)((nslots + 3) / 4), 128, 0, L.stream>>>(segs, nsegs, nslots, part, partd, range, range2,
+                                                                     ranged, code, factor, out);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

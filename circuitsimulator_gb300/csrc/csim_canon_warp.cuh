@@ -1,6 +1,6 @@
 // csim_canon_warp.cuh — a stabilizer state in pivot coordinates by one warp:
 // pc::canon_theta's steps with lane l holding variables l and l + 32 (rows of G
-// and J).  Shared by k_canon (csim_terms_tp.cu) and k_tree_root (csim_tree.cu).
+// and J).  Shared by k_canon (csim_terms_tp.cu) and k_tree_draw (csim_tree.cu).
 #pragma once
 
 #include <cstdint>

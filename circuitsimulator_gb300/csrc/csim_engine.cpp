@@ -8,14 +8,15 @@
 // Work is cut into rounds.  A round takes the next states of the admitted
 // evaluations (one evaluation = one projector of one query), up to a budget
 // of inner products, and runs:
+//   k_tree_*        states drawn, projected and summed over all terms as trees of
+//                   shared contractions
+//   k_seg_values    the states' values from their exact Z[w] sums
+// or, where a pair kernel is asked for, and for rows of a code with dependent rows,
 //   k_draw_project  draw or copy every state, then project it (innerprod.c:97-116)
 //   k_canon         the states of direct-restriction evaluations in pivot form
 //   k_items_tp      (state, |L> term range) items, thread per pair
 //   k_items_direct  the same items by direct restriction, thread per pair
 //   k_items_warp    (state, prepH term range) items, warp per pair
-//   k_tree_*        sampled terms of |L> as trees of shared contractions, one group
-//                   of states per decomposition
-//   k_reduce_slots  exact Z[w] sums per state
 // Two round buffers alternate.  The host builds round r+1 and queues it behind
 // round r, then reads round r's results.
 //
@@ -121,7 +122,7 @@ struct Decomp {
     int kern = 0;                // the tuner's kernel: 3 = direct restriction, else the block-prefix kernel
     csim_state* phis = nullptr;  // term states: prepH (exact == 1), prepL (exact projector on |L>)
     uint64_t* dL = nullptr;
-    csim::tree::Plan plan;             // the tree sum's chain of subcodes (exact == 0, sampled estimators)
+    csim::tree::Plan plan;             // the tree sum's order of contractions
     unsigned char* dplan = nullptr;    // and its device arrays
     size_t bytes = 0;
     int refs = 0;
@@ -148,7 +149,7 @@ struct Eval {
     int which = 0;  // 0 G', 1 H'
     int kind = 1;   // 1 sampled (multiSampledProjector), 2 exactProjector
     int t = 0;
-    bool tree = false;  // summed by the tree kernels (sampled, terms of |L>)
+    bool tree = false;  // summed by the tree kernels
     int64_t chi = 0, ns = 0;
     int samples = 0, bins = 1;
     int64_t next = 0, done = 0;
@@ -183,9 +184,10 @@ struct QueryRec {
     Clock::time_point t_submit;
 };
 
-struct Slot {
+// consecutive states s0 .. s0 + n - 1 of an evaluation in a round, in slots slot0 ..
+struct Seg {
     Eval* e;
-    int64_t s;
+    int64_t s0, n, slot0;
 };
 
 // one round's buffers and contents
@@ -193,9 +195,9 @@ struct RoundSet {
     DevBuf up, work, down;
     HostBuf hup, hdown;
     cudaEvent_t ev[4] = {};  // start, pair kernels start, pair kernels end, end
-    std::vector<Slot> slots;
+    std::vector<Seg> segs;
     int64_t pairs = 0;
-    size_t off_codes = 0, off_sum = 0, off_sumd = 0;
+    size_t off_codes = 0, off_val = 0;
 };
 
 }  // namespace
@@ -234,8 +236,10 @@ class Engine {
         for (auto& rs : sets_)
             for (auto& e : rs.ev)
                 if (cudaEventCreate(&e) != cudaSuccess) return fail(ctx_, CSIM_ERR_CUDA, "event create failed");
-        // randomStabilizerState's cumulative tables for every n (stabilizer.c:694-716)
+        // the projection factors (row 0), randomStabilizerState's cumulative tables for every n
+        // (stabilizer.c:694-716)
         std::vector<double> cum(65 * 65, 0.0);
+        for (int c = 0; c <= CSIM_MAX_QUBITS; c++) cum[c] = sqrt_half_power(c);
         for (int t = 1; t <= CSIM_MAX_QUBITS; t++) cum_table(t, &cum[65 * t]);
         if (cum_.ensure(cum.size() * 8)) return fail(ctx_, CSIM_ERR_NOMEM, "cum table");
         CK(cudaMemcpy(cum_.p, cum.data(), cum.size() * 8, cudaMemcpyHostToDevice));
@@ -297,7 +301,7 @@ class Engine {
     int nbuckets_ = 0;
 
     csim::Launch launch_on(int* d_err) { return csim::Launch{ctx_->stream, d_err, &ctx_->launches, ctx_->num_sms}; }
-    int ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp** out);
+    int ensure_decomp(QueryRec* r, bool rows, bool* tree, bool force, Decomp** out);
     void finish_eval(Eval* e);
     void finish_query(QueryRec* r);
     void fail_query(QueryRec* r, int status);
@@ -368,9 +372,10 @@ static bool plan_query(csim_ctx* ctx, QueryRec* r) {
     return true;
 }
 
-// rows: the exactProjector's evaluations (term order, term states); otherwise the
-// sampled estimators', as a tree or with a pair kernel
-int Engine::ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp** out) {
+// rows: for the exactProjector's evaluations; otherwise for the sampled estimators'.
+// *tree: whether they may be summed as a tree, on return whether they are; otherwise
+// the pair kernels' tables and term states are made.
+int Engine::ensure_decomp(QueryRec* r, bool rows, bool* tree, bool force, Decomp** out) {
     csim_ctx* const ctx = ctx_;  // for CK
     *out = nullptr;
     std::vector<uint64_t> key = {(uint64_t)r->q.t, (uint64_t)r->exact, (uint64_t)(r->exact ? 0 : r->k)};
@@ -378,11 +383,18 @@ int Engine::ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp*
     auto it = decomps_.find(key);
     Decomp* d = it == decomps_.end() ? nullptr : it->second.get();
     const int64_t chi = r->chi;
-    const bool want_cw = !r->exact && rows, want_cws = !r->exact && !rows && !tree, want_plan = !r->exact && tree,
-               want_phis = r->exact || rows;
+    csim::tree::Plan plan;
+    if (*tree && !(d && d->dplan)) {
+        if (r->exact) csim::tree::build_pairs(r->q.t, plan);
+        else csim::tree::build_chain(r->L, r->k, r->q.t, plan);
+    }
+    if (*tree && rows) *tree = tree_rows_ok(d && d->dplan ? d->plan : plan);
+    const bool want_plan = *tree, want_cw = !r->exact && rows && !*tree, want_cws = !r->exact && !rows && !*tree,
+               want_phis = (r->exact || rows) && !*tree, want_dL = want_cw || (!r->exact && rows);
     const size_t table = align_up((size_t)chi * 8);
     size_t add = 0;
-    if (want_cw && !(d && d->cw)) add += table + kAlign;
+    if (want_cw && !(d && d->cw)) add += table;
+    if (want_dL && !(d && d->dL)) add += align_up(8 * CSIM_MAX_QUBITS);
     if (want_cws && !(d && d->cws)) add += table;
     if (want_plan && !(d && d->dplan)) add += align_up(kTreePlanBytes);
     if (want_phis && !(d && d->phis)) add += align_up((size_t)chi * sizeof(csim_state));
@@ -422,7 +434,7 @@ int Engine::ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp*
         return 0;
     };
     if (want_plan && !d->dplan) {
-        csim::tree::build_chain(d->L.data(), d->k, d->t, d->plan);
+        d->plan = plan;
         unsigned char image[kTreePlanBytes];
         tree_plan_image(d->plan, image);
         CKR(grow((void**)&d->dplan, kTreePlanBytes));
@@ -444,11 +456,13 @@ int Engine::ensure_decomp(QueryRec* r, bool rows, bool tree, bool force, Decomp*
         CKR(grow((void**)&d->cws, (size_t)chi * 8));
         CK(cudaMemcpy(d->cws, ordered.data(), (size_t)chi * 8, cudaMemcpyHostToDevice));
     }
-    if (want_cw && !d->cw) {
+    if (want_dL && !d->dL) {
         uint64_t code_rows[CSIM_MAX_QUBITS] = {0};
         for (int i = 0; i < d->k; i++) code_rows[i] = d->L[i];
-        if (!d->dL) CKR(grow((void**)&d->dL, sizeof(code_rows)));
-        CK(cudaMemcpy(d->dL, code_rows, sizeof(code_rows), cudaMemcpyHostToDevice));
+        CKR(grow((void**)&d->dL, sizeof(code_rows)));
+        CK(cudaMemcpyAsync(d->dL, code_rows, sizeof(code_rows), cudaMemcpyHostToDevice, ctx_->stream));
+    }
+    if (want_cw && !d->cw) {
         CKR(grow((void**)&d->cw, (size_t)chi * 8));
         if (csim::launch_codewords(launch_of(ctx_), d->dL, d->k, 0, chi, d->cw))
             return fail(ctx_, CSIM_ERR_CUDA, "codeword launch failed");
@@ -488,9 +502,8 @@ int Engine::admit(QueryRec* r, bool force, bool* admitted) {
         return 0;
     }
     Decomp* d = nullptr;
-    // sampled terms of |L>: the tree sum, unless a pair kernel is asked for
-    const bool tree = !r->exact && !r->noapprox && ctx_->pair_kernel == 0 && r->k <= kTreeMaxRows;
-    const int rc = ensure_decomp(r, r->noapprox != 0, tree, force, &d);
+    bool tree = use_tree(ctx_, r->q.t, r->exact, r->k);
+    const int rc = ensure_decomp(r, r->noapprox != 0, &tree, force, &d);
     if (rc) {
         fail_query(r, rc);
         *admitted = true;
@@ -567,65 +580,88 @@ bool Engine::schedulable() const {
     return false;
 }
 
+// One round: the next states of every admitted evaluation, as segments (runs of
+// consecutive states of one evaluation).  Evaluations summed as trees are grouped by
+// decomposition for the choice of levels and share the tree launches; their states
+// never leave the GPU's registers.  The others (a pair kernel was asked for, or a
+// code whose rows are dependent) go through state descriptors and item tables.
 int Engine::launch_round() {
     csim_ctx* const ctx = ctx_;  // for CK
     RoundSet& rs = sets_[next_set_];
     next_set_ ^= 1;
-    rs.slots.clear();
+    rs.segs.clear();
     rs.pairs = 0;
     // pick states: a fair share per evaluation first, then first come first served
     int nready = 0;
     for (Eval* e : active_) nready += eval_ready(e) ? 1 : 0;
     const int64_t share = std::max<int64_t>(1, round_pairs_ / std::max(1, nready));
-    auto cost = [](const Eval* e) { return e->kind == 1 ? e->chi : e->chi - e->next; };
+    int64_t ns = 0;
     for (int pass = 0; pass < 2; pass++) {
         for (Eval* e : active_) {
-            int64_t mine = 0;
-            while (eval_ready(e) && (int64_t)rs.slots.size() < round_states_) {
-                const int64_t c = cost(e);
-                if (!rs.slots.empty() && rs.pairs + c > round_pairs_) break;
-                if (pass == 0 && mine > 0 && mine + c > share) break;
-                rs.slots.push_back(Slot{e, e->next});
-                e->q->inflight++;
-                e->next++;
-                rs.pairs += c;
-                mine += c;
-            }
+            if (!eval_ready(e) || ns >= round_states_) continue;
+            int64_t n = (round_pairs_ - rs.pairs) / e->chi;
+            if (pass == 0) n = std::min(n, std::max<int64_t>(1, share / e->chi));
+            if (ns == 0) n = std::max<int64_t>(n, 1);
+            n = std::min({n, e->ns - e->next, round_states_ - ns});
+            if (n <= 0) continue;
+            rs.segs.push_back(Seg{e, e->next, n, 0});
+            e->q->inflight += n;
+            e->next += n;
+            rs.pairs += n * e->chi;
+            ns += n;
         }
     }
-    const int64_t ns = (int64_t)rs.slots.size();
     if (ns == 0) return 0;
+    // slots: the states of the other evaluations first, then the trees'
+    std::stable_sort(rs.segs.begin(), rs.segs.end(),
+                     [](const Seg& a, const Seg& b) { return !a.e->tree && b.e->tree; });
+    int64_t nother = 0;
+    {
+        int64_t at = 0;
+        for (Seg& sg : rs.segs) {
+            sg.slot0 = at;
+            at += sg.n;
+            if (!sg.e->tree) nother = at;
+        }
+    }
+    const size_t nseg = rs.segs.size();
 
-    // rand() words of the sampled states with the C library's draws, each query's states in its own
+    // words of the sampled states with the C library's draws, each query's states in its own
     // stream order (G' then H'); queries are independent streams, so they are drawn on host threads
     // of their own (at t = 64 a state takes about 2000 words)
-    std::vector<std::pair<int64_t, int64_t>> wr(ns, {0, 0});
     struct WordJob {
         QueryRec* q;
         int t;
-        std::vector<int64_t> slots;
+        std::vector<size_t> segs;
+        int64_t states;
         std::vector<uint32_t> words;  // raw words, history first
         size_t nwords;                // without the history
         std::vector<int64_t> ends;
+        int64_t base;                 // its first word in the round's
     };
     std::vector<WordJob> jobs;
+    std::vector<std::pair<size_t, int64_t>> job_of(nseg);  // segment -> its job and first state in it
     {
         std::map<QueryRec*, size_t> jix;
-        for (int64_t i = 0; i < ns; i++) {
-            Eval* e = rs.slots[i].e;
+        for (size_t i = 0; i < nseg; i++) {
+            const Seg& sg = rs.segs[i];
+            Eval* e = sg.e;
             if (e->kind != 1 || e->q->q.rng != CSIM_RNG_LIBC) continue;
             auto it = jix.find(e->q);
             if (it == jix.end()) {
                 it = jix.emplace(e->q, jobs.size()).first;
-                jobs.push_back(WordJob{e->q, e->t, {}, {}, 0, {}});
+                jobs.push_back(WordJob{e->q, e->t, {}, 0, {}, 0, {}, 0});
             }
-            jobs[it->second].slots.push_back(i);
+            WordJob& j = jobs[it->second];
+            job_of[i] = {it->second, j.states};
+            j.segs.push_back(i);
+            j.states += sg.n;
         }
         auto run_job = [](WordJob& j) {
             double cum[CSIM_MAX_QUBITS + 1];
             cum_table(j.t, cum);
-            j.ends.reserve(j.slots.size());
-            j.words.resize(kRawHistory + j.slots.size() * state_words(j.t));
+            j.ends.reserve((size_t)j.states);
+            j.words.resize(kRawHistory + (size_t)j.states * state_words(j.t));
             RawWords w{j.words.data(), kRawHistory, j.words.size()};
             j.q->lr.history(w.p);
             auto grow = [&](size_t more) {
@@ -634,7 +670,7 @@ int Engine::launch_round() {
                 w.cap = j.words.size();
                 return true;
             };
-            for (size_t k = 0; k < j.slots.size(); k++) {
+            for (int64_t k = 0; k < j.states; k++) {
                 draw_state_words(w, j.t, cum, grow);
                 j.ends.push_back((int64_t)(w.n - kRawHistory));
             }
@@ -654,13 +690,14 @@ int Engine::launch_round() {
             for (auto& th : pool) th.join();
         }
     }
-    int64_t nwords = 0;
+    int64_t nwords = 0, noffs = 0;
     for (auto& j : jobs) {
-        for (size_t k = 0; k < j.slots.size(); k++)
-            wr[j.slots[k]] = {nwords + (k ? j.ends[k - 1] : 0), nwords + j.ends[k]};
+        j.base = nwords;
         nwords += (int64_t)j.nwords;
+        noffs += j.states + (int64_t)j.segs.size();
     }
     std::map<Eval*, int> evix;  // evaluations in this round -> projector block
+    for (const Seg& sg : rs.segs) evix.emplace(sg.e, (int)evix.size());
     // thread-per-pair items are grouped by t bucket: each bucket's launch sizes
     // its shared memory for that bucket's largest t, not the round's
     int64_t nbucket[kBuckets] = {0};
@@ -669,37 +706,31 @@ int Engine::launch_round() {
     // a launch runs as many rows per thread as its longest items need
     auto span_tp_of = [this](const Eval* e) { return 64 * (int64_t)(per_thread_ > 0 ? per_thread_ : e->q->dec->pt); };
     const int launch_pt = per_thread_ > 0 ? per_thread_ : 32;  // the largest item any t is tuned to
-    std::map<Decomp*, std::vector<int32_t>> tree_slots;  // slots of the tree sums, by decomposition
     int lzmax[kBuckets] = {0};  // per light launch: the largest light bound of its items
     const int64_t span_w = 64;
-    for (int64_t i = 0; i < ns; i++) {
-        Eval* e = rs.slots[i].e;
-        if (!evix.count(e)) {
-            const int ix = (int)evix.size();
-            evix[e] = ix;
-        }
-        if (e->tree) {
-            tree_slots[e->q->dec].push_back((int32_t)i);
-            continue;
-        }
-        const int64_t jb = e->kind == 2 ? rs.slots[i].s : 0;
-        const int64_t nj = e->chi - jb;
-        if (!e->q->exact) {
-            const int b = 4 * bucket_of_[e->t];
-            const int64_t span_tp = span_tp_of(e);
-            const int64_t nall = (nj + span_tp - 1) / span_tp;
-            if (e->q->dec->kern == 3) {
-                const int64_t nn = direct_narrow_items(e, span_tp);
-                nbucket[b + 2] += nn;
-                nbucket[b + 3] += nall - nn;
-                continue;
+    for (const Seg& sg : rs.segs) {
+        Eval* e = sg.e;
+        if (e->tree) continue;
+        for (int64_t i = 0; i < sg.n; i++) {
+            const int64_t jb = e->kind == 2 ? sg.s0 + i : 0;
+            const int64_t nj = e->chi - jb;
+            if (!e->q->exact) {
+                const int b = 4 * bucket_of_[e->t];
+                const int64_t span_tp = span_tp_of(e);
+                const int64_t nall = (nj + span_tp - 1) / span_tp;
+                if (e->q->dec->kern == 3) {
+                    const int64_t nn = direct_narrow_items(e, span_tp);
+                    nbucket[b + 2] += nn;
+                    nbucket[b + 3] += nall - nn;
+                    continue;
+                }
+                const int64_t nlight = e->kind == 1 ? nall - light_first_item(e, span_tp) : 0;
+                nbucket[b] += nall - nlight;
+                nbucket[b + 1] += nlight;
+                if (nlight) lzmax[b + 1] = std::max(lzmax[b + 1], e->q->dec->lz);
+            } else {
+                niw += (nj + span_w - 1) / span_w;
             }
-            const int64_t nlight = e->kind == 1 ? nall - light_first_item(e, span_tp) : 0;
-            nbucket[b] += nall - nlight;
-            nbucket[b + 1] += nlight;
-            if (nlight) lzmax[b + 1] = std::max(lzmax[b + 1], e->q->dec->lz);
-        } else {
-            niw += (nj + span_w - 1) / span_w;
         }
     }
     int64_t bstart[kBuckets + 1];
@@ -707,54 +738,67 @@ int Engine::launch_round() {
     for (int b = 0; b < kBuckets; b++) bstart[b + 1] = bstart[b] + nbucket[b];
     const int64_t nitp = bstart[kBuckets];
     const int64_t nitems = nitp + niw;
-    // tree sums: a group of states per decomposition, its partial sums behind the items'
+    // tree sums: levels by a decomposition's states in the round, a group of launches' jobs per
+    // segment; partial sums and diagonals behind the items'
+    std::map<Decomp*, int64_t> dec_states;
+    for (const Seg& sg : rs.segs)
+        if (sg.e->tree) dec_states[sg.e->q->dec] += sg.n;
+    for (auto& kv : dec_states) csim::tree::choose_levels(kv.first->plan, kv.second);
     std::vector<TreeGroup> groups;
-    std::vector<int64_t> group_parts;  // each group's partial sums per state
-    int64_t ntree = 0, nparts = nitems;
-    for (auto& kv : tree_slots) {
-        Decomp* d = kv.first;
-        const int64_t c = (int64_t)kv.second.size();
-        csim::tree::choose_levels(d->plan, c);
+    std::vector<csim::ValueSeg> vsegs(nseg);
+    int64_t nparts = nitems, ndiags = nitems;
+    for (size_t i = 0; i < nseg; i++) {
+        const Seg& sg = rs.segs[i];
+        Eval* e = sg.e;
+        csim::ValueSeg& v = vsegs[i];
+        v = csim::ValueSeg{sg.slot0, 0, 0, 0, e->t, e->kind == 2};
+        if (!e->tree) continue;
+        Decomp* d = e->q->dec;
         TreeGroup g;
         g.plan = &d->plan;
         g.dplan = d->dplan;
-        g.count = c;
+        g.count = sg.n;
+        g.shape_count = dec_states[d];
+        g.rows = e->kind == 2;
+        g.row0 = sg.s0;
         groups.push_back(g);
-        group_parts.push_back(tree_leaf_shape(d->plan, c).parts_per_state);
-        ntree += c;
-        nparts += c * group_parts.back();
+        v.parts = tree_leaf_shape(d->plan, g.shape_count).parts_per_state;
+        v.part0 = nparts;
+        nparts += sg.n * v.parts;
+        v.diag0 = ndiags;
+        if (g.rows) ndiags += sg.n;
     }
     const size_t scratch_bytes = tree_run_.layout(groups, kTreeScratchMax);
     std::vector<unsigned char> tree_jobs;
     tree_run_.build(nullptr, tree_jobs);  // for its size
-    // upload block: desc | proj | words | items | ranges | tree slots | tree jobs
-    const size_t o_desc = 0;
-    const size_t o_proj = align_up(o_desc + (size_t)ns * sizeof(csim::DrawDesc));
-    const size_t o_words = align_up(o_proj + evix.size() * 192 * 8);
-    const size_t o_items = align_up(o_words + (size_t)nwords * 4);
+    // upload block: projectors | segments | tree jobs | words | word offsets | state descriptors | items | ranges
+    const size_t o_proj = 0;
+    const size_t o_vsegs = align_up(o_proj + evix.size() * 192 * 8);
+    const size_t o_tjobs = align_up(o_vsegs + nseg * sizeof(csim::ValueSeg));
+    const size_t o_words = align_up(o_tjobs + tree_jobs.size());
+    const size_t o_offs = align_up(o_words + (size_t)nwords * 4);
+    const size_t o_desc = align_up(o_offs + (size_t)noffs * 8);
+    const size_t o_items = align_up(o_desc + (size_t)nother * sizeof(csim::DrawDesc));
     const size_t o_range = align_up(o_items + (size_t)nitems * sizeof(csim::PairItem));
-    const size_t o_range2 = align_up(o_range + (size_t)ns * 16);
-    const size_t o_ranged = align_up(o_range2 + (size_t)ns * 16);
-    const size_t o_tslots = align_up(o_ranged + (size_t)ns * 16);
-    const size_t o_tjobs = align_up(o_tslots + (size_t)ntree * 4);
-    const size_t up_bytes = align_up(o_tjobs + tree_jobs.size());
+    const size_t o_range2 = align_up(o_range + (size_t)nother * 16);
+    const size_t o_ranged = align_up(o_range2 + (size_t)nother * 16);
+    const size_t up_bytes = align_up(o_ranged + (size_t)nother * 16);
     bool any_direct = false;
     for (int b = 0; b < kBuckets; b++) any_direct |= b % 4 >= 2 && nbucket[b] > 0;
     // work block: states | parts | parts diag | pivot forms | direct and rest codes (direct launches)
     const size_t w_states = 0;
-    const size_t w_part = align_up((size_t)ns * sizeof(csim_state));
+    const size_t w_part = align_up((size_t)nother * sizeof(csim_state));
     const size_t w_partd = align_up(w_part + (size_t)std::max<int64_t>(nparts, 1) * 64);
-    const size_t w_canon = align_up(w_partd + (size_t)std::max<int64_t>(nitems, 1) * 64);
-    const size_t w_cdir = align_up(w_canon + (any_direct ? (size_t)ns * csim::canon_bytes() : 0));
-    const size_t w_crest = align_up(w_cdir + (any_direct ? (size_t)ns * 4 : 0));
-    const size_t work_bytes = align_up(w_crest + (any_direct ? (size_t)ns * 4 : 0));
-    // download block: err (16 B), the pair launches' work-queue counter (kQueueOffset) | codes | sums | sums diag
+    const size_t w_canon = align_up(w_partd + (size_t)std::max<int64_t>(ndiags, 1) * 64);
+    const size_t w_cdir = align_up(w_canon + (any_direct ? (size_t)nother * csim::canon_bytes() : 0));
+    const size_t w_crest = align_up(w_cdir + (any_direct ? (size_t)nother * 4 : 0));
+    const size_t work_bytes = align_up(w_crest + (any_direct ? (size_t)nother * 4 : 0));
+    // download block: err (16 B), the pair launches' work-queue counter (kQueueOffset) | codes | values
     rs.off_codes = 256;
-    rs.off_sum = align_up(rs.off_codes + (size_t)ns * 4);
-    rs.off_sumd = align_up(rs.off_sum + (size_t)ns * 64);
-    const size_t down_bytes = align_up(rs.off_sumd + (size_t)ns * 64);
-    if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) || tree_scratch_.ensure(scratch_bytes) || rs.down.ensure(down_bytes) ||
-        rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes))
+    rs.off_val = align_up(rs.off_codes + (size_t)ns * 4);
+    const size_t down_bytes = align_up(rs.off_val + (size_t)ns * 16);
+    if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) || tree_scratch_.ensure(scratch_bytes) ||
+        rs.down.ensure(down_bytes) || rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes))
         return fail(ctx_, CSIM_ERR_NOMEM, "round buffers (%lld states, %lld items)", (long long)ns,
                     (long long)nitems);
     unsigned char* hb = (unsigned char*)rs.hup.p;
@@ -769,15 +813,13 @@ int Engine::launch_round() {
         memcpy(blk + 64, kv.first->pz, 8 * kv.first->nstabs);
         memcpy(blk + 128, kv.first->px, 8 * kv.first->nstabs);
     }
-    {
-        size_t o = 0;
-        for (auto& j : jobs) {
-            if (j.nwords) memcpy(hb + o_words + 4 * o, j.words.data() + kRawHistory, j.nwords * 4);
-            o += j.nwords;
-        }
-    }
+    memcpy(hb + o_vsegs, vsegs.data(), nseg * sizeof(csim::ValueSeg));
+    for (auto& j : jobs)
+        if (j.nwords) memcpy(hb + o_words + 4 * (size_t)j.base, j.words.data() + kRawHistory, j.nwords * 4);
     const uint64_t* dproj = (const uint64_t*)(db + o_proj);
     const uint32_t* dwords = (const uint32_t*)(db + o_words);
+    int64_t* hoffs = (int64_t*)(hb + o_offs);
+    const int64_t* doffs = (const int64_t*)(db + o_offs);
     csim::DrawDesc* hdesc = (csim::DrawDesc*)(hb + o_desc);
     csim::PairItem* hitems = (csim::PairItem*)(hb + o_items);
     int64_t* hrange = (int64_t*)(hb + o_range);    // a slot's items in its heavy or warp launch
@@ -785,122 +827,142 @@ int Engine::launch_round() {
     int64_t* hranged = (int64_t*)(hb + o_ranged);  // items with a diagonal term (exactProjector rows)
     const double* dcum = (const double*)cum_.p;
     const csim::GState* dstates = (const csim::GState*)(wb + w_states);
+    __int128* const part = (__int128*)(wb + w_part);
+    __int128* const partd = (__int128*)(wb + w_partd);
+    int* const dcode = (int*)(dd + rs.off_codes);
     int64_t cur[kBuckets];
     for (int b = 0; b < kBuckets; b++) cur[b] = bstart[b];
-    int64_t iw = nitp;
-    for (int64_t i = 0; i < ns; i++) {
-        Eval* e = rs.slots[i].e;
-        const int64_t s = rs.slots[i].s;
+    int64_t iw = nitp, io = 0;
+    size_t gi = 0;
+    for (size_t si = 0; si < nseg; si++) {
+        const Seg& sg = rs.segs[si];
+        Eval* e = sg.e;
         const QueryRec* r = e->q;
-        const int b = evix[e];
-        csim::DrawDesc d{};
-        d.n = e->t;
-        d.nstabs = e->nstabs;
-        d.cum = dcum + 65 * e->t;
-        d.pm = (const int32_t*)(dproj + 192 * b);
-        d.pz = dproj + 192 * b + 64;
-        d.px = dproj + 192 * b + 128;
-        if (e->kind == 2) {
-            d.mode = 2;
-            d.src = (const csim::GState*)(r->dec->phis + s);
-        } else if (r->q.rng == CSIM_RNG_LIBC) {
-            d.mode = 3;
-            d.words = dwords;
-            d.wbegin = wr[i].first;
-            d.wend = wr[i].second;
-        } else {
-            d.mode = 0;
-            d.seed = r->q.seed;
-            d.id = e->id0 + (uint64_t)s;
+        const uint64_t* const pblk = dproj + 192 * evix[e];
+        const bool libc = e->kind == 1 && r->q.rng == CSIM_RNG_LIBC;
+        const int64_t* seg_offs = nullptr;  // host view of the segment's word offsets
+        const int64_t* seg_doffs = nullptr;
+        if (libc) {
+            const WordJob& j = jobs[job_of[si].first];
+            const int64_t k0 = job_of[si].second;
+            seg_offs = hoffs + io;
+            seg_doffs = doffs + io;
+            hoffs[io++] = j.base + (k0 ? j.ends[(size_t)k0 - 1] : 0);
+            for (int64_t k = 0; k < sg.n; k++) hoffs[io++] = j.base + j.ends[(size_t)(k0 + k)];
         }
-        hdesc[i] = d;
-        hranged[2 * i] = hranged[2 * i + 1] = 0;
-        if (e->tree) continue;  // ranges below, by group
-        const int64_t jb = e->kind == 2 ? s : 0;
-        const int64_t diag = e->kind == 2 ? s : -1;
-        if (!r->exact && r->dec->kern == 3) {
-            // a slot's items in its bucket's direct launches: narrow ones, then wide ones
-            const int64_t span_tp = span_tp_of(e);
-            const int b = 4 * bucket_of_[e->t];
-            const int64_t jn = jb + direct_narrow_items(e, span_tp) * span_tp;
-            const uint64_t* cw = e->kind == 1 ? r->dec->cws : r->dec->cw;
-            int64_t& cn = cur[b + 2];
-            int64_t& cd = cur[b + 3];
-            hrange[2 * i] = cn;
-            for (int64_t j = jb; j < jn; j += span_tp)
-                hitems[cn++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, cw, nullptr};
-            hrange[2 * i + 1] = cn;
-            hrange2[2 * i] = cd;
-            for (int64_t j = jn; j < e->chi; j += span_tp)
-                hitems[cd++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, cw, nullptr};
-            hrange2[2 * i + 1] = cd;
-            if (e->kind == 2) {  // no narrow items
-                hranged[2 * i] = hrange2[2 * i];
-                hranged[2 * i + 1] = cd;
-            }
-        } else if (!r->exact) {
-            // heavy items first, then light ones; a slot's items may sit in two
-            // launches, so its range is kept per slot in each (see below)
-            const int b = 4 * bucket_of_[e->t];
-            const int64_t span_tp = span_tp_of(e);
-            const int64_t jl = e->kind == 1 ? light_first_item(e, span_tp) * span_tp : e->chi;
-            int64_t& ch = cur[b];
-            int64_t& cl = cur[b + 1];
-            hrange[2 * i] = ch;
-            for (int64_t j = jb; j < std::min(jl, e->chi); j += span_tp)
-                hitems[ch++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag,
-                                              e->kind == 1 ? r->dec->cws : r->dec->cw, nullptr};
-            hrange[2 * i + 1] = ch;
-            hrange2[2 * i] = cl;
-            for (int64_t j = std::max(jl, jb); j < e->chi; j += span_tp)
-                hitems[cl++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, r->dec->cws, nullptr};
-            hrange2[2 * i + 1] = cl;
-            if (e->kind == 2) {  // no light items
-                hranged[2 * i] = hrange[2 * i];
-                hranged[2 * i + 1] = hrange[2 * i + 1];
-            }
-        } else {
-            hrange2[2 * i] = hrange2[2 * i + 1] = 0;
-            hrange[2 * i] = iw;
-            for (int64_t j = jb; j < e->chi; j += span_w)
-                hitems[iw++] = csim::PairItem{i, j, std::min(span_w, e->chi - j), diag, nullptr,
-                                              (const csim::GState*)r->dec->phis};
-            hrange[2 * i + 1] = iw;
+        if (e->tree) {
+            TreeGroup& g = groups[gi++];
+            const csim::ValueSeg& v = vsegs[si];
+            const Decomp* dec = r->dec;
+            g.draw = csim::TreeDraw{e->kind == 2 ? 3 : (libc ? 2 : 0),
+                                    e->nstabs,
+                                    r->q.seed,
+                                    e->kind == 2 ? (uint64_t)sg.s0 : e->id0 + (uint64_t)sg.s0,
+                                    dwords,
+                                    seg_doffs,
+                                    dcum + 65 * e->t,
+                                    (const int*)pblk,
+                                    pblk + 64,
+                                    pblk + 128,
+                                    dcode + sg.slot0,
+                                    dec->dL,
+                                    dec->exact ? -1 : dec->k,
+                                    0};
+            g.part = part + 4 * v.part0;
+            g.diag = partd + 4 * v.diag0;
+            continue;
+        }
+        for (int64_t k = 0; k < sg.n; k++) {
+            const int64_t i = sg.slot0 + k, s = sg.s0 + k;
+            csim::DrawDesc d{};
+            d.n = e->t;
+            d.nstabs = e->nstabs;
+            d.cum = dcum + 65 * e->t;
+            d.pm = (const int32_t*)pblk;
+            d.pz = pblk + 64;
+            d.px = pblk + 128;
             if (e->kind == 2) {
-                hranged[2 * i] = hrange[2 * i];
-                hranged[2 * i + 1] = iw;
+                d.mode = 2;
+                d.src = (const csim::GState*)(r->dec->phis + s);
+            } else if (libc) {
+                d.mode = 3;
+                d.words = dwords;
+                d.wbegin = seg_offs[k];
+                d.wend = seg_offs[k + 1];
+            } else {
+                d.mode = 0;
+                d.seed = r->q.seed;
+                d.id = e->id0 + (uint64_t)s;
             }
-        }
-    }
-    {
-        int32_t* hslots = (int32_t*)(hb + o_tslots);
-        int64_t at = 0, p0 = nitems;
-        size_t gi = 0;
-        for (auto& kv : tree_slots) {
-            groups[gi].index = (const int32_t*)(db + o_tslots) + at;
-            groups[gi].part = (__int128*)(wb + w_part) + 4 * p0;
-            const int64_t pp = group_parts[gi];
-            for (int32_t i : kv.second) {
-                hslots[at++] = i;
-                hrange[2 * i] = p0;
-                hrange[2 * i + 1] = p0 += pp;
+            hdesc[i] = d;
+            const int64_t jb = e->kind == 2 ? s : 0;
+            const int64_t diag = e->kind == 2 ? s : -1;
+            hranged[2 * i] = hranged[2 * i + 1] = 0;
+            if (!r->exact && r->dec->kern == 3) {
+                // a slot's items in its bucket's direct launches: narrow ones, then wide ones
+                const int64_t span_tp = span_tp_of(e);
+                const int b = 4 * bucket_of_[e->t];
+                const int64_t jn = jb + direct_narrow_items(e, span_tp) * span_tp;
+                const uint64_t* cw = e->kind == 1 ? r->dec->cws : r->dec->cw;
+                int64_t& cn = cur[b + 2];
+                int64_t& cd = cur[b + 3];
+                hrange[2 * i] = cn;
+                for (int64_t j = jb; j < jn; j += span_tp)
+                    hitems[cn++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, cw, nullptr};
+                hrange[2 * i + 1] = cn;
+                hrange2[2 * i] = cd;
+                for (int64_t j = jn; j < e->chi; j += span_tp)
+                    hitems[cd++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, cw, nullptr};
+                hrange2[2 * i + 1] = cd;
+                if (e->kind == 2) {  // no narrow items
+                    hranged[2 * i] = hrange2[2 * i];
+                    hranged[2 * i + 1] = cd;
+                }
+            } else if (!r->exact) {
+                // heavy items first, then light ones; a slot's items may sit in two
+                // launches, so its range is kept per slot in each (see below)
+                const int b = 4 * bucket_of_[e->t];
+                const int64_t span_tp = span_tp_of(e);
+                const int64_t jl = e->kind == 1 ? light_first_item(e, span_tp) * span_tp : e->chi;
+                int64_t& ch = cur[b];
+                int64_t& cl = cur[b + 1];
+                hrange[2 * i] = ch;
+                for (int64_t j = jb; j < std::min(jl, e->chi); j += span_tp)
+                    hitems[ch++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag,
+                                                  e->kind == 1 ? r->dec->cws : r->dec->cw, nullptr};
+                hrange[2 * i + 1] = ch;
+                hrange2[2 * i] = cl;
+                for (int64_t j = std::max(jl, jb); j < e->chi; j += span_tp)
+                    hitems[cl++] = csim::PairItem{i, j, std::min(span_tp, e->chi - j), diag, r->dec->cws, nullptr};
+                hrange2[2 * i + 1] = cl;
+                if (e->kind == 2) {  // no light items
+                    hranged[2 * i] = hrange[2 * i];
+                    hranged[2 * i + 1] = hrange[2 * i + 1];
+                }
+            } else {
                 hrange2[2 * i] = hrange2[2 * i + 1] = 0;
+                hrange[2 * i] = iw;
+                for (int64_t j = jb; j < e->chi; j += span_w)
+                    hitems[iw++] = csim::PairItem{i, j, std::min(span_w, e->chi - j), diag, nullptr,
+                                                  (const csim::GState*)r->dec->phis};
+                hrange[2 * i + 1] = iw;
+                if (e->kind == 2) {
+                    hranged[2 * i] = hrange[2 * i];
+                    hranged[2 * i + 1] = iw;
+                }
             }
-            gi++;
         }
-        tree_run_.layout(groups, kTreeScratchMax);
-        tree_run_.build((unsigned char*)tree_scratch_.p, tree_jobs);
-        if (!tree_jobs.empty()) memcpy(hb + o_tjobs, tree_jobs.data(), tree_jobs.size());
     }
+    tree_run_.layout(groups, kTreeScratchMax);
+    tree_run_.build((unsigned char*)tree_scratch_.p, tree_jobs);
+    if (!tree_jobs.empty()) memcpy(hb + o_tjobs, tree_jobs.data(), tree_jobs.size());
     int* derr = (int*)dd;
     const csim::Launch L = launch_on(derr);
     CK(cudaEventRecord(rs.ev[0], ctx_->stream));
     CK(cudaMemcpyAsync(db, hb, up_bytes, cudaMemcpyHostToDevice, ctx_->stream));
     CK(cudaMemsetAsync(derr, 0, 16, ctx_->stream));
-    __int128* part = (__int128*)(wb + w_part);
-    __int128* partd = (__int128*)(wb + w_partd);
-    int* dcode = (int*)(dd + rs.off_codes);
-    if (csim::launch_draw_project(L, (const csim::DrawDesc*)(db + o_desc), ns, (csim::GState*)(wb + w_states), dcode))
+    if (csim::launch_draw_project(L, (const csim::DrawDesc*)(db + o_desc), nother, (csim::GState*)(wb + w_states),
+                                  dcode))
         return fail(ctx_, CSIM_ERR_CUDA, "draw/project launch failed");
     CK(cudaEventRecord(rs.ev[1], ctx_->stream));
     const csim::PairItem* ditems = (const csim::PairItem*)(db + o_items);
@@ -914,7 +976,7 @@ int Engine::launch_round() {
     int* const rest_count = (int*)(dd + kRestCountOffset);
     if (any_direct) {
         CK(cudaMemsetAsync(rest_count, 0, 4, ctx_->stream));
-        if (csim::launch_canon(L, dstates, dcode, ns, dslots_max, canon, cdir, crest, rest_count))
+        if (csim::launch_canon(L, dstates, dcode, nother, dslots_max, canon, cdir, crest, rest_count))
             return fail(ctx_, CSIM_ERR_CUDA, "pivot form launch failed");
     }
     for (int b = 0; b < 4 * nbuckets_; b++) {
@@ -940,15 +1002,14 @@ int Engine::launch_round() {
         }
         if (rc) return fail(ctx_, CSIM_ERR_CUDA, "pair launch failed");
     }
-    if (!groups.empty() && tree_run_.launch(L, db + o_tjobs, dstates, dcode))
-        return fail(ctx_, CSIM_ERR_CUDA, "tree launch failed");
     if (csim::launch_items_warp(L, ditems + nitp, niw, dstates, dcode, part + 4 * nitp, partd + 4 * nitp))
         return fail(ctx_, CSIM_ERR_CUDA, "pair launch failed");
+    if (ndiags > nitems) CK(cudaMemsetAsync(partd + 4 * nitems, 0, (size_t)(ndiags - nitems) * 64, ctx_->stream));
+    if (!groups.empty() && tree_run_.launch(L, db + o_tjobs)) return fail(ctx_, CSIM_ERR_CUDA, "tree launch failed");
     CK(cudaEventRecord(rs.ev[2], ctx_->stream));
-    const int64_t* drange = (const int64_t*)(db + o_range);
-    const int64_t* drange2 = (const int64_t*)(db + o_range2);
-    if (csim::launch_reduce_slots(L, part, drange, drange2, ns, (__int128*)(dd + rs.off_sum)) ||
-        csim::launch_reduce_slots(L, partd, (const int64_t*)(db + o_ranged), nullptr, ns, (__int128*)(dd + rs.off_sumd)))
+    if (csim::launch_seg_values(L, (const csim::ValueSeg*)(db + o_vsegs), (int)nseg, ns, part, partd,
+                                (const int64_t*)(db + o_range), (const int64_t*)(db + o_range2),
+                                (const int64_t*)(db + o_ranged), dcode, dcum, (double*)(dd + rs.off_val)))
         return fail(ctx_, CSIM_ERR_CUDA, "reduce launch failed");
     CK(cudaMemcpyAsync(rs.hdown.p, dd, down_bytes, cudaMemcpyDeviceToHost, ctx_->stream));
     CK(cudaEventRecord(rs.ev[3], ctx_->stream));
@@ -973,45 +1034,39 @@ int Engine::complete_round() {
     const unsigned char* hd = (const unsigned char*)rs.hdown.p;
     const int err = *(const int*)hd;
     const int* code = (const int*)(hd + rs.off_codes);
-    const __int128* sum = (const __int128*)(hd + rs.off_sum);
-    const __int128* sumd = (const __int128*)(hd + rs.off_sumd);
+    const double* val = (const double*)(hd + rs.off_val);
     if (err) {
         fail(ctx_, CSIM_ERR_DEVICE, "kernel flagged error bits 0x%x (1 range, 2 replay, 4 expsum, 8 gamma, 16 arg)",
              err);
-        for (const Slot& sl : rs.slots)
-            if (!sl.e->q->done) fail_query(sl.e->q, CSIM_ERR_DEVICE);
-        for (const Slot& sl : rs.slots) sl.e->q->inflight--;
+        for (const Seg& sg : rs.segs)
+            if (!sg.e->q->done) fail_query(sg.e->q, CSIM_ERR_DEVICE);
+        for (const Seg& sg : rs.segs) sg.e->q->inflight -= sg.n;
         return 0;
     }
-    for (size_t i = 0; i < rs.slots.size(); i++) {
-        Eval* e = rs.slots[i].e;
-        const int64_t s = rs.slots[i].s;
-        e->q->inflight--;
+    for (const Seg& sg : rs.segs) {
+        Eval* e = sg.e;
+        e->q->inflight -= sg.n;
         if (e->q->done) continue;  // failed in an earlier round
-        const int P2 = 2 * e->t;
-        states++;
-        if (code[i] >= 0) {
-            states_live++;
-            const int64_t np = e->kind == 1 ? e->chi : e->chi - s;
-            pairs += np;
-            e->q->res.pairs += np;
-            const double pf = sqrt_half_power(code[i]);
-            double re, im;
+        const int* c = code + sg.slot0;
+        const double* v = val + 2 * sg.slot0;
+        int64_t np = 0;
+        for (int64_t i = 0; i < sg.n; i++) {
+            const int64_t s = sg.s0 + i;
             if (e->kind == 1) {  // singleProjectorSample's value, innerprod.c:142
-                zomega_to_complex(&sum[4 * i], P2, &re, &im);
-                const double x = re * pf, y = im * pf;
-                e->val[s] = pow(2, e->t) * (x * x + y * y);
-            } else {  // exactProjector row s: diag + 2 Re(off), innerprod.c:187-195
-                const __int128* o = &sum[4 * i];
-                const __int128* d = &sumd[4 * i];
-                const __int128 z[4] = {d[0] + 2 * o[0], d[1] + (o[1] - o[3]), d[2], d[3] - (o[1] - o[3])};
-                zomega_to_complex(z, P2, &re, &im);
-                e->val[2 * s] = re * pf;
-                e->val[2 * s + 1] = im * pf;
-                e->live[s] = 1;
+                e->val[s] = v[2 * i];
+            } else {  // exactProjector row s, innerprod.c:187-195
+                e->val[2 * s] = v[2 * i];
+                e->val[2 * s + 1] = v[2 * i + 1];
             }
+            if (c[i] < 0) continue;
+            states_live++;
+            np += e->kind == 1 ? e->chi : e->chi - s;
+            if (e->kind == 2) e->live[s] = 1;
         }
-        e->done++;
+        states += sg.n;
+        pairs += np;
+        e->q->res.pairs += np;
+        e->done += sg.n;
         if (e->done == e->ns) finish_eval(e);
     }
     return 0;

@@ -542,11 +542,6 @@ void tree_plan_for(csim_ctx* ctx, int exact, const uint64_t* L, int k, int t, in
     csim::tree::choose_levels(ctx->tree_plan, count);
 }
 
-// whether a decomposition's terms are summed as a tree: unless a pair kernel is asked for
-bool use_tree(const csim_ctx* ctx, int t, int exact, int k) {
-    return ctx->pair_kernel == 0 && !ctx->tuning && (exact ? (t + 1) / 2 : k) <= kTreeMaxRows;
-}
-
 // A sampler call's inputs on the device, one upload: the projector's rows, the
 // d-distribution of randomStabilizerState, the projection factors, the tree plan, the code
 struct CallInputs {
@@ -742,6 +737,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
                 TreeGroup g;
                 g.plan = &ctx->tree_plan;
                 g.dplan = in.plan;
+                g.draw = draw;
                 g.count = cs;
                 g.shape_count = shape_count;
                 g.part = spart;
@@ -751,7 +747,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
                 run.build((unsigned char*)scratch, jobs);
                 CKR(staged_put(ctx, 4 + (sb & 1), kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
                 // the event that starts the pair kernels' time is recorded behind the first roots
-                rc = run.launch(launch_of(ctx), djobs, nullptr, nullptr, &draw, first_sub ? ctx->ev[1] : nullptr);
+                rc = run.launch(launch_of(ctx), djobs, first_sub ? ctx->ev[1] : nullptr);
             } else if (tp && tn.kernel == 2) {
                 // one launch per occupancy class; class c's launch starts at its first whole item
                 const int64_t span = 64 * (int64_t)pt;
@@ -1123,6 +1119,8 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     g.rows = true;
     g.row0 = i0;
     g.diag = ddiag;
+    g.draw = csim::TreeDraw{3,     P->nstabs, 0,     (uint64_t)i0, nullptr, nullptr,        nullptr, in.pm,
+                            in.pz, in.px,     dcode, in.L,         exact ? -1 : k, 0};
     TreeRun run;
     std::vector<unsigned char> jobs;
     void* scratch;
@@ -1130,9 +1128,7 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
     run.build((unsigned char*)scratch, jobs);
     CKR(staged_put(ctx, 4, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
-    const csim::TreeDraw draw{3,       P->nstabs, 0,     (uint64_t)i0, nullptr, nullptr,        nullptr, in.pm,
-                              in.pz,   in.px,     dcode, in.L,         exact ? -1 : k, 0};
-    if (run.launch(launch_of(ctx), djobs, nullptr, nullptr, &draw, ctx->ev[1]))
+    if (run.launch(launch_of(ctx), djobs, ctx->ev[1]))
         return fail(ctx, CSIM_ERR_CUDA, "tree launch failed");
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
     // results: the live rows' count, the error word, the live rows' terms, re, im

@@ -632,6 +632,11 @@ inline int check_states(csim_ctx* ctx, const csim_state* s, int64_t count, int* 
 constexpr int64_t kBatch = 1 << 18;  // states per device round trip in the batched primitives
 
 
+// whether a decomposition's terms are summed as a tree: unless a pair kernel is asked for
+inline bool use_tree(const csim_ctx* ctx, int t, int exact, int k) {
+    return ctx->pair_kernel == 0 && !ctx->tuning && (exact ? (t + 1) / 2 : k) <= kTreeMaxRows;
+}
+
 inline int check_projector(csim_ctx* ctx, const csim_projector* P) {
     if (!P || P->nstabs < 0 || P->nqubits < 0 || P->nqubits > CSIM_MAX_QUBITS)
         return fail(ctx, CSIM_ERR_ARG, "bad projector");

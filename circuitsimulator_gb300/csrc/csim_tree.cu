@@ -1,8 +1,8 @@
 // csim_tree.cu — kernels of the tree sum (csim_tree.cuh): all terms of a
 // decomposition, |L> or |H^t>, for many states.
-//   k_tree_root   one warp per state: its graph form (csim_canon_warp.cuh) on
-//                 coordinates in the plan's order, as a root node
-//   k_tree_draw   the same for states that the warp draws and projects itself
+//   k_tree_draw   one warp per state: draws (or makes) it, projects it, and writes
+//                 its graph form (csim_canon_warp.cuh) on coordinates in the plan's
+//                 order as a root node
 //   k_tree_stage  one thread per node of the next written level: contracts the
 //                 coordinates between the two levels for its own message bits
 //   k_tree_leaf   one thread per node of the last written level (or a part of
@@ -18,6 +18,7 @@
 #include "csim_rng.cuh"
 #include "csim_tree.cuh"
 #include "csim_tree.h"
+#include "csim_values.cuh"
 #include "csim_warp.cuh"
 
 namespace csim {
@@ -140,47 +141,19 @@ __device__ void store_root(const TreeRootJob& J, int64_t i, const WS<NR>& st, Ro
 
 }  // namespace
 
-// roots of states that another kernel left in memory, projected
-__global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_root(const TreeRootJob* jobs, int njobs,
-                                                                   const GState* states, const int* code, int* err) {
-    __shared__ RootShared sh;
-    const TreeRootJob& J = job_of(jobs, njobs, blockIdx.x);
-    if ((int)threadIdx.x < J.t) sh.perm[threadIdx.x] = J.perm[threadIdx.x];
-    __syncthreads();
-    const int64_t i = ((int64_t)blockIdx.x - J.block0) * kTreeRootWarps + (threadIdx.x >> 5);
-    if (i >= J.count) return;  // warp-uniform
-    const int64_t a = J.index ? J.index[i] : J.first + i;
-    const int n = states[a].n, k = states[a].k;
-    const bool bad = n != J.t || k < 0 || k > n;
-    if (bad || code[a] < 0) {
-        if (bad && code[a] >= 0 && lane_id() == 0) atomicOr(err, kErrArg);
-        dead_root(J, i);
-        return;
-    }
-    if (n <= 32) {
-        WS<1> st;
-        load_state<1>(states + a, st);
-        store_root<1>(J, i, st, sh);
-    } else {
-        WS<2> st;
-        load_state<2>(states + a, st);
-        store_root<2>(J, i, st, sh);
-    }
-}
-
-// roots of states drawn and projected here (jobs of one decomposition):
-// k_random_states, k_project and k_tree_root in one launch, the state never
-// leaving the warp's registers.  Bound by the latency of a warp's serial steps:
-// 1024 states of 40 qubits take 44 us, the three launches 11 + 29 + 26 us.
+// Drawing, projecting and the graph form in one launch, the state never leaving the
+// warp's registers.  Bound by the latency of a warp's serial steps: 1024 states of
+// 40 qubits take 44 us; k_random_states, k_project and a kernel for the graph form
+// took 11 + 29 + 26 us.  NR = 1: jobs of up to 32 qubits, 2: the others.
 template <int NR>
-__global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRootJob* jobs, int njobs, TreeDraw d,
-                                                                   int* err) {
+__global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRootJob* jobs, int njobs, int* err) {
     __shared__ RootShared sh;
     const TreeRootJob& J = job_of(jobs, njobs, blockIdx.x);
     if ((int)threadIdx.x < J.t) sh.perm[threadIdx.x] = J.perm[threadIdx.x];
     __syncthreads();
     const int64_t i = ((int64_t)blockIdx.x - J.block0) * kTreeRootWarps + (threadIdx.x >> 5);
     if (i >= J.count) return;  // warp-uniform
+    const TreeDraw& d = J.draw;
     const int64_t a = J.first + i;
     int e = 0;
     const bool replay = d.mode == 1 || d.mode == 2;
@@ -443,7 +416,7 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
         int64_t state = 0, row = 0, term = 0;  // ROWS: the state, its row, and the term index so far
         if constexpr (ROWS) {
             state = node >> J.nodes_log2;
-            row = J.row ? J.row[state] : J.row0 + state;
+            row = J.row0 + state;
             for (int b = 0; b < J.nodes_log2; b++)
                 if ((node >> b) & 1) term ^= (int64_t)J.term[J.je + b];
             for (int b = 0; b < J.split; b++)
@@ -577,31 +550,7 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
 }
 
 // ---------------------------------------------------------------- values
-// z to double, to nearest even as the host's conversion: the top 64 bits with the
-// rest folded into the lowest one convert with a single rounding
-__device__ __forceinline__ double int128_to_double(__int128 z) {
-    const bool neg = z < 0;
-    const unsigned __int128 a = neg ? -(unsigned __int128)z : (unsigned __int128)z;
-    const uint64_t hi = (uint64_t)(a >> 64), lo = (uint64_t)a;
-    double d;
-    if (hi == 0ull) {
-        d = __ull2double_rn(lo);
-    } else {
-        const int s = 64 - __clzll((long long)hi);  // 1..64
-        const uint64_t top = s == 64 ? hi : ((hi << (64 - s)) | (lo >> s));
-        const uint64_t rest = s == 64 ? lo : lo << (64 - s);
-        d = __dmul_rn(__ull2double_rn(top | (rest != 0ull ? 1ull : 0ull)), __hiloint2double((1023 + s) << 20, 0));
-    }
-    return neg ? -d : d;
-}
-
-__device__ __forceinline__ __int128 shfl_xor_i128(__int128 v, int m) {
-    const uint64_t lo = shfl_xor64((uint64_t)v, m), hi = shfl_xor64((uint64_t)((unsigned __int128)v >> 64), m);
-    return (__int128)(((unsigned __int128)hi << 64) | lo);
-}
-
-// One warp per state: the sum of its partial sums as a double, with the host's own
-// roundings (csim_host::zomega_to_complex: no fused multiply-adds).  factor[c]: the
+// One warp per state: the sum of its partial sums as a double.  factor[c]: the
 // projection factor of c measurements that halved the norm.  *live counts the
 // states that the projector left alive (0 for the others).  Without diag: out is
 // singleProjectorSample's value 2^t |projfactor sum|^2 (innerprod.c:142); with it
@@ -619,49 +568,30 @@ __global__ void __launch_bounds__(128) k_tree_values(const __int128* part, const
     for (int64_t p = lane >> 2; p < parts; p += 8) z += part[4 * (i * parts + p) + q];
 #pragma unroll
     for (int o = 4; o < 32; o <<= 1) z += shfl_xor_i128(z, o);
-    // lanes 0..3 hold coordinates 0..3 and need z0, z1 - z3, z2, z1 + z3
-    const __int128 other = shfl_xor_i128(z, 2);
-    __int128 v = q == 1 ? z - other : (q == 3 ? other + z : z);
-    if (diag) {  // 2 Re(o) = 2 o0 + (o1 - o3) (w - w^3)
-        const __int128 d = c >= 0 ? diag[4 * i + q] : 0, dother = shfl_xor_i128(d, 2);
-        v = q == 0 ? d + 2 * z : (q == 1 ? d - dother + 2 * v : (q == 2 ? d : dother + d));
-    }
-    const double x = int128_to_double(v);
-    const double s = 0.70710678118654752440;
-    const double x0 = __shfl_sync(kFull, x, 0), x1 = __shfl_sync(kFull, x, 1), x2 = __shfl_sync(kFull, x, 2),
-                 x3 = __shfl_sync(kFull, x, 3);
+    const __int128 d = diag && c >= 0 ? diag[4 * i + q] : 0;
+    double a, b;
+    warp_value(z, diag != nullptr, d, t, factor[c >= 0 ? c : 0], a, b);
     if (lane != 0) return;
-    double a = 0, b = 0;
     if (c >= 0) {
-        const double unit = __hiloint2double((1023 - t) << 20, 0);  // 2^-t
-        a = __dmul_rn(__dmul_rn(__dadd_rn(x0, __dmul_rn(x1, s)), unit), factor[c]);
-        b = __dmul_rn(__dmul_rn(__dadd_rn(x2, __dmul_rn(x3, s)), unit), factor[c]);
         atomicAdd(live, 1ull);
         if (diag) atomicAdd(live + 2, (unsigned long long)(row_terms - i));
+    } else {
+        a = b = 0;
     }
     if (im_out) {
         out[i] = a;
         im_out[i] = b;
     } else {
-        out[i] = __dmul_rn(__hiloint2double((1023 + t) << 20, 0), __dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)));
+        out[i] = sample_value(a, b, t);
     }
 }
 
 // ---------------------------------------------------------------- launchers
-int launch_tree_root(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, const GState* states,
-                     const int* code) {
+int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, bool wide) {
     if (njobs <= 0 || blocks <= 0) return 0;
     if (blocks > 0x7fffffff) return -1;
-    k_tree_root<<<(unsigned)blocks, 32 * kTreeRootWarps, 0, L.stream>>>(jobs, njobs, states, code, L.d_err);
-    (*L.launches)++;
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, int t, const TreeDraw& d) {
-    if (njobs <= 0 || blocks <= 0) return 0;
-    if (blocks > 0x7fffffff || t < 1 || t > 64) return -1;
-    if (t <= 32) k_tree_draw<1><<<(unsigned)blocks, 32 * kTreeRootWarps, 0, L.stream>>>(jobs, njobs, d, L.d_err);
-    else k_tree_draw<2><<<(unsigned)blocks, 32 * kTreeRootWarps, 0, L.stream>>>(jobs, njobs, d, L.d_err);
+    if (wide) k_tree_draw<2><<<(unsigned)blocks, 32 * kTreeRootWarps, 0, L.stream>>>(jobs, njobs, L.d_err);
+    else k_tree_draw<1><<<(unsigned)blocks, 32 * kTreeRootWarps, 0, L.stream>>>(jobs, njobs, L.d_err);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

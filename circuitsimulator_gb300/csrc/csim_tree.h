@@ -13,9 +13,27 @@ namespace csim {
 // Every launch runs a table of jobs (one per group of states that share a
 // decomposition); a job's blocks are [block0, the next job's block0).
 
-// root nodes of `count` states: state i of the job is states[index ? index[i] : first + i]
+// How k_tree_draw makes states (k_random_states, k_project): state a is state id + a
+// of Philox stream `seed` (mode 0) or replays words [offsets[a], offsets[a + 1])
+// (mode 1: rand() values, 2: raw words, csim_rng.cuh).  Mode 3: exactProjector's term states,
+// state a is term id + a of the k-row code `words64` or (k < 0) of |H^t>.  code[a]
+// as k_project writes it.
+struct TreeDraw {
+    int32_t mode, nstabs;
+    uint64_t seed, id;
+    const uint32_t* words;
+    const int64_t* offsets;
+    const double* cum;
+    const int* pm;
+    const uint64_t *pz, *px;
+    int* code;
+    const uint64_t* words64;
+    int32_t k, pad;
+};
+
+// root nodes of `count` states: state i of the job is state first + i of draw
 struct TreeRootJob {
-    const int32_t* index;
+    TreeDraw draw;
     int64_t first;
     const uint8_t* perm;  // position -> coordinate (t of them)
     uint32_t* out;        // node planes, one node per state
@@ -45,40 +63,20 @@ struct TreeLeafJob {
     int32_t m, je, tv, tj;
     int32_t split, reps, group, shift;  // sums are scaled by 2^{shift / 2}
     uint16_t gen[16];     // generators of the levels below je, positions < m
-    // exactProjector rows: state a is row row[a] (or row0 + a); only its terms j > row are
-    // summed, term j == row is written to diag + 4 a
-    const int32_t* row;
+    // exactProjector rows: state a is row row0 + a; only its terms j > row are summed, term
+    // j == row is written to diag + 4 a
     const uint64_t* term; // the generators' parts of the term index, all levels
     __int128* diag;
     int64_t row0;
     int32_t nodes_log2, pad;  // log2 of the nodes per state
 };
 
-// How k_tree_draw makes its states (k_random_states, k_project): state a of the
-// call is state id + a of Philox stream `seed` (mode 0) or replays words
-// [offsets[a], offsets[a + 1]) (mode 1).  Mode 3: exactProjector's term states,
-// state a is term id + a of the k-row code `words64` or (k < 0) of |H^t>.  code[a]
-// as k_project writes it.
-struct TreeDraw {
-    int32_t mode, nstabs;  // mode 2: the words are raw (csim_rng.cuh)
-    uint64_t seed, id;
-    const uint32_t* words;
-    const int64_t* offsets;
-    const double* cum;
-    const int* pm;
-    const uint64_t *pz, *px;
-    int* code;
-    const uint64_t* words64;
-    int32_t k, pad;
-};
-
 constexpr int kTreeRootWarps = 4;      // states per root block
 constexpr int kTreeStageThreads = 64;
 constexpr int kTreeLeafThreads = 128;
 
-int launch_tree_root(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, const GState* states,
-                     const int* code);
-int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, int t, const TreeDraw& d);
+// wide: the jobs' states have more than 32 qubits
+int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, bool wide);
 // wide: the jobs' parents have more than 32 vertices (two words per row); mmax: the largest mp
 int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax,
                       bool pairs);

@@ -21,14 +21,13 @@ constexpr size_t kTreePlanBytes = 2 * 64 * 8 + 64;
 struct TreeGroup {
     const csim::tree::Plan* plan = nullptr;
     const unsigned char* dplan = nullptr;  // the plan's device arrays (kTreePlanBytes)
-    const int32_t* index = nullptr;        // device: states of the group (null: first, first + 1, ...)
-    int64_t first = 0, count = 0;
+    csim::TreeDraw draw{};                 // its states are draw's states 0 .. count - 1
+    int64_t count = 0;
     int64_t shape_count = 0;               // states that tree_leaf_shape is asked for (0: count)
     __int128* part = nullptr;              // device: parts_per_state partial sums for each state
-    // exactProjector rows (TreeLeafJob): the states' rows (device; null: row0, row0 + 1, ...), and 4
-    // int128 per state that are zero before the launches
+    // exactProjector rows (TreeLeafJob) row0, row0 + 1, ..., and 4 int128 per state that are zero
+    // before the launches
     bool rows = false;
-    const int32_t* row = nullptr;
     int64_t row0 = 0;
     __int128* diag = nullptr;
 };
@@ -126,23 +125,24 @@ class TreeRun {
         blob.clear();
         steps_.clear();
         for (const Chunk& ch : chunks_) {
-            std::vector<csim::TreeRootJob> roots;
+            std::vector<csim::TreeRootJob> roots[2];    // up to 32 qubits, more
             std::vector<csim::TreeLeafJob> leaves[16];  // by table words (1, 2, 4, 8), rows, pairs
-            int64_t rb = 0, lb[16] = {};
+            int64_t rb[2] = {}, lb[16] = {};
             size_t depth = 0;
             for (const Piece& p : ch.pieces) {
                 const csim::tree::Plan& pl = *p.g.plan;
                 csim::TreeRootJob r{};
-                r.index = p.g.index ? p.g.index + p.first : nullptr;
-                r.first = p.g.first + p.first;
+                const int wide = pl.t > 32;
+                r.draw = p.g.draw;
+                r.first = p.first;
                 r.perm = p.g.dplan + 2 * 64 * 8;
                 r.x0 = pl.x0;
                 r.out = (uint32_t*)(scratch + p.off[0]);
                 r.count = p.count;
-                r.block0 = rb;
+                r.block0 = rb[wide];
                 r.t = pl.t;
-                rb += (p.count + csim::kTreeRootWarps - 1) / csim::kTreeRootWarps;
-                roots.push_back(r);
+                rb[wide] += (p.count + csim::kTreeRootWarps - 1) / csim::kTreeRootWarps;
+                roots[wide].push_back(r);
                 depth = std::max(depth, pl.level.size());
                 const TreeLeafShape s = tree_leaf_shape(pl, p.g.shape_count ? p.g.shape_count : p.g.count);
                 csim::TreeLeafJob l{};
@@ -163,7 +163,6 @@ class TreeRun {
                 l.shift = pl.t - pl.tv + 2 * (pl.k - pl.r);  // each codeword 2^{k - r} times
                 for (int j = 0; j < je; j++) l.gen[j] = (uint16_t)pl.gen[j];
                 if (p.g.rows) {
-                    l.row = p.g.row ? p.g.row + p.first : nullptr;
                     l.row0 = p.g.row0 + p.first;
                     l.term = (const uint64_t*)p.g.dplan + 64;
                     l.diag = p.g.diag + 4 * p.first;
@@ -172,7 +171,8 @@ class TreeRun {
                 lb[wc] += (l.threads + csim::kTreeLeafThreads - 1) / csim::kTreeLeafThreads;
                 leaves[wc].push_back(l);
             }
-            add(blob, Step{0, 0, ch.pieces[0].g.plan->t, (int)roots.size(), rb, 0}, roots);
+            for (int wide = 0; wide < 2; wide++)
+                if (!roots[wide].empty()) add(blob, Step{0, wide, 0, (int)roots[wide].size(), rb[wide], 0}, roots[wide]);
             for (size_t d = 1; d < depth; d++)
                 for (int kind = 0; kind < 4; kind++) {  // bit 0 wide, bit 1 pairs
                     std::vector<csim::TreeStageJob> st;
@@ -204,18 +204,15 @@ class TreeRun {
         }
     }
 
-    // Queues the launches; `djobs`: build()'s tables on the device.  The states are in
-    // memory (states, code), or with `draw` made by the root launches (one group).
-    // after_first (optional) is recorded behind the first launch.
-    int launch(const csim::Launch& L, const unsigned char* djobs, const csim::GState* states, const int* code,
-               const csim::TreeDraw* draw = nullptr, cudaEvent_t after_first = nullptr) const {
+    // Queues the launches; `djobs`: build()'s tables on the device.  after_first (optional)
+    // is recorded behind the first launch.
+    int launch(const csim::Launch& L, const unsigned char* djobs, cudaEvent_t after_first = nullptr) const {
         for (size_t i = 0; i < steps_.size(); i++) {
             const Step& s = steps_[i];
             const void* j = djobs + s.off;
             if (i == 1 && after_first && cudaEventRecord(after_first, L.stream) != cudaSuccess) return -1;
             const int rc =
-                s.kind == 0 && draw ? csim::launch_tree_draw(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, s.size, *draw)
-                : s.kind == 0 ? csim::launch_tree_root(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, states, code)
+                s.kind == 0   ? csim::launch_tree_draw(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, s.flags & 1)
                 : s.kind == 1 ? csim::launch_tree_stage(L, (const csim::TreeStageJob*)j, s.njobs, s.blocks, s.flags & 1, s.size,
                                                           s.flags & 2)
                               : csim::launch_tree_leaf(L, (const csim::TreeLeafJob*)j, s.njobs, s.blocks, s.size,
@@ -236,8 +233,8 @@ class TreeRun {
     };
     struct Step {
         int kind;  // 0 roots, 1 a stage, 2 leaves
-        int flags;  // stages: bit 0 wide, bit 1 pairs; leaves: bit 0 rows, bit 1 pairs
-        int size;  // roots: the first group's qubits; a stage's largest parent; the leaves' table words
+        int flags;  // roots and stages: bit 0 wide, bit 1 pairs; leaves: bit 0 rows, bit 1 pairs
+        int size;   // a stage's largest parent; the leaves' table words
         int njobs;
         int64_t blocks;
         size_t off;
