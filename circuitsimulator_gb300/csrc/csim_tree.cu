@@ -46,40 +46,42 @@ __device__ __forceinline__ uint64_t permute_bits(uint64_t v, const unsigned char
     return r;
 }
 
+// vector v of node i among `count` nodes, tail u, the status word of m > 16
+__device__ __forceinline__ uint32_t* vector_at(uint32_t* base, int64_t count, int v, uint32_t i) {
+    return base + 4 * ((int64_t)v * count + i);
+}
+__device__ __forceinline__ uint32_t* tail_at(uint32_t* base, int64_t count, int m, int u, uint32_t i) {
+    return base + 4 * node_vectors(m) * count + ((int64_t)u * count + i) * row_tail(m);
+}
+__device__ __forceinline__ uint32_t* status_at(uint32_t* base, int64_t count, int m, uint32_t i) {
+    return base + (int64_t)(node_words(m) - 1) * count + i;
+}
+__device__ __forceinline__ void store_vector(uint32_t* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    *reinterpret_cast<uint4*>(p) = make_uint4(a, b, c, d);
+}
+
 // stores row `pos` of node i among `count` nodes of m vertices
-__device__ __forceinline__ void store_row(uint32_t* base, int64_t count, int64_t i, int m, int pos, uint64_t row) {
-    if (m > 32) {
-        base[(int64_t)(2 * pos) * count + i] = (uint32_t)row;
-        base[(int64_t)(2 * pos + 1) * count + i] = (uint32_t)(row >> 32);
-    } else if (m > 16) {
-        base[(int64_t)pos * count + i] = (uint32_t)row;
-    } else {
-        reinterpret_cast<uint16_t*>(base + (int64_t)(pos >> 1) * count + i)[pos & 1] = (uint16_t)row;
+__device__ __forceinline__ void store_row(uint32_t* base, int64_t count, uint32_t i, int m, int pos, uint64_t row) {
+    const int pl = row_planes(m), u = pos >> 2;
+    for (int k = 0; k < pl; k++) {
+        uint32_t* w = pl == 2 ? vector_at(base, count, node_scalars(m) + (u >> 1), i) + 2 * (u & 1) + k
+                              : (k < 4 ? vector_at(base, count, node_scalars(m) + u, i) + k
+                                       : tail_at(base, count, m, u, i) + (k - 4));
+        reinterpret_cast<uint8_t*>(w)[pos & 3] = (uint8_t)(row >> (8 * k));
     }
 }
-__device__ __forceinline__ void store_scalars(uint32_t* base, int64_t count, int64_t i, int m, uint64_t d1, uint64_t d2,
+__device__ __forceinline__ void store_scalars(uint32_t* base, int64_t count, uint32_t i, int m, uint64_t d1, uint64_t d2,
                                               uint64_t h, uint64_t x, uint32_t status) {
-    uint32_t* p = base + (int64_t)node_row_words(m) * count + i;
+    uint32_t* p = vector_at(base, count, 0, i);
     if (m > 32) {
-        p[0] = (uint32_t)d1;
-        p[count] = (uint32_t)(d1 >> 32);
-        p[2 * count] = (uint32_t)d2;
-        p[3 * count] = (uint32_t)(d2 >> 32);
-        p[4 * count] = (uint32_t)h;
-        p[5 * count] = (uint32_t)(h >> 32);
-        p[6 * count] = (uint32_t)x;
-        p[7 * count] = (uint32_t)(x >> 32);
-        p[8 * count] = status;
+        store_vector(p, (uint32_t)d1, (uint32_t)(d1 >> 32), (uint32_t)d2, (uint32_t)(d2 >> 32));
+        store_vector(p + 4 * count, (uint32_t)h, (uint32_t)(h >> 32), (uint32_t)x, (uint32_t)(x >> 32));
+        *status_at(base, count, m, i) = status;
     } else if (m > 16) {
-        p[0] = (uint32_t)d1;
-        p[count] = (uint32_t)d2;
-        p[2 * count] = (uint32_t)h;
-        p[3 * count] = (uint32_t)x;
-        p[4 * count] = status;
+        store_vector(p, (uint32_t)d1, (uint32_t)d2, (uint32_t)h, (uint32_t)x);
+        *status_at(base, count, m, i) = status;
     } else {
-        p[0] = (uint32_t)d1 | ((uint32_t)d2 << 16);
-        p[count] = (uint32_t)h | ((uint32_t)x << 16);
-        p[2 * count] = status;
+        store_vector(p, (uint32_t)d1 | ((uint32_t)d2 << 16), (uint32_t)h | ((uint32_t)x << 16), status, 0u);
     }
 }
 
@@ -95,13 +97,13 @@ struct RootShared {
 };
 
 // a state that the projector annihilates, or a bad one: its sum is 0
-__device__ __forceinline__ void dead_root(const TreeRootJob& J, int64_t i) {
+__device__ __forceinline__ void dead_root(const TreeRootJob& J, uint32_t i) {
     if (lane_id() == 0) store_scalars(J.out, J.count, i, J.t, 0, 0, 0, 0, pack_status(0, 0, 1));
 }
 
 // Node i of the job from a state held by the warp
 template <int NR>
-__device__ void store_root(const TreeRootJob& J, int64_t i, const WS<NR>& st, RootShared& sh) {
+__device__ void store_root(const TreeRootJob& J, uint32_t i, const WS<NR>& st, RootShared& sh) {
     unsigned char* const piv = sh.piv[threadIdx.x >> 5];
     const int t = J.t, k = st.k;
     const uint64_t km = pc::lowmask(k), nm = pc::lowmask(t);
@@ -184,80 +186,150 @@ __global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRoo
         if (res == 2) c++;
     }
     if (lane_id() == 0) d.code[a] = c;
-    if (c < 0) dead_root(J, i);
-    else store_root<NR>(J, i, st, sh);
+    if (c < 0) dead_root(J, (uint32_t)i);
+    else store_root<NR>(J, (uint32_t)i, st, sh);
     e = (int)__reduce_or_sync(kFull, (unsigned)e);
     if (e && lane_id() == 0) atomicOr(err, e);
 }
 
 // ---------------------------------------------------------------- stages
-template <class W>
-struct StageRows;
-template <>
-struct StageRows<uint32_t> {
-    using Rows = Rows32;
-    static constexpr int words = 1;
-    __device__ __forceinline__ static Rows at(uint32_t* smem, int, int tid) { return Rows{smem + 4 * tid, kTreeStageThreads}; }
-};
-template <>
-struct StageRows<uint64_t> {
-    using Rows = Rows64;
-    static constexpr int words = 2;
-    __device__ __forceinline__ static Rows at(uint32_t* smem, int units, int tid) {
-        return Rows{smem + 4 * tid, smem + (size_t)units * 4 * kTreeStageThreads + 4 * tid, kTreeStageThreads};
+// n vectors of V from the planes `from`, from + step, ... to two copies in shared memory
+// (`copy` words apart), the vectors of one `stride` words apart: through registers, eight
+// loads in flight
+template <class V>
+__device__ __forceinline__ void copy_twice(uint32_t* to, size_t copy, int stride, const uint32_t* from, int64_t step, int n) {
+    for (int u = 0; u < n; u += 8) {
+        V v[8];
+#pragma unroll
+        for (int b = 0; b < 8; b++)
+            if (u + b < n) v[b] = *reinterpret_cast<const V*>(from + b * step);
+#pragma unroll
+        for (int b = 0; b < 8; b++)
+            if (u + b < n) {
+                *reinterpret_cast<V*>(to + b * stride) = v[b];
+                *reinterpret_cast<V*>(to + copy + b * stride) = v[b];
+            }
+        from += 8 * step;
+        to += 8 * stride;
     }
-};
+}
+// The same past the registers, all in flight.  Rows from 33 vertices up: at t = 64 (2^14
+// terms) their stages are 2 to 10% faster so, where few blocks fit an SM and a warp reads
+// many parents; narrower rows are as fast or slower (a stage from 32 vertices whose warps
+// read one parent each: 80 us, 60 through registers).
+template <int BYTES>
+__device__ __forceinline__ void copy_async_twice(uint32_t* to, size_t copy, int stride, const uint32_t* from, int64_t step,
+                                                 int n) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(to);
+    const uint32_t second = (uint32_t)(4 * copy);
+    for (int u = 0; u < n; u++) {
+        asm volatile("cp.async.ca.shared.global [%0], [%2], %3;\n\tcp.async.ca.shared.global [%1], [%2], %3;" ::"r"(a),
+                     "r"(a + second), "l"(from), "n"(BYTES)
+                     : "memory");
+        from += step;
+        a += 4 * (uint32_t)stride;
+    }
+}
 
-// two words of a plane, for two adjacent nodes (counts are even, so they are aligned)
-__device__ __forceinline__ void store_two(uint32_t* plane, uint32_t at, uint32_t a, uint32_t b) {
-    *reinterpret_cast<uint2*>(plane + at) = make_uint2(a, b);
+// A node's rows (of `m` vertices, from rows of PL planes and `units` units) and scalars
+template <int PL, class W>
+__device__ __forceinline__ void store_node(uint32_t* out, int64_t count, uint32_t i, int m, const Rows<PL>& rows, int units,
+                                           const Node<W>& s, W x) {
+    const W cm = wlow<W>(m);
+    const uint32_t status = pack_status(s.q, s.iso, s.dead);
+    store_scalars(out, count, i, m, (uint64_t)(s.d1 & cm), (uint64_t)(s.d2 & cm), (uint64_t)(s.h & cm), (uint64_t)(x & cm),
+                  status);
+    if (s.dead) return;
+    const int cu = row_units(m);
+    uint32_t* p = vector_at(out, count, node_scalars(m), i);
+    if (PL > 2 && m <= 16) {  // two units to a vector
+        for (int u = 0; u < cu; u += 2) {
+            const U32x4 a = *rows.chunk(u), b = *rows.chunk(u + 1 < units ? u + 1 : u);
+            store_vector(p, a.a, a.b, b.a, b.b);
+            p += 4 * count;
+        }
+        return;
+    }
+    const int n = PL == 2 ? Rows<2>::chunks(cu) : cu;
+#pragma unroll 4
+    for (int u = 0; u < n; u++) {
+        const U32x4 v = *rows.chunk(u);
+        store_vector(p, v.a, v.b, v.c, v.d);
+        p += 4 * count;
+    }
+    if constexpr (PL > 4) {
+        const int tw = row_tail(m);
+        if (tw == 0) return;
+        p = tail_at(out, count, m, 0, i);
+        for (int u = 0; u < cu; u++) {
+            const U32x4 v = rows.get_tail(u);
+            if (tw == 1) *p = v.a;
+            else if (tw == 2) *reinterpret_cast<uint2*>(p) = make_uint2(v.a, v.b);
+            else store_vector(p, v.a, v.b, v.c, v.d);
+            p += tw * count;
+        }
+    }
 }
 
 // One thread per pair of siblings (nodes 2 i and 2 i + 1, whose messages differ in
-// the lowest bit).  ALU-bound (90% of the pipe): a pair of 28 -> 15 vertices runs
-// about 8 steps over some 20 rows.  The parent's rows are copied to shared memory
-// twice, so a lane moves on from one sibling to the other without a load: a stage
-// from 28 to 15 vertices took 985 us for 14.3e6 nodes with a node per thread, 576
-// with a pair.
-template <class W, bool PAIRS>
+// the lowest bit).  The parent's rows are copied to shared memory twice, so a lane
+// moves on from one sibling to the other without a load: a stage from 28 to 15
+// vertices took 985 us for 14.3e6 nodes with a node per thread, 576 with a pair.
+// Up to 32 vertices ALU-bound (83 to 90% of the pipe), above it by the latency of few
+// resident warps: shared memory holds 3 to 9 blocks (17% of the warps at 48 vertices).
+// Nodes move as 16-byte vectors and several loads at a time: with a load per word and
+// no more than four in flight, rows of 64, 48 and 40 vertices took 39, 213 and 191 us
+// (300 states of 64 qubits, 2^14 terms), now 26, 107 and 92.
+template <int PL, bool PAIRS>
 __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStageJob* jobs, int njobs) {
+    using W = typename RowWord<PL>::type;
     extern __shared__ __align__(16) uint32_t smem[];
     const TreeStageJob& J = job_of(jobs, njobs, blockIdx.x);
     const int mp = J.mp, mc = J.mc, sub = J.sub;
-    const int units = (mp + 3) / 4;
-    const size_t copy = (size_t)units * 4 * kTreeStageThreads * StageRows<W>::words;  // words of a copy
-    const auto rows = StageRows<W>::at(smem, units, threadIdx.x);
+    const int units = row_units(mp);
+    const size_t copy = Rows<PL>::words(units, kTreeStageThreads);
+    const Rows<PL> rows = Rows<PL>::at(smem, threadIdx.x, units, kTreeStageThreads);
+    Rows<PL> two = rows;
+    two.shift(copy);
     const bool both = sub > 0;  // a stage of no message bits (a code without rows) has no siblings
     const uint32_t pairs = (uint32_t)(both ? J.count >> 1 : J.count);
     const uint32_t i = (uint32_t)((int64_t)blockIdx.x - J.block0) * kTreeStageThreads + threadIdx.x;
     const bool valid = i < pairs;
     const uint32_t pi = valid ? (both ? i >> (sub - 1) : i) : 0u;  // the parent
     const int64_t np = J.in_count;
+    // rows into shared memory, two copies (a dead parent's were never written: nothing uses them)
+    const uint32_t* const vectors = J.in + 4 * ((int64_t)node_scalars(mp) * np + pi);
+    if constexpr (PL <= 4) {
+        copy_twice<uint4>(rows.p, copy, 4 * kTreeStageThreads, vectors, 4 * np, Rows<PL>::chunks(units));
+    } else {
+        constexpr int tw = Rows<PL>::tail;
+        copy_async_twice<16>(rows.p, copy, 4 * kTreeStageThreads, vectors, 4 * np, units);
+        copy_async_twice<4 * tw>(rows.tp, copy, tw * kTreeStageThreads, J.in + 4 * node_vectors(mp) * np + (int64_t)pi * tw,
+                                 tw * np, units);
+    }
     Work<W> a;
     W x;
     uint32_t status;
     {
-        const uint32_t* p = J.in + (int64_t)node_row_words(mp) * np;  // uniform plane bases, 32-bit lane offset
+        const uint4 s0 = *reinterpret_cast<const uint4*>(J.in + 4 * (int64_t)pi);
         if constexpr (sizeof(W) == 8) {
-            a.s.d1 = (W)p[pi] | ((W)(p + np)[pi] << 32);
-            a.s.d2 = (W)(p + 2 * np)[pi] | ((W)(p + 3 * np)[pi] << 32);
-            a.s.h = (W)(p + 4 * np)[pi] | ((W)(p + 5 * np)[pi] << 32);
-            x = (W)(p + 6 * np)[pi] | ((W)(p + 7 * np)[pi] << 32);
-            status = (p + 8 * np)[pi];
-        } else if (mp > 16) {
-            a.s.d1 = p[pi];
-            a.s.d2 = (p + np)[pi];
-            a.s.h = (p + 2 * np)[pi];
-            x = (p + 3 * np)[pi];
-            status = (p + 4 * np)[pi];
+            const uint4 s1 = *reinterpret_cast<const uint4*>(J.in + 4 * (np + pi));
+            a.s.d1 = (W)s0.x | ((W)s0.y << 32);
+            a.s.d2 = (W)s0.z | ((W)s0.w << 32);
+            a.s.h = (W)s1.x | ((W)s1.y << 32);
+            x = (W)s1.z | ((W)s1.w << 32);
+        } else if (PL > 2) {
+            a.s.d1 = s0.x;
+            a.s.d2 = s0.y;
+            a.s.h = s0.z;
+            x = s0.w;
         } else {
-            const uint32_t dd = p[pi], hx = (p + np)[pi];
-            a.s.d1 = dd & 0xFFFFu;
-            a.s.d2 = dd >> 16;
-            a.s.h = hx & 0xFFFFu;
-            x = hx >> 16;
-            status = (p + 2 * np)[pi];
+            a.s.d1 = s0.x & 0xFFFFu;
+            a.s.d2 = s0.x >> 16;
+            a.s.h = s0.y & 0xFFFFu;
+            x = s0.y >> 16;
         }
+        status = PL > 2 ? J.in[(int64_t)(node_words(mp) - 1) * np + pi] : s0.z;
     }
     const bool alive = valid && !(status & 0x80000000u);
     a.s.q = (int)(status & 7u);
@@ -265,41 +337,12 @@ __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStag
     a.s.dead = alive ? 0 : 1;
     for (int b = 1; b < sub; b++)
         if ((i >> (b - 1)) & 1u) x ^= (W)J.gen[b];
-    // rows into shared memory, four to a unit (a dead parent's rows were never written)
-    for (int u = 0; u < units; u++) {
-        uint32_t lo[4], hi[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int r = 4 * u + q;
-            lo[q] = hi[q] = 0u;
-            if (r < mp && alive) {
-                if constexpr (sizeof(W) == 8) {
-                    lo[q] = (J.in + (int64_t)(2 * r) * np)[pi];
-                    hi[q] = (J.in + (int64_t)(2 * r + 1) * np)[pi];
-                } else if (mp > 16) {
-                    lo[q] = (J.in + (int64_t)r * np)[pi];
-                } else {
-                    const uint32_t v = (J.in + (int64_t)(r >> 1) * np)[pi];
-                    lo[q] = (r & 1) ? v >> 16 : v & 0xFFFFu;
-                }
-            }
-        }
-        auto second = rows;
-        second.shift(copy);
-        if constexpr (sizeof(W) == 8) {
-            *rows.unit_lo(u) = *second.unit_lo(u) = U32x4{lo[0], lo[1], lo[2], lo[3]};
-            *rows.unit_hi(u) = *second.unit_hi(u) = U32x4{hi[0], hi[1], hi[2], hi[3]};
-        } else {
-            *rows.unit(u) = *second.unit(u) = U32x4{lo[0], lo[1], lo[2], lo[3]};
-        }
-    }
+    if constexpr (PL > 4) asm volatile("cp.async.wait_all;" ::: "memory");  // a lane reads only what it copied itself
     const W pm = wlow<W>(mp), cm = wlow<W>(mc), block = pm & ~cm;
     Work<W> c = a;
     const W xc = both ? x ^ (W)J.gen[0] : x;
     a.sum = alive ? (x ^ a.s.h) & block : (W)0;  // the others of the block are set to 0
     c.sum = (alive && both) ? (xc ^ c.s.h) & block : (W)0;
-    auto two = rows;
-    two.shift(copy);
     if constexpr (PAIRS) {
         const int hi = J.paired < mp ? J.paired : mp;
         const W pm2 = wlow<W>(hi) & block;  // the block's paired positions
@@ -313,60 +356,10 @@ __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStag
         a.live = cm | a.sum;
         c.live = cm | c.sum;
     }
-    contract_pair(rows, copy, a, c, mc);
+    contract_pair<PL>(rows, copy, a, c, mc);
     if (!valid) return;
-    const uint32_t sa = pack_status(a.s.q, a.s.iso, a.s.dead), sc = pack_status(c.s.q, c.s.iso, c.s.dead);
-    uint32_t* const out = J.out;
-    const int64_t nc = J.count;
-    if (!both) {  // (a code without rows: one node per state)
-        for (int r = 0; r < mc; r++) store_row(out, nc, i, mc, r, (uint64_t)(rows.get(r) & cm));
-        store_scalars(out, nc, i, mc, (uint64_t)(a.s.d1 & cm), (uint64_t)(a.s.d2 & cm), (uint64_t)(a.s.h & cm),
-                      (uint64_t)(x & cm), sa);
-        return;
-    }
-    const uint32_t at = 2u * i;
-    if (!(a.s.dead && c.s.dead)) {
-        if (mc > 32) {
-            for (int r = 0; r < mc; r++) {
-                const uint64_t v = (uint64_t)(rows.get(r) & cm), w = (uint64_t)(two.get(r) & cm);
-                store_two(out + (int64_t)(2 * r) * nc, at, (uint32_t)v, (uint32_t)w);
-                store_two(out + (int64_t)(2 * r + 1) * nc, at, (uint32_t)(v >> 32), (uint32_t)(w >> 32));
-            }
-        } else if (mc > 16) {
-            for (int r = 0; r < mc; r++)
-                store_two(out + (int64_t)r * nc, at, (uint32_t)(rows.get(r) & cm), (uint32_t)(two.get(r) & cm));
-        } else {
-            for (int r = 0; r < mc; r += 2) {  // row mc, if mc is odd, lies within the parent's and is cleared by cm's bits
-                const uint32_t hi = r + 1 < mc ? 0xFFFFFFFFu : 0xFFFFu;
-                const uint32_t v = (uint32_t)(rows.get(r) & cm) | ((uint32_t)(rows.get(r + 1 < mc ? r + 1 : r) & cm) << 16);
-                const uint32_t w = (uint32_t)(two.get(r) & cm) | ((uint32_t)(two.get(r + 1 < mc ? r + 1 : r) & cm) << 16);
-                store_two(out + (int64_t)(r >> 1) * nc, at, v & hi, w & hi);
-            }
-        }
-    }
-    uint32_t* p = out + (int64_t)node_row_words(mc) * nc;
-    const W xa = x & cm, xb = xc & cm;
-    if (mc > 32) {
-        const W va[4] = {a.s.d1 & cm, a.s.d2 & cm, a.s.h & cm, xa}, vc[4] = {c.s.d1 & cm, c.s.d2 & cm, c.s.h & cm, xb};
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            store_two(p + (int64_t)(2 * q) * nc, at, (uint32_t)va[q], (uint32_t)vc[q]);
-            store_two(p + (int64_t)(2 * q + 1) * nc, at, (uint32_t)((uint64_t)va[q] >> 32),
-                      (uint32_t)((uint64_t)vc[q] >> 32));
-        }
-        store_two(p + 8 * nc, at, sa, sc);
-    } else if (mc > 16) {
-        store_two(p, at, (uint32_t)(a.s.d1 & cm), (uint32_t)(c.s.d1 & cm));
-        store_two(p + nc, at, (uint32_t)(a.s.d2 & cm), (uint32_t)(c.s.d2 & cm));
-        store_two(p + 2 * nc, at, (uint32_t)(a.s.h & cm), (uint32_t)(c.s.h & cm));
-        store_two(p + 3 * nc, at, (uint32_t)xa, (uint32_t)xb);
-        store_two(p + 4 * nc, at, sa, sc);
-    } else {
-        store_two(p, at, (uint32_t)(a.s.d1 & cm) | ((uint32_t)(a.s.d2 & cm) << 16),
-                  (uint32_t)(c.s.d1 & cm) | ((uint32_t)(c.s.d2 & cm) << 16));
-        store_two(p + nc, at, (uint32_t)(a.s.h & cm) | ((uint32_t)xa << 16), (uint32_t)(c.s.h & cm) | ((uint32_t)xb << 16));
-        store_two(p + 2 * nc, at, sa, sc);
-    }
+    store_node<PL, W>(J.out, J.count, both ? 2u * i : i, mc, rows, units, a.s, x);
+    if (both) store_node<PL, W>(J.out, J.count, 2u * i + 1u, mc, two, units, c.s, xc);
 }
 
 // ---------------------------------------------------------------- leaves
@@ -390,8 +383,8 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
     __syncthreads();
     const int m = J.m, tv = J.tv;
     const int64_t ti = ((int64_t)blockIdx.x - J.block0) * kTreeLeafThreads + tid;  // thread of the job
-    const size_t copy = 8 * kTreeLeafThreads;
-    const Rows16 rows{wrows + 4 * tid, kTreeLeafThreads}, rows2{wrows + copy + 4 * tid, kTreeLeafThreads};
+    const size_t copy = Rows<2>::words(4, kTreeLeafThreads);
+    const Rows<2> rows = Rows<2>::at(wrows, tid, 4, kTreeLeafThreads), rows2 = Rows<2>::at(wrows + copy, tid, 4, kTreeLeafThreads);
     const uint32_t mm = wlow<uint32_t>(m), vm = wlow<uint32_t>(tv);
     const int64_t np = J.in_count;
     // a part's levels: table nodes, and leaves of a table (fewer than 2^tj if the part is smaller)
@@ -401,14 +394,13 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
         const int64_t part = ((int64_t)blockIdx.x - J.block0) * kTreeLeafThreads * J.reps + rep * kTreeLeafThreads + tid;
         const bool valid = ti < J.threads;
         const int64_t node = valid ? part >> J.split : 0;
-        const uint32_t* const p = J.in + (int64_t)((m + 1) / 2) * np + node;
-        const uint32_t status = p[2 * np];
+        const uint4* const p = reinterpret_cast<const uint4*>(J.in) + node;
+        const uint4 sc = *p;
+        const uint32_t dd = sc.x, hx = sc.y, status = sc.z;
         const bool alive = valid && !(status & 0x80000000u);
         if (!uniform_any(alive)) continue;
-        uint32_t w[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) w[q] = (2 * q < m && alive) ? J.in[(int64_t)q * np + node] : 0u;
-        const uint32_t dd = p[0], hx = p[np];
+        const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+        const uint4 w0 = alive && m > 0 ? p[np] : none, w1 = alive && m > 8 ? p[2 * np] : none;
         const int iso0 = (int)((status >> 8) & 0xFFu);
         uint32_t x = hx >> 16;
         for (int b = 0; b < J.split; b++)
@@ -433,8 +425,8 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
             wa.s = Node<uint32_t>{dd & 0xFFFFu, dd >> 16, hx & 0xFFFFu, (int)(status & 7u), 0, 0};
             wb = wa;
             if (m > tv) {
-                *rows.unit(0) = *rows2.unit(0) = U32x4{w[0], w[1], w[2], w[3]};
-                if (m > 8) *rows.unit(1) = *rows2.unit(1) = U32x4{w[4], w[5], w[6], w[7]};
+                *rows.chunk(0) = *rows2.chunk(0) = U32x4{w0.x, w0.y, w0.z, w0.w};
+                if (m > 8) *rows.chunk(1) = *rows2.chunk(1) = U32x4{w1.x, w1.y, w1.z, w1.w};
                 if constexpr (PAIRS) {  // every position below paired is a pair's, a single qubit above them
                     const uint32_t pm = wlow<uint32_t>(m & ~1);
                     wa.sum = alive ? (x ^ wa.s.h) & mm & ~pm : 0u;
@@ -461,9 +453,13 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
                 nd.q = e ? wb.s.q : wa.s.q;
                 nd.iso = e ? wb.s.iso : wa.s.iso;
                 nd.dead = e ? wb.s.dead : wa.s.dead;
-                U32x4 u = U32x4{w[0], w[1], w[2], w[3]};
-                if (m > tv) u = e ? *rows2.unit(0) : *rows.unit(0);
-                const uint32_t r[kTableVars] = {u.a, u.a >> 16, u.b, u.b >> 16, u.c, u.c >> 16, u.d, u.d >> 16};
+                uint32_t r0 = w0.x, r4 = w0.z;  // rows 0..3 and 4..7, a byte each
+                if (m > tv) {
+                    const U32x4 u = e ? *rows2.chunk(0) : *rows.chunk(0);
+                    r0 = u.a;
+                    r4 = u.c;
+                }
+                const uint32_t r[kTableVars] = {r0, r0 >> 8, r0 >> 16, r0 >> 24, r4, r4 >> 8, r4 >> 16, r4 >> 24};
                 const uint32_t d1 = nd.d1 & vm;
                 Table<WORDS> tb;
                 build_table<WORDS>(r, d1, nd.d2 & vm, lin, tb);
@@ -596,14 +592,31 @@ int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax,
+namespace {
+template <bool PAIRS>
+void (*stage_kernel(int planes))(const TreeStageJob*, int) {
+    switch (planes) {
+    case 2: return k_tree_stage<2, PAIRS>;
+    case 3: return k_tree_stage<3, PAIRS>;
+    case 4: return k_tree_stage<4, PAIRS>;
+    case 5: return k_tree_stage<5, PAIRS>;
+    case 6: return k_tree_stage<6, PAIRS>;
+    case 7: return k_tree_stage<7, PAIRS>;
+    case 8: return k_tree_stage<8, PAIRS>;
+    default: return nullptr;
+    }
+}
+}  // namespace
+
+int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, int planes, int mmax,
                       bool pairs) {
     if (njobs <= 0 || blocks <= 0) return 0;
-    if (blocks > 0x7fffffff || mmax < 1 || mmax > (wide ? 64 : 32)) return -1;
+    const auto kernel = pairs ? stage_kernel<true>(planes) : stage_kernel<false>(planes);
+    if (blocks > 0x7fffffff || !kernel || mmax < 1 || row_planes(mmax) != planes) return -1;
     // two copies of every lane's rows: at most 64 KB
-    const size_t smem = 2 * (size_t)((mmax + 3) / 4) * 16 * kTreeStageThreads * (wide ? 2 : 1);
-    const auto kernel = wide ? (pairs ? k_tree_stage<uint64_t, true> : k_tree_stage<uint64_t, false>)
-                             : (pairs ? k_tree_stage<uint32_t, true> : k_tree_stage<uint32_t, false>);
+    const int units = row_units(mmax);
+    const int chunks = planes == 2 ? Rows<2>::chunks(units) : units;
+    const size_t smem = (size_t)2 * 4 * (4 * chunks + row_tail(mmax) * units) * kTreeStageThreads;
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess)
         return -1;

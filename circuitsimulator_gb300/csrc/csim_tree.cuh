@@ -45,36 +45,20 @@ using pc::wbit;
 using pc::wlow;
 using pc::wmask;
 
-// The four bits of a nibble as the bytes 0 or 1 of a word (one multiply puts bit
-// i at bit 8 i).  A row update is then v ^ P * bit ^ R * bit: the products run on
-// the FMA pipe and one three-input XOR takes them in, where masking P and R takes
-// two logic ops (the ALU pipe is the busy one: 90% in a stage).
-CSIM_HD_INLINE uint32_t row_bits(uint32_t nib) { return (nib * 0x00204081u) & 0x01010101u; }
-// all-ones masks of the four rows of a unit (one prmt per row replicates a sign)
-CSIM_HD_INLINE void row_masks(uint32_t nib, uint32_t (&m)[4]) {
+// A byte mask of the bits of a nibble: byte q is 0xFF if bit q is set (one multiply
+// puts bit q at the sign of byte q, one prmt replicates the signs)
+CSIM_HD_INLINE uint32_t byte_mask(uint32_t nib) {
 #ifdef __CUDA_ARCH__
-    const uint32_t s = nib * 0x10204080u;
-    asm("prmt.b32 %0, %1, 0, 0x8888;" : "=r"(m[0]) : "r"(s));
-    asm("prmt.b32 %0, %1, 0, 0x9999;" : "=r"(m[1]) : "r"(s));
-    asm("prmt.b32 %0, %1, 0, 0xAAAA;" : "=r"(m[2]) : "r"(s));
-    asm("prmt.b32 %0, %1, 0, 0xBBBB;" : "=r"(m[3]) : "r"(s));
+    uint32_t m;
+    asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(m) : "r"(nib * 0x10204080u));
+    return m;
 #else
-    for (int i = 0; i < 4; i++) m[i] = (nib >> i) & 1u ? ~0u : 0u;
+    uint32_t m = 0;
+    for (int q = 0; q < 4; q++) m |= ((nib >> q) & 1u ? 0xFFu : 0u) << (8 * q);
+    return m;
 #endif
 }
-// the same for rows of 16 bits, two to a word (row 2i in the low half)
-CSIM_HD_INLINE void half_masks(uint32_t nib, uint32_t& m01, uint32_t& m23) {
-#ifdef __CUDA_ARCH__
-    const uint32_t s = nib * 0x10204080u;
-    asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(m01) : "r"(s));
-    asm("prmt.b32 %0, %1, 0, 0xBBAA;" : "=r"(m23) : "r"(s));
-#else
-    m01 = ((nib & 1u) ? 0xFFFFu : 0u) | ((nib & 2u) ? 0xFFFF0000u : 0u);
-    m23 = ((nib & 4u) ? 0xFFFFu : 0u) | ((nib & 8u) ? 0xFFFF0000u : 0u);
-#endif
-}
-
-// byte i of w, zero-extended
+// byte i of w: zero-extended, and in all four bytes
 CSIM_HD_INLINE uint32_t pick_byte(uint32_t w, int i) {
 #ifdef __CUDA_ARCH__
     return __byte_perm(w, 0u, 0x4440u | (unsigned)i);
@@ -82,94 +66,156 @@ CSIM_HD_INLINE uint32_t pick_byte(uint32_t w, int i) {
     return (w >> (8 * i)) & 0xFFu;
 #endif
 }
+CSIM_HD_INLINE uint32_t repeat_byte(uint32_t w, int i) {
+#ifdef __CUDA_ARCH__
+    return __byte_perm(w, 0u, 0x1111u * (unsigned)i);
+#else
+    return ((w >> (8 * i)) & 0xFFu) * 0x01010101u;
+#endif
+}
+// byte q of each of four words, as a word
+CSIM_HD_INLINE uint32_t gather_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d, int q) {
+#ifdef __CUDA_ARCH__
+    const unsigned sel = 0x40u + 0x11u * (unsigned)q;
+    return __byte_perm(__byte_perm(a, b, sel), __byte_perm(c, d, sel), 0x5410u);
+#else
+    return pick_byte(a, q) | (pick_byte(b, q) << 8) | (pick_byte(c, q) << 16) | (pick_byte(d, q) << 24);
+#endif
+}
 
-// One thread's J rows in memory laid out [unit][thread], 16-byte units `st`
-// units apart.  rank2(n, U, P, V, R): row x ^= (x in U ? P : 0) ^ (x in V ? R : 0)
-// for the rows x < n (whole units; rows past n hold nothing that is read).
-struct Rows32 {  // four 32-bit rows to a unit
-    uint32_t* p;
+// Byte planes of m-bit rows: 2 (at least) to 8
+CSIM_HD_INLINE int row_planes(int m) { return m <= 16 ? 2 : (m + 7) / 8; }
+CSIM_HD_INLINE int row_units(int m) { return (m + 3) / 4; }
+
+// One thread's J rows, four to a unit, as byte planes: plane k of unit u is a word
+// whose byte q is byte k of row 4 u + q.  A rank-two update of a unit is then two
+// byte masks (of the rows in U, of those in V) and two logic ops per plane, for as
+// many planes as the rows have bytes; with a word per row it was two masks and three
+// or four ops per row, and two words per row from 33 vertices up.  Stage 22 -> 13
+// vertices: 3,425 instructions per warp and pair of nodes before.
+// Memory is laid out [16-byte chunk][thread]: a chunk holds planes 0..3 of a unit, or
+// (two planes) those of two units.  Planes from 4 up follow as [unit][thread] tails of
+// no more words than they need: shared memory limits the blocks per SM from 33
+// vertices up.  Consecutive chunks (tails) of a lane are `st` chunks (tails) apart.
+template <int PL>
+struct Rows {
+    static constexpr int tail = PL <= 4 ? 0 : (PL == 5 ? 1 : (PL == 6 ? 2 : 4));  // words
+    uint32_t *p, *tp;  // this lane's first chunk, first tail
     int st;
-    CSIM_HD_INLINE uint32_t get(int i) const { return p[(size_t)(i >> 2) * 4 * st + (i & 3)]; }
-    CSIM_HD_INLINE U32x4* unit(int u) const { return reinterpret_cast<U32x4*>(p + (size_t)u * 4 * st); }
-    CSIM_HD_INLINE void shift(size_t words) { p += words; }
-    CSIM_HD_INLINE void rank2(int n, uint32_t U, uint32_t P, uint32_t V, uint32_t R) const {
-        // nibble u of a mask: byte u/2 of its even or odd nibbles
-        const uint32_t Ue = U & 0x0F0F0F0Fu, Uo = (U >> 4) & 0x0F0F0F0Fu, Ve = V & 0x0F0F0F0Fu, Vo = (V >> 4) & 0x0F0F0F0Fu;
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (4 * u >= n) break;
-            U32x4 v = *unit(u);
-            const uint32_t a = row_bits(pick_byte((u & 1) ? Uo : Ue, u >> 1));
-            const uint32_t b = row_bits(pick_byte((u & 1) ? Vo : Ve, u >> 1));
-            v.a = v.a ^ (P * pick_byte(a, 0)) ^ (R * pick_byte(b, 0));
-            v.b = v.b ^ (P * pick_byte(a, 1)) ^ (R * pick_byte(b, 1));
-            v.c = v.c ^ (P * pick_byte(a, 2)) ^ (R * pick_byte(b, 2));
-            v.d = v.d ^ (P * (a >> 24)) ^ (R * (b >> 24));
-            *unit(u) = v;
-        }
+    CSIM_HD static int chunks(int units) { return PL == 2 ? (units + 1) / 2 : units; }
+    // words a copy of `units` units takes in a block of `st` threads
+    CSIM_HD static size_t words(int units, int st) { return (size_t)(4 * chunks(units) + tail * units) * st; }
+    CSIM_HD static Rows at(uint32_t* base, int lane, int units, int st) {
+        return Rows{base + 4 * lane, base + (size_t)4 * chunks(units) * st + tail * lane, st};
     }
-};
-struct Rows64 {  // low and high halves of four rows in a unit each
-    uint32_t *lo, *hi;
-    int st;
-    CSIM_HD_INLINE uint64_t get(int i) const {
-        const size_t o = (size_t)(i >> 2) * 4 * st + (i & 3);
-        return (uint64_t)lo[o] | ((uint64_t)hi[o] << 32);
-    }
+    CSIM_HD_INLINE U32x4* chunk(int i) const { return reinterpret_cast<U32x4*>(p + (size_t)i * 4 * st); }
+    CSIM_HD_INLINE uint32_t* tails(int u) const { return tp + (size_t)u * tail * st; }
     CSIM_HD_INLINE void shift(size_t words) {
-        lo += words;
-        hi += words;
+        p += words;
+        tp += words;
     }
-    CSIM_HD_INLINE U32x4* unit_lo(int u) const { return reinterpret_cast<U32x4*>(lo + (size_t)u * 4 * st); }
-    CSIM_HD_INLINE U32x4* unit_hi(int u) const { return reinterpret_cast<U32x4*>(hi + (size_t)u * 4 * st); }
+    // planes 4 .. PL - 1 of unit u
+    CSIM_HD_INLINE U32x4 get_tail(int u) const {
+        if constexpr (tail == 1) return U32x4{*tails(u), 0u, 0u, 0u};
+        else if constexpr (tail == 2) {
+            const uint64_t v = *reinterpret_cast<const uint64_t*>(tails(u));
+            return U32x4{(uint32_t)v, (uint32_t)(v >> 32), 0u, 0u};
+        } else
+            return *reinterpret_cast<const U32x4*>(tails(u));
+    }
+    CSIM_HD_INLINE void set_tail(int u, const U32x4& v) const {
+        if constexpr (tail == 1) *tails(u) = v.a;
+        else if constexpr (tail == 2) *reinterpret_cast<uint64_t*>(tails(u)) = (uint64_t)v.a | ((uint64_t)v.b << 32);
+        else *reinterpret_cast<U32x4*>(tails(u)) = v;
+    }
+    // row i; bits from 8 PL up (PL = 2, 3) are not the row's
+    CSIM_HD_INLINE uint64_t get(int i) const {
+        const int u = i >> 2, q = i & 3;
+        if constexpr (PL == 2) {
+            const uint32_t* w = p + (size_t)(u >> 1) * 4 * st + 2 * (u & 1);
+            return gather_bytes(w[0], w[1], 0u, 0u, q);
+        } else {
+            const U32x4 v = *chunk(u);
+            const uint32_t lo = gather_bytes(v.a, v.b, v.c, v.d, q);
+            if constexpr (PL <= 4) return lo;
+            else if constexpr (tail == 1) return (uint64_t)lo | ((uint64_t)pick_byte(*tails(u), q) << 32);
+            else {
+                const U32x4 w = get_tail(u);
+                return (uint64_t)lo | ((uint64_t)gather_bytes(w.a, w.b, w.c, w.d, q) << 32);
+            }
+        }
+    }
+    // row x ^= (x in U ? P : 0) ^ (x in V ? R : 0) for the rows x < n (whole units; rows past
+    // n hold nothing that is read)
     CSIM_HD_INLINE void rank2(int n, uint64_t U, uint64_t P, uint64_t V, uint64_t R) const {
-        const uint32_t Pl = (uint32_t)P, Ph = (uint32_t)(P >> 32), Rl = (uint32_t)R, Rh = (uint32_t)(R >> 32);
-        for (int u = 0; 4 * u < n; u++) {
-            U32x4 a = *unit_lo(u), b = *unit_hi(u);
-            uint32_t mu[4], mv[4];
-            row_masks((uint32_t)U & 15u, mu);
-            row_masks((uint32_t)V & 15u, mv);
-            a.a ^= (Pl & mu[0]) ^ (Rl & mv[0]);
-            a.b ^= (Pl & mu[1]) ^ (Rl & mv[1]);
-            a.c ^= (Pl & mu[2]) ^ (Rl & mv[2]);
-            a.d ^= (Pl & mu[3]) ^ (Rl & mv[3]);
-            b.a ^= (Ph & mu[0]) ^ (Rh & mv[0]);
-            b.b ^= (Ph & mu[1]) ^ (Rh & mv[1]);
-            b.c ^= (Ph & mu[2]) ^ (Rh & mv[2]);
-            b.d ^= (Ph & mu[3]) ^ (Rh & mv[3]);
-            *unit_lo(u) = a;
-            *unit_hi(u) = b;
-            U >>= 4;
-            V >>= 4;
+        uint32_t pk[PL], rk[PL];
+#pragma unroll
+        for (int k = 0; k < PL; k++) {
+            pk[k] = repeat_byte((uint32_t)(k < 4 ? P : P >> 32), k & 3);
+            rk[k] = repeat_byte((uint32_t)(k < 4 ? R : R >> 32), k & 3);
+        }
+        // nibble u of a mask: byte u / 2 of its even or odd nibbles
+        constexpr uint64_t nibs = 0x0F0F0F0F0F0F0F0Full;
+        const uint64_t ue = U & nibs, uo = (U >> 4) & nibs, ve = V & nibs, vo = (V >> 4) & nibs;
+#pragma unroll
+        for (int u = 0; u < 2 * PL; u += 2) {  // two units at a time
+            if (4 * u >= n) break;
+            const uint32_t me = byte_mask(pick_byte((uint32_t)(u < 8 ? ue : ue >> 32), (u >> 1) & 3)),
+                           mo = byte_mask(pick_byte((uint32_t)(u < 8 ? uo : uo >> 32), (u >> 1) & 3)),
+                           ne = byte_mask(pick_byte((uint32_t)(u < 8 ? ve : ve >> 32), (u >> 1) & 3)),
+                           no = byte_mask(pick_byte((uint32_t)(u < 8 ? vo : vo >> 32), (u >> 1) & 3));
+            if constexpr (PL == 2) {
+                U32x4 v = *chunk(u >> 1);
+                v.a ^= (me & pk[0]) ^ (ne & rk[0]);
+                v.b ^= (me & pk[1]) ^ (ne & rk[1]);
+                v.c ^= (mo & pk[0]) ^ (no & rk[0]);
+                v.d ^= (mo & pk[1]) ^ (no & rk[1]);
+                *chunk(u >> 1) = v;
+            } else {
+                update(u, me, ne, pk, rk);
+                if (4 * (u + 1) < n) update(u + 1, mo, no, pk, rk);
+            }
+        }
+    }
+
+  private:
+    CSIM_HD_INLINE void update(int u, uint32_t mu, uint32_t mv, const uint32_t (&pk)[PL], const uint32_t (&rk)[PL]) const {
+        U32x4 v = *chunk(u);
+        v.a ^= (mu & pk[0]) ^ (mv & rk[0]);
+        v.b ^= (mu & pk[1]) ^ (mv & rk[1]);
+        if constexpr (PL > 2) v.c ^= (mu & pk[2]) ^ (mv & rk[2]);
+        if constexpr (PL > 3) v.d ^= (mu & pk[3]) ^ (mv & rk[3]);
+        *chunk(u) = v;
+        if constexpr (PL > 4) {
+            U32x4 w = get_tail(u);
+            w.a ^= (mu & pk[4]) ^ (mv & rk[4]);
+            if constexpr (PL > 5) w.b ^= (mu & pk[5]) ^ (mv & rk[5]);
+            if constexpr (PL > 6) w.c ^= (mu & pk[6]) ^ (mv & rk[6]);
+            if constexpr (PL > 7) w.d ^= (mu & pk[7]) ^ (mv & rk[7]);
+            set_tail(u, w);
         }
     }
 };
-struct Rows16 {  // eight 16-bit rows to a unit
-    uint32_t* p;
-    int st;
-    CSIM_HD_INLINE uint32_t get(int i) const {
-        return reinterpret_cast<const uint16_t*>(p)[(size_t)(i >> 3) * 8 * st + (i & 7)];
-    }
-    CSIM_HD_INLINE U32x4* unit(int u) const { return reinterpret_cast<U32x4*>(p + (size_t)u * 4 * st); }
-    CSIM_HD_INLINE void shift(size_t words) { p += words; }
-    CSIM_HD_INLINE void rank2(int n, uint32_t U, uint32_t P, uint32_t V, uint32_t R) const {
-        const uint32_t PP = P * 0x10001u, RR = R * 0x10001u;
-        for (int u = 0; 8 * u < n; u++) {
-            U32x4 v = *unit(u);
-            uint32_t u0, u1, u2, u3, v0, v1, v2, v3;
-            half_masks(U & 15u, u0, u1);
-            half_masks((U >> 4) & 15u, u2, u3);
-            half_masks(V & 15u, v0, v1);
-            half_masks((V >> 4) & 15u, v2, v3);
-            v.a ^= (PP & u0) ^ (RR & v0);
-            v.b ^= (PP & u1) ^ (RR & v1);
-            v.c ^= (PP & u2) ^ (RR & v2);
-            v.d ^= (PP & u3) ^ (RR & v3);
-            *unit(u) = v;
-            U >>= 8;
-            V >>= 8;
-        }
-    }
+// the word that holds a row of PL bytes
+template <int PL>
+struct RowWord {
+    using type = uint32_t;
+};
+template <>
+struct RowWord<5> {
+    using type = uint64_t;
+};
+template <>
+struct RowWord<6> {
+    using type = uint64_t;
+};
+template <>
+struct RowWord<7> {
+    using type = uint64_t;
+};
+template <>
+struct RowWord<8> {
+    using type = uint64_t;
 };
 
 // The scalar part of a node: bit c of d1, d2, h belongs to vertex c
@@ -178,6 +224,29 @@ struct Node {
     W d1, d2, h;
     int q, iso, dead;  // w^q 2^{iso/2}; dead: the amplitude is 0
 };
+
+// all ones if x is not 0; the highest bit of x, and its index (0 for x = 0)
+template <class W>
+CSIM_HD_INLINE W some(W x) {
+    return wmask<W>(x != (W)0);
+}
+CSIM_HD_INLINE uint32_t top_bit(uint32_t x) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_rc(0x80000000u, 0u, (unsigned)__clz((int)x));  // 0 for a shift by 32
+#else
+    return x ? 0x80000000u >> __builtin_clz(x) : 0u;
+#endif
+}
+CSIM_HD_INLINE uint64_t top_bit(uint64_t x) {
+    const uint32_t hi = (uint32_t)(x >> 32);
+    return hi ? (uint64_t)top_bit(hi) << 32 : (uint64_t)top_bit((uint32_t)x);
+}
+template <class W>
+CSIM_HD_INLINE int top_index(W x) {
+    using T = WordTraits<W>;
+    const int i = T::bits - 1 - T::clz(x);
+    return i < 0 ? 0 : i;
+}
 
 // A node being contracted: the vertices of `sum` are to be summed out (2^{-1/2}
 // sum over z_c each) on the vertices `live` (sum within live; vertices outside
@@ -194,59 +263,47 @@ struct Work {
 // takes c alone).  The rows keep stale bits in the columns of vertices that are
 // gone and on the diagonal: every row is masked by `live` when it is read.  All
 // lanes of a warp call it together; a lane with nothing to sum changes nothing.
+// Written in masks (all ones or zero) and without branches: lanes differ in every
+// condition, and a select by mask is one three-input logic op with what it selects for.
 template <class W, class R>
 CSIM_HD_INLINE void sum_step(const R& rows, Work<W>& w) {
-    using T = WordTraits<W>;
     Node<W>& s = w.s;
-    W sum = w.sum, live = w.live;
-    const bool act = sum != (W)0;
-    const int c = act ? T::bits - 1 - T::clz(sum) : 0;
-    const W mc = act ? wbit<W>(c) : (W)0;
-    sum ^= mc;
-    live &= ~mc;
-    const W N0 = act ? ((W)rows.get(c) & live) : (W)0;
-    const bool odd = (s.d1 & mc) != (W)0, d = (s.d2 & mc) != (W)0;
-    const W near = N0 & sum;
-    const W pick = odd ? sum & (s.d1 ^ N0) : (near != (W)0 ? near : N0);
-    const bool two = pick != (W)0;
-    const int b = two ? T::bits - 1 - T::clz(pick) : 0;
-    const W mb = two ? wbit<W>(b) : (W)0;
-    const W gone = mb & sum;  // a pivot's b that is summed too: its new bit is contracted to 0
+    const W act = some(w.sum), mc = top_bit(w.sum);
+    const W sum1 = w.sum ^ mc, live1 = w.live & ~mc;
+    const W N0 = (W)rows.get(top_index(w.sum)) & live1 & act;
+    const W odd = some(s.d1 & mc), d = some(s.d2 & mc);
+    const W near = N0 & sum1;
+    const W even_pick = near != (W)0 ? near : N0;
+    const W pick = (odd & sum1 & (s.d1 ^ N0)) | (~odd & even_pick);
+    const W two = some(pick), mb = top_bit(pick);
+    const W M0 = (W)rows.get(top_index(pick)) & live1 & ~mb & two;
     const W N = N0 & ~mb;
-    W M = two ? ((W)rows.get(b) & live & ~mb) : (W)0;
-    const bool db1 = (s.d1 & mb) != (W)0;
+    const W db1 = some(s.d1 & mb);
     // D on N: odd adds 6 (d = 0) or 2 (d = 1); a pivot adds D_b's odd part times (1 - 2 d)
-    const W plus = wmask<W>(odd != d);
-    s.d2 ^= (odd ? N0 : (W)0) & mb & (s.d1 ^ plus);  // b's own D after an odd c
-    const bool db2 = (s.d2 & mb) != (W)0;
-    const W wn = (odd || db1) ? N : (W)0;
-    s.d2 ^= wn & (s.d1 ^ plus);
-    s.d1 ^= wn;
-    if (odd) {
-        M ^= (N0 & mb) ? N : (W)0;
-        s.q += (d ? 7 : 1) + (two ? (db2 ? 7 : 1) : 0);
-        s.d2 ^= M & (s.d1 ^ wmask<W>(!db2));
-        s.d1 ^= M;
-    } else {
-        if (act && !two) {
-            s.dead |= d ? 1 : 0;
-            s.iso++;
-        }
-        s.q += d ? (db1 ? 2 : 0) + (db2 ? 4 : 0) : 0;
-        s.d2 ^= (db2 ? N : (W)0) ^ (d ? M : (W)0) ^ (N & M);
-    }
+    const W plus = s.d1 ^ odd ^ d;
+    const W joined = N0 & mb & odd;  // b's own D after an odd c
+    const W d2 = s.d2 ^ (joined & plus);
+    const W db2 = some(d2 & mb);
+    const W wn = N & (odd | db1);
+    const W M = M0 ^ (N & some(joined));
+    const W d1 = s.d1 ^ wn;
+    const W more = (odd & M & (d1 ^ ~db2)) | (~odd & ((N & (db2 ^ M)) ^ (M & d)));
     // a pivot's new bit at b: D = 4 d, neighbourhood N, Hadamard toggled
-    s.d1 &= ~mb;
-    s.d2 = (s.d2 & ~mb) | (d ? mb : (W)0);
+    s.d1 = (d1 ^ (M & odd)) & ~mb;
+    s.d2 = ((d2 ^ (wn & plus) ^ more) & ~mb) | (d & mb);
     s.h ^= mb;
-    sum &= ~mb;
-    live &= ~gone;
+    // w^{1 - 2 d} and, with a second odd vertex, w^{1 - 2 d_b}; a pivot's w^{d D_b}
+    const int o = (int)odd, di = (int)d, b1 = (int)db1, b2 = (int)db2, t = (int)two;
+    s.q += (o & (1 + 2 * di + (t & (1 + 2 * b2)))) - (~o & di & (2 * b1 + 4 * b2));
+    const int lone = (int)act & ~o & ~t;  // an even vertex without neighbours: 2 or 0, times 2^{-1/2}
+    s.dead |= lone & di;
+    s.iso -= lone;
+    w.sum = sum1 & ~mb;
+    w.live = live1 & ~(mb & sum1);  // a b that is summed too is gone: its new bit is contracted to 0
     // odd: rows of N get N, rows of M get M.  Pivot: rows of N get M (and N when D_b is odd),
     // rows of M get N, column b of both changes and row b becomes N
-    const int n = uniform_max(T::bits - T::clz(live));
-    rows.rank2(n, N | mb, odd ? N : M ^ wn ^ mb, M | (db1 ? (W)0 : mb), odd ? M : N ^ mb);
-    w.sum = sum;
-    w.live = live;
+    const int n = uniform_max(WordTraits<W>::bits - WordTraits<W>::clz(w.live));
+    rows.rank2(n, N | mb, wn ^ (~odd & (M ^ mb)), M | (mb & ~db1), (odd & M) | (~odd & (N ^ mb)));
 }
 
 // Steps until no lane has a vertex of `until` left to sum
@@ -305,30 +362,33 @@ CSIM_HD_INLINE void join_pairs(const R& rows, Work<W>& w, W x, int lo, int hi, b
     }
 }
 
-// Sums two sibling nodes down to their first mc vertices.  With rows of two words
-// and mc <= 32 the second words are needed only until the vertices from 32 up are gone.
-CSIM_HD_INLINE void contract_pair(const Rows32& rows, size_t words, Work<uint32_t>& a, Work<uint32_t>& b, int) {
-    sum_out_pair<uint32_t>(rows, words, a, b, ~0u);
-}
-CSIM_HD_INLINE void contract_pair(const Rows64& rows, size_t words, Work<uint64_t>& a, Work<uint64_t>& b, int mc) {
-    if (mc > 32) {
-        sum_out_pair<uint64_t>(rows, words, a, b, ~0ull);
-        return;
+// Sums two sibling nodes down to their first mc vertices.  With more than four
+// planes and mc <= 32 the upper planes are needed only until the vertices from 32
+// up are gone.
+template <int PL, class W>
+CSIM_HD_INLINE void contract_pair(const Rows<PL>& rows, size_t words, Work<W>& a, Work<W>& b, int mc) {
+    if constexpr (PL <= 4) {
+        sum_out_pair<W>(rows, words, a, b, ~(W)0);
+    } else {
+        if (mc > 32) {
+            sum_out_pair<W>(rows, words, a, b, ~(W)0);
+            return;
+        }
+        sum_out_pair<W>(rows, words, a, b, ~(W)0xFFFFFFFFu);
+        auto low = [](const Work<W>& w) {
+            return Work<uint32_t>{{(uint32_t)w.s.d1, (uint32_t)w.s.d2, (uint32_t)w.s.h, w.s.q, w.s.iso, w.s.dead},
+                                  (uint32_t)w.sum, (uint32_t)w.live};
+        };
+        auto back = [](Work<W>& w, const Work<uint32_t>& n) {
+            w.s = Node<W>{n.s.d1, n.s.d2, n.s.h, n.s.q, n.s.iso, n.s.dead};
+            w.sum = n.sum;
+            w.live = n.live;
+        };
+        Work<uint32_t> a32 = low(a), b32 = low(b);
+        sum_out_pair<uint32_t>(Rows<4>{rows.p, rows.tp, rows.st}, words, a32, b32, ~0u);  // without the tails
+        back(a, a32);
+        back(b, b32);
     }
-    sum_out_pair<uint64_t>(rows, words, a, b, ~0xFFFFFFFFull);
-    auto low = [](const Work<uint64_t>& w) {
-        return Work<uint32_t>{{(uint32_t)w.s.d1, (uint32_t)w.s.d2, (uint32_t)w.s.h, w.s.q, w.s.iso, w.s.dead},
-                              (uint32_t)w.sum, (uint32_t)w.live};
-    };
-    auto back = [](Work<uint64_t>& w, const Work<uint32_t>& n) {
-        w.s = Node<uint64_t>{n.s.d1, n.s.d2, n.s.h, n.s.q, n.s.iso, n.s.dead};
-        w.sum = n.sum;
-        w.live = n.live;
-    };
-    Work<uint32_t> a32 = low(a), b32 = low(b);
-    sum_out_pair<uint32_t>(Rows32{rows.lo, rows.st}, words, a32, b32, ~0u);
-    back(a, a32);
-    back(b, b32);
 }
 
 // ---------------------------------------------------------------- the last vertices
@@ -443,14 +503,17 @@ CSIM_HD_INLINE void times_omega(I (&y)[4], int q) {
 }
 
 // ---------------------------------------------------------------- node records
-// Nodes lie in planes of 32-bit words: word w of node i at base[w * count + i].
-// m > 32 vertices: two words per row (low, high), then D1, D2, H, X (two words
-// each), then the status; m > 16: one word per row, then D1, D2, H, X, status;
-// else rows two to a word, then D1 | D2 << 16, H | X << 16, status.  X: the
-// codeword bits of the node's message so far (positions < m are still to come).
-CSIM_HD_INLINE int node_class(int m) { return m > 32 ? 64 : (m > 16 ? 32 : 16); }
-CSIM_HD_INLINE int node_row_words(int m) { return m > 32 ? 2 * m : (m > 16 ? m : (m + 1) / 2); }
-CSIM_HD_INLINE int node_words(int m) { return node_row_words(m) + (m > 32 ? 9 : (m > 16 ? 5 : 3)); }
+// `count` nodes of m vertices lie in planes: first planes of 16-byte vectors, vector v
+// of node i at word 4 (v count + i), then the rows' tails (Rows<row_planes(m)>), tail u
+// of node i at (u count + i) tail words, then (m > 16) a word with the status.  The
+// vectors are the scalars D1, D2, H, X (m > 32: two, D1 D2 and H X, low word first;
+// m <= 16: D1 | D2 << 16, H | X << 16, status, 0) and the rows' chunks.  X: the codeword
+// bits of the node's message so far (positions < m are still to come).  Row and column
+// bits from m up are not zero: whoever reads a row masks it.
+CSIM_HD_INLINE int node_scalars(int m) { return m > 32 ? 2 : 1; }  // vectors
+CSIM_HD_INLINE int node_vectors(int m) { return node_scalars(m) + (m > 16 ? row_units(m) : Rows<2>::chunks(row_units(m))); }
+CSIM_HD_INLINE int row_tail(int m) { return m <= 32 ? 0 : (m <= 40 ? 1 : (m <= 48 ? 2 : 4)); }
+CSIM_HD_INLINE int node_words(int m) { return 4 * node_vectors(m) + row_tail(m) * row_units(m) + (m > 16 ? 1 : 0); }
 CSIM_HD_INLINE uint32_t pack_status(int q, int iso, int dead) {
     return (uint32_t)(q & 7) | ((uint32_t)iso << 8) | (dead ? 0x80000000u : 0u);
 }

@@ -77,8 +77,8 @@ constexpr int kTreeLeafThreads = 128;
 
 // wide: the jobs' states have more than 32 qubits
 int launch_tree_draw(const Launch& L, const TreeRootJob* jobs, int njobs, int64_t blocks, bool wide);
-// wide: the jobs' parents have more than 32 vertices (two words per row); mmax: the largest mp
-int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, bool wide, int mmax,
+// planes: the jobs' parents' byte planes (tree::row_planes(mp)); mmax: the largest mp
+int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int64_t blocks, int planes, int mmax,
                       bool pairs);
 // words: the jobs' table words (tree::table_words(tv)); rows: exactProjector rows; pairs: terms of |H^t> (one word)
 int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words, bool rows,

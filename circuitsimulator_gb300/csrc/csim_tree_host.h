@@ -174,13 +174,14 @@ class TreeRun {
             for (int wide = 0; wide < 2; wide++)
                 if (!roots[wide].empty()) add(blob, Step{0, wide, 0, (int)roots[wide].size(), rb[wide], 0}, roots[wide]);
             for (size_t d = 1; d < depth; d++)
-                for (int kind = 0; kind < 4; kind++) {  // bit 0 wide, bit 1 pairs
+                for (int kind = 2 * 8 + 1; kind >= 2 * 2; kind--) {  // 2 * byte planes + pairs
                     std::vector<csim::TreeStageJob> st;
                     int64_t sb = 0;
                     int mmax = 0;
                     for (const Piece& p : ch.pieces) {
                         const csim::tree::Plan& pl = *p.g.plan;
-                        if (pl.level.size() <= d || (pl.vert[d - 1] > 32) + 2 * pl.pairs != kind) continue;
+                        if (pl.level.size() <= d || 2 * csim::tree::row_planes(pl.vert[d - 1]) + pl.pairs != kind)
+                            continue;
                         csim::TreeStageJob j{};
                         j.in = (const uint32_t*)(scratch + p.off[(d - 1) & 1]);
                         j.out = (uint32_t*)(scratch + p.off[d & 1]);
@@ -213,8 +214,8 @@ class TreeRun {
             if (i == 1 && after_first && cudaEventRecord(after_first, L.stream) != cudaSuccess) return -1;
             const int rc =
                 s.kind == 0   ? csim::launch_tree_draw(L, (const csim::TreeRootJob*)j, s.njobs, s.blocks, s.flags & 1)
-                : s.kind == 1 ? csim::launch_tree_stage(L, (const csim::TreeStageJob*)j, s.njobs, s.blocks, s.flags & 1, s.size,
-                                                          s.flags & 2)
+                : s.kind == 1 ? csim::launch_tree_stage(L, (const csim::TreeStageJob*)j, s.njobs, s.blocks, s.flags >> 1, s.size,
+                                                          s.flags & 1)
                               : csim::launch_tree_leaf(L, (const csim::TreeLeafJob*)j, s.njobs, s.blocks, s.size,
                                                          s.flags & 1, s.flags & 2);
             if (rc) return rc;
@@ -233,7 +234,7 @@ class TreeRun {
     };
     struct Step {
         int kind;  // 0 roots, 1 a stage, 2 leaves
-        int flags;  // roots and stages: bit 0 wide, bit 1 pairs; leaves: bit 0 rows, bit 1 pairs
+        int flags;  // roots: 1 wide; stages: 2 * byte planes + pairs; leaves: bit 0 rows, bit 1 pairs
         int size;   // a stage's largest parent; the leaves' table words
         int njobs;
         int64_t blocks;

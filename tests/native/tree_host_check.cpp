@@ -50,44 +50,44 @@ void join(const R& rows, Work<W>& w, const HostNode& n, int mp, int mc, int pair
     w.live = wlow<W>(mc) | w.sum | pm;
     join_pairs<W>(rows, w, (W)n.x, mc, hi, true);
 }
-// contracts positions [mc, mp) of two siblings with the row type that the
-// kernels use for mp vertices (`leaf`: the leaf kernel's 16-bit rows)
-void stage(HostNode& a, HostNode& b, int mp, int mc, bool leaf, int paired) {
-    alignas(16) uint32_t w[256] = {0};
-    const HostNode* n[2] = {&a, &b};
-    if (leaf) {
-        const Rows16 r0{w, 1}, r1{w + 8, 1};
-        for (int e = 0; e < 2; e++)
-            for (int i = 0; i < mp; i++) reinterpret_cast<uint16_t*>(w + 8 * e)[i] = (uint16_t)n[e]->row[i];
-        auto wa = work_of<uint32_t>(a, mp, mc), wb = work_of<uint32_t>(b, mp, mc);
-        join(r0, wa, a, mp, mc, paired);
-        join(r1, wb, b, mp, mc, paired);
-        sum_out_pair<uint32_t>(r0, 8, wa, wb, ~0u);
-        take(a, wa, r0, mc);
-        take(b, wb, r1, mc);
-    } else if (mp > 32) {
-        const Rows64 r0{w, w + 64, 1}, r1{w + 128, w + 192, 1};
-        for (int e = 0; e < 2; e++)
-            for (int i = 0; i < mp; i++) {
-                w[128 * e + i] = (uint32_t)n[e]->row[i];
-                w[128 * e + 64 + i] = (uint32_t)(n[e]->row[i] >> 32);
-            }
-        auto wa = work_of<uint64_t>(a, mp, mc), wb = work_of<uint64_t>(b, mp, mc);
-        join(r0, wa, a, mp, mc, paired);
-        join(r1, wb, b, mp, mc, paired);
-        contract_pair(r0, 128, wa, wb, mc);
-        take(a, wa, r0, mc);
-        take(b, wb, r1, mc);
-    } else {
-        const Rows32 r0{w, 1}, r1{w + 32, 1};
-        for (int e = 0; e < 2; e++)
-            for (int i = 0; i < mp; i++) w[32 * e + i] = (uint32_t)n[e]->row[i];
-        auto wa = work_of<uint32_t>(a, mp, mc), wb = work_of<uint32_t>(b, mp, mc);
-        join(r0, wa, a, mp, mc, paired);
-        join(r1, wb, b, mp, mc, paired);
-        contract_pair(r0, 32, wa, wb, mc);
-        take(a, wa, r0, mc);
-        take(b, wb, r1, mc);
+// row i of rows laid out as Rows<PL>
+template <int PL>
+void put_row(const Rows<PL>& rows, int i, uint64_t v) {
+    const int u = i >> 2;
+    for (int k = 0; k < PL; k++) {
+        uint32_t* w = PL == 2 ? rows.p + 4 * (u >> 1) + 2 * (u & 1) + k : (k < 4 ? rows.p + 4 * u + k : rows.tails(u) + k - 4);
+        reinterpret_cast<uint8_t*>(w)[i & 3] = (uint8_t)(v >> (8 * k));
+    }
+}
+
+// contracts positions [mc, mp) of two siblings with the rows that the kernels
+// use for mp vertices
+template <int PL>
+void stage_planes(HostNode& a, HostNode& b, int mp, int mc, int paired) {
+    using W = typename RowWord<PL>::type;
+    const size_t copy = (Rows<PL>::words(row_units(mp), 1) + 3) / 4 * 4;  // 16-byte chunks
+    alignas(16) uint32_t w[2 * 16 * 8] = {0};
+    const Rows<PL> r0 = Rows<PL>::at(w, 0, row_units(mp), 1), r1 = Rows<PL>::at(w + copy, 0, row_units(mp), 1);
+    for (int i = 0; i < mp; i++) {
+        put_row(r0, i, a.row[i]);
+        put_row(r1, i, b.row[i]);
+    }
+    auto wa = work_of<W>(a, mp, mc), wb = work_of<W>(b, mp, mc);
+    join(r0, wa, a, mp, mc, paired);
+    join(r1, wb, b, mp, mc, paired);
+    contract_pair<PL>(r0, copy, wa, wb, mc);
+    take(a, wa, r0, mc);
+    take(b, wb, r1, mc);
+}
+void stage(HostNode& a, HostNode& b, int mp, int mc, int paired) {
+    switch (row_planes(mp)) {
+    case 2: return stage_planes<2>(a, b, mp, mc, paired);
+    case 3: return stage_planes<3>(a, b, mp, mc, paired);
+    case 4: return stage_planes<4>(a, b, mp, mc, paired);
+    case 5: return stage_planes<5>(a, b, mp, mc, paired);
+    case 6: return stage_planes<6>(a, b, mp, mc, paired);
+    case 7: return stage_planes<7>(a, b, mp, mc, paired);
+    default: return stage_planes<8>(a, b, mp, mc, paired);
     }
 }
 
@@ -155,7 +155,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
                         if ((c >> b) & 1) n.x ^= p.gen[p.level[s] + b];
                     HostNode o = n;
                     if (sb) o.x ^= p.gen[p.level[s]];
-                    if (!par.dead) stage(n, o, p.vert[s - 1], p.vert[s], false, paired);
+                    if (!par.dead) stage(n, o, p.vert[s - 1], p.vert[s], paired);
                     next.push_back(n);
                     if (sb) next.push_back(o);
                 }
@@ -172,7 +172,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
                 n.x = x;
                 n.iso = 0;
                 HostNode o = n;
-                if (m > p.tv) stage(n, o, m, p.tv, true, paired);
+                if (m > p.tv) stage(n, o, m, p.tv, paired);
                 uint32_t r[kTableVars] = {0};
                 for (int i = 0; i < kTableVars && i < m; i++) r[i] = (uint32_t)n.row[i];
                 const uint32_t vm = wlow<uint32_t>(p.tv), d1 = (uint32_t)n.d1 & vm;
