@@ -371,15 +371,12 @@ __device__ __forceinline__ int64_t shfl_xor_i64(int64_t v, int m) { return (int6
 // ROWS: exactProjector rows, PAIRS: terms of |H^t> (TreeLeafJob).
 template <int WORDS, bool ROWS, bool PAIRS>
 __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(const TreeLeafJob* jobs, int njobs) {
-    __shared__ uint32_t lin[32], sub[32];
+    __shared__ TableWords words;
     __shared__ __align__(16) uint32_t wrows[2 * 8 * kTreeLeafThreads];
     __shared__ int64_t red[kTreeLeafThreads / 32][4];
     const TreeLeafJob& J = job_of(jobs, njobs, blockIdx.x);
     const int tid = threadIdx.x;
-    if (tid < 32) {
-        lin[tid] = linear_word((uint32_t)tid);
-        sub[tid] = subset_word((uint32_t)tid);
-    }
+    if (tid < 32) words.fill(tid);
     __syncthreads();
     const int m = J.m, tv = J.tv;
     const int64_t ti = ((int64_t)blockIdx.x - J.block0) * kTreeLeafThreads + tid;  // thread of the job
@@ -459,10 +456,9 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
                     r0 = u.a;
                     r4 = u.c;
                 }
-                const uint32_t r[kTableVars] = {r0, r0 >> 8, r0 >> 16, r0 >> 24, r4, r4 >> 8, r4 >> 16, r4 >> 24};
                 const uint32_t d1 = nd.d1 & vm;
                 Table<WORDS> tb;
-                build_table<WORDS>(r, d1, nd.d2 & vm, lin, tb);
+                build_table<WORDS>(r0, r4, d1, nd.d2 & vm, words, tb);
                 int evr = 0, evi = 0, odr = 0, odi = 0;
                 uint32_t S = ((e ? x2 : x) ^ nd.h) & vm;
                 // (evr + i evi) + sqrt2 (odr + i odi), times w^q 2^{iso / 2}
@@ -484,11 +480,11 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
                             S ^= J.gen[__ffs(l) - 1] & vm;
                             j ^= (int64_t)J.term[__ffs(l) - 1];
                         }
-                        if (j > row) table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
+                        if (j > row) table_leaf<WORDS>(tb, S, d1, tv, words.sub, evr, evi, odr, odi);
                         if (j == row && alive) {  // one leaf of a state
                             const int keep[4] = {evr, evi, odr, odi};
                             evr = evi = odr = odi = 0;
-                            if (!nd.dead) table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
+                            if (!nd.dead) table_leaf<WORDS>(tb, S, d1, tv, words.sub, evr, evi, odr, odi);
                             node_sum(v);
                             int64_t dz[4];
                             if (iso0 & 1) times_sqrt2(v);
@@ -504,7 +500,7 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
                 } else {
                     for (int l = 0; l < (1 << tj); l++) {
                         if (l) S ^= J.gen[__ffs(l) - 1] & vm;
-                        table_leaf<WORDS>(tb, S, d1, tv, sub, evr, evi, odr, odi);
+                        table_leaf<WORDS>(tb, S, d1, tv, words.sub, evr, evi, odr, odi);
                     }
                 }
                 if (alive && !nd.dead) {

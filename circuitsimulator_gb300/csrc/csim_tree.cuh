@@ -45,20 +45,9 @@ using pc::wbit;
 using pc::wlow;
 using pc::wmask;
 
-// A byte mask of the bits of a nibble: byte q is 0xFF if bit q is set (one multiply
-// puts bit q at the sign of byte q, one prmt replicates the signs)
-CSIM_HD_INLINE uint32_t byte_mask(uint32_t nib) {
-#ifdef __CUDA_ARCH__
-    uint32_t m;
-    asm("prmt.b32 %0, %1, 0, 0xBA98;" : "=r"(m) : "r"(nib * 0x10204080u));
-    return m;
-#else
-    uint32_t m = 0;
-    for (int q = 0; q < 4; q++) m |= ((nib >> q) & 1u ? 0xFFu : 0u) << (8 * q);
-    return m;
-#endif
-}
-// byte i of w: zero-extended, and in all four bytes
+// The bits of a nibble, one to a byte: times a byte, that byte where a bit is set
+CSIM_HD_INLINE uint32_t spread_bits(uint32_t nib) { return (nib * 0x00204081u) & 0x01010101u; }
+// byte i of w
 CSIM_HD_INLINE uint32_t pick_byte(uint32_t w, int i) {
 #ifdef __CUDA_ARCH__
     return __byte_perm(w, 0u, 0x4440u | (unsigned)i);
@@ -66,11 +55,20 @@ CSIM_HD_INLINE uint32_t pick_byte(uint32_t w, int i) {
     return (w >> (8 * i)) & 0xFFu;
 #endif
 }
-CSIM_HD_INLINE uint32_t repeat_byte(uint32_t w, int i) {
+// byte q of a, then byte q of b; the upper half is not 0
+CSIM_HD_INLINE uint32_t pick_bytes(uint32_t a, uint32_t b, int q) {
 #ifdef __CUDA_ARCH__
-    return __byte_perm(w, 0u, 0x1111u * (unsigned)i);
+    return __byte_perm(a, b, 0x40u + 0x11u * (unsigned)q);
 #else
-    return ((w >> (8 * i)) & 0xFFu) * 0x01010101u;
+    return ((a >> (8 * q)) & 0xFFu) | (((b >> (8 * q)) & 0xFFu) << 8);
+#endif
+}
+// w with byte q of c as its third byte; the fourth is not 0
+CSIM_HD_INLINE uint32_t set_third(uint32_t w, uint32_t c, int q) {
+#ifdef __CUDA_ARCH__
+    return __byte_perm(w, c, 0x0410u + 0x100u * (unsigned)q);
+#else
+    return (w & 0xFFFFu) | (((c >> (8 * q)) & 0xFFu) << 16);
 #endif
 }
 // byte q of each of four words, as a word
@@ -89,10 +87,10 @@ CSIM_HD_INLINE int row_units(int m) { return (m + 3) / 4; }
 
 // One thread's J rows, four to a unit, as byte planes: plane k of unit u is a word
 // whose byte q is byte k of row 4 u + q.  A rank-two update of a unit is then two
-// byte masks (of the rows in U, of those in V) and two logic ops per plane, for as
-// many planes as the rows have bytes; with a word per row it was two masks and three
-// or four ops per row, and two words per row from 33 vertices up.  Stage 22 -> 13
-// vertices: 3,425 instructions per warp and pair of nodes before.
+// words of a bit per byte (the rows in U, those in V), their products with a byte of
+// each pattern and one three-input XOR per plane, for as many planes as the rows have
+// bytes.  The products run on the multiply-add pipe beside the logic ops: byte masks and
+// two logic ops per plane are 2 to 3% slower, a word per row 3 to 10% (t = 32 to 57).
 // Memory is laid out [16-byte chunk][thread]: a chunk holds planes 0..3 of a unit, or
 // (two planes) those of two units.  Planes from 4 up follow as [unit][thread] tails of
 // no more words than they need: shared memory limits the blocks per SM from 33
@@ -133,9 +131,10 @@ struct Rows {
         const int u = i >> 2, q = i & 3;
         if constexpr (PL == 2) {
             const uint32_t* w = p + (size_t)(u >> 1) * 4 * st + 2 * (u & 1);
-            return gather_bytes(w[0], w[1], 0u, 0u, q);
+            return pick_bytes(w[0], w[1], q);
         } else {
             const U32x4 v = *chunk(u);
+            if constexpr (PL == 3) return set_third(pick_bytes(v.a, v.b, q), v.c, q);
             const uint32_t lo = gather_bytes(v.a, v.b, v.c, v.d, q);
             if constexpr (PL <= 4) return lo;
             else if constexpr (tail == 1) return (uint64_t)lo | ((uint64_t)pick_byte(*tails(u), q) << 32);
@@ -151,8 +150,8 @@ struct Rows {
         uint32_t pk[PL], rk[PL];
 #pragma unroll
         for (int k = 0; k < PL; k++) {
-            pk[k] = repeat_byte((uint32_t)(k < 4 ? P : P >> 32), k & 3);
-            rk[k] = repeat_byte((uint32_t)(k < 4 ? R : R >> 32), k & 3);
+            pk[k] = pick_byte((uint32_t)(k < 4 ? P : P >> 32), k & 3);
+            rk[k] = pick_byte((uint32_t)(k < 4 ? R : R >> 32), k & 3);
         }
         // nibble u of a mask: byte u / 2 of its even or odd nibbles
         constexpr uint64_t nibs = 0x0F0F0F0F0F0F0F0Full;
@@ -160,16 +159,16 @@ struct Rows {
 #pragma unroll
         for (int u = 0; u < 2 * PL; u += 2) {  // two units at a time
             if (4 * u >= n) break;
-            const uint32_t me = byte_mask(pick_byte((uint32_t)(u < 8 ? ue : ue >> 32), (u >> 1) & 3)),
-                           mo = byte_mask(pick_byte((uint32_t)(u < 8 ? uo : uo >> 32), (u >> 1) & 3)),
-                           ne = byte_mask(pick_byte((uint32_t)(u < 8 ? ve : ve >> 32), (u >> 1) & 3)),
-                           no = byte_mask(pick_byte((uint32_t)(u < 8 ? vo : vo >> 32), (u >> 1) & 3));
+            const uint32_t me = spread_bits(pick_byte((uint32_t)(u < 8 ? ue : ue >> 32), (u >> 1) & 3)),
+                           mo = spread_bits(pick_byte((uint32_t)(u < 8 ? uo : uo >> 32), (u >> 1) & 3)),
+                           ne = spread_bits(pick_byte((uint32_t)(u < 8 ? ve : ve >> 32), (u >> 1) & 3)),
+                           no = spread_bits(pick_byte((uint32_t)(u < 8 ? vo : vo >> 32), (u >> 1) & 3));
             if constexpr (PL == 2) {
                 U32x4 v = *chunk(u >> 1);
-                v.a ^= (me & pk[0]) ^ (ne & rk[0]);
-                v.b ^= (me & pk[1]) ^ (ne & rk[1]);
-                v.c ^= (mo & pk[0]) ^ (no & rk[0]);
-                v.d ^= (mo & pk[1]) ^ (no & rk[1]);
+                v.a ^= (me * pk[0]) ^ (ne * rk[0]);
+                v.b ^= (me * pk[1]) ^ (ne * rk[1]);
+                v.c ^= (mo * pk[0]) ^ (no * rk[0]);
+                v.d ^= (mo * pk[1]) ^ (no * rk[1]);
                 *chunk(u >> 1) = v;
             } else {
                 update(u, me, ne, pk, rk);
@@ -181,17 +180,17 @@ struct Rows {
   private:
     CSIM_HD_INLINE void update(int u, uint32_t mu, uint32_t mv, const uint32_t (&pk)[PL], const uint32_t (&rk)[PL]) const {
         U32x4 v = *chunk(u);
-        v.a ^= (mu & pk[0]) ^ (mv & rk[0]);
-        v.b ^= (mu & pk[1]) ^ (mv & rk[1]);
-        if constexpr (PL > 2) v.c ^= (mu & pk[2]) ^ (mv & rk[2]);
-        if constexpr (PL > 3) v.d ^= (mu & pk[3]) ^ (mv & rk[3]);
+        v.a ^= (mu * pk[0]) ^ (mv * rk[0]);
+        v.b ^= (mu * pk[1]) ^ (mv * rk[1]);
+        if constexpr (PL > 2) v.c ^= (mu * pk[2]) ^ (mv * rk[2]);
+        if constexpr (PL > 3) v.d ^= (mu * pk[3]) ^ (mv * rk[3]);
         *chunk(u) = v;
         if constexpr (PL > 4) {
             U32x4 w = get_tail(u);
-            w.a ^= (mu & pk[4]) ^ (mv & rk[4]);
-            if constexpr (PL > 5) w.b ^= (mu & pk[5]) ^ (mv & rk[5]);
-            if constexpr (PL > 6) w.c ^= (mu & pk[6]) ^ (mv & rk[6]);
-            if constexpr (PL > 7) w.d ^= (mu & pk[7]) ^ (mv & rk[7]);
+            w.a ^= (mu * pk[4]) ^ (mv * rk[4]);
+            if constexpr (PL > 5) w.b ^= (mu * pk[5]) ^ (mv * rk[5]);
+            if constexpr (PL > 6) w.c ^= (mu * pk[6]) ^ (mv * rk[6]);
+            if constexpr (PL > 7) w.d ^= (mu * pk[7]) ^ (mv * rk[7]);
             set_tail(u, w);
         }
     }
@@ -225,27 +224,41 @@ struct Node {
     int q, iso, dead;  // w^q 2^{iso/2}; dead: the amplitude is 0
 };
 
-// all ones if x is not 0; the highest bit of x, and its index (0 for x = 0)
+// all ones if x is not 0
 template <class W>
 CSIM_HD_INLINE W some(W x) {
     return wmask<W>(x != (W)0);
 }
-CSIM_HD_INLINE uint32_t top_bit(uint32_t x) {
+// the index of x's highest bit, -1 for x = 0; bit i as a word, 0 for i = -1
+CSIM_HD_INLINE int top_index(uint32_t x) {
 #ifdef __CUDA_ARCH__
-    return __funnelshift_rc(0x80000000u, 0u, (unsigned)__clz((int)x));  // 0 for a shift by 32
+    int i;
+    asm("bfind.u32 %0, %1;" : "=r"(i) : "r"(x));
+    return i;
 #else
-    return x ? 0x80000000u >> __builtin_clz(x) : 0u;
+    return x ? 31 - __builtin_clz(x) : -1;
 #endif
 }
-CSIM_HD_INLINE uint64_t top_bit(uint64_t x) {
+CSIM_HD_INLINE int top_index(uint64_t x) {
     const uint32_t hi = (uint32_t)(x >> 32);
-    return hi ? (uint64_t)top_bit(hi) << 32 : (uint64_t)top_bit((uint32_t)x);
+    const int i = top_index(hi ? hi : (uint32_t)x);
+    return hi ? i + 32 : i;
 }
 template <class W>
-CSIM_HD_INLINE int top_index(W x) {
-    using T = WordTraits<W>;
-    const int i = T::bits - 1 - T::clz(x);
-    return i < 0 ? 0 : i;
+CSIM_HD_INLINE W bit_at(int i);
+template <>
+CSIM_HD_INLINE uint32_t bit_at<uint32_t>(int i) {
+#ifdef __CUDA_ARCH__
+    uint32_t m;
+    asm("shl.b32 %0, 1, %1;" : "=r"(m) : "r"(i));  // 0 for a shift by 32 or more
+    return m;
+#else
+    return (unsigned)i < 32u ? 1u << i : 0u;
+#endif
+}
+template <>
+CSIM_HD_INLINE uint64_t bit_at<uint64_t>(int i) {
+    return (uint64_t)bit_at<uint32_t>(i) | ((uint64_t)bit_at<uint32_t>((int)((unsigned)i - 32u)) << 32);
 }
 
 // A node being contracted: the vertices of `sum` are to be summed out (2^{-1/2}
@@ -268,15 +281,17 @@ struct Work {
 template <class W, class R>
 CSIM_HD_INLINE void sum_step(const R& rows, Work<W>& w) {
     Node<W>& s = w.s;
-    const W act = some(w.sum), mc = top_bit(w.sum);
+    const int ic = top_index(w.sum), none = ic >> 31;  // nothing to sum: ic -1, none all ones
+    const W mc = bit_at<W>(ic);
     const W sum1 = w.sum ^ mc, live1 = w.live & ~mc;
-    const W N0 = (W)rows.get(top_index(w.sum)) & live1 & act;
+    const W N0 = (W)rows.get(ic < 0 ? 0 : ic) & live1 & ~(W)none;
     const W odd = some(s.d1 & mc), d = some(s.d2 & mc);
     const W near = N0 & sum1;
     const W even_pick = near != (W)0 ? near : N0;
     const W pick = (odd & sum1 & (s.d1 ^ N0)) | (~odd & even_pick);
-    const W two = some(pick), mb = top_bit(pick);
-    const W M0 = (W)rows.get(top_index(pick)) & live1 & ~mb & two;
+    const int ib = top_index(pick), single = ib >> 31;
+    const W mb = bit_at<W>(ib);
+    const W M0 = (W)rows.get(ib < 0 ? 0 : ib) & live1 & ~(mb | (W)single);
     const W N = N0 & ~mb;
     const W db1 = some(s.d1 & mb);
     // D on N: odd adds 6 (d = 0) or 2 (d = 1); a pivot adds D_b's odd part times (1 - 2 d)
@@ -292,29 +307,25 @@ CSIM_HD_INLINE void sum_step(const R& rows, Work<W>& w) {
     s.d1 = (d1 ^ (M & odd)) & ~mb;
     s.d2 = ((d2 ^ (wn & plus) ^ more) & ~mb) | (d & mb);
     s.h ^= mb;
-    // w^{1 - 2 d} and, with a second odd vertex, w^{1 - 2 d_b}; a pivot's w^{d D_b}
-    const int o = (int)odd, di = (int)d, b1 = (int)db1, b2 = (int)db2, t = (int)two;
-    s.q += (o & (1 + 2 * di + (t & (1 + 2 * b2)))) - (~o & di & (2 * b1 + 4 * b2));
-    const int lone = (int)act & ~o & ~t;  // an even vertex without neighbours: 2 or 0, times 2^{-1/2}
+    // w^{1 - 2 d} and, with a second odd vertex, w^{1 - 2 d_b}; a pivot's w^{d D_b}.  Products of
+    // the masks (0 or -1): multiply-adds run beside the logic ops
+    const int o = (int)odd, di = (int)d, b1 = (int)db1, b2 = (int)db2;
+    s.q -= o * (1 + 2 * di + ~single * -(1 + 2 * b2));
+    s.q += (~o & di) * (2 * b1 + 4 * b2);
+    const int lone = ~none & ~o & single;  // an even vertex without neighbours: 2 or 0, times 2^{-1/2}
     s.dead |= lone & di;
     s.iso -= lone;
     w.sum = sum1 & ~mb;
     w.live = live1 & ~(mb & sum1);  // a b that is summed too is gone: its new bit is contracted to 0
     // odd: rows of N get N, rows of M get M.  Pivot: rows of N get M (and N when D_b is odd),
     // rows of M get N, column b of both changes and row b becomes N
-    const int n = uniform_max(WordTraits<W>::bits - WordTraits<W>::clz(w.live));
+    const int n = uniform_max(top_index(w.live) + 1);
     rows.rank2(n, N | mb, wn ^ (~odd & (M ^ mb)), M | (mb & ~db1), (odd & M) | (~odd & (N ^ mb)));
 }
 
-// Steps until no lane has a vertex of `until` left to sum
-template <class W, class R>
-CSIM_HD_INLINE void sum_out(const R& rows, Work<W>& w, W until) {
-    while (uniform_any((w.sum & until) != (W)0)) sum_step<W>(rows, w);
-}
-
-// The same for two nodes of a lane, whose rows lie `words` apart: a lane goes on
-// to its second node when it is done with its first, without waiting for the
-// other lanes.  The number of steps varies between lanes (13 vertices, half of
+// Steps for two nodes of a lane, whose rows lie `words` apart, until neither has a
+// vertex of `until` left to sum: a lane goes on to its second node when it is done
+// with its first, without waiting for the other lanes.  The number of steps varies between lanes (13 vertices, half of
 // them to be summed: 3.9 on average, 5.9 in a warp's slowest lane), that of a
 // pair of siblings much less: their x agree or are complements on most positions.
 template <class W, class R>
@@ -343,7 +354,6 @@ CSIM_HD_INLINE void sum_out_pair(R rows, size_t words, Work<W>& a, Work<W>& b, W
 // each of a pair's positions); they are all in w.live before, in w.sum after.
 template <class W, class R>
 CSIM_HD_INLINE void join_pairs(const R& rows, Work<W>& w, W x, int lo, int hi, bool act) {
-    using T = WordTraits<W>;
     Node<W>& s = w.s;
     for (int a = lo; a < hi; a += 2) {  // uniform
         const W ma = act ? wbit<W>(a) : (W)0, mb = act ? wbit<W>(a + 1) : (W)0;
@@ -358,7 +368,7 @@ CSIM_HD_INLINE void join_pairs(const R& rows, Work<W>& w, W x, int lo, int hi, b
             w.live &= ~ma;
         }
         w.sum |= bell ? mb : ma | mb;
-        rows.rank2(uniform_max(T::bits - T::clz(w.live)), N, mb, mb, N);
+        rows.rank2(uniform_max(top_index(w.live) + 1), N, mb, mb, N);
     }
 }
 
@@ -399,40 +409,62 @@ CSIM_HD_INLINE void contract_pair(const Rows<PL>& rows, size_t words, Work<W>& a
 // all leaves of the node share the table.
 constexpr int kTableVars = 8;
 
-// entry r < 32: the truth table over five bits z of parity(r & z); of z within r
+// Lookup tables, by entry r < 32: the truth table over five bits z of parity(r & z); of
+// z within r.  By r < 64, the edges among four of the bits (edge j i, j < i, in bit
+// i (i - 1) / 2 + j): of sum of z_j z_i over the edges, mod 2.
+CSIM_HD_INLINE uint32_t coordinate_word(int i) {  // of z_i
+    return i == 0 ? 0xAAAAAAAAu : (i == 1 ? 0xCCCCCCCCu : (i == 2 ? 0xF0F0F0F0u : (i == 3 ? 0xFF00FF00u : 0xFFFF0000u)));
+}
 CSIM_HD_INLINE uint32_t linear_word(uint32_t r) {
     uint32_t w = 0;
-    for (uint32_t z = 0; z < 32; z++) w |= (uint32_t)(WordTraits<uint32_t>::popc(r & z) & 1) << z;
+#pragma unroll
+    for (int i = 0; i < 5; i++) w ^= coordinate_word(i) & wmask<uint32_t>((r >> i) & 1u);
     return w;
 }
 CSIM_HD_INLINE uint32_t subset_word(uint32_t r) {
-    uint32_t w = 0;
-    for (uint32_t z = 0; z < 32; z++) w |= (uint32_t)((z & ~r) == 0u) << z;
+    uint32_t w = 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < 5; i++) w &= ~coordinate_word(i) | wmask<uint32_t>((r >> i) & 1u);
     return w;
 }
+CSIM_HD_INLINE uint32_t edges_word(uint32_t r) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 1; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < i; j++)
+            w ^= coordinate_word(i) & coordinate_word(j) & wmask<uint32_t>((r >> (i * (i - 1) / 2 + j)) & 1u);
+    return w;
+}
+struct TableWords {
+    uint32_t lin[32], sub[32], edges[64];
+    CSIM_HD_INLINE void fill(int i) {  // i = 0 .. 31
+        lin[i] = linear_word((uint32_t)i);
+        sub[i] = subset_word((uint32_t)i);
+        edges[i] = edges_word((uint32_t)i);
+        edges[32 + i] = edges_word((uint32_t)(32 + i));
+    }
+};
 
 template <int WORDS>
 struct Table {
     uint32_t a[WORDS], c[WORDS];  // points with p1 = 1 and p0 = 0; p0 = 1
 };
-// rows r[i]: J row i of vertex i (bits below i are used)
+// r0, r4: the J rows of vertices 0..3 and 4..7, a byte each (bits below the vertex's are used)
 template <int WORDS>
-CSIM_HD_INLINE void build_table(const uint32_t (&r)[kTableVars], uint32_t d1, uint32_t d2, const uint32_t* lin,
-                                Table<WORDS>& t) {
-    const uint32_t zw[5] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
+CSIM_HD_INLINE void build_table(uint32_t r0, uint32_t r4, uint32_t d1, uint32_t d2, const TableWords& tw, Table<WORDS>& t) {
+    // D1_i D1_j joins the edges; vertices 0..3 are looked up at once
+    r0 = (r0 ^ (spread_bits(d1 & 15u) * d1)) & 0x07030100u;
+    r4 = (r4 ^ (spread_bits(d1 >> 4) * d1)) & 0x7F3F1F0Fu;
     uint32_t q1[WORDS], q0[WORDS];
-    q1[0] = 0u;
-#pragma unroll
-    for (int i = 0; i < 5; i++) {
-        const uint32_t row = (r[i] ^ (((d1 >> i) & 1u) ? d1 : 0u)) & ((1u << i) - 1u);
-        q1[0] ^= zw[i] & ((i ? lin[row] : 0u) ^ wmask<uint32_t>((d2 >> i) & 1u));
-    }
-    q0[0] = lin[d1 & 31u];
+    q1[0] = tw.edges[(r0 * ((1u << 18) | (1u << 11) | (1u << 5))) >> 26] ^ (tw.lin[pick_byte(r4, 0)] & 0xFFFF0000u) ^
+            tw.lin[d2 & 31u];
+    q0[0] = tw.lin[d1 & 31u];
 #pragma unroll
     for (int i = 5; (32 << (i - 5)) < 32 * WORDS; i++) {  // vertex i doubles the table: its linear form where z_i = 1
         const int half = 1 << (i - 5);
-        const uint32_t row = r[i] ^ (((d1 >> i) & 1u) ? d1 : 0u);
-        const uint32_t l = lin[row & 31u] ^ wmask<uint32_t>((d2 >> i) & 1u), o = wmask<uint32_t>((d1 >> i) & 1u);
+        const uint32_t row = pick_byte(r4, i - 4);
+        const uint32_t l = tw.lin[row & 31u] ^ wmask<uint32_t>((d2 >> i) & 1u), o = wmask<uint32_t>((d1 >> i) & 1u);
         const uint32_t l5 = wmask<uint32_t>((row >> 5) & 1u), l6 = wmask<uint32_t>((row >> 6) & 1u);
 #pragma unroll
         for (int w = 0; w < half; w++) {

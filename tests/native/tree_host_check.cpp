@@ -137,11 +137,8 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
         info[2] = (int)p.level.size();
         for (size_t i = 0; i < p.level.size(); i++) info[3 + i] = p.vert[i];
     }
-    uint32_t lin[32], sub[32];
-    for (uint32_t i = 0; i < 32; i++) {
-        lin[i] = linear_word(i);
-        sub[i] = subset_word(i);
-    }
+    TableWords tables;
+    for (int i = 0; i < 32; i++) tables.fill(i);
     const int words = table_words(p.tv);
     for (int a = 0; a < ntheta; a++) {
         std::vector<HostNode> cur{root_of(theta[a], p)};
@@ -173,16 +170,16 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
                 n.iso = 0;
                 HostNode o = n;
                 if (m > p.tv) stage(n, o, m, p.tv, paired);
-                uint32_t r[kTableVars] = {0};
-                for (int i = 0; i < kTableVars && i < m; i++) r[i] = (uint32_t)n.row[i];
+                uint32_t r[2] = {0, 0};
+                for (int i = 0; i < kTableVars && i < m; i++) r[i >> 2] |= (uint32_t)(n.row[i] & 0xFFu) << (8 * (i & 3));
                 const uint32_t vm = wlow<uint32_t>(p.tv), d1 = (uint32_t)n.d1 & vm;
                 int e0 = 0, e1 = 0, o0 = 0, o1 = 0;
                 uint32_t S = ((uint32_t)(x ^ n.h)) & vm;
                 auto leaves = [&](auto tb) {
-                    build_table(r, d1, (uint32_t)n.d2 & vm, lin, tb);
+                    build_table(r[0], r[1], d1, (uint32_t)n.d2 & vm, tables, tb);
                     for (int l = 0; l < (1 << p.tj); l++) {
                         if (l) S ^= (uint32_t)p.gen[__builtin_ctz((unsigned)l)] & vm;
-                        table_leaf(tb, S, d1, p.tv, sub, e0, e1, o0, o1);
+                        table_leaf(tb, S, d1, p.tv, tables.sub, e0, e1, o0, o1);
                     }
                 };
                 if (words == 1) leaves(Table<1>());
