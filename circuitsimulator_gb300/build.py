@@ -25,8 +25,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # the same bits on x86 and Arm hosts and in every code path.
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2,-ffp-contract=off",
                   "-I" + os.path.join(ROOT, "include")]
-SOURCES = ["csim_kernels.cu", "csim_terms_tp.cu", "csim_tree.cu", "csim_static.cu", "csim_batch_kernels.cu", "csim_host.cpp",
-           "csim_engine.cpp", "csim_backend.cpp"]
+SOURCES = ["csim_kernels.cu", "csim_terms_tp.cu", "csim_tree.cu", "csim_rand.cu", "csim_static.cu",
+           "csim_batch_kernels.cu", "csim_host.cpp", "csim_engine.cpp", "csim_backend.cpp"]
 
 
 def _nvcc():

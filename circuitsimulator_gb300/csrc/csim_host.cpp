@@ -558,7 +558,7 @@ int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Pl
                  o_plan = o_factor + 8 * (n + 1), o_L = o_plan + kTreePlanBytes, o_pm = o_L + 8 * (size_t)k,
                  bytes = o_pm + 4 * n;
     void* v;
-    CKR(staged_room(ctx, 6, bytes, &v));
+    CKR(staged_room(ctx, 1, bytes, &v));
     unsigned char* const h = (unsigned char*)v;
     if (n) memcpy(h, P->zs, 8 * n);
     if (n) memcpy(h + o_px, P->xs, 8 * n);
@@ -568,7 +568,7 @@ int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Pl
     else memset(h + o_plan, 0, kTreePlanBytes);
     if (k) memcpy(h + o_L, L, 8 * (size_t)k);
     for (size_t r = 0; r < n; r++) ((int32_t*)(h + o_pm))[r] = phase_m(P->phase[r]);
-    CKR(staged_send(ctx, 6, kBufCall, bytes, &v));
+    CKR(staged_send(ctx, 1, kBufCall, bytes, &v));
     const unsigned char* const d = (const unsigned char*)v;
     in->pz = (const uint64_t*)d;
     in->px = (const uint64_t*)(d + o_px);
@@ -581,9 +581,9 @@ int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Pl
 }
 
 // The raw words of the next `count` states in pinned slots `slot` (words) and
-// slot + 1 (offsets), and their upload
+// slot + 1 (offsets), and their upload; *chain: where they end
 int put_state_words(csim_ctx* ctx, int slot, int t, const double* cum, int64_t count, const uint32_t** dwords,
-                    const int64_t** doffs) {
+                    const int64_t** doffs, csim::DrawChain* chain) {
     void *v, *o;
     CKR(staged_room(ctx, slot, (kRawHistory + (size_t)count * state_words(t)) * 4, &v));
     CKR(staged_room(ctx, slot + 1, (size_t)(count + 1) * 8, &o));
@@ -602,11 +602,55 @@ int put_state_words(csim_ctx* ctx, int slot, int t, const double* cum, int64_t c
         if (!draw_state_words(w, t, cum, grow)) return CSIM_ERR_NOMEM;
     }
     offs[count] = (int64_t)w.n;
-    ctx->lr.set_history(w.p + w.n - kRawHistory);
+    chain->states = count;
+    memcpy(chain->history, w.p + w.n - kRawHistory, sizeof(chain->history));
     CKR(staged_send(ctx, slot, kBufWords, w.n * 4, &v));
     *dwords = (const uint32_t*)v;
     CKR(staged_send(ctx, slot + 1, kBufOffsets, (size_t)(count + 1) * 8, &v));
     *doffs = (const int64_t*)v;
+    return 0;
+}
+
+// Words of the longest sequence for a state of t qubits that draws at most two vectors again
+int most_words(int t) {
+    const int bytes = (t + 7) / 8;
+    int most = 0;
+    for (int d = 0; d <= t; d++) most = std::max(most, 1 + (5 + d) * bytes + (t - d) * (t - d - 1) / 2);
+    return most;
+}
+
+// The same on the device, from `words` words: *chain (device memory) counts the states that these
+// suffice for
+int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, int64_t words, const uint32_t** dwords,
+                     const int64_t** doffs, csim::DrawChain* chain) {
+    const int entries = most_words(t);
+    csim::RawStart start;
+    csim::raw_jumps(start);
+    ctx->lr.history(start.history);
+    csim::DrawTable table;
+    csim::draw_table(t, cum, table);
+    const int segment = csim::chain_segment(count, entries);
+    const int64_t padded = csim::chain_padded(words, segment);
+    void *w, *len, *map, *offs;
+    CKR(dbuf(ctx, kBufWords, (kRawHistory + (size_t)words) * 4, &w));
+    CKR(dbuf(ctx, kBufLengths, (size_t)padded * 2, &len));
+    CKR(dbuf(ctx, kBufChainMaps, (size_t)(padded / segment) * entries * 4, &map));
+    CKR(dbuf(ctx, kBufOffsets, (size_t)(count + 1) * 8, &offs));
+    if (csim::launch_raw_words(launch_of(ctx), start, words, (uint32_t*)w) ||
+        csim::launch_draw_lengths(launch_of(ctx), table, (const uint32_t*)w, words, padded, (uint16_t*)len) ||
+        csim::launch_draw_chain(launch_of(ctx), (const uint16_t*)len, padded, segment, (const uint32_t*)w, entries,
+                                (uint32_t*)map, count, (int64_t*)offs, chain))
+        return fail(ctx, CSIM_ERR_CUDA, "word launch failed");
+    *dwords = (const uint32_t*)w;
+    *doffs = (const int64_t*)offs;
+    return 0;
+}
+
+// A batch whose states took more words than there were: its draws flagged that, and it runs
+// again with twice as many
+int more_words(csim_ctx* ctx, int* more) {
+    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+    if (++*more > 2) return fail(ctx, CSIM_ERR_DEVICE, "random states took more words than four times the longest");
     return 0;
 }
 
@@ -663,9 +707,14 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     std::vector<unsigned char> jobs;
     std::vector<int> code;
     std::vector<__int128> acc;
-    for (int64_t o = 0; o < count; o += batch) {
+    const bool libc = rng == CSIM_RNG_LIBC;
+    constexpr size_t head = 16 + (sizeof(csim::DrawChain) + 15) / 16 * 16;  // results: live states, error, chain, values
+    int more = 0;  // a batch that ran out of words runs again with twice as many
+    for (int64_t o = 0; o < count;) {
         const int64_t c = std::min(batch, count - o);
         void* v;
+        CKR(dbuf(ctx, kBufResults, head + (size_t)c * 8, &v));
+        unsigned char* const dres = (unsigned char*)v;
         csim::GState* dth = nullptr;  // the tree's states stay in registers
         if (!tree) {
             CKR(dbuf(ctx, kBufA, c * sizeof(csim_state), &v));
@@ -681,7 +730,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             dcode_dir = (int*)v;
             CKR(dbuf(ctx, kBufCodeRest, c * 4, &v));
             dcode_rest = (int*)v;
-            CKR(dbuf(ctx, kBufRestCount, 4, &v));  // live states of a sub-batch left to the block-prefix kernel
+            CKR(dbuf(ctx, kBufRestCount, 4, &v));  // live states of a batch left to the block-prefix kernel
             drest = (int*)v;
         }
         const size_t nparts = (size_t)c * nchunks * 4;
@@ -689,146 +738,138 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         __int128* dpart = (__int128*)v;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
         if (!tree) CK(cudaMemsetAsync(dpart, 0, nparts * sizeof(__int128), ctx->stream));
-        // With the C library's draws the host makes every state's words.  The batch
-        // goes in sub-batches: the host draws sub-batch s+1 while the GPU works on
-        // sub-batch s, all launches queued on the stream.  The sub-batches grow 128,
-        // 512, 2048 states, so the GPU starts after a short draw and each draw stays
-        // shorter than the GPU's work on the one before.
-        int64_t ramp = rng == CSIM_RNG_LIBC ? 128 : c;
-        bool first = true;
-        for (int64_t s0 = 0, sb = 0; s0 < c; sb++) {
-            const int64_t cs = std::min(ramp, c - s0);
-            ramp = std::min<int64_t>(4 * ramp, rng == CSIM_RNG_LIBC ? 2048 : c);
-            csim::GState* sth = tree ? nullptr : (csim::GState*)((csim_state*)dth + s0);
-            int* scode = dcode + s0;
-            csim::TreeDraw draw{};
-            if (rng == CSIM_RNG_LIBC) {
-                // alternating pinned slots: the upload does not wait for the sub-batch before it, so
-                // the host goes on to draw the next one
-                const uint32_t* dw;
-                const int64_t* doff;
-                CKR(put_state_words(ctx, 2 * (sb & 1), t, hcum, cs, &dw, &doff));
-                draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, scode, nullptr, 0, 0};
-                if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 2, 0, 0, dw, doff, in.cum, sth, nullptr))
-                    return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
-            } else {
-                draw = csim::TreeDraw{0, P->nstabs, ctx->philox_seed, ctx->philox_next, nullptr, nullptr, in.cum, in.pm,
-                                      in.pz, in.px, scode, nullptr, 0, 0};
-                if (!tree && csim::launch_random_states(launch_of(ctx), t, cs, 0, ctx->philox_seed, ctx->philox_next,
-                                                        nullptr, nullptr, in.cum, sth, nullptr))
-                    return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
-                ctx->philox_next += cs;
-            }
-            if (!tree && csim::launch_project(launch_of(ctx), nr, sth, cs, P->nstabs, in.pm, in.pz, in.px, scode))
-                return fail(ctx, CSIM_ERR_CUDA, "projection launch failed");
-            if (tp && tn.kernel == 3) {
-                CK(cudaMemsetAsync(drest, 0, 4, ctx->stream));
-                if (csim::launch_canon(launch_of(ctx), sth, scode, cs, dsl,
-                                       (unsigned char*)dcanon + (size_t)s0 * csim::canon_bytes(), dcode_dir + s0,
-                                       dcode_rest + s0, drest))
-                    return fail(ctx, CSIM_ERR_CUDA, "pivot-form launch failed");
-            }
-            if (first && !tree) CK(cudaEventRecord(ctx->ev[1], ctx->stream));
-            const bool first_sub = first;
-            first = false;
-            __int128* spart = dpart + (size_t)s0 * nchunks * 4;
-            int rc = 0;
-            if (tree) {
-                TreeGroup g;
-                g.plan = &ctx->tree_plan;
-                g.dplan = in.plan;
-                g.draw = draw;
-                g.count = cs;
-                g.shape_count = shape_count;
-                g.part = spart;
-                void* scratch;
-                unsigned char* djobs;
-                CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
-                run.build((unsigned char*)scratch, jobs);
-                CKR(staged_put(ctx, 4 + (sb & 1), kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
-                // the event that starts the pair kernels' time is recorded behind the first roots
-                rc = run.launch(launch_of(ctx), djobs, first_sub ? ctx->ev[1] : nullptr);
-            } else if (tp && tn.kernel == 2) {
-                // one launch per occupancy class; class c's launch starts at its first whole item
-                const int64_t span = 64 * (int64_t)pt;
-                const int nc = (int)ctx->cw_bounds.size();
-                for (int c = 0; c < nc; c++) {
-                    const int64_t a0 = c == 0 ? 0 : (ctx->cw_starts[(size_t)c] + span - 1) / span * span;
-                    const int64_t b0 = c + 1 < nc ? (ctx->cw_starts[(size_t)c + 1] + span - 1) / span * span : chi;
-                    const int64_t aa = std::min(a0, chi), bb = std::min(b0, chi);
-                    if (aa < bb)
-                        rc |= csim::launch_terms_tp(launch_of(ctx), t, ctx->cw_bounds[(size_t)c], dcw + aa, sth,
-                                                    scode, cs, aa, bb - aa, pt, P2, spart, nchunks, aa / span,
-                                                    nullptr, nullptr, nullptr);
-                }
-            } else if (tp && tn.kernel == 1) {
-                // run kernel: terms [0, jb) in heavy runs, [jb, chi) in runs whose codewords have at most
-                // tn.light zeros below their run's agreed top bits
-                const int64_t span = 64 * (int64_t)pt;
-                const int64_t jb = ctx->cw_split;
-                if (jb > 0)
-                    rc |= csim::launch_terms_runs(launch_of(ctx), t, t, dcw, sth, scode, cs, 0, jb, pt, P2, spart,
-                                                  nchunks, 0, dscr, scr_bytes);
-                if (jb < chi)
-                    rc |= csim::launch_terms_runs(launch_of(ctx), t, std::min(t, tn.light), dcw + jb, sth, scode, cs,
-                                                  jb, chi - jb, pt, P2, spart, nchunks, jb / span, dscr, scr_bytes);
-            } else if (tp) {
-                // direct kernel: every term of the states it takes; the rest (or all, for kernel 0) below
-                const int* rcode = scode;
-                if (tn.kernel == 3) {
-                    // above 32 qubits the table's heavy part [0, cw_split) holds the codewords of at most 32
-                    // ones (direct_light), whose pairs need 32 J rows: a launch of its own with smaller
-                    // per-pair memory; the rest (from its first whole item) with rows for every coordinate
-                    const unsigned char* cb = (const unsigned char*)dcanon + (size_t)s0 * csim::canon_bytes();
-                    const int64_t span = 64 * (int64_t)pt;
-                    const int64_t jn = t > 32 ? std::min(chi, ctx->cw_split / span * span) : 0;
-                    if (jn > 0)
-                        rc |= csim::launch_terms_direct(launch_of(ctx), t, 32, dsl, dcw, cb, dcode_dir + s0, cs, 0,
-                                                        jn, pt, P2, spart, nchunks, 0);
-                    if (jn < chi)
-                        rc |= csim::launch_terms_direct(launch_of(ctx), t, t, dsl, dcw + jn, cb, dcode_dir + s0, cs,
-                                                        jn, chi - jn, pt, P2, spart, nchunks, jn / span);
-                    rcode = dcode_rest + s0;
-                }
-                // terms [0, jb): every zero count; terms [jb, chi): at most tn.light zeros (for the direct
-                // kernel's fallback, gated on the sub-batch having a state left to it)
-                const int64_t span = 64 * (int64_t)pt;
-                const int64_t jb = std::min(chi, (ctx->cw_split + span - 1) / span * span);
-                if (jb > 0)
-                    rc |= csim::launch_terms_tp(launch_of(ctx), t, t, dcw, sth, rcode, cs, 0, jb, pt, P2, spart,
-                                                nchunks, 0, nullptr, nullptr, nullptr, drest);
-                if (jb < chi)
-                    rc |= csim::launch_terms_tp(launch_of(ctx), t, tn.light, dcw + jb, sth, rcode, cs, jb,
-                                                chi - jb, pt, P2, spart, nchunks, jb / span, nullptr, nullptr,
-                                                nullptr, drest);
-            } else {
-                rc = csim::launch_terms(launch_of(ctx), nr, exact ? 1 : 0, dcw, (const csim::GState*)dphis, sth,
-                                        scode, cs, 0, chi, (int)chunk, P2, spart, nullptr, nullptr, nullptr, nullptr);
-            }
-            if (rc) return fail(ctx, CSIM_ERR_CUDA, "term launch failed");
-            s0 += cs;
+        // The C library's words: a few on the host, 0.4 ns each and 60 ns a state, from 30 us on on the
+        // device, whose four launches take that long (a call of 256 states: t = 24 185 us with the host's
+        // words, 145 with the device's, t = 40 349 and 246; of 64: t = 24 122 and 138, t = 40 212 and 219)
+        const int64_t most = (int64_t)most_words(t) * c;
+        const bool on_host = libc && most + 150 * c <= 75000;
+        csim::DrawChain chain{};
+        csim::TreeDraw draw{};
+        if (libc) {
+            const uint32_t* dw;
+            const int64_t* doff;
+            if (on_host) CKR(put_state_words(ctx, 3, t, hcum, c, &dw, &doff, &chain));
+            else CKR(make_state_words(ctx, t, hcum, c, (most + 4096) << more, &dw, &doff, (csim::DrawChain*)(dres + 16)));
+            draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, dcode, nullptr, 0, 0};
+            if (!tree && csim::launch_random_states(launch_of(ctx), t, c, 2, 0, 0, dw, doff, in.cum, dth, nullptr))
+                return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
+        } else {
+            draw = csim::TreeDraw{0, P->nstabs, ctx->philox_seed, ctx->philox_next, nullptr, nullptr, in.cum, in.pm,
+                                  in.pz, in.px, dcode, nullptr, 0, 0};
+            if (!tree && csim::launch_random_states(launch_of(ctx), t, c, 0, ctx->philox_seed, ctx->philox_next,
+                                                    nullptr, nullptr, in.cum, dth, nullptr))
+                return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
+            ctx->philox_next += c;
         }
+        if (!tree && csim::launch_project(launch_of(ctx), nr, dth, c, P->nstabs, in.pm, in.pz, in.px, dcode))
+            return fail(ctx, CSIM_ERR_CUDA, "projection launch failed");
+        if (tp && tn.kernel == 3) {
+            CK(cudaMemsetAsync(drest, 0, 4, ctx->stream));
+            if (csim::launch_canon(launch_of(ctx), dth, dcode, c, dsl, (unsigned char*)dcanon, dcode_dir, dcode_rest,
+                                   drest))
+                return fail(ctx, CSIM_ERR_CUDA, "pivot-form launch failed");
+        }
+        if (!tree) CK(cudaEventRecord(ctx->ev[1], ctx->stream));
+        int rc = 0;
+        if (tree) {
+            TreeGroup g;
+            g.plan = &ctx->tree_plan;
+            g.dplan = in.plan;
+            g.draw = draw;
+            g.count = c;
+            g.shape_count = shape_count;
+            g.part = dpart;
+            void* scratch;
+            unsigned char* djobs;
+            CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
+            run.build((unsigned char*)scratch, jobs);
+            CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+            // the event that starts the pair kernels' time is recorded behind the first roots
+            rc = run.launch(launch_of(ctx), djobs, ctx->ev[1]);
+        } else if (tp && tn.kernel == 2) {
+            // one launch per occupancy class; class c's launch starts at its first whole item
+            const int64_t span = 64 * (int64_t)pt;
+            const int nc = (int)ctx->cw_bounds.size();
+            for (int cl = 0; cl < nc; cl++) {
+                const int64_t a0 = cl == 0 ? 0 : (ctx->cw_starts[(size_t)cl] + span - 1) / span * span;
+                const int64_t b0 = cl + 1 < nc ? (ctx->cw_starts[(size_t)cl + 1] + span - 1) / span * span : chi;
+                const int64_t aa = std::min(a0, chi), bb = std::min(b0, chi);
+                if (aa < bb)
+                    rc |= csim::launch_terms_tp(launch_of(ctx), t, ctx->cw_bounds[(size_t)cl], dcw + aa, dth,
+                                                dcode, c, aa, bb - aa, pt, P2, dpart, nchunks, aa / span,
+                                                nullptr, nullptr, nullptr);
+            }
+        } else if (tp && tn.kernel == 1) {
+            // run kernel: terms [0, jb) in heavy runs, [jb, chi) in runs whose codewords have at most
+            // tn.light zeros below their run's agreed top bits
+            const int64_t span = 64 * (int64_t)pt;
+            const int64_t jb = ctx->cw_split;
+            if (jb > 0)
+                rc |= csim::launch_terms_runs(launch_of(ctx), t, t, dcw, dth, dcode, c, 0, jb, pt, P2, dpart,
+                                              nchunks, 0, dscr, scr_bytes);
+            if (jb < chi)
+                rc |= csim::launch_terms_runs(launch_of(ctx), t, std::min(t, tn.light), dcw + jb, dth, dcode, c,
+                                              jb, chi - jb, pt, P2, dpart, nchunks, jb / span, dscr, scr_bytes);
+        } else if (tp) {
+            // direct kernel: every term of the states it takes; the rest (or all, for kernel 0) below
+            const int* rcode = dcode;
+            if (tn.kernel == 3) {
+                // above 32 qubits the table's heavy part [0, cw_split) holds the codewords of at most 32
+                // ones (direct_light), whose pairs need 32 J rows: a launch of its own with smaller
+                // per-pair memory; the rest (from its first whole item) with rows for every coordinate
+                const unsigned char* cb = (const unsigned char*)dcanon;
+                const int64_t span = 64 * (int64_t)pt;
+                const int64_t jn = t > 32 ? std::min(chi, ctx->cw_split / span * span) : 0;
+                if (jn > 0)
+                    rc |= csim::launch_terms_direct(launch_of(ctx), t, 32, dsl, dcw, cb, dcode_dir, c, 0,
+                                                    jn, pt, P2, dpart, nchunks, 0);
+                if (jn < chi)
+                    rc |= csim::launch_terms_direct(launch_of(ctx), t, t, dsl, dcw + jn, cb, dcode_dir, c,
+                                                    jn, chi - jn, pt, P2, dpart, nchunks, jn / span);
+                rcode = dcode_rest;
+            }
+            // terms [0, jb): every zero count; terms [jb, chi): at most tn.light zeros (for the direct
+            // kernel's fallback, gated on the batch having a state left to it)
+            const int64_t span = 64 * (int64_t)pt;
+            const int64_t jb = std::min(chi, (ctx->cw_split + span - 1) / span * span);
+            if (jb > 0)
+                rc |= csim::launch_terms_tp(launch_of(ctx), t, t, dcw, dth, rcode, c, 0, jb, pt, P2, dpart,
+                                            nchunks, 0, nullptr, nullptr, nullptr, drest);
+            if (jb < chi)
+                rc |= csim::launch_terms_tp(launch_of(ctx), t, tn.light, dcw + jb, dth, rcode, c, jb,
+                                            chi - jb, pt, P2, dpart, nchunks, jb / span, nullptr, nullptr,
+                                            nullptr, drest);
+        } else {
+            rc = csim::launch_terms(launch_of(ctx), nr, exact ? 1 : 0, dcw, (const csim::GState*)dphis, dth,
+                                    dcode, c, 0, chi, (int)chunk, P2, dpart, nullptr, nullptr, nullptr, nullptr);
+        }
+        if (rc) return fail(ctx, CSIM_ERR_CUDA, "term launch failed");
         CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-        if (tree) {  // results: the live states' count, the error word, the values
-            CKR(dbuf(ctx, kBufResults, 16 + (size_t)c * 8, &v));
-            unsigned char* const dres = (unsigned char*)v;
+        if (tree) {
             CK(cudaMemsetAsync(dres, 0, 16, ctx->stream));
-            if (csim::launch_tree_values(launch_of(ctx), dpart, c, nchunks, t, dcode, in.factor, (double*)(dres + 16),
+            if (csim::launch_tree_values(launch_of(ctx), dpart, c, nchunks, t, dcode, in.factor, (double*)(dres + head),
                                          (unsigned long long*)dres))
                 return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
             CK(cudaMemcpyAsync(dres + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
             CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-            CKR(staged_room(ctx, 7, 16 + (size_t)c * 8, &v));
-            CKR(dget(ctx, (unsigned char*)v, dres, 16 + (size_t)c * 8));
+            CKR(staged_room(ctx, 2, head + (size_t)c * 8, &v));
+            CKR(dget(ctx, (unsigned char*)v, dres, head + (size_t)c * 8));
             CK(cudaStreamSynchronize(ctx->stream));
             CK(cudaGetLastError());
+            if (libc && !on_host) memcpy(&chain, (const unsigned char*)v + 16, sizeof(chain));
+            if (libc && chain.states < c) {
+                CKR(more_words(ctx, &more));
+                continue;
+            }
             CKR(error_status(ctx, ((const int*)v)[2]));
             CKR(stats_batch(ctx));
             const int64_t live = *(const int64_t*)v;
-            memcpy(values + o, (const unsigned char*)v + 16, (size_t)c * 8);
+            memcpy(values + o, (const unsigned char*)v + head, (size_t)c * 8);
+            if (libc) ctx->lr.set_history(chain.history);
             ctx->stats.states += c;
             ctx->stats.states_live += live;
             ctx->stats.pairs += live * chi;
+            o += c;
             continue;
         }
         CKR(dbuf(ctx, kBufAcc, (size_t)c * 4 * sizeof(__int128), &v));
@@ -840,7 +881,16 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         acc.resize(c * 4);
         CKR(dget(ctx, code.data(), dcode, c));
         CKR(dget(ctx, acc.data(), dacc, c * 4));
+        if (libc && !on_host) {
+            CKR(dget(ctx, &chain, (const csim::DrawChain*)(dres + 16), 1));
+            CK(cudaStreamSynchronize(ctx->stream));
+            if (chain.states < c) {
+                CKR(more_words(ctx, &more));
+                continue;
+            }
+        }
         CKR(finish(ctx));
+        if (libc) ctx->lr.set_history(chain.history);
         CKR(stats_batch(ctx));
         const double scale = pow(2, t);
         ctx->stats.states += c;
@@ -857,11 +907,10 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             const double a = re * pf, b = im * pf;
             values[o + i] = scale * (a * a + b * b);
         }
+        o += c;
     }
     return 0;
 }
-
-
 
 }  // namespace
 
@@ -1127,7 +1176,7 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     unsigned char* djobs;
     CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
     run.build((unsigned char*)scratch, jobs);
-    CKR(staged_put(ctx, 4, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+    CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
     if (run.launch(launch_of(ctx), djobs, ctx->ev[1]))
         return fail(ctx, CSIM_ERR_CUDA, "tree launch failed");
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
@@ -1141,7 +1190,7 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
         return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
     CK(cudaMemcpyAsync(dres + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
-    CKR(staged_room(ctx, 7, bytes, &v));
+    CKR(staged_room(ctx, 2, bytes, &v));
     CKR(dget(ctx, (unsigned char*)v, dres, bytes));
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());

@@ -18,6 +18,7 @@
 
 #include "../../include/csim.h"
 #include "csim_internal.h"
+#include "csim_rand.h"
 #include "csim_tree_host.h"
 
 namespace csim_host {
@@ -87,7 +88,7 @@ struct RawWords {
         for (; e < end; e++) *e = e[-3] + e[-31];
     }
 };
-constexpr size_t kRawHistory = 34;
+constexpr size_t kRawHistory = csim::kRawHistory;
 
 // ---------------------------------------------------------------- helpers
 inline int popc(uint64_t x) { return __builtin_popcountll(x); }
@@ -411,10 +412,10 @@ enum BufId {
     kBufA, kBufB, kBufEps, kBufP, kBufM, kBufXi, kBufZeta, kBufAlpha, kBufCode, kBufWords, kBufOffsets,
     kBufCum, kBufCodewords, kBufAcc, kBufAccDiag, kBufPhis, kBufIdx, kBufConsumed, kBufPm, kBufPz, kBufPx,
     kBufL, kBufParts, kBufPartsDiag, kBufCwOrdered, kBufRunScratch, kBufCanon, kBufCodeDirect, kBufCodeRest,
-    kBufRestCount, kBufTreeJobs, kBufTreeScratch, kBufCall, kBufResults, kNumBufs
+    kBufRestCount, kBufTreeJobs, kBufTreeScratch, kBufCall, kBufResults, kBufLengths, kBufChainMaps, kNumBufs
 };
 
-constexpr int kPinSlots = 8;      // words and offsets twice, jobs twice, a call's inputs, its results
+constexpr int kPinSlots = 5;      // tree jobs, a call's inputs, its results, words, offsets
 
 class Engine;                     // csim_engine.cpp: the batched query engine
 void engine_free(Engine* engine);  // releases it and its device memory

@@ -1,0 +1,38 @@
+"""The C library's draws on the device (csim_rand.cu): the states' places in the
+generator's sequence are the same however many states a call draws."""
+import numpy as np
+import pytest
+
+from circuitsimulator_gb300 import backend
+from helpers import rand_word, random_projector_rows
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    g = backend.Backend(0)
+    yield g
+    g.close()
+
+
+# few words are made on the host, more on the device (a batch is 2^14 states); with few qubits
+# many vectors are drawn again
+@pytest.mark.parametrize("t,count", [(1, 700), (2, 513), (3, 3000), (5, 17000), (8, 512), (9, 1100), (31, 1500), (33, 600),
+                                     (64, 1300)])
+def test_draws_of_one_call_equal_those_of_several(gpu, t, count):
+    rs = np.random.RandomState(t)
+    rows = random_projector_rows(rs, t, max(1, t // 3))
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    L = [rand_word(rs, t) for _ in range(2)]
+    whole = gpu.singleProjectorSample(P, L, False, count, backend.RNG_LIBC, 77)
+    after = gpu.singleProjectorSample(P, L, False, 3, backend.RNG_LIBC)
+    parts, left = [], count
+    for i, n in enumerate([1, 2, 509, 1, 20, 513] * 40):
+        n = min(n, left)
+        if not n:
+            break
+        parts.append(gpu.singleProjectorSample(P, L, False, n, backend.RNG_LIBC, *([77] if i == 0 else [])))
+        left -= n
+    assert (np.concatenate(parts) == whole).all()
+    assert (gpu.singleProjectorSample(P, L, False, 3, backend.RNG_LIBC) == after).all()
