@@ -768,7 +768,8 @@ int Engine::launch_round() {
         v.diag0 = ndiags;
         if (g.rows) ndiags += sg.n;
     }
-    const size_t scratch_bytes = tree_run_.layout(groups, kTreeScratchMax);
+    if (tree_run_.reserve(groups, [&](size_t bytes) { return tree_scratch_.ensure(bytes); }))
+        return fail(ctx_, CSIM_ERR_NOMEM, "tree sum buffers (%lld states)", (long long)ns);
     std::vector<unsigned char> tree_jobs;
     tree_run_.build(nullptr, tree_jobs);  // for its size
     // upload block: projectors | segments | tree jobs | words | word offsets | state descriptors | items | ranges
@@ -797,7 +798,7 @@ int Engine::launch_round() {
     rs.off_codes = 256;
     rs.off_val = align_up(rs.off_codes + (size_t)ns * 4);
     const size_t down_bytes = align_up(rs.off_val + (size_t)ns * 16);
-    if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) || tree_scratch_.ensure(scratch_bytes) ||
+    if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) ||
         rs.down.ensure(down_bytes) || rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes))
         return fail(ctx_, CSIM_ERR_NOMEM, "round buffers (%lld states, %lld items)", (long long)ns,
                     (long long)nitems);
@@ -953,7 +954,7 @@ int Engine::launch_round() {
             }
         }
     }
-    tree_run_.layout(groups, kTreeScratchMax);
+    tree_run_.layout(groups);
     tree_run_.build((unsigned char*)tree_scratch_.p, tree_jobs);
     if (!tree_jobs.empty()) memcpy(hb + o_tjobs, tree_jobs.data(), tree_jobs.size());
     int* derr = (int*)dd;

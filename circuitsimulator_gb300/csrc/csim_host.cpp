@@ -781,7 +781,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             g.part = dpart;
             void* scratch;
             unsigned char* djobs;
-            CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
+            CKR(run.reserve({g}, [&](size_t bytes) { return dbuf(ctx, kBufTreeScratch, bytes, &scratch); }));
             run.build((unsigned char*)scratch, jobs);
             CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
             // the event that starts the pair kernels' time is recorded behind the first roots
@@ -1174,7 +1174,7 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     std::vector<unsigned char> jobs;
     void* scratch;
     unsigned char* djobs;
-    CKR(dbuf(ctx, kBufTreeScratch, run.layout({g}, kTreeScratchMax), &scratch));
+    CKR(run.reserve({g}, [&](size_t bytes) { return dbuf(ctx, kBufTreeScratch, bytes, &scratch); }));
     run.build((unsigned char*)scratch, jobs);
     CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
     if (run.launch(launch_of(ctx), djobs, ctx->ev[1]))

@@ -64,15 +64,20 @@ inline void tree_scratch_per_state(const csim::tree::Plan& p, int64_t (&half)[2]
     }
 }
 
-constexpr size_t kTreeScratchMax = (size_t)1 << 30;
+// Scratch of a run's node planes: every chunk pays the latency of its draws and first stages,
+// about 0.2 ms at 40 to 64 qubits (256 states of 57 qubits, 2^18 terms: 5.36 ms with 1 GB, 5.05 with
+// 2, 4.93 with 4; 4096 of 40, 2^16 terms: 7.96, 7.74, 7.62).  Where the memory is not to be had,
+// a quarter of it will do, down to kTreeScratchMin.
+constexpr size_t kTreeScratchMax = (size_t)4 << 30, kTreeScratchMin = (size_t)64 << 20;
 // decompositions of more than 2^30 terms run on the pair kernels (node indices are 32 bits)
 constexpr int kTreeMaxRows = 30;
 
 class TreeRun {
   public:
-    // Splits the groups into chunks whose node planes fit `budget` bytes (one
+    // Splits the groups into chunks whose node planes fit reserve()'s budget (one
     // state at least).  Returns the scratch bytes needed.
-    size_t layout(const std::vector<TreeGroup>& groups, size_t budget) {
+    size_t layout(const std::vector<TreeGroup>& groups) {
+        const size_t budget = budget_;
         chunks_.clear();
         scratch_ = 0;
         size_t used = 0;
@@ -118,6 +123,16 @@ class TreeRun {
             scratch_ = std::max(scratch_, used);
         }
         return scratch_;
+    }
+
+    // layout() for the largest budget whose scratch `alloc` (bytes -> 0 or an error) finds memory for
+    template <class Alloc>
+    int reserve(const std::vector<TreeGroup>& groups, Alloc alloc) {
+        for (budget_ = kTreeScratchMax;; budget_ /= 4) {
+            const int rc = alloc(layout(groups));
+            if (rc == 0 || budget_ <= kTreeScratchMin) return rc;
+            cudaGetLastError();  // the failed allocation's
+        }
     }
 
     // The job tables, to be copied to the device (`scratch`: the device scratch)
@@ -250,7 +265,7 @@ class TreeRun {
     }
     std::vector<Chunk> chunks_;
     std::vector<Step> steps_;
-    size_t scratch_ = 0;
+    size_t scratch_ = 0, budget_ = kTreeScratchMax;
 };
 
 // A plan's device image (kTreePlanBytes)

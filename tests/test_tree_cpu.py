@@ -162,3 +162,26 @@ def test_tree_sum_on_extreme_states(tree_sums, oracle):
                     w["J"][x] = int(w["J"][x]) & ~(1 << x)
             states.append(w)
         _check(tree_sums, oracle, t, L, np.array(states))
+
+
+@pytest.mark.parametrize("t,k,count", [(40, 16, 4096), (57, 18, 256), (24, 8, 60), (64, 18, 1)])
+@pytest.mark.parametrize("room", [1 << 40, 1 << 32, (1 << 30) + 4096, 100 << 20, 1 << 20])
+def test_scratch_of_the_memory_there_is(t, k, count, room):
+    """Chunks fit the memory that the allocator finds, in quarters of the largest budget
+    down to the smallest; then a run of more than one state fails, as one state's planes do."""
+    src, so = os.path.join(HERE, "native", "tree_layout_check.cpp"), os.path.join(HERE, "native", "_build", "liblayout.so")
+    os.makedirs(os.path.dirname(so), exist_ok=True)
+    deps = [src] + [os.path.join(CSRC, f) for f in ("csim_tree.h", "csim_tree_host.h", "csim_tree.cuh", "csim_tree_plan.h")]
+    if not os.path.exists(so) or os.path.getmtime(so) < max(os.path.getmtime(f) for f in deps):
+        subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", src, "-o", so])
+    lib = C.CDLL(so)
+    rs = np.random.RandomState(t)
+    L = np.array([int(rand_word(rs, t)) for _ in range(k)], dtype=np.uint64)
+    out = np.zeros(5, dtype=np.int64)
+    lib.tree_layout(C.c_void_p(L.ctypes.data), k, t, C.c_int64(count), C.c_int64(room), C.c_void_p(out.ctypes.data))
+    status, used, tried, first, per = out.tolist()
+    budget = (4 << 30) >> (2 * (tried - 1))
+    assert 1 <= tried <= 4 and budget >= 64 << 20
+    assert used <= max(budget, per) + 1024 and first == min(count, max(1, -(-count // max(1, -(-count // max(1, budget // per))))))
+    assert (status == 0) == (used <= room)
+    assert status == 0 or budget == 64 << 20
