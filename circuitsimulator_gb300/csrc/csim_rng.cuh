@@ -142,7 +142,7 @@ __device__ void random_state(WS<NR>& s, int n, DevRng& rng, const double* cum, i
         }
     }
     __syncwarp();
-    uint64_t low[NR];  // J[x][c], c < x
+    RW<NR> low[NR];  // J[x][c], c < x
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
@@ -150,16 +150,16 @@ __device__ void random_state(WS<NR>& s, int n, DevRng& rng, const double* cum, i
         if (x >= 1 && x < k) {
             const int at = lead + x * (x - 1) / 2, w = at >> 5, sh = at & 31;
             const uint64_t v = (uint64_t)tri[w] | ((uint64_t)tri[w + 1] << 32);
-            low[sl] = ((v >> sh) | (sh ? (uint64_t)tri[w + 2] << (64 - sh) : 0ull)) & lowmask(x);
+            low[sl] = (RW<NR>)((v >> sh) | (sh ? (uint64_t)tri[w + 2] << (64 - sh) : 0ull)) & low_mask<NR>(x);
         }
     }
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        s.J[sl] = x < k ? low[sl] | ((uint64_t)getbit(s.D1, x) << x) : 0ull;  // J[x][x] = ((2 D[x]) mod 8) / 4
+        s.J[sl] = x < k ? low[sl] | ((RW<NR>)getbit(s.D1, x) << x) : (RW<NR>)0;  // J[x][x] = ((2 D[x]) mod 8) / 4
     }
     for (int x = 0; x < k; x++) {
-        const uint64_t col = ballot_bit<NR>(low, x);  // rows c > x with J[c][x] = 1
+        const RW<NR> col = ballot_bit<NR>(low, x);  // rows c > x with J[c][x] = 1
         if (lane == (x & 31)) {
             if (NR == 2 && x >= 32) s.J[NR - 1] |= col;
             else s.J[0] |= col;

@@ -179,17 +179,17 @@ __global__ void __launch_bounds__(64) k_canon(const GState* theta, const int* co
     CanonG& o = out[a0];
     const uint64_t nm = pc::lowmask(n), km = pc::lowmask(k);
     const int r0 = lane, r1 = lane + 32;  // this lane's variables
-    CanonWarp w;
-    w.g0 = r0 < k ? g->G[r0] & nm : 0ull;
-    w.g1 = r1 < k ? g->G[r1] & nm : 0ull;
-    w.j0 = r0 < k ? g->J[r0] & km : 0ull;
-    w.j1 = r1 < k ? g->J[r1] & km : 0ull;
+    CanonWarp<2> w;
+    w.g[0] = r0 < k ? g->G[r0] & nm : 0ull;
+    w.g[1] = r1 < k ? g->G[r1] & nm : 0ull;
+    w.j[0] = r0 < k ? g->J[r0] & km : 0ull;
+    w.j[1] = r1 < k ? g->J[r1] & km : 0ull;
     w.D1 = g->D1 & km;
     w.D2 = g->D2 & km;
-    canon_warp(w, k, g->h);
+    canon_warp<2>(w, k, g->h);
     // to coordinate indexing
-    piv[r0] = (unsigned char)(r0 < k ? w.p0 : 0);
-    piv[r1] = (unsigned char)(r1 < k ? w.p1 : 0);
+    piv[r0] = (unsigned char)(r0 < k ? w.p[0] : 0);
+    piv[r1] = (unsigned char)(r1 < k ? w.p[1] : 0);
     __syncwarp();
     const uint64_t P = w.P;
     o.Jc[r0] = 0ull;
@@ -197,14 +197,14 @@ __global__ void __launch_bounds__(64) k_canon(const GState* theta, const int* co
     o.acol[r0] = 0ull;
     o.acol[r1] = 0ull;
     __syncwarp();
-    if (r0 < k) o.Jc[w.p0] = to_coords(w.j0, piv);
-    if (r1 < k) o.Jc[w.p1] = to_coords(w.j1, piv);
+    if (r0 < k) o.Jc[w.p[0]] = to_coords(w.j[0], piv);
+    if (r1 < k) o.Jc[w.p[1]] = to_coords(w.j[1], piv);
     // each non-pivot coordinate: the variables its coordinate depends on, and the constraint's bit
     uint64_t bm = 0ull;
     for (uint64_t np = ~P & nm; np;) {
         const int cc = __ffsll((long long)np) - 1;
         np &= np - 1ull;
-        const uint64_t av = ballot64(r0 < k && ((w.g0 >> cc) & 1ull), r1 < k && ((w.g1 >> cc) & 1ull));
+        const uint64_t av = ballot_i<2>(r0 < k && ((w.g[0] >> cc) & 1ull), r1 < k && ((w.g[1] >> cc) & 1ull));
         if (lane == (cc & 31)) o.acol[cc] = to_coords(av, piv);
         if ((((g->h >> cc) & 1ull) ^ (uint64_t)(__popcll(w.wv & av) & 1)) != 0ull) bm |= 1ull << cc;
     }

@@ -40,9 +40,10 @@ __device__ __forceinline__ const J& job_of(const J* jobs, int njobs, int64_t b) 
 }
 
 // bits of v in the plan's order (position -> coordinate)
-__device__ __forceinline__ uint64_t permute_bits(uint64_t v, const unsigned char* perm, int t) {
-    uint64_t r = 0ull;
-    for (int i = 0; i < t; i++) r |= ((v >> perm[i]) & 1ull) << i;
+template <class W>
+__device__ __forceinline__ W permute_bits(W v, const unsigned char* perm, int t) {
+    W r = 0;
+    for (int i = 0; i < t; i++) r |= ((v >> perm[i]) & (W)1) << i;
     return r;
 }
 
@@ -104,40 +105,54 @@ __device__ __forceinline__ void dead_root(const TreeRootJob& J, uint32_t i) {
 // Node i of the job from a state held by the warp
 template <int NR>
 __device__ void store_root(const TreeRootJob& J, uint32_t i, const WS<NR>& st, RootShared& sh) {
+    using W = RW<NR>;
     unsigned char* const piv = sh.piv[threadIdx.x >> 5];
     const int t = J.t, k = st.k;
-    const uint64_t km = pc::lowmask(k), nm = pc::lowmask(t);
-    const int r0 = lane_id(), r1 = r0 + 32;  // this lane's variables
-    CanonWarp w;
-    w.g0 = r0 < k ? permute_bits(st.G[0], sh.perm, t) : 0ull;
-    w.g1 = NR == 2 && r1 < k ? permute_bits(st.G[NR - 1], sh.perm, t) : 0ull;
-    w.j0 = r0 < k ? st.J[0] & km : 0ull;
-    w.j1 = NR == 2 && r1 < k ? st.J[NR - 1] & km : 0ull;
+    const W km = low_mask<NR>(k), nm = low_mask<NR>(t);
+    CanonWarp<NR> w;
+#pragma unroll
+    for (int q = 0; q < NR; q++) {  // this lane's variables
+        const bool in = row_of<NR>(q) < k;
+        w.g[q] = in ? permute_bits<W>(st.G[q], sh.perm, t) : (W)0;
+        w.j[q] = in ? st.J[q] & km : (W)0;
+    }
     w.D1 = st.D1 & km;
     w.D2 = st.D2 & km;
-    const uint64_t h = permute_bits(st.h, sh.perm, t);
-    canon_warp(w, k, h);
+    const W h = permute_bits<W>(st.h, sh.perm, t);
+    canon_warp<NR>(w, k, h);
     __syncwarp();
-    piv[r0] = (unsigned char)(r0 < k ? w.p0 : 0);
-    piv[r1] = (unsigned char)(r1 < k ? w.p1 : 0);
+#pragma unroll
+    for (int q = 0; q < NR; q++) piv[row_of<NR>(q)] = (unsigned char)w.p[q];
     __syncwarp();
     // pivots: vertices with J and D; a non-pivot coordinate y = b + a.v is Had on a vertex
     // joined to the variables in a, with D = 4 b
-    uint64_t row0 = to_coords(w.j0, piv), row1 = to_coords(w.j1, piv), bm = 0ull;
-    for (uint64_t np = ~w.P & nm; np;) {
-        const int c = __ffsll((long long)np) - 1;
-        np &= np - 1ull;
-        const bool in0 = r0 < k && ((w.g0 >> c) & 1ull), in1 = r1 < k && ((w.g1 >> c) & 1ull);
-        const uint64_t av = ballot64(in0, in1);
-        if (in0) row0 |= 1ull << c;
-        if (in1) row1 |= 1ull << c;
-        if (r0 == (c & 31)) store_row(J.out, J.count, i, t, c, to_coords(av, piv));
-        if ((((h >> c) & 1ull) ^ (uint64_t)(__popcll(w.wv & av) & 1)) != 0ull) bm |= 1ull << c;
+    W row[NR], had[NR] = {}, bm = 0;  // rows of this lane's variables, of its coordinates
+#pragma unroll
+    for (int q = 0; q < NR; q++) row[q] = to_coords<W>(w.j[q], piv);
+    for (W np = ~w.P & nm; np;) {  // uniform
+        const int c = first_bit(np);
+        np &= np - (W)1;
+        bool in[2] = {};
+#pragma unroll
+        for (int q = 0; q < NR; q++) {
+            in[q] = row_of<NR>(q) < k && ((w.g[q] >> c) & (W)1);
+            if (in[q]) row[q] |= bit_of<NR>(c);
+        }
+        const W av = ballot_i<NR>(in[0], in[NR - 1]);
+#pragma unroll
+        for (int q = 0; q < NR; q++)
+            if (row_of<NR>(q) == c) had[q] = av;
+        if ((getbit(h, c) ^ parity(w.wv & av)) != 0) bm |= bit_of<NR>(c);
     }
-    if (r0 < k) store_row(J.out, J.count, i, t, w.p0, row0);
-    if (r1 < k) store_row(J.out, J.count, i, t, w.p1, row1);
-    if (r0 == 0)
-        store_scalars(J.out, J.count, i, t, to_coords(w.D1, piv), to_coords(w.D2, piv) | bm, ~w.P & nm, J.x0,
+#pragma unroll
+    for (int q = 0; q < NR; q++) {
+        const int r = row_of<NR>(q);
+        if (r < k) store_row(J.out, J.count, i, t, w.p[q], row[q]);
+        had[q] = to_coords<W>(had[q], piv);
+        if (r < t && !getbit(w.P, r)) store_row(J.out, J.count, i, t, r, had[q]);
+    }
+    if (lane_id() == 0)
+        store_scalars(J.out, J.count, i, t, to_coords<W>(w.D1, piv), to_coords<W>(w.D2, piv) | bm, ~w.P & nm, J.x0,
                       pack_status(st.Q + w.dq, 0, 0));
 }
 
@@ -146,7 +161,8 @@ __device__ void store_root(const TreeRootJob& J, uint32_t i, const WS<NR>& st, R
 // Drawing, projecting and the graph form in one launch, the state never leaving the
 // warp's registers.  Bound by the latency of a warp's serial steps: 1024 states of
 // 40 qubits take 44 us; k_random_states, k_project and a kernel for the graph form
-// took 11 + 29 + 26 us.  NR = 1: jobs of up to 32 qubits, 2: the others.
+// took 11 + 29 + 26 us.  NR = 1: jobs of up to 32 qubits, 2: the others.  Many states
+// are bound by the instructions: 64,400 of up to 23 qubits 347 us (NR = 1).
 template <int NR>
 __global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRootJob* jobs, int njobs, int* err) {
     __shared__ RootShared sh;

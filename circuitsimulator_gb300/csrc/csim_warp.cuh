@@ -2,7 +2,7 @@
 //
 // One warp holds one stabilizer state (CircuitSimulator's struct
 // StabilizerState, libcirc/stabilizer/stabilizer.h:5-16) with lane l owning
-// rows l and l+32 of G, Gbar and J as uint64 words (bit c = column c).  The
+// rows l and l+32 of G, Gbar and J as words (bit c = column c; RW).  The
 // vectors h, D1, D2 and the scalars n, k, Q are warp-uniform.  Rows >= n are
 // kept zero.  NR = rows per lane (1 for n <= 32, 2 for n <= 64).
 //
@@ -36,10 +36,39 @@ enum : int {
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint64_t bit1(int i) { return 1ull << i; }
 __device__ __forceinline__ uint64_t lowmask(int k) { return k >= 64 ? ~0ull : ((1ull << k) - 1ull); }
-__device__ __forceinline__ int getbit(uint64_t w, int i) { return (int)((w >> i) & 1ull); }
+template <class W>
+__device__ __forceinline__ int getbit(W w, int i) {
+    return (int)((w >> i) & (W)1);
+}
+// the same for rows of either width (RW)
+template <int NR>
+__device__ __forceinline__ auto bit_of(int i) {
+    if constexpr (NR == 1) return 1u << i;
+    else return bit1(i);
+}
+template <int NR>
+__device__ __forceinline__ auto low_mask(int k) {
+    if constexpr (NR == 1) {
+        uint32_t m;
+        asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(m) : "r"(k));
+        return m;
+    } else {
+        return lowmask(k);
+    }
+}
+__device__ __forceinline__ int popcount(uint32_t w) { return __popc(w); }
+__device__ __forceinline__ int popcount(uint64_t w) { return __popcll(w); }
+__device__ __forceinline__ int parity(uint32_t w) { return __popc(w) & 1; }
+__device__ __forceinline__ int parity(uint64_t w) { return __popcll(w) & 1; }
+// of a word that is not 0
+__device__ __forceinline__ int first_bit(uint32_t w) { return __ffs((int)w) - 1; }
+__device__ __forceinline__ int first_bit(uint64_t w) { return __ffsll((long long)w) - 1; }
+__device__ __forceinline__ int last_bit(uint32_t w) { return 31 - __clz((int)w); }
+__device__ __forceinline__ int last_bit(uint64_t w) { return 63 - __clzll((long long)w); }
 __device__ __forceinline__ int par64(uint64_t w) { return __popcll(w) & 1; }
-__device__ __forceinline__ uint64_t swapbits(uint64_t w, int i, int j) {
-    const uint64_t t = ((w >> i) ^ (w >> j)) & 1ull;
+template <class W>
+__device__ __forceinline__ W swapbits(W w, int i, int j) {
+    const W t = ((w >> i) ^ (w >> j)) & (W)1;
     return w ^ ((t << i) | (t << j));
 }
 
@@ -55,22 +84,43 @@ __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
     return ((uint64_t)hi << 32) | lo;
 }
 
+__device__ __forceinline__ uint32_t shfl_row(uint32_t v, int src) { return __shfl_sync(kFull, v, src); }
+__device__ __forceinline__ uint64_t shfl_row(uint64_t v, int src) { return shfl64(v, src); }
+
 // Reductions of the warp in one instruction per 32 bits instead of five shuffles:
 // a warp's steps are one serial chain, so their latency is what a state costs.
 __device__ __forceinline__ int warp_sum(int v) { return (int)__reduce_add_sync(kFull, (unsigned)v); }
 __device__ __forceinline__ uint64_t warp_xor64(uint64_t v) {
     return (uint64_t)__reduce_xor_sync(kFull, (uint32_t)v) | ((uint64_t)__reduce_xor_sync(kFull, (uint32_t)(v >> 32)) << 32);
 }
+__device__ __forceinline__ uint32_t warp_xor(uint32_t v) { return __reduce_xor_sync(kFull, v); }
+__device__ __forceinline__ uint64_t warp_xor(uint64_t v) { return warp_xor64(v); }
+__device__ __forceinline__ uint32_t warp_or(uint32_t v) { return __reduce_or_sync(kFull, v); }
 __device__ __forceinline__ uint64_t warp_or64(uint64_t v) {
     return (uint64_t)__reduce_or_sync(kFull, (uint32_t)v) | ((uint64_t)__reduce_or_sync(kFull, (uint32_t)(v >> 32)) << 32);
 }
+__device__ __forceinline__ uint64_t warp_or(uint64_t v) { return warp_or64(v); }
 
 // ------------------------------------------------------------------ state
+// A row of a state with NR rows per lane.  Up to 32 qubits a row is one 32-bit word,
+// and so are the masks over rows: half the instructions of 64-bit rows (drawing and
+// projecting 64,400 states of up to 23 qubits: 347 us, 696 with 64-bit rows).
+template <int NR>
+struct RowType {
+    using type = uint64_t;
+};
+template <>
+struct RowType<1> {
+    using type = uint32_t;
+};
+template <int NR>
+using RW = typename RowType<NR>::type;
+
 template <int NR>
 struct WS {
     int n, k, Q;
-    uint64_t h, D1, D2;
-    uint64_t G[NR], B[NR], J[NR];  // B = Gbar
+    RW<NR> h, D1, D2;
+    RW<NR> G[NR], B[NR], J[NR];  // B = Gbar
 };
 
 template <int NR>
@@ -80,14 +130,14 @@ __device__ __forceinline__ int row_of(int slot) {
 
 // broadcast row idx (uniform) of a lane-distributed matrix
 template <int NR>
-__device__ __forceinline__ uint64_t row_get(const uint64_t (&m)[NR], int idx) {
-    uint64_t v = m[0];
+__device__ __forceinline__ RW<NR> row_get(const RW<NR> (&m)[NR], int idx) {
+    RW<NR> v = m[0];
     if constexpr (NR == 2) v = (idx >= 32) ? m[1] : m[0];
-    return shfl64(v, idx & 31);
+    return shfl_row(v, idx & 31);
 }
 
 template <int NR>
-__device__ __forceinline__ void row_set(uint64_t (&m)[NR], int idx, uint64_t v) {
+__device__ __forceinline__ void row_set(RW<NR> (&m)[NR], int idx, RW<NR> v) {
     if ((idx & 31) == lane_id()) {
         if constexpr (NR == 2) {
             if (idx >= 32) m[1] = v;
@@ -99,48 +149,48 @@ __device__ __forceinline__ void row_set(uint64_t (&m)[NR], int idx, uint64_t v) 
 }
 
 template <int NR>
-__device__ __forceinline__ void row_swap(uint64_t (&m)[NR], int i, int j) {
+__device__ __forceinline__ void row_swap(RW<NR> (&m)[NR], int i, int j) {
     if (i == j) return;
-    const uint64_t ri = row_get<NR>(m, i), rj = row_get<NR>(m, j);
+    const RW<NR> ri = row_get<NR>(m, i), rj = row_get<NR>(m, j);
     row_set<NR>(m, i, rj);
     row_set<NR>(m, j, ri);
 }
 
 // mask over rows x: bit c of row x
 template <int NR>
-__device__ __forceinline__ uint64_t ballot_bit(const uint64_t (&m)[NR], int c) {
-    uint64_t r = __ballot_sync(kFull, (unsigned)((m[0] >> c) & 1ull));
-    if constexpr (NR == 2) r |= (uint64_t)__ballot_sync(kFull, (unsigned)((m[1] >> c) & 1ull)) << 32;
+__device__ __forceinline__ RW<NR> ballot_bit(const RW<NR> (&m)[NR], int c) {
+    RW<NR> r = __ballot_sync(kFull, (unsigned)((m[0] >> c) & 1ull));
+    if constexpr (NR == 2) r |= (RW<NR>)__ballot_sync(kFull, (unsigned)((m[1] >> c) & 1ull)) << 32;
     return r;
 }
 
 // mask over rows x: parity(row_x & v)
 template <int NR>
-__device__ __forceinline__ uint64_t ballot_par(const uint64_t (&m)[NR], uint64_t v) {
-    uint64_t r = __ballot_sync(kFull, (unsigned)par64(m[0] & v));
-    if constexpr (NR == 2) r |= (uint64_t)__ballot_sync(kFull, (unsigned)par64(m[1] & v)) << 32;
+__device__ __forceinline__ RW<NR> ballot_par(const RW<NR> (&m)[NR], RW<NR> v) {
+    RW<NR> r = __ballot_sync(kFull, (unsigned)parity(m[0] & v));
+    if constexpr (NR == 2) r |= (RW<NR>)__ballot_sync(kFull, (unsigned)parity(m[1] & v)) << 32;
     return r;
 }
 
 // XOR of the rows selected by mask
 template <int NR>
-__device__ __forceinline__ uint64_t xor_rows(const uint64_t (&m)[NR], uint64_t mask) {
+__device__ __forceinline__ RW<NR> xor_rows(const RW<NR> (&m)[NR], RW<NR> mask) {
     const int l = lane_id();
-    uint64_t acc = getbit(mask, l) ? m[0] : 0ull;
+    RW<NR> acc = getbit(mask, l) ? m[0] : 0ull;
     if constexpr (NR == 2) acc ^= getbit(mask, l + 32) ? m[1] : 0ull;
-    return warp_xor64(acc);
+    return warp_xor(acc);
 }
 
 template <int NR>
-__device__ __forceinline__ uint64_t ballot_i(int pred0, int pred1) {
-    uint64_t r = __ballot_sync(kFull, (unsigned)pred0);
-    if constexpr (NR == 2) r |= (uint64_t)__ballot_sync(kFull, (unsigned)pred1) << 32;
+__device__ __forceinline__ RW<NR> ballot_i(int pred0, int pred1) {
+    RW<NR> r = __ballot_sync(kFull, (unsigned)pred0);
+    if constexpr (NR == 2) r |= (RW<NR>)__ballot_sync(kFull, (unsigned)pred1) << 32;
     return r;
 }
 
 template <int NR>
-__device__ __forceinline__ bool any_row_nonzero(const uint64_t (&m)[NR]) {
-    uint64_t v = m[0];
+__device__ __forceinline__ bool any_row_nonzero(const RW<NR> (&m)[NR]) {
+    RW<NR> v = m[0];
     if constexpr (NR == 2) v |= m[1];
     return __any_sync(kFull, v != 0ull) != 0;
 }
@@ -156,15 +206,15 @@ __device__ __forceinline__ void setD(WS<NR>& s, int i, int val) {
     const int v2 = val / 2;
     const int d1 = (v2 % 2) & 1;
     const int d2 = (((v2 - v2 % 2) / 2) % 2) & 1;
-    s.D1 = (s.D1 & ~bit1(i)) | ((uint64_t)d1 << i);
-    s.D2 = (s.D2 & ~bit1(i)) | ((uint64_t)d2 << i);
+    s.D1 = (s.D1 & ~bit_of<NR>(i)) | ((RW<NR>)d1 << i);
+    s.D2 = (s.D2 & ~bit_of<NR>(i)) | ((RW<NR>)d2 << i);
 }
 
 // D[x] += d (d in {0,2,4,6} as bits d1, d2) for rows in u, mod 8, bit-sliced
 template <int NR>
-__device__ __forceinline__ void add_D(WS<NR>& s, uint64_t u, int d1, int d2) {
-    const uint64_t a1 = d1 ? u : 0ull, a2 = d2 ? u : 0ull;
-    const uint64_t carry = s.D1 & a1;
+__device__ __forceinline__ void add_D(WS<NR>& s, RW<NR> u, int d1, int d2) {
+    const RW<NR> a1 = d1 ? u : 0ull, a2 = d2 ? u : 0ull;
+    const RW<NR> carry = s.D1 & a1;
     s.D1 ^= a1;
     s.D2 ^= a2 ^ carry;
 }
@@ -173,10 +223,10 @@ __device__ __forceinline__ void add_D(WS<NR>& s, uint64_t u, int d1, int d2) {
 // updateDJ (stabilizer.c:129-160) for R = I + u1 e_c1^T + u2 e_c2^T (c2 < 0: absent).
 // Requires c1, c2 < k and u1, u2 subsets of [0,k) \ {c1, c2}.
 template <int NR>
-__device__ __forceinline__ void apply_R(WS<NR>& s, int c1, uint64_t u1, int c2, uint64_t u2) {
-    const uint64_t km = lowmask(s.k);
-    const uint64_t row1 = row_get<NR>(s.J, c1), col1 = ballot_bit<NR>(s.J, c1);
-    uint64_t row2 = 0ull, col2 = 0ull;
+__device__ __forceinline__ void apply_R(WS<NR>& s, int c1, RW<NR> u1, int c2, RW<NR> u2) {
+    const RW<NR> km = low_mask<NR>(s.k);
+    const RW<NR> row1 = row_get<NR>(s.J, c1), col1 = ballot_bit<NR>(s.J, c1);
+    RW<NR> row2 = 0ull, col2 = 0ull;
     if (c2 >= 0) {
         row2 = row_get<NR>(s.J, c2);
         col2 = ballot_bit<NR>(s.J, c2);
@@ -193,9 +243,9 @@ __device__ __forceinline__ void apply_R(WS<NR>& s, int c1, uint64_t u1, int c2, 
     s.D1 &= km;
     s.D2 &= km;
     // + diag(R J R^T) lower-triangle parity, into D2
-    uint64_t flip = u1 & ((col1 & ~lowmask(c1 + 1)) | (row1 & lowmask(c1)));
+    RW<NR> flip = u1 & ((col1 & ~low_mask<NR>(c1 + 1)) | (row1 & low_mask<NR>(c1)));
     if (c2 >= 0) {
-        flip ^= u2 & ((col2 & ~lowmask(c2 + 1)) | (row2 & lowmask(c2)));
+        flip ^= u2 & ((col2 & ~low_mask<NR>(c2 + 1)) | (row2 & low_mask<NR>(c2)));
         const int jc = (c1 > c2) ? getbit(row1, c2) : getbit(row2, c1);
         if (jc) flip ^= u1 & u2;
     }
@@ -204,10 +254,10 @@ __device__ __forceinline__ void apply_R(WS<NR>& s, int c1, uint64_t u1, int c2, 
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        uint64_t r = s.J[sl];
+        RW<NR> r = s.J[sl];
         if (getbit(u1, x)) r ^= row1;
         if (c2 >= 0 && getbit(u2, x)) r ^= row2;
-        uint64_t r2 = r;
+        RW<NR> r2 = r;
         if (getbit(r, c1)) r2 ^= u1;
         if (c2 >= 0 && getbit(r, c2)) r2 ^= u2;
         s.J[sl] = r2;
@@ -217,7 +267,7 @@ __device__ __forceinline__ void apply_R(WS<NR>& s, int c1, uint64_t u1, int c2, 
 // updateDJ for the permutation swapping basis vectors i and j (both < k)
 template <int NR>
 __device__ __forceinline__ void apply_swap(WS<NR>& s, int i, int j) {
-    const uint64_t km = lowmask(s.k);
+    const RW<NR> km = low_mask<NR>(s.k);
     if (i != j) {
         s.D1 = swapbits(s.D1, i, j);
         s.D2 = swapbits(s.D2, i, j);
@@ -231,41 +281,41 @@ __device__ __forceinline__ void apply_swap(WS<NR>& s, int i, int j) {
 
 // dense updateDJ for a general R (lane-distributed rows), stabilizer.c:129-160
 template <int NR>
-__device__ void update_dj_dense(WS<NR>& s, const uint64_t (&R)[NR]) {
+__device__ void update_dj_dense(WS<NR>& s, const RW<NR> (&R)[NR]) {
     const int n = s.n;
-    const uint64_t km = lowmask(s.k);
+    const RW<NR> km = low_mask<NR>(s.k);
     int v[NR];
 #pragma unroll
     for (int sl = 0; sl < NR; sl++)
-        v[sl] = (__popcll(R[sl] & s.D1 & km) + 2 * __popcll(R[sl] & s.D2 & km)) & 3;
-    const uint64_t nd1 = ballot_i<NR>(v[0] & 1, NR == 2 ? (v[NR - 1] & 1) : 0);
-    const uint64_t nd2 = ballot_i<NR>((v[0] >> 1) & 1, NR == 2 ? ((v[NR - 1] >> 1) & 1) : 0);
+        v[sl] = (popcount(R[sl] & s.D1 & km) + 2 * popcount(R[sl] & s.D2 & km)) & 3;
+    const RW<NR> nd1 = ballot_i<NR>(v[0] & 1, NR == 2 ? (v[NR - 1] & 1) : 0);
+    const RW<NR> nd2 = ballot_i<NR>((v[0] >> 1) & 1, NR == 2 ? ((v[NR - 1] >> 1) & 1) : 0);
     int fl[NR];
-    uint64_t RJ[NR];
+    RW<NR> RJ[NR];
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         fl[sl] = 0;
         RJ[sl] = 0ull;
     }
     for (int b = 0; b < n; b++) {
-        const uint64_t jb = row_get<NR>(s.J, b);
+        const RW<NR> jb = row_get<NR>(s.J, b);
 #pragma unroll
         for (int sl = 0; sl < NR; sl++)
             if (getbit(R[sl], b)) {
-                fl[sl] += __popcll(jb & R[sl] & lowmask(b));
+                fl[sl] += popcount(jb & R[sl] & low_mask<NR>(b));
                 RJ[sl] ^= jb;
             }
     }
-    const uint64_t flip = ballot_i<NR>(fl[0] & 1, NR == 2 ? (fl[NR - 1] & 1) : 0);
+    const RW<NR> flip = ballot_i<NR>(fl[0] & 1, NR == 2 ? (fl[NR - 1] & 1) : 0);
     s.D1 = nd1;
     s.D2 = nd2 ^ flip;
-    uint64_t Jn[NR];
+    RW<NR> Jn[NR];
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) Jn[sl] = 0ull;
     for (int y = 0; y < n; y++) {
-        const uint64_t ry = row_get<NR>(R, y);
+        const RW<NR> ry = row_get<NR>(R, y);
 #pragma unroll
-        for (int sl = 0; sl < NR; sl++) Jn[sl] |= (uint64_t)par64(RJ[sl] & ry) << y;
+        for (int sl = 0; sl < NR; sl++) Jn[sl] |= (RW<NR>)parity(RJ[sl] & ry) << y;
     }
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) s.J[sl] = Jn[sl];
@@ -273,16 +323,16 @@ __device__ void update_dj_dense(WS<NR>& s, const uint64_t (&R)[NR]) {
 
 // updateQD (stabilizer.c:163-177) for a general y
 template <int NR>
-__device__ void update_qd(WS<NR>& s, uint64_t y) {
-    const uint64_t km = lowmask(s.k);
+__device__ void update_qd(WS<NR>& s, RW<NR> y) {
+    const RW<NR> km = low_mask<NR>(s.k);
     int quad = 0;
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        if (x < s.k && getbit(y, x)) quad += __popcll(s.J[sl] & y & km & ~lowmask(x + 1));
+        if (x < s.k && getbit(y, x)) quad += popcount(s.J[sl] & y & km & ~low_mask<NR>(x + 1));
     }
     quad = warp_sum(quad);
-    const int lin = 2 * __popcll(s.D1 & y & km) + 4 * __popcll(s.D2 & y & km);
+    const int lin = 2 * popcount(s.D1 & y & km) + 4 * popcount(s.D2 & y & km);
     s.Q = (s.Q + lin + 4 * quad) % 8;
     s.D2 ^= ballot_par<NR>(s.J, y);
 }
@@ -291,11 +341,11 @@ __device__ void update_qd(WS<NR>& s, uint64_t y) {
 // shrink (stabilizer.c:500-585).  LAZY skips the D/J/Q updates; TRACK_B keeps
 // Gbar up to date (it is dead in the term-product inner loop).
 template <int NR, bool LAZY, bool TRACK_B>
-__device__ __forceinline__ int shrink_core(WS<NR>& s, uint64_t S, int beta) {
+__device__ __forceinline__ int shrink_core(WS<NR>& s, RW<NR> S, int beta) {
     if (S == 0ull) return 1 - beta;
-    const int i = 63 - __clzll((long long)S);
-    const uint64_t U = S & ~bit1(i);
-    const uint64_t gi = row_get<NR>(s.G, i);
+    const int i = last_bit(S);
+    const RW<NR> U = S & ~bit_of<NR>(i);
+    const RW<NR> gi = row_get<NR>(s.G, i);
 #pragma unroll
     for (int sl = 0; sl < NR; sl++)
         if (getbit(U, row_of<NR>(sl))) s.G[sl] ^= gi;
@@ -303,7 +353,7 @@ __device__ __forceinline__ int shrink_core(WS<NR>& s, uint64_t S, int beta) {
     if (!LAZY && !U) {  // updateDJ is still called |S|-1 = 0 times: nothing to do
     }
     if (TRACK_B) {
-        const uint64_t bi = row_get<NR>(s.B, i) ^ xor_rows<NR>(s.B, U);
+        const RW<NR> bi = row_get<NR>(s.B, i) ^ xor_rows<NR>(s.B, U);
         row_set<NR>(s.B, i, bi);
     }
     const int kk = s.k - 1;
@@ -324,16 +374,16 @@ __device__ __forceinline__ int shrink_core(WS<NR>& s, uint64_t S, int beta) {
 }
 
 template <int NR, bool LAZY, bool TRACK_B>
-__device__ __forceinline__ int shrink(WS<NR>& s, uint64_t xi, int alpha) {
-    const uint64_t S = ballot_par<NR>(s.G, xi) & lowmask(s.k);
-    const int beta = (alpha + __popcll(xi & s.h)) % 2;
+__device__ __forceinline__ int shrink(WS<NR>& s, RW<NR> xi, int alpha) {
+    const RW<NR> S = ballot_par<NR>(s.G, xi) & low_mask<NR>(s.k);
+    const int beta = (alpha + popcount(xi & s.h)) % 2;
     return shrink_core<NR, LAZY, TRACK_B>(s, S, beta);
 }
 
 // shrink by the unit vector e_q with alpha = 0
 template <int NR, bool TRACK_B>
 __device__ __forceinline__ int shrink_unit(WS<NR>& s, int q) {
-    const uint64_t S = ballot_bit<NR>(s.G, q) & lowmask(s.k);
+    const RW<NR> S = ballot_bit<NR>(s.G, q) & low_mask<NR>(s.k);
     return shrink_core<NR, false, TRACK_B>(s, S, getbit(s.h, q));
 }
 
@@ -381,13 +431,13 @@ __device__ __forceinline__ void gamma_ab(int A, int B, int& e, int& p, int& m, i
 // (a in DA, partner[a] = b).  The reference accumulates p and m in order and
 // stops at the first zero factor; sums mod 8 make the order irrelevant.
 template <int NR>
-__device__ void wsigma(const WS<NR>& s, int sigma, int sidx, uint64_t Mm, uint64_t DA, const int (&partner)[NR],
+__device__ void wsigma(const WS<NR>& s, int sigma, int sidx, RW<NR> Mm, RW<NR> DA, const int (&partner)[NR],
                        int& e, int& p, int& m, int& err) {
     if (s.k == 0) {
         e = 1; p = 0; m = s.Q;
         return;
     }
-    const uint64_t cs = (sigma && sidx >= 0) ? ballot_bit<NR>(s.J, sidx) : 0ull;
+    const RW<NR> cs = (sigma && sidx >= 0) ? ballot_bit<NR>(s.J, sidx) : 0ull;
     const int tM0 = s.Q + sigma * getD<NR>(s, sidx >= 0 ? sidx : 0);
     int zero = 0, P = 0, Ms = 0;
 #pragma unroll
@@ -427,12 +477,12 @@ __device__ void wsigma(const WS<NR>& s, int sigma, int sidx, uint64_t Mm, uint64
 template <int NR>
 __device__ void exp_sum(WS<NR>& s, int& eps, int& p, int& m, int& err) {
     const int k = s.k;
-    const uint64_t km = lowmask(k);
-    const uint64_t Sm = s.D1 & km;  // D[a] in {2, 6}
+    const RW<NR> km = low_mask<NR>(k);
+    const RW<NR> Sm = s.D1 & km;  // D[a] in {2, 6}
     int sidx = -1;
     if (Sm) {
-        const int a = __ffsll((long long)Sm) - 1;
-        const uint64_t U = Sm & ~bit1(a);
+        const int a = first_bit(Sm);
+        const RW<NR> U = Sm & ~bit_of<NR>(a);
         if (U) apply_R<NR>(s, a, U, -1, 0ull);
         else {
             s.D1 &= km;  // updateDJ with R = I still clears D beyond k
@@ -441,29 +491,29 @@ __device__ void exp_sum(WS<NR>& s, int& eps, int& p, int& m, int& err) {
         apply_swap<NR>(s, a, k - 1);
         sidx = k - 1;
     }
-    uint64_t E = km & ~(sidx >= 0 ? bit1(sidx) : 0ull);
-    uint64_t Mm = 0ull, DA = 0ull;
+    RW<NR> E = km & ~(sidx >= 0 ? bit_of<NR>(sidx) : 0ull);
+    RW<NR> Mm = 0ull, DA = 0ull;
     int partner[NR];
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) partner[sl] = 0;
     while (E) {
-        const int a = __ffsll((long long)E) - 1;
-        const uint64_t ra = row_get<NR>(s.J, a);
-        const uint64_t K = ra & E & ~bit1(a);
+        const int a = first_bit(E);
+        const RW<NR> ra = row_get<NR>(s.J, a);
+        const RW<NR> K = ra & E & ~bit_of<NR>(a);
         if (!K) {
-            Mm |= bit1(a);
-            E &= ~bit1(a);
+            Mm |= bit_of<NR>(a);
+            E &= ~bit_of<NR>(a);
         } else {
-            const int b = __ffsll((long long)K) - 1;
-            const uint64_t Ep = E & ~bit1(a) & ~bit1(b);
-            const uint64_t rb = row_get<NR>(s.J, b);
-            const uint64_t vb = ra & Ep, va = rb & Ep;
+            const int b = first_bit(K);
+            const RW<NR> Ep = E & ~bit_of<NR>(a) & ~bit_of<NR>(b);
+            const RW<NR> rb = row_get<NR>(s.J, b);
+            const RW<NR> vb = ra & Ep, va = rb & Ep;
             if (vb | va) apply_R<NR>(s, b, vb, a, va);
             else {
                 s.D1 &= km;
                 s.D2 &= km;
             }
-            DA |= bit1(a);
+            DA |= bit_of<NR>(a);
 #pragma unroll
             for (int sl = 0; sl < NR; sl++)
                 if (row_of<NR>(sl) == a) partner[sl] = b;
@@ -506,8 +556,8 @@ template <int NR>
 __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int& p, int& m, int& err) {
     const int n = s2.n;
     for (int b = s2.k; b < n; b++) {
-        const uint64_t v = row_get<NR>(s2.B, b);
-        const int alpha = __popcll(s2.h & v) % 2;
+        const RW<NR> v = row_get<NR>(s2.B, b);
+        const int alpha = popcount(s2.h & v) % 2;
         eps = shrink<NR, false, false>(st, v, alpha);
         if (eps == 0) {
             p = 0; m = 0;
@@ -518,14 +568,14 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
     const bool trivial = (s2.Q == 0) && (s2.D1 == 0ull) && (s2.D2 == 0ull) && !any_row_nonzero<NR>(s2.J);
     WS<NR> t2 = s2;
     if (!trivial) {
-        const uint64_t y = ballot_par<NR>(s2.B, st.h ^ s2.h);
-        uint64_t R[NR];
+        const RW<NR> y = ballot_par<NR>(s2.B, st.h ^ s2.h);
+        RW<NR> R[NR];
 #pragma unroll
         for (int sl = 0; sl < NR; sl++) R[sl] = 0ull;
         for (int a = 0; a < n; a++) {
-            const uint64_t g2a = row_get<NR>(s2.B, a);
+            const RW<NR> g2a = row_get<NR>(s2.B, a);
 #pragma unroll
-            for (int sl = 0; sl < NR; sl++) R[sl] |= (uint64_t)par64(st.G[sl] & g2a) << a;
+            for (int sl = 0; sl < NR; sl++) R[sl] |= (RW<NR>)parity(st.G[sl] & g2a) << a;
         }
         update_qd<NR>(t2, y);
         update_dj_dense<NR>(t2, R);
@@ -533,10 +583,10 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
     st.Q -= t2.Q;
     if (st.Q < 0) st.Q += 8;
     {  // D <- (D - D2temp) mod 8 on all n entries, bit-sliced on D/2 mod 4
-        const uint64_t a0 = st.D1, a1 = st.D2, b0 = t2.D1, b1 = t2.D2;
-        const uint64_t borrow = ~a0 & b0;
-        st.D1 = (a0 ^ b0) & lowmask(n);
-        st.D2 = (a1 ^ b1 ^ borrow) & lowmask(n);
+        const RW<NR> a0 = st.D1, a1 = st.D2, b0 = t2.D1, b1 = t2.D2;
+        const RW<NR> borrow = ~a0 & b0;
+        st.D1 = (a0 ^ b0) & low_mask<NR>(n);
+        st.D2 = (a1 ^ b1 ^ borrow) & low_mask<NR>(n);
     }
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) st.J[sl] ^= t2.J[sl];
@@ -547,15 +597,15 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
 // ------------------------------------------------------------------ measurePauli
 // extend (stabilizer.c:759-825)
 template <int NR>
-__device__ void extend(WS<NR>& s, uint64_t xi) {
+__device__ void extend(WS<NR>& s, RW<NR> xi) {
     const int n = s.n, k = s.k;
-    const uint64_t S = ballot_par<NR>(s.B, xi) & lowmask(n);
-    const uint64_t T = (k < n) ? (S & ~lowmask(k)) : 0ull;
+    const RW<NR> S = ballot_par<NR>(s.B, xi) & low_mask<NR>(n);
+    const RW<NR> T = (k < n) ? (S & ~low_mask<NR>(k)) : 0ull;
     if (!T) return;
-    const int i = __ffsll((long long)T) - 1;
-    const uint64_t newS = S & ~bit1(i);
-    const uint64_t gbar_i = row_get<NR>(s.B, i);
-    const uint64_t g_i = row_get<NR>(s.G, i) ^ xor_rows<NR>(s.G, newS);
+    const int i = first_bit(T);
+    const RW<NR> newS = S & ~bit_of<NR>(i);
+    const RW<NR> gbar_i = row_get<NR>(s.B, i);
+    const RW<NR> g_i = row_get<NR>(s.G, i) ^ xor_rows<NR>(s.G, newS);
 #pragma unroll
     for (int sl = 0; sl < NR; sl++)
         if (getbit(newS, row_of<NR>(sl))) s.B[sl] ^= gbar_i;
@@ -571,37 +621,37 @@ __device__ void extend(WS<NR>& s, uint64_t xi) {
 template <int NR>
 __device__ int measure_pauli(WS<NR>& s, int m, uint64_t zeta, uint64_t xi) {
     const int n = s.n, k = s.k;
-    const uint64_t km = lowmask(k);
-    const uint64_t vXi = ballot_par<NR>(s.B, xi) & km;
-    const uint64_t vZeta = ballot_par<NR>(s.G, zeta) & km;
-    const uint64_t xiP = xor_rows<NR>(s.G, vXi);
+    const RW<NR> km = low_mask<NR>(k);
+    const RW<NR> vXi = ballot_par<NR>(s.B, xi) & km;
+    const RW<NR> vZeta = ballot_par<NR>(s.G, zeta) & km;
+    const RW<NR> xiP = xor_rows<NR>(s.G, vXi);
     int quad = 0;
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        if (x < k && getbit(vXi, x)) quad += __popcll(s.J[sl] & vXi & ~lowmask(x + 1));
+        if (x < k && getbit(vXi, x)) quad += popcount(s.J[sl] & vXi & ~low_mask<NR>(x + 1));
     }
     quad = warp_sum(quad);
-    int w = 2 * m + 4 * (__popcll(zeta & s.h) % 2) + 2 * __popcll(s.D1 & vXi) + 4 * __popcll(s.D2 & vXi) + 4 * quad;
+    int w = 2 * m + 4 * (popcount(zeta & s.h) % 2) + 2 * popcount(s.D1 & vXi) + 4 * popcount(s.D2 & vXi) + 4 * quad;
     w = w % 8;
-    const uint64_t eta = ballot_par<NR>(s.J, vXi) ^ vZeta;
+    const RW<NR> eta = ballot_par<NR>(s.J, vXi) ^ vZeta;
     if (xi == xiP) {
         if (w == 0 || w == 4) {
-            const uint64_t gam = xor_rows<NR>(s.B, eta & km);
-            const int alpha = (w / 4 + __popcll(gam & s.h)) % 2;
+            const RW<NR> gam = xor_rows<NR>(s.B, eta & km);
+            const int alpha = (w / 4 + popcount(gam & s.h)) % 2;
             return shrink<NR, false, true>(s, gam, alpha);  // 0 EMPTY, 1 SAME, 2 SUCCESS == result codes
         }
         if (w == 2 || w == 6) {
             const int sigma = 2 - w / 2;
             s.Q = (s.Q + sigma) % 8;
             while (s.Q < 0) s.Q += 8;
-            const uint64_t u = eta & km;  // D[a] -= 2 sigma eta_a  (mod 8, halves mod 4)
+            const RW<NR> u = eta & km;  // D[a] -= 2 sigma eta_a  (mod 8, halves mod 4)
             if (sigma == 1) {
-                const uint64_t borrow = ~s.D1 & u;
+                const RW<NR> borrow = ~s.D1 & u;
                 s.D1 ^= u;
                 s.D2 ^= borrow;
             } else {
-                const uint64_t carry = s.D1 & u;
+                const RW<NR> carry = s.D1 & u;
                 s.D1 ^= u;
                 s.D2 ^= carry;
             }
@@ -612,18 +662,18 @@ __device__ int measure_pauli(WS<NR>& s, int m, uint64_t zeta, uint64_t xi) {
         }
     }
     extend<NR>(s, xi);
-    const int newD = 2 * m + 4 * (__popcll(zeta & xi) % 2) + 4 * (__popcll(zeta & s.h) % 2);
+    const int newD = 2 * m + 4 * (popcount(zeta & xi) % 2) + 4 * (popcount(zeta & s.h) % 2);
     const int kk = s.k - 1;
     if (kk < 0) return -1;  // the reference would fail an assert in setD here
     setD<NR>(s, kk, newD);
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        s.J[sl] = (s.J[sl] & ~bit1(kk)) | ((uint64_t)getbit(vZeta, x) << kk);
+        s.J[sl] = (s.J[sl] & ~bit_of<NR>(kk)) | ((RW<NR>)getbit(vZeta, x) << kk);
     }
-    uint64_t rowk = vZeta;
-    if (m & 1) rowk |= bit1(kk);
-    else rowk &= ~bit1(kk);
+    RW<NR> rowk = vZeta;
+    if (m & 1) rowk |= bit_of<NR>(kk);
+    else rowk &= ~bit_of<NR>(kk);
     row_set<NR>(s.J, kk, rowk);
     return 2;
 }
@@ -693,7 +743,7 @@ __device__ __forceinline__ void init_identity(WS<NR>& s, int n) {
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
         const int x = row_of<NR>(sl);
-        s.G[sl] = x < n ? bit1(x) : 0ull;
+        s.G[sl] = x < n ? bit_of<NR>(x) : 0ull;
         s.B[sl] = s.G[sl];
         s.J[sl] = 0ull;
     }
@@ -711,16 +761,16 @@ __device__ void prep_h(WS<NR>& s, int t, int64_t idx) {
         if (x < t) {
             const int j = x / 2;
             const int bit = (int)((idx >> (size - 1 - j)) & 1);
-            if (bit == 0 && !((t % 2) && j == size - 1)) s.J[sl] |= bit1(x ^ 1);
+            if (bit == 0 && !((t % 2) && j == size - 1)) s.J[sl] |= bit_of<NR>(x ^ 1);
         }
     }
     for (int j = 0; j < size; j++) {
         const int bit = (int)((idx >> (size - 1 - j)) & 1);
         if ((t % 2) && j == size - 1) {
-            if (bit == 1) shrink<NR, false, true>(s, bit1(t - 1), 0);
+            if (bit == 1) shrink<NR, false, true>(s, bit_of<NR>(t - 1), 0);
             continue;
         }
-        if (bit == 1) shrink<NR, false, true>(s, bit1(2 * j + 1) | bit1(2 * j), 0);
+        if (bit == 1) shrink<NR, false, true>(s, bit_of<NR>(2 * j + 1) | bit_of<NR>(2 * j), 0);
     }
 }
 
