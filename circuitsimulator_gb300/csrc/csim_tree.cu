@@ -381,18 +381,25 @@ __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStag
 // ---------------------------------------------------------------- leaves
 __device__ __forceinline__ int64_t shfl_xor_i64(int64_t v, int m) { return (int64_t)shfl_xor64((uint64_t)v, m); }
 
-// ALU-bound (80% of the pipe; the counts run on the XU pipe).  Six blocks per SM:
-// 80 registers without spills; with 128 registers (four blocks) t = 40 is 1.5%
-// slower and t = 48 3.5%, with 72 (seven) within 0.4%.
+// ALU-bound (87% of the pipe at t = 40; the counts run on the XU pipe).  Six blocks per SM:
+// 80 registers; with 128 registers (four blocks) t = 40 is 1.5% slower and t = 48 3.5%, with
+// 72 (seven) within 0.4%.  With ROWS 24 light queries take 2.98 ms with four, 2.93 with five
+// and 2.90 with six, although tables of eight words then spill some registers.
 // ROWS: exactProjector rows, PAIRS: terms of |H^t> (TreeLeafJob).
 template <int WORDS, bool ROWS, bool PAIRS>
-__global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(const TreeLeafJob* jobs, int njobs) {
+__global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLeafJob* jobs, int njobs) {
     __shared__ TableWords words;
+    __shared__ uint32_t gen_s[16], term_s[ROWS ? 16 : 1];  // the levels' generators and their parts of the term index
     __shared__ __align__(16) uint32_t wrows[2 * 8 * kTreeLeafThreads];
     __shared__ int64_t red[kTreeLeafThreads / 32][4];
     const TreeLeafJob& J = job_of(jobs, njobs, blockIdx.x);
     const int tid = threadIdx.x;
-    if (tid < 32) words.fill(tid);
+    if (tid < 32) words.fill(tid, J.tv);
+    else if (tid < 48) {
+        const int b = tid - 32;
+        gen_s[b] = b < J.je ? J.gen[b] : 0u;
+        if constexpr (ROWS) term_s[b] = b < J.je ? (uint32_t)J.term[b] : 0u;
+    }
     __syncthreads();
     const int m = J.m, tv = J.tv;
     const int64_t ti = ((int64_t)blockIdx.x - J.block0) * kTreeLeafThreads + tid;  // thread of the job
@@ -416,24 +423,26 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
         const uint4 w0 = alive && m > 0 ? p[np] : none, w1 = alive && m > 8 ? p[2 * np] : none;
         const int iso0 = (int)((status >> 8) & 0xFFu);
         uint32_t x = hx >> 16;
+        const int split0 = J.je - J.split;  // levels from here up to je are split over threads
         for (int b = 0; b < J.split; b++)
-            if ((part >> b) & 1) x ^= J.gen[J.je - J.split + b];
-        int64_t state = 0, row = 0, term = 0;  // ROWS: the state, its row, and the term index so far
+            if ((part >> b) & 1) x ^= gen_s[split0 + b];
+        int state = 0;  // ROWS: the state, its row, and the term index so far (below 2^30)
+        uint32_t row = 0, term = 0;
         if constexpr (ROWS) {
-            state = node >> J.nodes_log2;
-            row = J.row0 + state;
+            state = (int)(node >> J.nodes_log2);
+            row = (uint32_t)(J.row0 + state);
             for (int b = 0; b < J.nodes_log2; b++)
-                if ((node >> b) & 1) term ^= (int64_t)J.term[J.je + b];
+                if ((node >> b) & 1) term ^= (uint32_t)J.term[J.je + b];
             for (int b = 0; b < J.split; b++)
-                if ((part >> b) & 1) term ^= (int64_t)J.term[J.je - J.split + b];
+                if ((part >> b) & 1) term ^= term_s[split0 + b];
         }
         int y[4] = {0, 0, 0, 0};  // this part's sum, relative to 2^{iso0 / 2}
         // table nodes two at a time, in Gray code order
         for (int s = 0; s < nsub; s += 2) {
-            if (s) x ^= J.gen[tj + __ffs(s) - 1];
+            if (s) x ^= gen_s[tj + __ffs(s) - 1];
             if constexpr (ROWS)
-                if (s) term ^= (int64_t)J.term[tj + __ffs(s) - 1];
-            const uint32_t x2 = nsub > 1 ? x ^ J.gen[tj] : x;
+                if (s) term ^= term_s[tj + __ffs(s) - 1];
+            const uint32_t x2 = nsub > 1 ? x ^ gen_s[tj] : x;
             Work<uint32_t> wa, wb;
             wa.s = Node<uint32_t>{dd & 0xFFFFu, dd >> 16, hx & 0xFFFFu, (int)(status & 7u), 0, 0};
             wb = wa;
@@ -490,23 +499,23 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
                 };
                 int v[4];
                 if constexpr (ROWS) {
-                    int64_t j = e ? term ^ (int64_t)J.term[tj] : term;
+                    uint32_t j = e ? term ^ term_s[tj] : term;
                     for (int l = 0; l < (1 << tj); l++) {
                         if (l) {
-                            S ^= J.gen[__ffs(l) - 1] & vm;
-                            j ^= (int64_t)J.term[__ffs(l) - 1];
+                            S ^= gen_s[__ffs(l) - 1] & vm;
+                            j ^= term_s[__ffs(l) - 1];
                         }
-                        if (j > row) table_leaf<WORDS>(tb, S, d1, tv, words.sub, evr, evi, odr, odi);
+                        if (j > row) table_leaf<WORDS>(tb, S, d1, words, evr, evi, odr, odi);
                         if (j == row && alive) {  // one leaf of a state
                             const int keep[4] = {evr, evi, odr, odi};
                             evr = evi = odr = odi = 0;
-                            if (!nd.dead) table_leaf<WORDS>(tb, S, d1, tv, words.sub, evr, evi, odr, odi);
+                            if (!nd.dead) table_leaf<WORDS>(tb, S, d1, words, evr, evi, odr, odi);
                             node_sum(v);
                             int64_t dz[4];
                             if (iso0 & 1) times_sqrt2(v);
                             for (int q = 0; q < 4; q++) dz[q] = (int64_t)v[q] << (iso0 >> 1);
                             if (J.shift & 1) times_sqrt2(dz);
-                            for (int q = 0; q < 4; q++) J.diag[4 * state + q] = (__int128)dz[q] << (J.shift >> 1);
+                            for (int q = 0; q < 4; q++) J.diag[4 * (int64_t)state + q] = (__int128)dz[q] << (J.shift >> 1);
                             evr = keep[0];
                             evi = keep[1];
                             odr = keep[2];
@@ -515,8 +524,8 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
                     }
                 } else {
                     for (int l = 0; l < (1 << tj); l++) {
-                        if (l) S ^= J.gen[__ffs(l) - 1] & vm;
-                        table_leaf<WORDS>(tb, S, d1, tv, words.sub, evr, evi, odr, odi);
+                        if (l) S ^= gen_s[__ffs(l) - 1] & vm;
+                        table_leaf<WORDS>(tb, S, d1, words, evr, evi, odr, odi);
                     }
                 }
                 if (alive && !nd.dead) {
@@ -527,7 +536,7 @@ __global__ void __launch_bounds__(kTreeLeafThreads, ROWS ? 4 : 6) k_tree_leaf(co
             }
             if (nsub > 1) {
                 x = x2;
-                if constexpr (ROWS) term ^= (int64_t)J.term[tj];
+                if constexpr (ROWS) term ^= term_s[tj];
             }
         }
         if (iso0 & 1) times_sqrt2(y);

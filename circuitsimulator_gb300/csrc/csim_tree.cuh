@@ -437,12 +437,22 @@ CSIM_HD_INLINE uint32_t edges_word(uint32_t r) {
     return w;
 }
 struct TableWords {
+    // by 2 |S| + (S meets D1): the points of S with p0 = 0 and p0 = 1, and 2^{(v - |S|) / 2} as
+    // c + sqrt2 d
+    U32x4 scale[2 * kTableVars + 2];
     uint32_t lin[32], sub[32], edges[64];
-    CSIM_HD_INLINE void fill(int i) {  // i = 0 .. 31
+    CSIM_HD_INLINE void fill(int i, int v) {  // i = 0 .. 31; tables of v vertices
         lin[i] = linear_word((uint32_t)i);
         sub[i] = subset_word((uint32_t)i);
         edges[i] = edges_word((uint32_t)i);
         edges[32 + i] = edges_word((uint32_t)(32 + i));
+        const int size = i >> 1;
+        if (size <= v && size <= kTableVars) {
+            const uint32_t n = 1u << size, n1 = (i & 1) ? n >> 1 : 0u;
+            const int e = v - size;
+            const uint32_t one = 1u << (e >> 1);
+            scale[i] = U32x4{n - n1, n1, (e & 1) ? 0u : one, (e & 1) ? one : 0u};
+        }
     }
 };
 
@@ -480,11 +490,11 @@ CSIM_HD_INLINE void build_table(uint32_t r0, uint32_t r4, uint32_t d1, uint32_t 
 }
 // 2^{-|S|/2} sum_{z in S} i^{p0 + 2 p1}, times 2^{v/2}, added to ev + sqrt2 od (re, im each)
 template <int WORDS>
-CSIM_HD_INLINE void table_leaf(const Table<WORDS>& t, uint32_t S, uint32_t d1, int v, const uint32_t* sub, int& evr,
-                               int& evi, int& odr, int& odi) {
+CSIM_HD_INLINE void table_leaf(const Table<WORDS>& t, uint32_t S, uint32_t d1, const TableWords& tw, int& evr, int& evi,
+                               int& odr, int& odi) {
     using T = WordTraits<uint32_t>;
     uint32_t mk[WORDS];
-    mk[0] = sub[S & 31u];
+    mk[0] = tw.sub[S & 31u];
     int na = T::popc(mk[0] & t.a[0]), nc = T::popc(mk[0] & t.c[0]);
 #pragma unroll
     for (int w = 1; w < WORDS; w++) {
@@ -493,14 +503,12 @@ CSIM_HD_INLINE void table_leaf(const Table<WORDS>& t, uint32_t S, uint32_t d1, i
         na += T::popc(mk[w] & t.a[w]);
         nc += T::popc(mk[w] & t.c[w]);
     }
-    const int size = T::popc(S), n = 1 << size;
-    const int n1 = (S & d1) ? n >> 1 : 0;  // points with p0 = 1
-    const int re = n - n1 - 2 * na, im = n1 - 2 * nc;
-    const int e = v - size, one = 1 << (e >> 1), mo = (e & 1) ? one : 0, me = one - mo;
-    evr += re * me;
-    evi += im * me;
-    odr += re * mo;
-    odi += im * mo;
+    const U32x4 sc = tw.scale[2 * T::popc(S) + ((S & d1) != 0u ? 1 : 0)];
+    const int re = (int)sc.a - 2 * na, im = (int)sc.b - 2 * nc;
+    evr += re * (int)sc.c;
+    evi += im * (int)sc.c;
+    odr += re * (int)sc.d;
+    odi += im * (int)sc.d;
 }
 CSIM_HD_INLINE int table_words(int v) { return v > 5 ? 1 << (v - 5) : 1; }
 

@@ -138,7 +138,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
         for (size_t i = 0; i < p.level.size(); i++) info[3 + i] = p.vert[i];
     }
     TableWords tables;
-    for (int i = 0; i < 32; i++) tables.fill(i);
+    for (int i = 0; i < 32; i++) tables.fill(i, p.tv);
     const int words = table_words(p.tv);
     for (int a = 0; a < ntheta; a++) {
         std::vector<HostNode> cur{root_of(theta[a], p)};
@@ -179,7 +179,7 @@ extern "C" int tree_host_sums(const csim_state* theta, int ntheta, const uint64_
                     build_table(r[0], r[1], d1, (uint32_t)n.d2 & vm, tables, tb);
                     for (int l = 0; l < (1 << p.tj); l++) {
                         if (l) S ^= (uint32_t)p.gen[__builtin_ctz((unsigned)l)] & vm;
-                        table_leaf(tb, S, d1, p.tv, tables.sub, e0, e1, o0, o1);
+                        table_leaf(tb, S, d1, tables, e0, e1, o0, o1);
                     }
                 };
                 if (words == 1) leaves(Table<1>());
