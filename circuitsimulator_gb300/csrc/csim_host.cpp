@@ -542,25 +542,32 @@ void tree_plan_for(csim_ctx* ctx, int exact, const uint64_t* L, int k, int t, in
     csim::tree::choose_levels(ctx->tree_plan, count);
 }
 
-// A sampler call's inputs on the device, one upload: the projector's rows, the
-// d-distribution of randomStabilizerState, the projection factors, the tree plan, the code
+// A call's inputs on the device, one upload: the tree's job tables, the projector's rows,
+// the d-distribution of randomStabilizerState, the projection factors, the tree plan, the
+// code and the zero head of the results, which lie behind them
 struct CallInputs {
     const int* pm;
     const uint64_t *pz, *px;
     const double *cum, *factor;
     const unsigned char* plan;
     const uint64_t* L;
+    unsigned char* results;  // `head` bytes that are zero once the inputs are sent, then the rest
+    unsigned char *host, *dev;
+    size_t bytes;
 };
-int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Plan* plan, CallInputs* in,
-                    const uint64_t* L = nullptr, int k = 0) {
+constexpr size_t kCallJobs = 16 << 10;  // room for job tables in front
+
+// Makes the inputs, with room for `results` bytes (head of them zero); send_inputs uploads them
+int make_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Plan* plan, size_t head, size_t results,
+                CallInputs* in, const uint64_t* L = nullptr, int k = 0) {
     const size_t n = (size_t)P->nstabs;
-    const size_t o_px = 8 * n, o_cum = 16 * n, o_factor = o_cum + 8 * (CSIM_MAX_QUBITS + 1),
+    const size_t o_pz = kCallJobs, o_px = o_pz + 8 * n, o_cum = o_px + 8 * n, o_factor = o_cum + 8 * (CSIM_MAX_QUBITS + 1),
                  o_plan = o_factor + 8 * (n + 1), o_L = o_plan + kTreePlanBytes, o_pm = o_L + 8 * (size_t)k,
-                 bytes = o_pm + 4 * n;
+                 o_res = (o_pm + 4 * n + 15) / 16 * 16;
     void* v;
-    CKR(staged_room(ctx, 1, bytes, &v));
+    CKR(staged_room(ctx, 1, o_res + head, &v));
     unsigned char* const h = (unsigned char*)v;
-    if (n) memcpy(h, P->zs, 8 * n);
+    if (n) memcpy(h + o_pz, P->zs, 8 * n);
     if (n) memcpy(h + o_px, P->xs, 8 * n);
     cum_table(P->nqubits, (double*)(h + o_cum));
     for (size_t c = 0; c <= n; c++) ((double*)(h + o_factor))[c] = sqrt_half_power((int)c);
@@ -568,46 +575,56 @@ int put_call_inputs(csim_ctx* ctx, const csim_projector* P, const csim::tree::Pl
     else memset(h + o_plan, 0, kTreePlanBytes);
     if (k) memcpy(h + o_L, L, 8 * (size_t)k);
     for (size_t r = 0; r < n; r++) ((int32_t*)(h + o_pm))[r] = phase_m(P->phase[r]);
-    CKR(staged_send(ctx, 1, kBufCall, bytes, &v));
-    const unsigned char* const d = (const unsigned char*)v;
-    in->pz = (const uint64_t*)d;
-    in->px = (const uint64_t*)(d + o_px);
-    in->cum = (const double*)(d + o_cum);
-    in->factor = (const double*)(d + o_factor);
-    in->plan = d + o_plan;
-    in->L = (const uint64_t*)(d + o_L);
-    in->pm = (const int*)(d + o_pm);
+    memset(h + o_pm + 4 * n, 0, o_res + head - (o_pm + 4 * n));
+    CKR(dbuf(ctx, kBufCall, o_res + results, &v));
+    unsigned char* const d = (unsigned char*)v;
+    *in = CallInputs{(const int*)(d + o_pm), (const uint64_t*)(d + o_pz), (const uint64_t*)(d + o_px),
+                     (const double*)(d + o_cum), (const double*)(d + o_factor), d + o_plan, (const uint64_t*)(d + o_L),
+                     d + o_res, h, d, o_res + head};
+    return 0;
+}
+// Uploads them with the job tables (*djobs; larger ones go alone)
+int send_inputs(csim_ctx* ctx, const CallInputs& in, const std::vector<unsigned char>& jobs, unsigned char** djobs) {
+    size_t from = kCallJobs;
+    if (!jobs.empty() && jobs.size() <= kCallJobs) {
+        from = (kCallJobs - jobs.size()) / 256 * 256;
+        memcpy(in.host + from, jobs.data(), jobs.size());
+        *djobs = in.dev + from;
+    } else if (!jobs.empty()) {
+        CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), djobs));
+    }
+    CK(cudaMemcpyAsync(in.dev + from, in.host + from, in.bytes - from, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaEventRecord(ctx->pin_ev[1], ctx->stream));
+    ctx->stats.h2d_bytes += (int64_t)(in.bytes - from);
     return 0;
 }
 
-// The raw words of the next `count` states in pinned slots `slot` (words) and
-// slot + 1 (offsets), and their upload; *chain: where they end
-int put_state_words(csim_ctx* ctx, int slot, int t, const double* cum, int64_t count, const uint32_t** dwords,
+// The raw words of the next `count` states and their offsets in pinned slot 3, and their
+// upload; *chain: where they end
+int put_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, const uint32_t** dwords,
                     const int64_t** doffs, csim::DrawChain* chain) {
-    void *v, *o;
-    CKR(staged_room(ctx, slot, (kRawHistory + (size_t)count * state_words(t)) * 4, &v));
-    CKR(staged_room(ctx, slot + 1, (size_t)(count + 1) * 8, &o));
-    RawWords w{(uint32_t*)v, kRawHistory, ctx->pin_cap[slot] / 4};
-    int64_t* const offs = (int64_t*)o;
+    const size_t head = (size_t)(count + 1) * 8;
+    void* v;
+    CKR(staged_room(ctx, 3, head + (kRawHistory + (size_t)count * state_words(t)) * 4, &v));
+    RawWords w{(uint32_t*)((unsigned char*)v + head), kRawHistory, (ctx->pin_cap[3] - head) / 4};
     ctx->lr.history(w.p);
     auto grow = [&](size_t more) {
         const size_t cap = w.cap + w.cap / 2 + more;
-        if (staged_grow(ctx, slot, cap * 4, w.n * 4, &v)) return false;
-        w.p = (uint32_t*)v;
+        if (staged_grow(ctx, 3, head + cap * 4, head + w.n * 4, &v)) return false;
+        w.p = (uint32_t*)((unsigned char*)v + head);
         w.cap = cap;
         return true;
     };
     for (int64_t i = 0; i < count; i++) {
-        offs[i] = (int64_t)w.n;
+        ((int64_t*)v)[i] = (int64_t)w.n;
         if (!draw_state_words(w, t, cum, grow)) return CSIM_ERR_NOMEM;
     }
-    offs[count] = (int64_t)w.n;
+    ((int64_t*)v)[count] = (int64_t)w.n;
     chain->states = count;
     memcpy(chain->history, w.p + w.n - kRawHistory, sizeof(chain->history));
-    CKR(staged_send(ctx, slot, kBufWords, w.n * 4, &v));
-    *dwords = (const uint32_t*)v;
-    CKR(staged_send(ctx, slot + 1, kBufOffsets, (size_t)(count + 1) * 8, &v));
+    CKR(staged_send(ctx, 3, kBufWords, head + w.n * 4, &v));
     *doffs = (const int64_t*)v;
+    *dwords = (const uint32_t*)((unsigned char*)v + head);
     return 0;
 }
 
@@ -685,8 +702,12 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int64_t nchunks = tree ? tree_leaf_shape(ctx->tree_plan, shape_count).parts_per_state
                                  : (tp ? csim::terms_tp_blocks(chi, pt) : (chi + chunk - 1) / chunk);
 
+    const bool libc = rng == CSIM_RNG_LIBC;
+    constexpr size_t head = 16 + (sizeof(csim::DrawChain) + 15) / 16 * 16;  // results: live states, error, chain, values
     CallInputs in;
-    CKR(put_call_inputs(ctx, P, tree ? &ctx->tree_plan : nullptr, &in));
+    CKR(make_inputs(ctx, P, tree ? &ctx->tree_plan : nullptr, 16, head + (size_t)std::min(count, batch) * 8, &in));
+    if (!tree) CKR(send_inputs(ctx, in, {}, nullptr));
+    unsigned char* const dres = in.results;
     double hcum[CSIM_MAX_QUBITS + 1];
     cum_table(t, hcum);
     uint64_t* dcw = nullptr;
@@ -707,14 +728,11 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     std::vector<unsigned char> jobs;
     std::vector<int> code;
     std::vector<__int128> acc;
-    const bool libc = rng == CSIM_RNG_LIBC;
-    constexpr size_t head = 16 + (sizeof(csim::DrawChain) + 15) / 16 * 16;  // results: live states, error, chain, values
+    bool sent = !tree;
     int more = 0;  // a batch that ran out of words runs again with twice as many
     for (int64_t o = 0; o < count;) {
         const int64_t c = std::min(batch, count - o);
         void* v;
-        CKR(dbuf(ctx, kBufResults, head + (size_t)c * 8, &v));
-        unsigned char* const dres = (unsigned char*)v;
         csim::GState* dth = nullptr;  // the tree's states stay in registers
         if (!tree) {
             CKR(dbuf(ctx, kBufA, c * sizeof(csim_state), &v));
@@ -748,7 +766,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         if (libc) {
             const uint32_t* dw;
             const int64_t* doff;
-            if (on_host) CKR(put_state_words(ctx, 3, t, hcum, c, &dw, &doff, &chain));
+            if (on_host) CKR(put_state_words(ctx, t, hcum, c, &dw, &doff, &chain));
             else CKR(make_state_words(ctx, t, hcum, c, (most + 4096) << more, &dw, &doff, (csim::DrawChain*)(dres + 16)));
             draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, dcode, nullptr, 0, 0};
             if (!tree && csim::launch_random_states(launch_of(ctx), t, c, 2, 0, 0, dw, doff, in.cum, dth, nullptr))
@@ -783,7 +801,13 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             unsigned char* djobs;
             CKR(run.reserve({g}, [&](size_t bytes) { return dbuf(ctx, kBufTreeScratch, bytes, &scratch); }));
             run.build((unsigned char*)scratch, jobs);
-            CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+            if (!sent) {
+                CKR(send_inputs(ctx, in, jobs, &djobs));
+                sent = true;
+            } else {
+                CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+                CK(cudaMemsetAsync(dres, 0, 16, ctx->stream));
+            }
             // the event that starts the pair kernels' time is recorded behind the first roots
             rc = run.launch(launch_of(ctx), djobs, ctx->ev[1]);
         } else if (tp && tn.kernel == 2) {
@@ -846,11 +870,9 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         if (rc) return fail(ctx, CSIM_ERR_CUDA, "term launch failed");
         CK(cudaEventRecord(ctx->ev[2], ctx->stream));
         if (tree) {
-            CK(cudaMemsetAsync(dres, 0, 16, ctx->stream));
             if (csim::launch_tree_values(launch_of(ctx), dpart, c, nchunks, t, dcode, in.factor, (double*)(dres + head),
                                          (unsigned long long*)dres))
                 return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
-            CK(cudaMemcpyAsync(dres + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
             CK(cudaEventRecord(ctx->ev[3], ctx->stream));
             CKR(staged_room(ctx, 2, head + (size_t)c * 8, &v));
             CKR(dget(ctx, (unsigned char*)v, dres, head + (size_t)c * 8));
@@ -1152,7 +1174,9 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     void* v;
     CallInputs in;
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
-    CKR(put_call_inputs(ctx, P, &plan, &in, exact ? nullptr : L, exact ? 0 : k));
+    // results: the live rows' count, the error word, the live rows' terms, re, im
+    const size_t head = 32, bytes = head + (size_t)nrow * 16;
+    CKR(make_inputs(ctx, P, &plan, head, bytes, &in, exact ? nullptr : L, exact ? 0 : k));
     CKR(dbuf(ctx, kBufCode, (size_t)nrow * 4, &v));
     int* const dcode = (int*)v;
     CKR(dbuf(ctx, kBufParts, (size_t)nrow * parts * 64, &v));
@@ -1176,19 +1200,14 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     unsigned char* djobs;
     CKR(run.reserve({g}, [&](size_t bytes) { return dbuf(ctx, kBufTreeScratch, bytes, &scratch); }));
     run.build((unsigned char*)scratch, jobs);
-    CKR(staged_put(ctx, 0, kBufTreeJobs, jobs.data(), jobs.size(), &djobs));
+    CKR(send_inputs(ctx, in, jobs, &djobs));
     if (run.launch(launch_of(ctx), djobs, ctx->ev[1]))
         return fail(ctx, CSIM_ERR_CUDA, "tree launch failed");
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    // results: the live rows' count, the error word, the live rows' terms, re, im
-    const size_t head = 32, bytes = head + (size_t)nrow * 16;
-    CKR(dbuf(ctx, kBufResults, bytes, &v));
-    unsigned char* const dres = (unsigned char*)v;
-    CK(cudaMemsetAsync(dres, 0, head, ctx->stream));
+    unsigned char* const dres = in.results;
     if (csim::launch_tree_rows(launch_of(ctx), dpart, ddiag, nrow, parts, t, dcode, in.factor, (double*)(dres + head),
                                (double*)(dres + head) + nrow, (unsigned long long*)dres, chi - i0))
         return fail(ctx, CSIM_ERR_CUDA, "reduce launch failed");
-    CK(cudaMemcpyAsync(dres + 8, ctx->d_err, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
     CKR(staged_room(ctx, 2, bytes, &v));
     CKR(dget(ctx, (unsigned char*)v, dres, bytes));

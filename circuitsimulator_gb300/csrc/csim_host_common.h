@@ -412,10 +412,10 @@ enum BufId {
     kBufA, kBufB, kBufEps, kBufP, kBufM, kBufXi, kBufZeta, kBufAlpha, kBufCode, kBufWords, kBufOffsets,
     kBufCum, kBufCodewords, kBufAcc, kBufAccDiag, kBufPhis, kBufIdx, kBufConsumed, kBufPm, kBufPz, kBufPx,
     kBufL, kBufParts, kBufPartsDiag, kBufCwOrdered, kBufRunScratch, kBufCanon, kBufCodeDirect, kBufCodeRest,
-    kBufRestCount, kBufTreeJobs, kBufTreeScratch, kBufCall, kBufResults, kBufLengths, kBufChainMaps, kNumBufs
+    kBufRestCount, kBufTreeJobs, kBufTreeScratch, kBufCall, kBufLengths, kBufChainMaps, kNumBufs
 };
 
-constexpr int kPinSlots = 5;      // tree jobs, a call's inputs, its results, words, offsets
+constexpr int kPinSlots = 4;      // tree jobs, a call's inputs, its results, words and offsets
 
 class Engine;                     // csim_engine.cpp: the batched query engine
 void engine_free(Engine* engine);  // releases it and its device memory

@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
 __global__ void __launch_bounds__(128) k_tree_values(const __int128* part, const __int128* diag, int64_t count,
                                                      int64_t parts, int t, const int* code, const double* factor,
                                                      double* out, double* im_out, unsigned long long* live,
-                                                     int64_t row_terms) {
+                                                     int64_t row_terms, const int* err) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= count) return;  // warp-uniform
     const int lane = lane_id(), q = lane & 3;
@@ -589,6 +589,7 @@ __global__ void __launch_bounds__(128) k_tree_values(const __int128* part, const
     double a, b;
     warp_value(z, diag != nullptr, d, t, factor[c >= 0 ? c : 0], a, b);
     if (lane != 0) return;
+    if (i == 0) *(int*)(live + 1) = *err;  // of the kernels before
     if (c >= 0) {
         atomicAdd(live, 1ull);
         if (diag) atomicAdd(live + 2, (unsigned long long)(row_terms - i));
@@ -650,7 +651,7 @@ int launch_tree_values(const Launch& L, const __int128* part, int64_t count, int
                        const double* factor, double* values, unsigned long long* live) {
     if (count <= 0) return 0;
     k_tree_values<<<(unsigned)((count + 3) / 4), 128, 0, L.stream>>>(part, nullptr, count, parts, t, code, factor, values,
-                                                                     nullptr, live, 0);
+                                                                     nullptr, live, 0, L.d_err);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -660,7 +661,7 @@ int launch_tree_rows(const Launch& L, const __int128* part, const __int128* diag
                      int64_t row_terms) {
     if (count <= 0) return 0;
     k_tree_values<<<(unsigned)((count + 3) / 4), 128, 0, L.stream>>>(part, diag, count, parts, t, code, factor, re, im,
-                                                                     live, row_terms);
+                                                                     live, row_terms, L.d_err);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -84,7 +84,8 @@ int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int6
 int launch_tree_leaf(const Launch& L, const TreeLeafJob* jobs, int njobs, int64_t blocks, int words, bool rows,
                      bool pairs);
 
-// values[i] of `count` states from `parts` partial sums each; factor: 65 doubles; *live is added to
+// values[i] of `count` states from `parts` partial sums each; factor: 65 doubles; *live is added to,
+// the low word of live[1] becomes the device error word
 int launch_tree_values(const Launch& L, const __int128* part, int64_t count, int64_t parts, int t, const int* code,
                        const double* factor, double* values, unsigned long long* live);
 // the rows' values of exactProjector: re[i] + i im[i] = factor (diag + 2 Re sum of the parts);
