@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256) k_exp_sum(GState* s, int64_t count, int* 
         load_state<NR>(s + i, st);
         int ee = 0, pp = 0, mm = 0;
         if (!n_ok(st.n, NR)) e |= kErrArg;
-        else exp_sum<NR>(st, ee, pp, mm, e);
+        else exp_sum<NR, true>(st, ee, pp, mm, e);
         store_state<NR>(s + i, st);
         if (lane_id() == 0) {
             eps[i] = ee;
@@ -270,7 +270,7 @@ __device__ __forceinline__ void pair_l(WS<NR> st, uint64_t x, int& eps, int& p, 
             return;
         }
     }
-    exp_sum<NR>(st, eps, p, m, err);
+    exp_sum<NR, false>(st, eps, p, m, err);
     p -= k1 + k2;
 }
 

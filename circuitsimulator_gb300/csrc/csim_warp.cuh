@@ -59,13 +59,13 @@ __device__ __forceinline__ auto low_mask(int k) {
 __device__ __forceinline__ int popcount(uint32_t w) { return __popc(w); }
 __device__ __forceinline__ int popcount(uint64_t w) { return __popcll(w); }
 __device__ __forceinline__ int parity(uint32_t w) { return __popc(w) & 1; }
-__device__ __forceinline__ int parity(uint64_t w) { return __popcll(w) & 1; }
+__device__ __forceinline__ int parity(uint64_t w) { return __popc((uint32_t)w ^ (uint32_t)(w >> 32)) & 1; }
+__device__ __forceinline__ int par64(uint64_t w) { return parity(w); }
 // of a word that is not 0
 __device__ __forceinline__ int first_bit(uint32_t w) { return __ffs((int)w) - 1; }
 __device__ __forceinline__ int first_bit(uint64_t w) { return __ffsll((long long)w) - 1; }
 __device__ __forceinline__ int last_bit(uint32_t w) { return 31 - __clz((int)w); }
 __device__ __forceinline__ int last_bit(uint64_t w) { return 63 - __clzll((long long)w); }
-__device__ __forceinline__ int par64(uint64_t w) { return __popcll(w) & 1; }
 template <class W>
 __device__ __forceinline__ W swapbits(W w, int i, int j) {
     const W t = ((w >> i) ^ (w >> j)) & (W)1;
@@ -279,46 +279,81 @@ __device__ __forceinline__ void apply_swap(WS<NR>& s, int i, int j) {
     s.D2 &= km;
 }
 
-// dense updateDJ for a general R (lane-distributed rows), stabilizer.c:129-160
+// Rows of a matrix for all lanes of the warp to read: a load from shared memory that all
+// lanes share is one instruction for two words, a row from a lane's registers four.
+template <int NR>
+struct alignas(2 * sizeof(RW<NR>)) RowPair {
+    RW<NR> a, b;
+};
+template <int NR>
+__device__ __forceinline__ RowPair<NR>* warp_rows() {
+    __shared__ RowPair<NR> rows_s[8][32 * NR];  // blocks have at most 8 warps
+    return rows_s[threadIdx.x >> 5];
+}
+template <int NR>
+__device__ __forceinline__ void share_rows(RowPair<NR>* rows, const RW<NR> (&a)[NR], const RW<NR> (&b)[NR]) {
+    __syncwarp();
+#pragma unroll
+    for (int sl = 0; sl < NR; sl++) rows[row_of<NR>(sl)] = RowPair<NR>{a[sl], b[sl]};
+    __syncwarp();
+}
+// out[x] bit y = parity(m[x] & row y) for the shared rows y < n
+template <int NR>
+__device__ __forceinline__ void parity_rows(const RowPair<NR>* rows, const RW<NR> (&m)[NR], int n, RW<NR> (&out)[NR]) {
+#pragma unroll
+    for (int sl = 0; sl < NR; sl++) out[sl] = 0;
+#pragma unroll
+    for (int h = 0; h < NR; h++) {  // 32 bits of the result at a time, the highest first
+        uint32_t w[NR] = {};
+#pragma unroll 4
+        for (int y = (n < 32 * (h + 1) ? n : 32 * (h + 1)) - 1; y >= 32 * h; y--) {
+            const RW<NR> r = rows[y].a;
+#pragma unroll
+            for (int sl = 0; sl < NR; sl++) w[sl] = 2u * w[sl] + (uint32_t)parity(m[sl] & r);
+        }
+#pragma unroll
+        for (int sl = 0; sl < NR; sl++) out[sl] |= (RW<NR>)w[sl] << (32 * h);
+    }
+}
+
+// updateDJ (stabilizer.c:129-160) for a general R (lane-distributed rows) of columns < s.k: D and J
+// of the rows of R
 template <int NR>
 __device__ void update_dj_dense(WS<NR>& s, const RW<NR> (&R)[NR]) {
-    const int n = s.n;
-    const RW<NR> km = low_mask<NR>(s.k);
+    const int k = s.k;
+    const RW<NR> km = low_mask<NR>(k);
     int v[NR];
 #pragma unroll
-    for (int sl = 0; sl < NR; sl++)
-        v[sl] = (popcount(R[sl] & s.D1 & km) + 2 * popcount(R[sl] & s.D2 & km)) & 3;
+    for (int sl = 0; sl < NR; sl++) v[sl] = (popcount(R[sl] & s.D1 & km) + 2 * popcount(R[sl] & s.D2 & km)) & 3;
     const RW<NR> nd1 = ballot_i<NR>(v[0] & 1, NR == 2 ? (v[NR - 1] & 1) : 0);
     const RW<NR> nd2 = ballot_i<NR>((v[0] >> 1) & 1, NR == 2 ? ((v[NR - 1] >> 1) & 1) : 0);
-    int fl[NR];
-    RW<NR> RJ[NR];
+    // R J, and R times J's part below the diagonal (whose product with R is the sum over pairs)
+    RowPair<NR>* const rows = warp_rows<NR>();
+    RW<NR> below[NR], RJ[NR], RL[NR];
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) {
-        fl[sl] = 0;
-        RJ[sl] = 0ull;
+        below[sl] = s.J[sl] & low_mask<NR>(row_of<NR>(sl));
+        RJ[sl] = RL[sl] = 0;
     }
-    for (int b = 0; b < n; b++) {
-        const RW<NR> jb = row_get<NR>(s.J, b);
+    share_rows<NR>(rows, s.J, below);
 #pragma unroll
-        for (int sl = 0; sl < NR; sl++)
-            if (getbit(R[sl], b)) {
-                fl[sl] += popcount(jb & R[sl] & low_mask<NR>(b));
-                RJ[sl] ^= jb;
-            }
+    for (int h = 0; h < NR; h++) {
+        const int end = k < 32 * (h + 1) ? k - 32 * h : 32;
+#pragma unroll 4
+        for (int b = 0; b < end; b++) {
+            const RowPair<NR> r = rows[32 * h + b];
+#pragma unroll
+            for (int sl = 0; sl < NR; sl++)
+                if (((uint32_t)(R[sl] >> (32 * h)) >> b) & 1u) {
+                    RJ[sl] ^= r.a;
+                    RL[sl] ^= r.b;
+                }
+        }
     }
-    const RW<NR> flip = ballot_i<NR>(fl[0] & 1, NR == 2 ? (fl[NR - 1] & 1) : 0);
     s.D1 = nd1;
-    s.D2 = nd2 ^ flip;
-    RW<NR> Jn[NR];
-#pragma unroll
-    for (int sl = 0; sl < NR; sl++) Jn[sl] = 0ull;
-    for (int y = 0; y < n; y++) {
-        const RW<NR> ry = row_get<NR>(R, y);
-#pragma unroll
-        for (int sl = 0; sl < NR; sl++) Jn[sl] |= (RW<NR>)parity(RJ[sl] & ry) << y;
-    }
-#pragma unroll
-    for (int sl = 0; sl < NR; sl++) s.J[sl] = Jn[sl];
+    s.D2 = nd2 ^ ballot_i<NR>(parity(RL[0] & R[0]), NR == 2 ? parity(RL[NR - 1] & R[NR - 1]) : 0);
+    share_rows<NR>(rows, R, R);
+    parity_rows<NR>(rows, RJ, 32 * NR < s.n ? 32 * NR : s.n, s.J);
 }
 
 // updateQD (stabilizer.c:163-177) for a general y
@@ -472,9 +507,9 @@ __device__ void wsigma(const WS<NR>& s, int sigma, int sidx, RW<NR> Mm, RW<NR> D
     m = (Mm | DA) ? (tM0 + Ms) % 8 : tM0;
 }
 
-// exponentialSumExact (stabilizer.c:300-481); modifies s like the reference.
-// eps/p/m are left untouched on the reference's error-return path.
-template <int NR>
+// exponentialSumExact (stabilizer.c:300-481); with STATE modifies s like the
+// reference.  eps/p/m are left untouched on the reference's error-return path.
+template <int NR, bool STATE>
 __device__ void exp_sum(WS<NR>& s, int& eps, int& p, int& m, int& err) {
     const int k = s.k;
     const RW<NR> km = low_mask<NR>(k);
@@ -508,8 +543,19 @@ __device__ void exp_sum(WS<NR>& s, int& eps, int& p, int& m, int& err) {
             const RW<NR> Ep = E & ~bit_of<NR>(a) & ~bit_of<NR>(b);
             const RW<NR> rb = row_get<NR>(s.J, b);
             const RW<NR> vb = ra & Ep, va = rb & Ep;
-            if (vb | va) apply_R<NR>(s, b, vb, a, va);
-            else {
+            if constexpr (!STATE) {
+                // the same on what is read later: J among Ep and in column sidx gets va in the rows of vb and vb
+                // in those of va (both D are even), D_x += vb_x D_b + va_x D_a + 4 vb_x va_x
+                const RW<NR> keep = Ep | (sidx >= 0 ? bit_of<NR>(sidx) : (RW<NR>)0), jb = rb & keep, ja = ra & keep;
+#pragma unroll
+                for (int sl = 0; sl < NR; sl++) {
+                    const int x = row_of<NR>(sl);
+                    s.J[sl] ^= (getbit(vb, x) ? jb : (RW<NR>)0) ^ (getbit(va, x) ? ja : (RW<NR>)0);
+                }
+                s.D2 ^= (getbit(s.D2, b) ? vb : (RW<NR>)0) ^ (getbit(s.D2, a) ? va : (RW<NR>)0) ^ (vb & va);
+            } else if (vb | va) {
+                apply_R<NR>(s, b, vb, a, va);
+            } else {
                 s.D1 &= km;
                 s.D2 &= km;
             }
@@ -568,15 +614,12 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
     const bool trivial = (s2.Q == 0) && (s2.D1 == 0ull) && (s2.D2 == 0ull) && !any_row_nonzero<NR>(s2.J);
     WS<NR> t2 = s2;
     if (!trivial) {
+        // (a < s2.k: G_b lies in the space of s2)
         const RW<NR> y = ballot_par<NR>(s2.B, st.h ^ s2.h);
         RW<NR> R[NR];
-#pragma unroll
-        for (int sl = 0; sl < NR; sl++) R[sl] = 0ull;
-        for (int a = 0; a < n; a++) {
-            const RW<NR> g2a = row_get<NR>(s2.B, a);
-#pragma unroll
-            for (int sl = 0; sl < NR; sl++) R[sl] |= (RW<NR>)parity(st.G[sl] & g2a) << a;
-        }
+        RowPair<NR>* const rows = warp_rows<NR>();
+        share_rows<NR>(rows, s2.B, s2.B);
+        parity_rows<NR>(rows, st.G, s2.k, R);
         update_qd<NR>(t2, y);
         update_dj_dense<NR>(t2, R);
     }
@@ -590,7 +633,7 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
     }
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) st.J[sl] ^= t2.J[sl];
-    exp_sum<NR>(st, eps, p, m, err);
+    exp_sum<NR, false>(st, eps, p, m, err);
     p -= k1 + s2.k;
 }
 
