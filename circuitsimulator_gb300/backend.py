@@ -331,7 +331,7 @@ class Backend:
         self._check(self.lib.csim_extend(self.ctx, n, _p(s), _p(x)))
 
     def randomStabilizerState(self, n, count=1, seed=0, first=0):
-        out = np.zeros(int(count), dtype=STATE_DTYPE)
+        out = np.empty(int(count), dtype=STATE_DTYPE)  # the download writes every byte
         self._check(self.lib.csim_random_states(self.ctx, int(n), int(count), int(seed), int(first), _p(out)))
         return out
 

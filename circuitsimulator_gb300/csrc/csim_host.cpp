@@ -37,7 +37,8 @@ extern "C" int csim_ctx_create(int device, csim_ctx** out) {
     ctx->num_sms = prop.multiProcessorCount;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) !=
                                                     cudaSuccess ||
-        cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess || cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess ||
+        cudaMallocHost(&ctx->h_err, sizeof(int)) != cudaSuccess || cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) {
         delete ctx;
         return CSIM_ERR_CUDA;
     }
@@ -64,6 +65,7 @@ extern "C" void csim_ctx_destroy(csim_ctx* ctx) {
     for (int i = 0; i < kNumBufs + 32; i++)
         if (ctx->buf[i]) cudaFree(ctx->buf[i]);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->h_err) cudaFreeHost(ctx->h_err);
     for (int i = 0; i < 4; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     for (int i = 0; i < kPinSlots; i++) {
@@ -132,20 +134,17 @@ extern "C" int csim_inner_product_exact(csim_ctx* ctx, int64_t count, const csim
     for (int64_t o = 0; o < count; o += kBatch) {
         const int64_t c = std::min(kBatch, count - o);
         csim_state *da, *db;
-        int *de, *dp, *dm;
-        void* v;
+        void *d, *v;
         CKR(dput(ctx, kBufA, a + o, c, &da));
         CKR(dput(ctx, kBufB, b + o, c, &db));
-        CKR(dbuf(ctx, kBufEps, c * 4, &v)); de = (int*)v;
-        CKR(dbuf(ctx, kBufP, c * 4, &v)); dp = (int*)v;
-        CKR(dbuf(ctx, kBufM, c * 4, &v)); dm = (int*)v;
-        if (csim::launch_inner_product(launch_of(ctx), nr, (const csim::GState*)da, (const csim::GState*)db, c, de, dp,
-                                       dm))
+        CKR(dbuf(ctx, kBufEps, 3 * c * 4, &d));  // eps, p, m
+        if (csim::launch_inner_product(launch_of(ctx), nr, (const csim::GState*)da, (const csim::GState*)db, c, (int*)d,
+                                       (int*)d + c, (int*)d + 2 * c))
             return fail(ctx, CSIM_ERR_CUDA, "inner product launch failed");
-        CKR(dget(ctx, eps + o, de, c));
-        CKR(dget(ctx, p + o, dp, c));
-        CKR(dget(ctx, m + o, dm, c));
-        CKR(finish(ctx));
+        CKR(finish_with(ctx, d, (size_t)(3 * c * 4), &v));
+        memcpy(eps + o, v, (size_t)(c * 4));
+        memcpy(p + o, (const int*)v + c, (size_t)(c * 4));
+        memcpy(m + o, (const int*)v + 2 * c, (size_t)(c * 4));
     }
     return CSIM_OK;
 }
@@ -211,24 +210,24 @@ extern "C" int csim_measure_pauli(csim_ctx* ctx, int64_t count, csim_state* s, c
     cudaSetDevice(ctx->device);
     int nr;
     CKR(check_states(ctx, s, count, &nr));
-    std::vector<int> code((size_t)std::min(count, kBatch));
     for (int64_t o = 0; o < count; o += kBatch) {
         const int64_t c = std::min(kBatch, count - o);
         csim_state* ds;
-        uint64_t *dx, *dz;
-        int32_t* dm;
-        int* dc;
-        void* v;
+        void *d, *v;
+        const size_t bytes = (size_t)c * 8;
+        CKR(staged_room(ctx, 1, 2 * bytes + bytes / 2, &v));  // xi, zeta, m
+        memcpy(v, xi + o, bytes);
+        memcpy((unsigned char*)v + bytes, zeta + o, bytes);
+        memcpy((unsigned char*)v + 2 * bytes, m + o, bytes / 2);
+        CKR(staged_send(ctx, 1, kBufXi, 2 * bytes + bytes / 2, &v));
+        const uint64_t* const dx = (const uint64_t*)v;
         CKR(dput(ctx, kBufA, s + o, c, &ds));
-        CKR(dput(ctx, kBufXi, xi + o, c, &dx));
-        CKR(dput(ctx, kBufZeta, zeta + o, c, &dz));
-        CKR(dput(ctx, kBufAlpha, m + o, c, &dm));
-        CKR(dbuf(ctx, kBufCode, c * 4, &v)); dc = (int*)v;
-        if (csim::launch_measure(launch_of(ctx), nr, (csim::GState*)ds, dm, dz, dx, c, dc))
+        CKR(dbuf(ctx, kBufCode, c * 4, &d));
+        if (csim::launch_measure(launch_of(ctx), nr, (csim::GState*)ds, (const int*)(dx + 2 * c), dx + c, dx, c, (int*)d))
             return fail(ctx, CSIM_ERR_CUDA, "measurePauli launch failed");
         CKR(dget(ctx, s + o, ds, c));
-        CKR(dget(ctx, code.data(), dc, c));
-        CKR(finish(ctx));
+        CKR(finish_with(ctx, d, bytes / 2, &v));
+        const int* const code = (const int*)v;
         for (int64_t i = 0; i < c; i++) norm[o + i] = code[i] == 0 ? 0.0 : (code[i] == 1 ? 1.0 : pow(2, -0.5));
     }
     return CSIM_OK;

@@ -409,7 +409,7 @@ inline double sqrt_half_power(int c) {  // projfactor of innerprod.c:104-111: c 
 
 // ---------------------------------------------------------------- context
 enum BufId {
-    kBufA, kBufB, kBufEps, kBufP, kBufM, kBufXi, kBufZeta, kBufAlpha, kBufCode, kBufWords, kBufOffsets,
+    kBufA, kBufB, kBufEps, kBufP, kBufM, kBufXi, kBufAlpha, kBufCode, kBufWords, kBufOffsets,
     kBufCum, kBufCodewords, kBufAcc, kBufAccDiag, kBufPhis, kBufIdx, kBufConsumed, kBufPm, kBufPz, kBufPx,
     kBufL, kBufParts, kBufPartsDiag, kBufCwOrdered, kBufRunScratch, kBufCanon, kBufCodeDirect, kBufCodeRest,
     kBufRestCount, kBufTreeJobs, kBufTreeScratch, kBufCall, kBufLengths, kBufChainMaps, kNumBufs
@@ -425,6 +425,7 @@ struct csim_ctx {
     int num_sms = 0;
     cudaStream_t stream = nullptr;
     int* d_err = nullptr;
+    int* h_err = nullptr;  // pinned: d_err's last download
     int64_t launches = 0;
     std::string last_error;
     void* buf[kNumBufs + 32] = {};
@@ -609,11 +610,17 @@ inline int error_status(csim_ctx* ctx, int h) {
 }
 // waits for the stream, then turns device error flags into a status
 inline int finish(csim_ctx* ctx) {
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->h_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     CK(cudaGetLastError());
-    return error_status(ctx, h);
+    return error_status(ctx, *ctx->h_err);
+}
+// finish() with `bytes` of results from the device, in pinned memory: copies to pageable memory
+// wait for the stream one by one
+inline int finish_with(csim_ctx* ctx, const void* results, size_t bytes, void** out) {
+    CKR(staged_room(ctx, 2, bytes, out));
+    CKR(dget(ctx, (unsigned char*)*out, (const unsigned char*)results, bytes));
+    return finish(ctx);
 }
 
 inline int check_states(csim_ctx* ctx, const csim_state* s, int64_t count, int* nr_out, int n_expect = -1) {
