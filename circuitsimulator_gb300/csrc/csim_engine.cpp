@@ -627,8 +627,10 @@ int Engine::launch_round() {
     const size_t nseg = rs.segs.size();
 
     // words of the sampled states with the C library's draws, each query's states in its own
-    // stream order (G' then H'); queries are independent streams, so they are drawn on host threads
-    // of their own (at t = 64 a state takes about 2000 words)
+    // stream order (G' then H').  Queries are independent streams.  A query whose last states these are
+    // (so that its stream need not go on) has its words made on the device, unless they are few or its
+    // states are not a tree's; the others are drawn on host threads of their own (at t = 64 a state takes
+    // about 2000 words)
     struct WordJob {
         QueryRec* q;
         int t;
@@ -638,6 +640,9 @@ int Engine::launch_round() {
         size_t nwords;                // without the history
         std::vector<int64_t> ends;
         int64_t base;                 // its first word in the round's
+        bool device = false;          // made on the device: `draw`, its memory from the work block's byte w_draw on
+        csim::DrawJob draw;
+        size_t w_draw;
     };
     std::vector<WordJob> jobs;
     std::vector<std::pair<size_t, int64_t>> job_of(nseg);  // segment -> its job and first state in it
@@ -650,14 +655,29 @@ int Engine::launch_round() {
             auto it = jix.find(e->q);
             if (it == jix.end()) {
                 it = jix.emplace(e->q, jobs.size()).first;
-                jobs.push_back(WordJob{e->q, e->t, {}, 0, {}, 0, {}, 0});
+                jobs.push_back(WordJob{e->q, e->t, {}, 0, {}, 0, {}, 0, false, {}, 0});
             }
             WordJob& j = jobs[it->second];
             job_of[i] = {it->second, j.states};
             j.segs.push_back(i);
             j.states += sg.n;
         }
+        for (WordJob& j : jobs) {
+            j.device = !words_on_host(j.t, j.states);
+            for (int w = 0; w < 2; w++)
+                if (!j.q->host_only[w]) {
+                    const Eval* e = j.q->ev[w].get();
+                    j.device &= e->kind == 1 && e->tree && e->next == e->ns;
+                }
+            if (!j.device) continue;
+            double cum[CSIM_MAX_QUBITS + 1];
+            cum_table(j.t, cum);
+            csim::draw_job(j.t, cum, j.states, 0, j.draw);
+            j.q->lr.history(j.draw.history);
+            j.nwords = 0;
+        }
         auto run_job = [](WordJob& j) {
+            if (j.device) return;
             double cum[CSIM_MAX_QUBITS + 1];
             cum_table(j.t, cum);
             j.ends.reserve((size_t)j.states);
@@ -692,6 +712,7 @@ int Engine::launch_round() {
     }
     int64_t nwords = 0, noffs = 0;
     for (auto& j : jobs) {
+        if (j.device) continue;
         j.base = nwords;
         nwords += (int64_t)j.nwords;
         noffs += j.states + (int64_t)j.segs.size();
@@ -793,7 +814,20 @@ int Engine::launch_round() {
     const size_t w_canon = align_up(w_partd + (size_t)std::max<int64_t>(ndiags, 1) * 64);
     const size_t w_cdir = align_up(w_canon + (any_direct ? (size_t)nother * csim::canon_bytes() : 0));
     const size_t w_crest = align_up(w_cdir + (any_direct ? (size_t)nother * 4 : 0));
-    const size_t work_bytes = align_up(w_crest + (any_direct ? (size_t)nother * 4 : 0));
+    size_t work_bytes = align_up(w_crest + (any_direct ? (size_t)nother * 4 : 0));
+    // a device job's words, lengths, maps, offsets and its end
+    auto draw_part = [](const csim::DrawJob& j, int part) {
+        size_t at = 0;
+        const size_t sizes[] = {(kRawHistory + (size_t)j.words) * 4, (size_t)j.padded() * 2, (size_t)j.map_words() * 4,
+                                (size_t)(j.states + 1) * 8, sizeof(csim::DrawChain)};
+        for (int i = 0; i < part; i++) at += align_up(sizes[i]);
+        return at;
+    };
+    for (auto& j : jobs)
+        if (j.device) {
+            j.w_draw = work_bytes;
+            work_bytes += draw_part(j.draw, 5);
+        }
     // download block: err (16 B), the pair launches' work-queue counter (kQueueOffset) | codes | values
     rs.off_codes = 256;
     rs.off_val = align_up(rs.off_codes + (size_t)ns * 4);
@@ -806,6 +840,17 @@ int Engine::launch_round() {
     unsigned char* db = (unsigned char*)rs.up.p;
     unsigned char* wb = (unsigned char*)rs.work.p;
     unsigned char* dd = (unsigned char*)rs.down.p;
+    std::vector<csim::DrawJob> draws;
+    for (auto& j : jobs)
+        if (j.device) {
+            unsigned char* const at = wb + j.w_draw;
+            j.draw.buf = (uint32_t*)(at + draw_part(j.draw, 0));
+            j.draw.len = (uint16_t*)(at + draw_part(j.draw, 1));
+            j.draw.map = (uint32_t*)(at + draw_part(j.draw, 2));
+            j.draw.offs = (int64_t*)(at + draw_part(j.draw, 3));
+            j.draw.chain = (csim::DrawChain*)(at + draw_part(j.draw, 4));
+            draws.push_back(j.draw);
+        }
     uint64_t* hproj = (uint64_t*)(hb + o_proj);
     for (auto& kv : evix) {
         uint64_t* blk = hproj + 192 * kv.second;
@@ -843,7 +888,12 @@ int Engine::launch_round() {
         const bool libc = e->kind == 1 && r->q.rng == CSIM_RNG_LIBC;
         const int64_t* seg_offs = nullptr;  // host view of the segment's word offsets
         const int64_t* seg_doffs = nullptr;
-        if (libc) {
+        const uint32_t* seg_words = dwords;
+        if (libc && jobs[job_of[si].first].device) {
+            const csim::DrawJob& j = jobs[job_of[si].first].draw;
+            seg_words = j.buf;
+            seg_doffs = j.offs + job_of[si].second;
+        } else if (libc) {
             const WordJob& j = jobs[job_of[si].first];
             const int64_t k0 = job_of[si].second;
             seg_offs = hoffs + io;
@@ -859,7 +909,7 @@ int Engine::launch_round() {
                                     e->nstabs,
                                     r->q.seed,
                                     e->kind == 2 ? (uint64_t)sg.s0 : e->id0 + (uint64_t)sg.s0,
-                                    dwords,
+                                    seg_words,
                                     seg_doffs,
                                     dcum + 65 * e->t,
                                     (const int*)pblk,
@@ -1005,6 +1055,8 @@ int Engine::launch_round() {
     }
     if (csim::launch_items_warp(L, ditems + nitp, niw, dstates, dcode, part + 4 * nitp, partd + 4 * nitp))
         return fail(ctx_, CSIM_ERR_CUDA, "pair launch failed");
+    if (!draws.empty() && csim::launch_draws(L, draws.data(), (int)draws.size()))
+        return fail(ctx_, CSIM_ERR_CUDA, "word launch failed");
     if (ndiags > nitems) CK(cudaMemsetAsync(partd + 4 * nitems, 0, (size_t)(ndiags - nitems) * 64, ctx_->stream));
     if (!groups.empty() && tree_run_.launch(L, db + o_tjobs)) return fail(ctx_, CSIM_ERR_CUDA, "tree launch failed");
     CK(cudaEventRecord(rs.ev[2], ctx_->stream));
@@ -1185,7 +1237,7 @@ extern "C" int csim_run_queries(csim_ctx* ctx, int64_t nq, const csim_query* q, 
     stats_begin(ctx);
     if (!ctx->engine || ctx->engine->per_thread() != ctx->per_thread) {
         if (ctx->engine) engine_free(ctx->engine);
-        ctx->engine = new Engine(ctx, (int64_t)1 << 28, (int64_t)1 << 16, ctx->per_thread, 0);
+        ctx->engine = new Engine(ctx, (int64_t)1 << 30, (int64_t)1 << 16, ctx->per_thread, 0);
         const int rc = ctx->engine->init();
         if (rc) {
             engine_free(ctx->engine);

@@ -627,38 +627,25 @@ int put_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, cons
     return 0;
 }
 
-// Words of the longest sequence for a state of t qubits that draws at most two vectors again
-int most_words(int t) {
-    const int bytes = (t + 7) / 8;
-    int most = 0;
-    for (int d = 0; d <= t; d++) most = std::max(most, 1 + (5 + d) * bytes + (t - d) * (t - d - 1) / 2);
-    return most;
-}
-
-// The same on the device, from `words` words: *chain (device memory) counts the states that these
-// suffice for
-int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, int64_t words, const uint32_t** dwords,
+// The same on the device: *chain (device memory) counts the states that the words suffice for
+int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, int more, const uint32_t** dwords,
                      const int64_t** doffs, csim::DrawChain* chain) {
-    const int entries = most_words(t);
-    csim::RawStart start;
-    csim::raw_jumps(start);
-    ctx->lr.history(start.history);
-    csim::DrawTable table;
-    csim::draw_table(t, cum, table);
-    const int segment = csim::chain_segment(count, entries);
-    const int64_t padded = csim::chain_padded(words, segment);
-    void *w, *len, *map, *offs;
-    CKR(dbuf(ctx, kBufWords, (kRawHistory + (size_t)words) * 4, &w));
-    CKR(dbuf(ctx, kBufLengths, (size_t)padded * 2, &len));
-    CKR(dbuf(ctx, kBufChainMaps, (size_t)(padded / segment) * entries * 4, &map));
-    CKR(dbuf(ctx, kBufOffsets, (size_t)(count + 1) * 8, &offs));
-    if (csim::launch_raw_words(launch_of(ctx), start, words, (uint32_t*)w) ||
-        csim::launch_draw_lengths(launch_of(ctx), table, (const uint32_t*)w, words, padded, (uint16_t*)len) ||
-        csim::launch_draw_chain(launch_of(ctx), (const uint16_t*)len, padded, segment, (const uint32_t*)w, entries,
-                                (uint32_t*)map, count, (int64_t*)offs, chain))
-        return fail(ctx, CSIM_ERR_CUDA, "word launch failed");
-    *dwords = (const uint32_t*)w;
-    *doffs = (const int64_t*)offs;
+    csim::DrawJob j{};
+    csim::draw_job(t, cum, count, more, j);
+    ctx->lr.history(j.history);
+    void* v;
+    CKR(dbuf(ctx, kBufWords, (kRawHistory + (size_t)j.words) * 4, &v));
+    j.buf = (uint32_t*)v;
+    CKR(dbuf(ctx, kBufLengths, (size_t)j.padded() * 2, &v));
+    j.len = (uint16_t*)v;
+    CKR(dbuf(ctx, kBufChainMaps, (size_t)j.map_words() * 4, &v));
+    j.map = (uint32_t*)v;
+    CKR(dbuf(ctx, kBufOffsets, (size_t)(count + 1) * 8, &v));
+    j.offs = (int64_t*)v;
+    j.chain = chain;
+    if (csim::launch_draws(launch_of(ctx), &j, 1)) return fail(ctx, CSIM_ERR_CUDA, "word launch failed");
+    *dwords = j.buf;
+    *doffs = j.offs;
     return 0;
 }
 
@@ -755,18 +742,14 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         __int128* dpart = (__int128*)v;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
         if (!tree) CK(cudaMemsetAsync(dpart, 0, nparts * sizeof(__int128), ctx->stream));
-        // The C library's words: a few on the host, 0.4 ns each and 60 ns a state, from 30 us on on the
-        // device, whose four launches take that long (a call of 256 states: t = 24 185 us with the host's
-        // words, 145 with the device's, t = 40 349 and 246; of 64: t = 24 122 and 138, t = 40 212 and 219)
-        const int64_t most = (int64_t)most_words(t) * c;
-        const bool on_host = libc && most + 150 * c <= 75000;
+        const bool on_host = libc && words_on_host(t, c);
         csim::DrawChain chain{};
         csim::TreeDraw draw{};
         if (libc) {
             const uint32_t* dw;
             const int64_t* doff;
             if (on_host) CKR(put_state_words(ctx, t, hcum, c, &dw, &doff, &chain));
-            else CKR(make_state_words(ctx, t, hcum, c, (most + 4096) << more, &dw, &doff, (csim::DrawChain*)(dres + 16)));
+            else CKR(make_state_words(ctx, t, hcum, c, more, &dw, &doff, (csim::DrawChain*)(dres + 16)));
             draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, dcode, nullptr, 0, 0};
             if (!tree && csim::launch_random_states(launch_of(ctx), t, c, 2, 0, 0, dw, doff, in.cum, dth, nullptr))
                 return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");

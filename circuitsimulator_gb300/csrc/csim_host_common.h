@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -107,7 +108,7 @@ inline double logeta(int d, int n) {
     return (-d * (d + 1) / 2) + product;
 }
 
-inline void cum_table(int n, double* cum) {
+inline void make_cum_table(int n, double* cum) {
     double dist[CSIM_MAX_QUBITS + 1];
     double sum = 0;
     for (int d = 0; d <= n; d++) {
@@ -120,6 +121,14 @@ inline void cum_table(int n, double* cum) {
         for (int d = 0; d <= i; d++) cum[i] += dist[d];
     }
     for (int i = 0; i <= n; i++) cum[i] /= cum[n];
+}
+
+// The same, made once per n and process (8,000 calls of libm at n = 64, 0.1 ms)
+inline void cum_table(int n, double* cum) {
+    static std::once_flag made[CSIM_MAX_QUBITS + 1];
+    static double table[CSIM_MAX_QUBITS + 1][CSIM_MAX_QUBITS + 1];
+    std::call_once(made[n], [n] { make_cum_table(n, table[n]); });
+    memcpy(cum, table[n], (size_t)(n + 1) * sizeof(double));
 }
 
 inline uint64_t codeword(int64_t j, const uint64_t* L, int k) {
@@ -185,6 +194,11 @@ bool draw_state_words(RawWords& w, int n, const double* cum, Grow grow) {
     w.extend(rest);
     return true;
 }
+
+// The C library's words: a few on the host, 0.4 ns each and 60 ns a state, from 30 us on on the
+// device, whose four launches take that long (a call of 256 states: t = 24 185 us with the host's
+// words, 145 with the device's, t = 40 349 and 246; of 64: t = 24 122 and 138, t = 40 212 and 219)
+inline bool words_on_host(int t, int64_t states) { return (csim::most_words(t) + 150) * states <= 75000; }
 
 // Zero bound of the "light" part of an ordered codeword table: codewords with
 // at most this many zeros run in a launch whose G-column slots are sized for

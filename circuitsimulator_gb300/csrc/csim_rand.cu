@@ -24,12 +24,13 @@ void poly_mul(const uint32_t (&a)[31], const uint32_t (&b)[31], uint32_t (&out)[
     for (int i = 0; i < 31; i++) out[i] = p[i];
 }
 
-}  // namespace
-
-void raw_jumps(RawStart& s) {
-    struct Jumps {
-        uint32_t p[kRawJumps][31];
-        Jumps() {
+// x^(kRawChunk 2^b), coefficient of x^m at m
+struct RawJumps {
+    uint32_t p[kRawJumps][31];
+};
+const RawJumps& raw_jumps() {
+    struct Made : RawJumps {
+        Made() {
             uint32_t r[31] = {1}, x[31] = {0, 1};
             for (int e = kRawChunk; e; e >>= 1) {
                 if (e & 1) poly_mul(r, x, r);
@@ -41,9 +42,8 @@ void raw_jumps(RawStart& s) {
             }
         }
     };
-    static const Jumps jumps;
-    for (int b = 0; b < kRawJumps; b++)
-        for (int m = 0; m < 31; m++) s.jump[b][m] = jumps.p[b][m];
+    static const Made jumps;
+    return jumps;
 }
 
 void draw_table(int n, const double* cum, DrawTable& t) {
@@ -58,6 +58,40 @@ void draw_table(int n, const double* cum, DrawTable& t) {
         }
         t.last[d] = (uint32_t)lo;
     }
+}
+
+// Words per segment of the chain of `states` states of up to `longest` words each: a power of two.
+// Following a chain within a segment takes 30 ns a state, twice, the walk 300 ns a segment, so
+// sqrt(5 states) states per segment are best.
+int chain_segment(int64_t states, int longest) {
+    int64_t s = 1 << 10;
+    while (s < kMaxSegment && s * s < 5 * states * longest * longest / 2) s *= 2;
+    return (int)s;
+}
+
+// The jobs of a launch, and the first block of each in the four kernels
+template <int N>
+struct DrawJobs {
+    int n;
+    int32_t raw0[N], len0[N], map0[N], place0[N];
+    DrawJob job[N];
+};
+template <int N>
+__device__ __forceinline__ int job_at(const int32_t (&first)[N], int n) {
+    int j = 0;
+    for (int i = 1; i < n; i++)
+        if ((int)blockIdx.x >= first[i]) j = i;
+    return j;
+}
+
+}  // namespace
+
+void draw_job(int t, const double* cum, int64_t states, int more, DrawJob& j) {
+    draw_table(t, cum, j.table);
+    j.entries = most_words(t);
+    j.segment = chain_segment(states, j.entries);
+    j.words = (j.entries * states + 4096) << more;
+    j.states = states;
 }
 
 // ---------------------------------------------------------------- words
@@ -78,11 +112,16 @@ constexpr int kRawThreads = 256;
 // A warp per kRawChunk words: jumps to its chunk (a jump: 31 products per word), then 31
 // words at a time from the 31 before.  Bound by the latency of its serial steps: 361,000
 // words in 10 us (the host makes one in 0.4 ns, 144 us).
-__global__ void __launch_bounds__(kRawThreads) k_raw_words(const __grid_constant__ RawStart s, int64_t count, uint32_t* buf) {
+template <int N>
+__global__ void __launch_bounds__(kRawThreads) k_raw_words(const __grid_constant__ RawJumps jumps,
+                                                           const __grid_constant__ DrawJobs<N> jobs) {
     __shared__ uint32_t win[kRawThreads / 32][64];
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, ji = job_at<N>(jobs.raw0, jobs.n);
+    const DrawJob& s = jobs.job[ji];
+    const int64_t count = s.words;
+    uint32_t* const buf = s.buf;
     uint32_t* const r = win[threadIdx.x >> 5];
-    const int64_t chunk = ((int64_t)blockIdx.x * kRawThreads + threadIdx.x) >> 5;
+    const int64_t chunk = ((int64_t)(blockIdx.x - jobs.raw0[ji]) * kRawThreads + threadIdx.x) >> 5;
     if (chunk == 0) {
         buf[lane] = s.history[lane];
         if (lane < kRawHistory - 32) buf[32 + lane] = s.history[32 + lane];
@@ -100,7 +139,7 @@ __global__ void __launch_bounds__(kRawThreads) k_raw_words(const __grid_constant
         __syncwarp();
         w = 0u;
 #pragma unroll
-        for (int m = 0; m < 31; m++) w += s.jump[b][m] * r[m + lane];  // lane 31: unused
+        for (int m = 0; m < 31; m++) w += jumps.p[b][m] * r[m + lane];  // lane 31: unused
     }
     uint32_t* const out = buf + kRawHistory + chunk * kRawChunk;
     const int64_t left = count - chunk * kRawChunk;
@@ -119,11 +158,16 @@ __global__ void __launch_bounds__(kRawThreads) k_raw_words(const __grid_constant
 // dimension: ALU-bound with few of them busy.
 constexpr int kLengthThreads = 256, kLengthReach = 256;  // words behind the block's that vectors are read from
 
-__global__ void __launch_bounds__(kLengthThreads) k_draw_lengths(const __grid_constant__ DrawTable t, const uint32_t* buf,
-                                                                 int64_t count, uint16_t* len) {
+template <int N>
+__global__ void __launch_bounds__(kLengthThreads) k_draw_lengths(const __grid_constant__ DrawJobs<N> jobs) {
     __shared__ uint64_t bytes_s[(kLengthThreads + kLengthReach) / 8 + 1];
-    const int64_t base = (int64_t)blockIdx.x * kLengthThreads, i = base + threadIdx.x;
-    const uint32_t* const w = buf + kRawHistory + base;
+    const int ji = job_at<N>(jobs.len0, jobs.n);
+    const DrawJob& s = jobs.job[ji];
+    const DrawTable& t = s.table;
+    const int64_t count = s.words;
+    uint16_t* const len = s.len;
+    const int64_t base = (int64_t)(blockIdx.x - jobs.len0[ji]) * kLengthThreads, i = base + threadIdx.x;
+    const uint32_t* const w = s.buf + kRawHistory + base;
     const int there = (int)(count - base < (1 << 20) ? count - base : (1 << 20));  // words from the block's first on
     for (int q = threadIdx.x; q < kLengthThreads + kLengthReach; q += kLengthThreads)
         reinterpret_cast<uint8_t*>(bytes_s)[q] = q < there ? (uint8_t)(w[q] >> 1) : 0;
@@ -203,9 +247,13 @@ __device__ __forceinline__ void load_segment(uint16_t* to, const uint16_t* from,
 
 // map[e] of the block's segment: where the chain from its word e leaves it (words behind
 // its end, kNoExit) and, in the upper half, how many states begin in it on the way
-__global__ void __launch_bounds__(kChainThreads) k_chain_maps(const uint16_t* len, int segment, int entries, uint32_t* map) {
+template <int N>
+__global__ void __launch_bounds__(kChainThreads) k_chain_maps(const __grid_constant__ DrawJobs<N> jobs) {
     extern __shared__ __align__(16) uint16_t seg_s[];
-    load_segment(seg_s, len + (int64_t)blockIdx.x * segment, segment);
+    const int ji = job_at<N>(jobs.map0, jobs.n), b = blockIdx.x - jobs.map0[ji];
+    const int segment = jobs.job[ji].segment, entries = jobs.job[ji].entries;
+    uint32_t* const map = jobs.job[ji].map + (int64_t)b * entries;
+    load_segment(seg_s, jobs.job[ji].len + (int64_t)b * segment, segment);
     __syncthreads();
     for (int e = threadIdx.x; e < entries; e += kChainThreads) {
         int p = e, states = 0;
@@ -216,7 +264,7 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_maps(const uint16_t* le
             states++;
         }
         const int out = p - segment;  // (below 0: the words end)
-        map[(int64_t)blockIdx.x * entries + e] = (out < 0 || out >= (int)kNoExit ? kNoExit : (uint32_t)out) | ((uint32_t)states << 16);
+        map[e] = (out < 0 || out >= (int)kNoExit ? kNoExit : (uint32_t)out) | ((uint32_t)states << 16);
     }
 }
 
@@ -225,18 +273,25 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_maps(const uint16_t* le
 // serial loads: 2000 states of 12 qubits 15 us with k_chain_maps' 8, 4096 of 40 qubits
 // 30 with 8; one thread over all segments, the next one loading meanwhile, took 72 and
 // 203 us.
-__global__ void __launch_bounds__(kChainThreads) k_chain_place(const uint16_t* len, int segment, const uint32_t* buf, int entries,
-                                                               const uint32_t* map, int64_t states, int64_t* offs,
-                                                               DrawChain* chain) {
+template <int N>
+__global__ void __launch_bounds__(kChainThreads) k_chain_place(const __grid_constant__ DrawJobs<N> jobs) {
     extern __shared__ __align__(16) uint16_t seg_s[];
     __shared__ int64_t at_s;
     __shared__ int last_s;
-    load_segment(seg_s, len + (int64_t)blockIdx.x * segment, segment);
+    const int ji = job_at<N>(jobs.place0, jobs.n), b = blockIdx.x - jobs.place0[ji];
+    const DrawJob& J = jobs.job[ji];
+    const int segment = J.segment, entries = J.entries;
+    const uint16_t* const len = J.len;
+    const uint32_t* const map = J.map;
+    const int64_t states = J.states;
+    int64_t* const offs = J.offs;
+    const bool last_segment = (int64_t)(b + 1) * segment >= J.words;
+    load_segment(seg_s, len + (int64_t)b * segment, segment);
     __syncthreads();
     if (threadIdx.x == 0) {
         int64_t state = 0, at = 0;
         bool out_of_words = false;
-        for (int s = 0; s < (int)blockIdx.x && state < states && !out_of_words; s++) {
+        for (int s = 0; s < b && state < states && !out_of_words; s++) {
             const int64_t end = (int64_t)(s + 1) * segment;
             const int64_t e = at - (end - segment);
             if (e >= segment) continue;  // a state longer than a segment
@@ -254,7 +309,7 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_place(const uint16_t* l
             }
         }
         // (state can have passed `states`: then a block before places the last one)
-        const int64_t seg = (int64_t)blockIdx.x * segment;
+        const int64_t seg = (int64_t)b * segment;
         int last = 0;
         if (state < states && !out_of_words) {
             int64_t rel = at - seg;
@@ -266,10 +321,10 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_place(const uint16_t* l
                 rel += l;
             }
             at = seg + rel;
-            last = state == states || out_of_words || blockIdx.x + 1 == gridDim.x;
+            last = state == states || out_of_words || last_segment;
             if (last) {
-                chain->states = state;
-                chain->words = at;
+                J.chain->states = state;
+                J.chain->words = at;
                 for (; state <= states; state++) offs[state] = kRawHistory + at;  // the end, or no words
             }
         }
@@ -277,43 +332,56 @@ __global__ void __launch_bounds__(kChainThreads) k_chain_place(const uint16_t* l
         last_s = last;
     }
     __syncthreads();
-    if (last_s && threadIdx.x < kRawHistory) chain->history[threadIdx.x] = buf[at_s + threadIdx.x];
+    if (last_s && threadIdx.x < kRawHistory) J.chain->history[threadIdx.x] = J.buf[at_s + threadIdx.x];
 }
 
 // ---------------------------------------------------------------- launchers
-int launch_raw_words(const Launch& L, const RawStart& s, int64_t count, uint32_t* buf) {
-    if (count <= 0 || count > kRawMax) return -1;
-    const int64_t chunks = (count + kRawChunk - 1) / kRawChunk, per = kRawThreads / 32;
-    k_raw_words<<<(unsigned)((chunks + per - 1) / per), kRawThreads, 0, L.stream>>>(s, count, buf);
-    (*L.launches)++;
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
+namespace {
 
-int launch_draw_lengths(const Launch& L, const DrawTable& t, const uint32_t* buf, int64_t count, int64_t padded,
-                        uint16_t* len) {
-    if (count <= 0 || padded <= 0 || padded > kRawMax || padded % kLengthThreads || t.n < 1 || t.n > 64) return -1;
-    k_draw_lengths<<<(unsigned)(padded / kLengthThreads), kLengthThreads, 0, L.stream>>>(t, buf, count, len);
-    (*L.launches)++;
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-int launch_draw_chain(const Launch& L, const uint16_t* len, int64_t padded, int segment, const uint32_t* buf, int entries,
-                      uint32_t* map, int64_t states, int64_t* offs, DrawChain* chain) {
-    if (states <= 0 || segment < 8 || segment % 8 || segment > kMaxSegment || padded <= 0 || padded % segment ||
-        padded > kRawMax || entries < 1)
-        return -1;
-    const unsigned segments = (unsigned)(padded / segment);
-    const int smem = segment * (int)sizeof(uint16_t), most = kMaxSegment * (int)sizeof(uint16_t);
-    if (cudaFuncSetAttribute(k_chain_maps, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
-        cudaFuncSetAttribute(k_chain_place, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
-        return -1;
-    if (segments > 1) {
-        k_chain_maps<<<segments - 1, kChainThreads, smem, L.stream>>>(len, segment, entries, map);
-        (*L.launches)++;
+template <int N>
+int launch_jobs(const Launch& L, const DrawJob* jobs, int njobs) {
+    DrawJobs<N> J;
+    J.n = njobs;
+    int64_t raw = 0, len = 0, maps = 0, place = 0;
+    int segment = 0;
+    for (int i = 0; i < njobs; i++) {
+        const DrawJob& j = J.job[i] = jobs[i];
+        if (j.states <= 0 || j.words <= 0 || j.words > kRawMax || j.table.n < 1 || j.table.n > 64 || j.entries < 1 ||
+            j.segment < kLengthThreads || j.segment % kLengthThreads || j.segment > kMaxSegment)
+            return -1;
+        const int64_t chunks = (j.words + kRawChunk - 1) / kRawChunk, segments = j.padded() / j.segment;
+        J.raw0[i] = (int32_t)raw;
+        J.len0[i] = (int32_t)len;
+        J.map0[i] = (int32_t)maps;
+        J.place0[i] = (int32_t)place;
+        raw += (chunks + kRawThreads / 32 - 1) / (kRawThreads / 32);
+        len += j.padded() / kLengthThreads;
+        maps += segments - 1;
+        place += segments;
+        segment = segment > j.segment ? segment : j.segment;
     }
-    k_chain_place<<<segments, kChainThreads, smem, L.stream>>>(len, segment, buf, entries, map, states, offs, chain);
-    (*L.launches)++;
+    if (raw > 0x7fffffff || len > 0x7fffffff) return -1;
+    const int smem = segment * (int)sizeof(uint16_t), most = kMaxSegment * (int)sizeof(uint16_t);
+    if (cudaFuncSetAttribute(k_chain_maps<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+        cudaFuncSetAttribute(k_chain_place<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+        return -1;
+    k_raw_words<N><<<(unsigned)raw, kRawThreads, 0, L.stream>>>(raw_jumps(), J);
+    k_draw_lengths<N><<<(unsigned)len, kLengthThreads, 0, L.stream>>>(J);
+    if (maps > 0) k_chain_maps<N><<<(unsigned)maps, kChainThreads, smem, L.stream>>>(J);
+    k_chain_place<N><<<(unsigned)place, kChainThreads, smem, L.stream>>>(J);
+    *L.launches += maps > 0 ? 4 : 3;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+}  // namespace
+
+int launch_draws(const Launch& L, const DrawJob* jobs, int njobs) {
+    for (int i = 0; i < njobs; i += kDrawJobs) {
+        const int n = njobs - i < kDrawJobs ? njobs - i : kDrawJobs;
+        const int rc = n == 1 ? launch_jobs<1>(L, jobs + i, 1) : launch_jobs<kDrawJobs>(L, jobs + i, n);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 }  // namespace csim

@@ -23,10 +23,6 @@ constexpr int kRawJumps = 18;                    // jumps of 2^b chunks
 constexpr int64_t kRawMax = (int64_t)kRawChunk << kRawJumps;
 constexpr int kMaxSegment = 1 << 16;             // words per segment, at most (16 bits each in shared memory)
 
-struct RawStart {
-    uint32_t jump[kRawJumps][31];  // x^(kRawChunk 2^b), coefficient of x^m at m
-    uint32_t history[kRawHistory];  // the last words before the buffer's
-};
 // randomStabilizerState's dimension from a rand() value x: the first d with x <= last[d]
 struct DrawTable {
     int n;
@@ -38,28 +34,39 @@ struct DrawChain {
     uint32_t history[kRawHistory];  // the last words before that point
 };
 
-void raw_jumps(RawStart& s);                                // fills jump
-void draw_table(int n, const double* cum, DrawTable& t);    // cum: csim_host::cum_table
+// The words of a batch of states from one stream, and the states' places in them
+struct DrawJob {
+    uint32_t history[kRawHistory];  // the last words before the batch's
+    DrawTable table;
+    int32_t segment, entries;       // words per segment; words from a segment's first that most states which begin
+                                    // before the segment end by
+    int64_t words, states;          // words to make
+    uint32_t* buf;                  // kRawHistory + words: the history, then the words
+    uint16_t* len;                  // padded(): the words of a state that starts at each word (scratch)
+    uint32_t* map;                  // map_words() (scratch)
+    int64_t* offs;                  // states + 1: the words that the states begin at (indices into buf) and the end of
+                                    // the last; states without enough words get none
+    DrawChain* chain;
+    int64_t padded() const { return (words + segment - 1) / segment * segment; }
+    int64_t map_words() const { return padded() / segment * entries; }
+};
 
-// words [0, count) of the sequence behind s.history into buf[kRawHistory ...], the history in front
-int launch_raw_words(const Launch& L, const RawStart& s, int64_t count, uint32_t* buf);
-// Words per segment of the chain of `states` states of up to `longest` words each: a power of two.
-// Following a chain within a segment takes 30 ns a state, twice, the walk 300 ns a segment, so
-// sqrt(5 states) states per segment are best.
-inline int chain_segment(int64_t states, int longest) {
-    int64_t s = 1 << 10;
-    while (s < kMaxSegment && s * s < 5 * states * longest * longest / 2) s *= 2;
-    return (int)s;
+// Words of the longest sequence for a state of t qubits that draws at most two vectors again
+inline int most_words(int t) {
+    const int bytes = (t + 7) / 8;
+    int most = 0;
+    for (int d = 0; d <= t; d++) {
+        const int w = 1 + (5 + d) * bytes + (t - d) * (t - d - 1) / 2;
+        most = w > most ? w : most;
+    }
+    return most;
 }
-inline int64_t chain_padded(int64_t count, int segment) { return (count + segment - 1) / segment * segment; }
-// len[i] for i < padded (a multiple of 256): the words of a state that starts at word i, 0 if they go
-// beyond `count`
-int launch_draw_lengths(const Launch& L, const DrawTable& t, const uint32_t* buf, int64_t count, int64_t padded,
-                        uint16_t* len);
-// offs[0 .. states]: the words that the states begin at (indices into buf) and the end of the last;
-// states without enough words get none.  entries: words from a segment's first that most states which
-// begin before the segment end by; map: padded / segment * entries words of scratch.
-int launch_draw_chain(const Launch& L, const uint16_t* len, int64_t padded, int segment, const uint32_t* buf, int entries,
-                      uint32_t* map, int64_t states, int64_t* offs, DrawChain* chain);
+// Fills a job but for its history and pointers.  cum: csim_host::cum_table.  Words: for that longest
+// sequence and a few thousand; 2^more times as many.
+void draw_job(int t, const double* cum, int64_t states, int more, DrawJob& j);
+
+// Four launches for up to kDrawJobs jobs
+constexpr int kDrawJobs = 16;
+int launch_draws(const Launch& L, const DrawJob* jobs, int njobs);
 
 }  // namespace csim
