@@ -36,3 +36,29 @@ def test_draws_of_one_call_equal_those_of_several(gpu, t, count):
         left -= n
     assert (np.concatenate(parts) == whole).all()
     assert (gpu.singleProjectorSample(P, L, False, 3, backend.RNG_LIBC) == after).all()
+
+
+@pytest.mark.parametrize("count", [1, 5, 16, 17])
+def test_batched_draws_on_the_device_equal_the_hosts(gpu, count):
+    """Queries whose states all fit a round have their words made on the device (sixteen
+    queries to a launch); in rounds of a few states the host draws them."""
+    rs = np.random.RandomState(count)
+    qs = []
+    for i in range(count):
+        t = int(rs.choice([5, 9, 17, 24, 33, 47, 64]))
+        g = random_projector_rows(rs, t, int(rs.randint(2, 6)))
+        h = (g[0][1:], g[1][1:], g[2][1:])
+        cfg = dict(quiet=1, verbose=0, noapprox=0, samples=int(rs.choice([60, 300, 600])), bins=1, t=t, k=3, exact=0,
+                   fidbound=1e-5, fidelity=0, rank=0, forceL=0, forceSample=1)
+        qs.append({"cfg": cfg, "projs": [(*g, t), (*h, t)], "seed": 50 + i, "rng": backend.RNG_LIBC})
+    batched = gpu.run_queries(qs, batched=True)
+    plain = gpu.run_queries(qs, batched=False)
+    srv = backend.Server(0, round_pairs=8 * 40)
+    try:
+        tickets = [srv.submit(q) for q in qs]
+        rounds = [srv.wait(t) for t in tickets]
+    finally:
+        srv.close()
+    for b, p, r in zip(batched, plain, rounds):
+        assert b["numerator"] == p["numerator"] == r["numerator"]
+        assert b["denominator"] == p["denominator"] == r["denominator"]
