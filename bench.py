@@ -126,6 +126,11 @@ ROWOPS_PER_PAIR_T40 = 2576.0
 DIRECT_ROWS_PER_PAIR_T40 = 151.1
 
 
+# The tree sum (csim_tree.cu), the default: thread instructions per pair and DRAM bytes
+# (read + write) per state of its kernels on c2, ncu over 512 states
+# (profiles/k_tree_small.md).
+TREE_INSTR_PER_PAIR_T40 = 827.0
+TREE_TRAFFIC_PER_STATE = 2.31e6
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of pair-kernel launches over
 # projected c2 states.  The block-prefix kernel: the light launch over 64 states
 # (profiles/k_terms_tp_c2_small.md: 657 KB read, 600 KB written), the codeword
@@ -140,8 +145,10 @@ DIRECT_TRAFFIC = ((64, 677888 + 843264), (256, 884736 + 1737472))
 
 
 def dram_bytes_per_launch(states, kernel="block prefix"):
-    """DRAM bytes of one pair-kernel launch over `states` states, from the
+    """DRAM bytes of the pair kernels' launches over `states` states, from the
     measured captures above."""
+    if kernel == "tree":
+        return TREE_TRAFFIC_PER_STATE * states
     if kernel == "direct":
         (s0, b0), (s1, b1) = DIRECT_TRAFFIC
         return b0 + (b1 - b0) / (s1 - s0) * (states - s0)
@@ -243,12 +250,16 @@ def run_ours(args, rank, world, local_rank):
         step(i, backend.RNG_PHILOX)
         flush.zero_()
     barrier()
-    if args.no_tune:  # the launch the fixed rules and the forcing options give
+    tree = not args.pair_kernel
+    if tree:
+        tuned = (0, 0, 0.0, None)
+    elif args.no_tune:  # the launch the fixed rules and the forcing options give
         forced = {2: 0, 3: 1, 4: 2, 5: 3}.get(args.pair_kernel, 0)
         tuned = (args.per_thread or 0, 0, 0.0, forced)
     else:  # done by the first warm-up step; this reads the choice
         tuned = gpu.autotune(cfg["t"], P[0], [int(x) for x in L])
-    kname = {0: "k_terms_tp (heavy and light launches)", 1: "k_terms_runs",
+    kname = {None: "k_tree_draw, k_tree_stage, k_tree_leaf (shared partial contractions)",
+             0: "k_terms_tp (heavy and light launches)", 1: "k_terms_runs",
              2: "k_terms_tp (one launch per occupancy class)",
              3: "k_terms_direct (each state restricted once in pivot form)"}[tuned[3]]
     clocks = ClockSampler(local_rank)
@@ -298,26 +309,34 @@ def run_ours(args, rank, world, local_rank):
     value = pairs / (dev_ms / 1e3)
     props = torch.cuda.get_device_properties(local_rank)
     mhz = clk.get("sm_mhz") or 2070.0
-    per_pair = ROWOPS_PER_PAIR_T40
-    kernel_rate = (pairs / world) / (pair_ms / 1e3)  # pairs/s of the pair kernel alone (rank 0 share)
-    achieved = kernel_rate * per_pair / 1e9 if per_pair else None
+    per_pair = TREE_INSTR_PER_PAIR_T40 if tree else ROWOPS_PER_PAIR_T40
+    kernel_rate = (pairs / world) / (pair_ms / 1e3)  # pairs/s of the pair kernels alone (rank 0 share)
+    achieved = kernel_rate * per_pair / 1e9
     peak = alu_peak_gops(props.multi_processor_count, clk.get("sm_max_mhz") or 2070.0)
-    roofline = {"bound": "alu", "kernel": kname + ": (theta, prepL term) pairs, one thread per pair",
-                "achieved": achieved, "peak": peak, "unit": "G packed row-ops/s",
-                "frac": (achieved / peak) if achieved else None,
+    roofline = {"bound": "alu", "kernel": kname + (": sums over all (theta, prepL term) pairs" if tree else
+                                                  ": (theta, prepL term) pairs, one thread per pair"),
+                "achieved": achieved, "peak": peak,
+                "unit": "G thread instructions/s" if tree else "G packed row-ops/s",
+                "frac": achieved / peak,
                 "traffic": dram_bytes_per_launch(samples * bins / world,
-                                                 "direct" if tuned[3] == 3 else "block prefix"),
-                "traffic_source": ("ncu dram bytes (read + write) of this kernel's launches over 64 and 256 states "
+                                                 "tree" if tree else ("direct" if tuned[3] == 3 else "block prefix")),
+                "traffic_source": ("ncu dram bytes (read + write) of these kernels' launches over 512 states "
+                                   "(profiles/k_tree_small.md), scaled to this launch's states" if tree else
+                                   "ncu dram bytes (read + write) of this kernel's launches over 64 and 256 states "
                                    "(profiles/k_terms_direct_c2_small.md), on the line through them"
                                    if tuned[3] == 3 else
                                    "ncu dram bytes (read + write) of a 64-state launch of this kernel "
                                    "(profiles/k_terms_tp_c2_small.md), scaled to this launch's states"),
-                "work_unit": "packed row-op of the reference's algorithm (one 64-bit row test/XOR/update of its "
+                "work_unit": "thread instruction of the tree sum's kernels (ncu smsp__inst_executed x 32 per pair on "
+                             "c2's t and k); the logic pipe takes half of the issue peak" if tree else
+                             "packed row-op of the reference's algorithm (one 64-bit row test/XOR/update of its "
                              "elementary updates), whichever kernel runs",
-                "rowops_per_pair": per_pair,
-                "kernel_rows_per_pair": DIRECT_ROWS_PER_PAIR_T40 if tuned[3] == 3 else per_pair,
+                "work_per_pair": per_pair,
+                "rowops_per_pair": ROWOPS_PER_PAIR_T40,
                 "peak_source": "SMs x 4 x 32 lanes x sm_max_mhz (MEASURED_PEAKS.json holds no integer peak)",
                 "pair_kernel_share": pair_ms / dev_ms}
+    if not tree:
+        roofline["kernel_rows_per_pair"] = DIRECT_ROWS_PER_PAIR_T40 if tuned[3] == 3 else per_pair
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True, "scaling": "strong",
@@ -331,7 +350,8 @@ def run_ours(args, rank, world, local_rank):
                    "last_query": {"numerator": result.get(0), "denominator": result.get(1)},
                    "l2": "flushed between steps (256 MiB write); hot data (codewords 512 KiB) is L2-resident",
                    "rng": "Philox on device (value); the C library's rand() sequence (e2e)",
-                   "launch": {"kernel": kname, "terms_per_thread": tuned[0] or "fixed rule (32)",
+                   "launch": {"kernel": kname} if tree else
+                             {"kernel": kname, "terms_per_thread": tuned[0] or "fixed rule (32)",
                               "light_zero_bound": tuned[1] or "fixed rule (24)",
                               "chosen_by": "fixed rules (--no-tune)" if args.no_tune else
                               "csim_autotune on this query's G' and code"}},
@@ -384,24 +404,6 @@ def c3_queries(light=True, every=1):
     return out, len(recs)
 
 
-def pretune(gpu, qs):
-    """Tunes the thread-per-pair launches (csim_autotune) for every t bucket
-    the queries use, on the first query of each bucket (its G' and code), so
-    that no timed arm pays for tuning."""
-    from circuitsimulator_gb300 import backend
-
-    seen = set()
-    for q in qs:
-        cfg, projs = q["cfg"], q["projs"]
-        if cfg["exact"] or cfg["t"] // 4 in seen or not projs[0][0]:
-            continue
-        seen.add(cfg["t"] // 4)
-        e, k, norm, L = backend.decompose(cfg["t"], cfg["fidbound"], cfg["rank"], cfg["fidelity"], cfg["forceL"],
-                                          cfg["exact"], cfg["k"])
-        if not e:
-            gpu.autotune(cfg["t"], backend.projector(*projs[0]), [int(x) for x in L])
-
-
 def batch_compare(gpu, reps=3, light=True, every=1):
     """Batched vs plain queries/s on the c3 queries (the light ones by default,
     all 256 with light=False, every every-th of them with every > 1): the
@@ -411,7 +413,6 @@ def batch_compare(gpu, reps=3, light=True, every=1):
     qs, total = c3_queries(light=light, every=every)
     gpu.run_queries(qs[:4], batched=True)
     gpu.run_queries(qs[:4], batched=False)
-    pretune(gpu, qs)
     tp, tb = [], []
     same = True
     pairs = 0
@@ -516,9 +517,6 @@ def serve_compare(rate, count, seed=5, c5=False):
         return {"p50_ms": 1e3 * float(np.percentile(v, 50)), "p99_ms": 1e3 * float(np.percentile(v, 99)),
                 "max_ms": 1e3 * float(v[-1])}
 
-    tuner = backend.Backend(0)
-    pretune(tuner, qs)  # tuned launches for every t of the stream, shared by the process
-    tuner.close()
     srv = backend.Server(0)
     for t in [srv.submit(q) for q in qs[:8]]:  # warm-up: decompositions resident, buffers sized
         srv.wait(t)

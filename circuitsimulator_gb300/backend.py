@@ -264,7 +264,7 @@ class Backend:
         return int(self.lib.csim_launch_count(self.ctx))
 
     def set_option(self, option, value):
-        """CSIM_OPT_PAIR_KERNEL = 1 (0 thread-per-pair, 1 warp-per-pair), CSIM_OPT_PER_THREAD = 2,
+        """CSIM_OPT_PAIR_KERNEL = 1 (0 tree sum, 1..5 pair kernels, csim.h), CSIM_OPT_PER_THREAD = 2,
         CSIM_OPT_AUTOTUNE = 3 (1 tune on first use, 0 fixed rules)."""
         self._check(self.lib.csim_set_option(self.ctx, int(option), int(value)))
 

@@ -1,6 +1,6 @@
 // csim_tree.cuh — the sum of <theta|phi_x> over all codewords x of |L> as a
 // walk over a binary tree of partial contractions, written once for the device
-// (csim_tree.cu) and the host (a checker the CPU tests build).
+// (csim_tree.cu) and the host (a program the CPU tests build).
 //
 // A term phi_x of |L> is a product of |0> (x_c = 0) and |+> (x_c = 1)
 // (libcirc/stateprep.c:85-120), so <theta|phi_x> contracts theta's qubits one
