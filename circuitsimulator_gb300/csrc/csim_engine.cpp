@@ -207,8 +207,9 @@ static bool plan_query(csim_ctx* ctx, QueryRec* r);
 
 class Engine {
   public:
-    Engine(csim_ctx* ctx, int64_t round_pairs, int64_t round_states, int per_thread, int64_t budget)
+    Engine(csim_ctx* ctx, int64_t round_pairs, int64_t round_states, int per_thread, int64_t budget, bool fair)
         : ctx_(ctx),
+          fair_(fair),
           round_pairs_(round_pairs > 0 ? round_pairs : ((int64_t)1 << 26)),
           round_states_(round_states > 0 ? round_states : ((int64_t)1 << 16)),
           per_thread_(per_thread > 0 ? per_thread : 0),
@@ -284,6 +285,7 @@ class Engine {
   private:
     csim_ctx* ctx_;
     int64_t round_pairs_, round_states_;
+    bool fair_;  // a share of each round for every evaluation; else first come, first served
     int per_thread_;
     int64_t budget_;
     int64_t resident_ = 0, use_clock_ = 0;
@@ -596,7 +598,7 @@ int Engine::launch_round() {
     for (Eval* e : active_) nready += eval_ready(e) ? 1 : 0;
     const int64_t share = std::max<int64_t>(1, round_pairs_ / std::max(1, nready));
     int64_t ns = 0;
-    for (int pass = 0; pass < 2; pass++) {
+    for (int pass = fair_ ? 0 : 1; pass < 2; pass++) {
         for (Eval* e : active_) {
             if (!eval_ready(e) || ns >= round_states_) continue;
             int64_t n = (round_pairs_ - rs.pairs) / e->chi;
@@ -1237,7 +1239,7 @@ extern "C" int csim_run_queries(csim_ctx* ctx, int64_t nq, const csim_query* q, 
     stats_begin(ctx);
     if (!ctx->engine || ctx->engine->per_thread() != ctx->per_thread) {
         if (ctx->engine) engine_free(ctx->engine);
-        ctx->engine = new Engine(ctx, (int64_t)1 << 30, (int64_t)1 << 16, ctx->per_thread, 0);
+        ctx->engine = new Engine(ctx, (int64_t)1 << 30, (int64_t)1 << 16, ctx->per_thread, 0, false);
         const int rc = ctx->engine->init();
         if (rc) {
             engine_free(ctx->engine);
@@ -1393,7 +1395,7 @@ extern "C" int csim_server_create(const csim_server_config* cfg, csim_server** o
     auto s = std::make_unique<csim_server>();
     s->ctx = ctx;
     s->eng = std::make_unique<Engine>(ctx, cfg->round_pairs, cfg->round_states, cfg->per_thread,
-                                      cfg->hbm_budget_bytes);
+                                      cfg->hbm_budget_bytes, true);
     rc = s->eng->init();
     if (rc) {
         s->eng.reset();
