@@ -270,7 +270,7 @@ __device__ __forceinline__ void pair_l(WS<NR> st, uint64_t x, int& eps, int& p, 
             return;
         }
     }
-    exp_sum<NR, false>(st, eps, p, m, err);
+    exp_sum<NR, true>(st, eps, p, m, err);  // (any J: the C ABI sends asymmetric ones here)
     p -= k1 + k2;
 }
 

@@ -596,6 +596,25 @@ __device__ void exp_sum(WS<NR>& s, int& eps, int& p, int& m, int& err) {
     }
 }
 
+// Whether J is symmetric with J_xx = D1_x on the k variables, as every stabilizer state's is
+template <int NR>
+__device__ __forceinline__ bool consistent(const WS<NR>& s) {
+    const RW<NR> km = low_mask<NR>(s.k);
+    bool bad = false;
+#pragma unroll 4
+    for (int c = 0; c < s.k; c++) {
+        const RW<NR> col = ballot_bit<NR>(s.J, c) & km;
+#pragma unroll
+        for (int sl = 0; sl < NR; sl++) bad |= row_of<NR>(sl) == c && (s.J[sl] & km) != col;
+    }
+#pragma unroll
+    for (int sl = 0; sl < NR; sl++) {
+        const int x = row_of<NR>(sl);
+        bad |= x < s.k && getbit(s.J[sl], x) != getbit(s.D1, x);
+    }
+    return __any_sync(kFull, bad) == 0;
+}
+
 // ------------------------------------------------------------------ inner product
 // innerProductExact (stabilizer.c:589-659); st is a working copy of state1.
 template <int NR>
@@ -633,7 +652,9 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
     }
 #pragma unroll
     for (int sl = 0; sl < NR; sl++) st.J[sl] ^= t2.J[sl];
-    exp_sum<NR, false>(st, eps, p, m, err);
+    // (a J that no state has gives what the reference makes of it)
+    if (consistent<NR>(st)) exp_sum<NR, false>(st, eps, p, m, err);
+    else exp_sum<NR, true>(st, eps, p, m, err);
     p -= k1 + s2.k;
 }
 

@@ -101,3 +101,20 @@ def test_tree_rows_equal_pair_kernel(gpu, t, k, kind):
     (re0, im0, v0, n0, l0), (re1, im1, v1, n1, l1) = out
     assert (re0 == re1).all() and (im0 == im1).all() and v0 == v1
     assert (n0, l0) == (n1, l1)
+
+
+def test_inner_product_of_any_symmetric_or_asymmetric_form(gpu, oracle):
+    """A J that no state has (asymmetric, or with a diagonal other than D's) takes the steps that keep
+    the whole form, as the reference does."""
+    rs = np.random.RandomState(11)
+    for n in (2, 5, 17, 31, 33, 40, 64):
+        a, b = gpu.randomStabilizerState(n, 6, n), gpu.randomStabilizerState(n, 6, n + 1000)
+        for i in range(6):
+            st = (a, b)[i % 2]
+            k = max(1, int(st["k"][i]))
+            x, y = (int(v) for v in rs.randint(k, size=2))
+            st["J"][i][x] ^= np.uint64(1 << (y if i < 4 else x))
+        for i in range(6):
+            want = oracle.inner_product(a[i:i + 1], b[i:i + 1])
+            got = tuple(int(v[0]) for v in gpu.innerProductExact(a[i:i + 1], b[i:i + 1]))
+            assert got == tuple(want), (n, i)
