@@ -665,7 +665,7 @@ int Engine::launch_round() {
             j.states += sg.n;
         }
         for (WordJob& j : jobs) {
-            j.device = !words_on_host(j.t, j.states);
+            j.device = !words_on_host(j.t, j.states) && (csim::most_words(j.t) + 1) * j.states + 4096 <= csim::kRawMax;
             for (int w = 0; w < 2; w++)
                 if (!j.q->host_only[w]) {
                     const Eval* e = j.q->ev[w].get();

@@ -19,7 +19,7 @@ namespace csim {
 
 constexpr int kRawHistory = 34;                  // words in front of a buffer of raw words
 constexpr int kRawChunk = 31 * 16;               // words a warp makes
-constexpr int kRawJumps = 18;                    // jumps of 2^b chunks
+constexpr int kRawJumps = 20;                    // jumps of 2^b chunks
 constexpr int64_t kRawMax = (int64_t)kRawChunk << kRawJumps;
 constexpr int kMaxSegment = 1 << 16;             // words per segment, at most (16 bits each in shared memory)
 

@@ -62,3 +62,14 @@ def test_batched_draws_on_the_device_equal_the_hosts(gpu, count):
     for b, p, r in zip(batched, plain, rounds):
         assert b["numerator"] == p["numerator"] == r["numerator"]
         assert b["denominator"] == p["denominator"] == r["denominator"]
+
+
+def test_the_most_draws_of_a_round(gpu):
+    """2^16 states of 64 qubits, 1.3e8 words of one stream."""
+    rs = np.random.RandomState(64)
+    g = random_projector_rows(rs, 64, 3)
+    cfg = dict(quiet=1, verbose=0, noapprox=0, samples=32768, bins=1, t=64, k=1, exact=0, fidbound=1e-5, fidelity=0,
+               rank=0, forceL=0, forceSample=1)
+    q = {"cfg": cfg, "projs": [(*g, 64), (g[0][1:], g[1][1:], g[2][1:], 64)], "seed": 9, "rng": backend.RNG_LIBC}
+    b, p = gpu.run_queries([q], batched=True)[0], gpu.run_queries([q], batched=False)[0]
+    assert b["numerator"] == p["numerator"] and b["denominator"] == p["denominator"]
