@@ -291,8 +291,8 @@ __device__ __forceinline__ void store_node(uint32_t* out, int64_t count, uint32_
 // the lowest bit).  The parent's rows are copied to shared memory twice, so a lane
 // moves on from one sibling to the other without a load: a stage from 28 to 15
 // vertices took 985 us for 14.3e6 nodes with a node per thread, 576 with a pair.
-// Up to 32 vertices ALU-bound (83 to 90% of the pipe), above it by the latency of few
-// resident warps: shared memory holds 3 to 9 blocks (17% of the warps at 48 vertices).
+// Up to 32 vertices ALU-bound (75 to 86% of the pipe), above it by the latency of few
+// resident warps: shared memory holds 7 to 18 (12 at 48 vertices).
 // Nodes move as 16-byte vectors and several loads at a time: with a load per word and
 // no more than four in flight, rows of 64, 48 and 40 vertices took 39, 213 and 191 us
 // (300 states of 64 qubits, 2^14 terms), now 26, 107 and 92.

@@ -72,7 +72,9 @@ struct TreeLeafJob {
 };
 
 constexpr int kTreeRootWarps = 4;      // states per root block
-constexpr int kTreeStageThreads = 64;
+// a warp: with rows above 32 vertices shared memory limits what an SM holds, and blocks of 64 threads are
+// 1 to 1.6% slower (t = 57 and 64; up to t = 48 within 0.5%)
+constexpr int kTreeStageThreads = 32;
 constexpr int kTreeLeafThreads = 128;
 
 // wide: the jobs' states have more than 32 qubits
