@@ -281,7 +281,12 @@ __device__ __forceinline__ void store_node(uint32_t* out, int64_t count, uint32_
             const U32x4 v = rows.get_tail(u);
             if (tw == 1) *p = v.a;
             else if (tw == 2) *reinterpret_cast<uint2*>(p) = make_uint2(v.a, v.b);
-            else store_vector(p, v.a, v.b, v.c, v.d);
+            else if (tw == 4) store_vector(p, v.a, v.b, v.c, v.d);
+            else {
+                p[0] = v.a;
+                p[1] = v.b;
+                p[2] = v.c;
+            }
             p += tw * count;
         }
     }
@@ -320,8 +325,13 @@ __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStag
     } else {
         constexpr int tw = Rows<PL>::tail;
         copy_async_twice<16>(rows.p, copy, 4 * kTreeStageThreads, vectors, 4 * np, units);
-        copy_async_twice<4 * tw>(rows.tp, copy, tw * kTreeStageThreads, J.in + 4 * node_vectors(mp) * np + (int64_t)pi * tw,
-                                 tw * np, units);
+        const uint32_t* const tails = J.in + 4 * node_vectors(mp) * np + (int64_t)pi * tw;
+        if constexpr (tw == 3) {
+            for (int j = 0; j < 3; j++)
+                copy_async_twice<4>(rows.tp + j, copy, tw * kTreeStageThreads, tails + j, tw * np, units);
+        } else {
+            copy_async_twice<4 * tw>(rows.tp, copy, tw * kTreeStageThreads, tails, tw * np, units);
+        }
     }
     Work<W> a;
     W x;

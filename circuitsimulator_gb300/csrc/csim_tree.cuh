@@ -97,7 +97,7 @@ CSIM_HD_INLINE int row_units(int m) { return (m + 3) / 4; }
 // vertices up.  Consecutive chunks (tails) of a lane are `st` chunks (tails) apart.
 template <int PL>
 struct Rows {
-    static constexpr int tail = PL <= 4 ? 0 : (PL == 5 ? 1 : (PL == 6 ? 2 : 4));  // words
+    static constexpr int tail = PL <= 4 ? 0 : PL - 4;  // words
     uint32_t *p, *tp;  // this lane's first chunk, first tail
     int st;
     CSIM_HD static int chunks(int units) { return PL == 2 ? (units + 1) / 2 : units; }
@@ -118,12 +118,21 @@ struct Rows {
         else if constexpr (tail == 2) {
             const uint64_t v = *reinterpret_cast<const uint64_t*>(tails(u));
             return U32x4{(uint32_t)v, (uint32_t)(v >> 32), 0u, 0u};
+        } else if constexpr (tail == 3) {
+            const uint32_t* t = tails(u);
+            return U32x4{t[0], t[1], t[2], 0u};
         } else
             return *reinterpret_cast<const U32x4*>(tails(u));
     }
     CSIM_HD_INLINE void set_tail(int u, const U32x4& v) const {
         if constexpr (tail == 1) *tails(u) = v.a;
         else if constexpr (tail == 2) *reinterpret_cast<uint64_t*>(tails(u)) = (uint64_t)v.a | ((uint64_t)v.b << 32);
+        else if constexpr (tail == 3) {
+            uint32_t* t = tails(u);
+            t[0] = v.a;
+            t[1] = v.b;
+            t[2] = v.c;
+        }
         else *reinterpret_cast<U32x4*>(tails(u)) = v;
     }
     // row i; bits from 8 PL up (PL = 2, 3) are not the row's
@@ -552,7 +561,7 @@ CSIM_HD_INLINE void times_omega(I (&y)[4], int q) {
 // bits from m up are not zero: whoever reads a row masks it.
 CSIM_HD_INLINE int node_scalars(int m) { return m > 32 ? 2 : 1; }  // vectors
 CSIM_HD_INLINE int node_vectors(int m) { return node_scalars(m) + (m > 16 ? row_units(m) : Rows<2>::chunks(row_units(m))); }
-CSIM_HD_INLINE int row_tail(int m) { return m <= 32 ? 0 : (m <= 40 ? 1 : (m <= 48 ? 2 : 4)); }
+CSIM_HD_INLINE int row_tail(int m) { return m <= 32 ? 0 : row_planes(m) - 4; }
 CSIM_HD_INLINE int node_words(int m) { return 4 * node_vectors(m) + row_tail(m) * row_units(m) + (m > 16 ? 1 : 0); }
 CSIM_HD_INLINE uint32_t pack_status(int q, int iso, int dead) {
     return (uint32_t)(q & 7) | ((uint32_t)iso << 8) | (dead ? 0x80000000u : 0u);
