@@ -300,7 +300,7 @@ __device__ __forceinline__ void store_node(uint32_t* out, int64_t count, uint32_
 // resident warps: shared memory holds 7 to 18 (12 at 48 vertices).
 // Nodes move as 16-byte vectors and several loads at a time: with a load per word and
 // no more than four in flight, rows of 64, 48 and 40 vertices took 39, 213 and 191 us
-// (300 states of 64 qubits, 2^14 terms), now 26, 107 and 92.
+// (300 states of 64 qubits, 2^14 terms), now 24, 98 and 85.
 template <int PL, bool PAIRS>
 __global__ void __launch_bounds__(kTreeStageThreads) k_tree_stage(const TreeStageJob* jobs, int njobs) {
     using W = typename RowWord<PL>::type;
