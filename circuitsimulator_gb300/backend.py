@@ -33,6 +33,7 @@ OPT_PAIR_KERNEL = 1
 OPT_PER_THREAD = 2
 OPT_AUTOTUNE = 3
 OPT_DIRECT_SLOTS = 4
+OPT_DRAW_WORDS = 5
 RNG_PHILOX = 0
 RNG_LIBC = 1
 SEED_CONTINUE = (1 << 64) - 1

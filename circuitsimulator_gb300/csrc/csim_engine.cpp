@@ -173,6 +173,7 @@ struct QueryRec {
     uint64_t L[CSIM_MAX_QUBITS] = {0};
     int64_t chi = 0;
     LibcRand lr;
+    bool host_words = false;  // its words ran out on the device once: from then on the host makes them
     Decomp* dec = nullptr;
     double host_value[2] = {0, 0};
     bool host_only[2] = {false, false};
@@ -196,8 +197,9 @@ struct RoundSet {
     HostBuf hup, hdown;
     cudaEvent_t ev[4] = {};  // start, pair kernels start, pair kernels end, end
     std::vector<Seg> segs;
+    std::vector<std::pair<QueryRec*, int64_t>> draws;  // queries whose words the device makes, and their states
     int64_t pairs = 0;
-    size_t off_codes = 0, off_val = 0;
+    size_t off_codes = 0, off_val = 0, off_chains = 0;  // chains: a csim::DrawChain for each of draws
 };
 
 }  // namespace
@@ -665,7 +667,8 @@ int Engine::launch_round() {
             j.states += sg.n;
         }
         for (WordJob& j : jobs) {
-            j.device = !words_on_host(j.t, j.states) && (csim::most_words(j.t) + 1) * j.states + 4096 <= csim::kRawMax;
+            j.device = !j.q->host_words && !words_on_host(j.t, j.states) &&
+                       (csim::most_words(j.t) + 1) * j.states + 4096 <= csim::kRawMax;
             for (int w = 0; w < 2; w++)
                 if (!j.q->host_only[w]) {
                     const Eval* e = j.q->ev[w].get();
@@ -674,7 +677,7 @@ int Engine::launch_round() {
             if (!j.device) continue;
             double cum[CSIM_MAX_QUBITS + 1];
             cum_table(j.t, cum);
-            csim::draw_job(j.t, cum, j.states, 0, j.draw);
+            csim::draw_job(j.t, cum, j.states, ctx_->draw_percent, j.draw);
             j.q->lr.history(j.draw.history);
             j.nwords = 0;
         }
@@ -817,23 +820,26 @@ int Engine::launch_round() {
     const size_t w_cdir = align_up(w_canon + (any_direct ? (size_t)nother * csim::canon_bytes() : 0));
     const size_t w_crest = align_up(w_cdir + (any_direct ? (size_t)nother * 4 : 0));
     size_t work_bytes = align_up(w_crest + (any_direct ? (size_t)nother * 4 : 0));
-    // a device job's words, lengths, maps, offsets and its end
+    // a device job's words, lengths, maps and offsets
     auto draw_part = [](const csim::DrawJob& j, int part) {
         size_t at = 0;
         const size_t sizes[] = {(kRawHistory + (size_t)j.words) * 4, (size_t)j.padded() * 2, (size_t)j.map_words() * 4,
-                                (size_t)(j.states + 1) * 8, sizeof(csim::DrawChain)};
+                                (size_t)(j.states + 1) * 8};
         for (int i = 0; i < part; i++) at += align_up(sizes[i]);
         return at;
     };
+    rs.draws.clear();
     for (auto& j : jobs)
         if (j.device) {
             j.w_draw = work_bytes;
-            work_bytes += draw_part(j.draw, 5);
+            work_bytes += draw_part(j.draw, 4);
+            rs.draws.push_back({j.q, j.states});
         }
-    // download block: err (16 B), the pair launches' work-queue counter (kQueueOffset) | codes | values
+    // download block: err (16 B), the pair launches' work-queue counter (kQueueOffset) | codes | values | chains
     rs.off_codes = 256;
     rs.off_val = align_up(rs.off_codes + (size_t)ns * 4);
-    const size_t down_bytes = align_up(rs.off_val + (size_t)ns * 16);
+    rs.off_chains = align_up(rs.off_val + (size_t)ns * 16);
+    const size_t down_bytes = align_up(rs.off_chains + rs.draws.size() * sizeof(csim::DrawChain));
     if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) ||
         rs.down.ensure(down_bytes) || rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes))
         return fail(ctx_, CSIM_ERR_NOMEM, "round buffers (%lld states, %lld items)", (long long)ns,
@@ -850,7 +856,7 @@ int Engine::launch_round() {
             j.draw.len = (uint16_t*)(at + draw_part(j.draw, 1));
             j.draw.map = (uint32_t*)(at + draw_part(j.draw, 2));
             j.draw.offs = (int64_t*)(at + draw_part(j.draw, 3));
-            j.draw.chain = (csim::DrawChain*)(at + draw_part(j.draw, 4));
+            j.draw.chain = (csim::DrawChain*)(dd + rs.off_chains) + draws.size();
             draws.push_back(j.draw);
         }
     uint64_t* hproj = (uint64_t*)(hb + o_proj);
@@ -1087,7 +1093,15 @@ int Engine::complete_round() {
     device_ms += a;
     pair_ms += b;
     const unsigned char* hd = (const unsigned char*)rs.hdown.p;
-    const int err = *(const int*)hd;
+    int err = *(const int*)hd;
+    const csim::DrawChain* chains = (const csim::DrawChain*)(hd + rs.off_chains);
+    std::vector<QueryRec*> again;  // queries whose words ran out: these states once more (their streams have not gone on)
+    for (size_t i = 0; i < rs.draws.size(); i++)
+        if (chains[i].states < rs.draws[i].second) {
+            again.push_back(rs.draws[i].first);
+            again.back()->host_words = true;
+            err &= ~csim::kErrReplay;  // flagged by their draws
+        }
     const int* code = (const int*)(hd + rs.off_codes);
     const double* val = (const double*)(hd + rs.off_val);
     if (err) {
@@ -1102,6 +1116,10 @@ int Engine::complete_round() {
         Eval* e = sg.e;
         e->q->inflight -= sg.n;
         if (e->q->done) continue;  // failed in an earlier round
+        if (std::find(again.begin(), again.end(), e->q) != again.end()) {
+            e->next = std::min(e->next, sg.s0);
+            continue;
+        }
         const int* c = code + sg.slot0;
         const double* v = val + 2 * sg.slot0;
         int64_t np = 0;

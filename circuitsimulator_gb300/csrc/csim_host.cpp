@@ -95,6 +95,10 @@ extern "C" int csim_set_option(csim_ctx* ctx, int32_t option, int64_t value) {
         if (value != 0 && value != 1) return fail(ctx, CSIM_ERR_ARG, "autotune must be 0 or 1");
         ctx->autotune = (int)value;
         return CSIM_OK;
+    case CSIM_OPT_DRAW_WORDS:
+        if (value < 1 || value > 100) return fail(ctx, CSIM_ERR_ARG, "draw words must be 1..100 percent");
+        ctx->draw_percent = (int)value;
+        return CSIM_OK;
     default:
         return fail(ctx, CSIM_ERR_ARG, "unknown option %d", option);
     }
@@ -628,10 +632,10 @@ int put_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, cons
 }
 
 // The same on the device: *chain (device memory) counts the states that the words suffice for
-int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, int more, const uint32_t** dwords,
+int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, const uint32_t** dwords,
                      const int64_t** doffs, csim::DrawChain* chain) {
     csim::DrawJob j{};
-    csim::draw_job(t, cum, count, more, j);
+    csim::draw_job(t, cum, count, ctx->draw_percent, j);
     ctx->lr.history(j.history);
     void* v;
     CKR(dbuf(ctx, kBufWords, (kRawHistory + (size_t)j.words) * 4, &v));
@@ -646,14 +650,6 @@ int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, int
     if (csim::launch_draws(launch_of(ctx), &j, 1)) return fail(ctx, CSIM_ERR_CUDA, "word launch failed");
     *dwords = j.buf;
     *doffs = j.offs;
-    return 0;
-}
-
-// A batch whose states took more words than there were: its draws flagged that, and it runs
-// again with twice as many
-int more_words(csim_ctx* ctx, int* more) {
-    CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    if (++*more > 2) return fail(ctx, CSIM_ERR_DEVICE, "random states took more words than four times the longest");
     return 0;
 }
 
@@ -715,7 +711,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     std::vector<int> code;
     std::vector<__int128> acc;
     bool sent = !tree;
-    int more = 0;  // a batch that ran out of words runs again with twice as many
+    bool ran_out = false;  // of the device's words: the batch runs again with the host's, and its draws' flag is cleared
     for (int64_t o = 0; o < count;) {
         const int64_t c = std::min(batch, count - o);
         void* v;
@@ -742,14 +738,14 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         __int128* dpart = (__int128*)v;
         CK(cudaEventRecord(ctx->ev[0], ctx->stream));
         if (!tree) CK(cudaMemsetAsync(dpart, 0, nparts * sizeof(__int128), ctx->stream));
-        const bool on_host = libc && words_on_host(t, c);
+        const bool on_host = libc && (ran_out || words_on_host(t, c));
         csim::DrawChain chain{};
         csim::TreeDraw draw{};
         if (libc) {
             const uint32_t* dw;
             const int64_t* doff;
             if (on_host) CKR(put_state_words(ctx, t, hcum, c, &dw, &doff, &chain));
-            else CKR(make_state_words(ctx, t, hcum, c, more, &dw, &doff, (csim::DrawChain*)(dres + 16)));
+            else CKR(make_state_words(ctx, t, hcum, c, &dw, &doff, (csim::DrawChain*)(dres + 16)));
             draw = csim::TreeDraw{2, P->nstabs, 0, 0, dw, doff, in.cum, in.pm, in.pz, in.px, dcode, nullptr, 0, 0};
             if (!tree && csim::launch_random_states(launch_of(ctx), t, c, 2, 0, 0, dw, doff, in.cum, dth, nullptr))
                 return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
@@ -862,7 +858,8 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             CK(cudaGetLastError());
             if (libc && !on_host) memcpy(&chain, (const unsigned char*)v + 16, sizeof(chain));
             if (libc && chain.states < c) {
-                CKR(more_words(ctx, &more));
+                CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+                ran_out = true;
                 continue;
             }
             CKR(error_status(ctx, ((const int*)v)[2]));
@@ -874,6 +871,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             ctx->stats.states_live += live;
             ctx->stats.pairs += live * chi;
             o += c;
+            ran_out = false;
             continue;
         }
         CKR(dbuf(ctx, kBufAcc, (size_t)c * 4 * sizeof(__int128), &v));
@@ -889,7 +887,8 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             CKR(dget(ctx, &chain, (const csim::DrawChain*)(dres + 16), 1));
             CK(cudaStreamSynchronize(ctx->stream));
             if (chain.states < c) {
-                CKR(more_words(ctx, &more));
+                CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
+                ran_out = true;
                 continue;
             }
         }
@@ -912,6 +911,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             values[o + i] = scale * (a * a + b * b);
         }
         o += c;
+        ran_out = false;
     }
     return 0;
 }

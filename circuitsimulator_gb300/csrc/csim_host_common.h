@@ -466,6 +466,7 @@ struct csim_ctx {
     // autotuner (CSIM_OPT_AUTOTUNE): the tuned launch parameters live in a
     // process-wide table per device (csim_host.cpp), filled a t bucket at a time
     int direct_slots = 0;  // CSIM_OPT_DIRECT_SLOTS; 0 = direct_slots(t)
+    int draw_percent = 100;  // CSIM_OPT_DRAW_WORDS
     int autotune = 1;
     bool tuning = false;      // a tuning pass is running on this context (its trials use `trial`)
     csim_host::TpTune trial;  // the parameters of the trial in progress

@@ -11,6 +11,15 @@ namespace csim {
 
 struct GState;  // device image of csim_state (csim_warp.cuh)
 
+// device error flags (OR-ed into the per-launch error word)
+enum : int {
+    kErrRange = 1,        // p or k outside the range a normalized state allows
+    kErrReplay = 2,       // a replayed state needed more rand() words than given
+    kErrExpSum = 4,       // exponentialSumExact's "p0 != p1" / "odd m1-m0" branch
+    kErrGamma = 8,        // partialGamma/Gamma given an odd argument (reference asserts)
+    kErrArg = 16,         // bad per-item argument (n out of range ...)
+};
+
 struct Launch {
     cudaStream_t stream;
     int* d_err;         // device error word, OR of csim::kErr* flags

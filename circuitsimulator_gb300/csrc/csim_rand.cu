@@ -86,11 +86,11 @@ __device__ __forceinline__ int job_at(const int32_t (&first)[N], int n) {
 
 }  // namespace
 
-void draw_job(int t, const double* cum, int64_t states, int more, DrawJob& j) {
+void draw_job(int t, const double* cum, int64_t states, int percent, DrawJob& j) {
     draw_table(t, cum, j.table);
     j.entries = most_words(t);
     j.segment = chain_segment(states, j.entries);
-    j.words = (j.entries * states + 4096) << more;
+    j.words = (j.entries * states + 4096) * percent / 100;
     j.states = states;
 }
 

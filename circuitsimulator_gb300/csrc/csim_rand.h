@@ -61,9 +61,9 @@ inline int most_words(int t) {
     }
     return most;
 }
-// Fills a job but for its history and pointers.  cum: csim_host::cum_table.  Words: for that longest
-// sequence and a few thousand; 2^more times as many.
-void draw_job(int t, const double* cum, int64_t states, int more, DrawJob& j);
+// Fills a job but for its history and pointers.  cum: csim_host::cum_table.  Words: `percent` of that
+// longest sequence and a few thousand.
+void draw_job(int t, const double* cum, int64_t states, int percent, DrawJob& j);
 
 // Four launches for up to kDrawJobs jobs
 constexpr int kDrawJobs = 16;

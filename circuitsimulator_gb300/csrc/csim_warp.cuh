@@ -20,18 +20,11 @@
 
 #include <cstdint>
 
+#include "csim_internal.h"
+
 namespace csim {
 
 constexpr unsigned kFull = 0xffffffffu;
-
-// device error flags (OR-ed into the per-launch error word)
-enum : int {
-    kErrRange = 1,        // p or k outside the range a normalized state allows
-    kErrReplay = 2,       // a replayed state needed more rand() words than given
-    kErrExpSum = 4,       // exponentialSumExact's "p0 != p1" / "odd m1-m0" branch
-    kErrGamma = 8,        // partialGamma/Gamma given an odd argument (reference asserts)
-    kErrArg = 16,         // bad per-item argument (n out of range ...)
-};
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint64_t bit1(int i) { return 1ull << i; }

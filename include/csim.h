@@ -132,6 +132,9 @@ int csim_rng_position(csim_ctx *ctx, uint64_t seed, uint64_t first);
                                    non-pivot coordinates (n - k) go to the block-prefix kernel */
 #define CSIM_OPT_AUTOTUNE 3    /* 1 (default): tuned thread-per-pair launches, a t bucket tuned on first use; 0: fixed rules
                                   (the tree needs no tuning) */
+#define CSIM_OPT_DRAW_WORDS 5   /* the words that a batch of CSIM_RNG_LIBC states has made on the device, in percent
+                                  (1..100, default 100) of what almost every batch needs; where they run out the batch
+                                  is drawn again with words from the host */
 int csim_set_option(csim_ctx *ctx, int32_t option, int64_t value);
 
 /* The autotuner of the thread-per-pair launches (no counterpart in the

@@ -73,3 +73,59 @@ def test_the_most_draws_of_a_round(gpu):
     q = {"cfg": cfg, "projs": [(*g, 64), (g[0][1:], g[1][1:], g[2][1:], 64)], "seed": 9, "rng": backend.RNG_LIBC}
     b, p = gpu.run_queries([q], batched=True)[0], gpu.run_queries([q], batched=False)[0]
     assert b["numerator"] == p["numerator"] and b["denominator"] == p["denominator"]
+
+
+# percent of the words that a batch needs: none of its states but the first have any; some; all but a few
+@pytest.mark.parametrize("percent", [1, 60, 96])
+@pytest.mark.parametrize("t,count,kernel", [(3, 3000, 0), (40, 700, 0), (64, 17000, 0), (24, 900, 5)])
+def test_states_that_run_out_of_words(gpu, percent, t, count, kernel):
+    """A batch whose words run out on the device is drawn again with the host's: the same
+    values, and the stream goes on behind them."""
+    rs = np.random.RandomState(t)
+    rows = random_projector_rows(rs, t, max(1, t // 3))
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    L = [rand_word(rs, t) for _ in range(2)]
+    out = []
+    try:
+        gpu.set_option(backend.OPT_PAIR_KERNEL, kernel)
+        gpu.singleProjectorSample(P, L, False, 1, backend.RNG_PHILOX, 1)  # a pair kernel is tuned
+        for p in (100, percent):
+            gpu.set_option(backend.OPT_DRAW_WORDS, p)
+            n0 = gpu.launches
+            a = gpu.singleProjectorSample(P, L, False, count, backend.RNG_LIBC, 7)
+            n1 = gpu.launches
+            out.append((a, gpu.singleProjectorSample(P, L, False, count, backend.RNG_LIBC), n1 - n0))
+    finally:
+        gpu.set_option(backend.OPT_PAIR_KERNEL, 0)
+        gpu.set_option(backend.OPT_DRAW_WORDS, 100)
+    assert (out[0][0] == out[1][0]).all() and (out[0][1] == out[1][1]).all()
+    if percent < 90:
+        assert out[1][2] > out[0][2]  # it did run out
+
+
+@pytest.mark.parametrize("percent", [1, 60, 97])
+def test_a_query_out_of_words_leaves_the_others_alone(gpu, percent):
+    """Queries of one round: those whose words run out on the device get their states
+    in another round, with the host's words; all have their usual results."""
+    rs = np.random.RandomState(percent)
+    qs = []
+    for i in range(12):
+        t = int(rs.choice([5, 9, 24, 33, 64]))
+        g = random_projector_rows(rs, t, 4)
+        cfg = dict(quiet=1, verbose=0, noapprox=0, samples=400, bins=1, t=t, k=3, exact=0, fidbound=1e-5, fidelity=0,
+                   rank=0, forceL=0, forceSample=1)
+        if i % 4 == 3:
+            cfg.update(noapprox=1, forceSample=0, samples=1000)
+        qs.append({"cfg": cfg, "projs": [(*g, t), (g[0][1:], g[1][1:], g[2][1:], t)], "seed": 50 + i,
+                   "rng": backend.RNG_LIBC if i % 3 else backend.RNG_PHILOX})
+    want = gpu.run_queries(qs, batched=True)
+    plain = gpu.run_queries(qs, batched=False)
+    try:
+        gpu.set_option(backend.OPT_DRAW_WORDS, percent)
+        got = gpu.run_queries(qs, batched=True)
+    finally:
+        gpu.set_option(backend.OPT_DRAW_WORDS, 100)
+    for a, b, c in zip(want, got, plain):
+        assert b["status"] == 0
+        assert (a["numerator"], a["denominator"], a["pairs"]) == (b["numerator"], b["denominator"], b["pairs"])
+        assert (a["numerator"], a["denominator"]) == (c["numerator"], c["denominator"])
