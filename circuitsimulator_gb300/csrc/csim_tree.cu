@@ -151,9 +151,13 @@ __device__ void store_root(const TreeRootJob& J, uint32_t i, const WS<NR>& st, R
         had[q] = to_coords<W>(had[q], piv);
         if (r < t && !getbit(w.P, r)) store_row(J.out, J.count, i, t, r, had[q]);
     }
-    if (lane_id() == 0)
-        store_scalars(J.out, J.count, i, t, to_coords<W>(w.D1, piv), to_coords<W>(w.D2, piv) | bm, ~w.P & nm, J.x0,
+    if (lane_id() == 0) {
+        uint64_t x = J.x0;
+        for (int b = 0; b < J.slice; b++)
+            if (((J.first + i) >> b) & 1) x ^= J.gen[b];
+        store_scalars(J.out, J.count, i, t, to_coords<W>(w.D1, piv), to_coords<W>(w.D2, piv) | bm, ~w.P & nm, x,
                       pack_status(st.Q + w.dq, 0, 0));
+    }
 }
 
 }  // namespace
@@ -172,7 +176,7 @@ __global__ void __launch_bounds__(32 * kTreeRootWarps) k_tree_draw(const TreeRoo
     const int64_t i = ((int64_t)blockIdx.x - J.block0) * kTreeRootWarps + (threadIdx.x >> 5);
     if (i >= J.count) return;  // warp-uniform
     const TreeDraw& d = J.draw;
-    const int64_t a = J.first + i;
+    const int64_t a = (J.first + i) >> J.slice;
     int e = 0;
     const bool replay = d.mode == 1 || d.mode == 2;
     DevRng rng = make_rng(replay ? d.mode : 0, d.seed, d.id + a, d.words, replay ? d.offsets[a] : 0,
@@ -439,10 +443,11 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
         int state = 0;  // ROWS: the state, its row, and the term index so far (below 2^30)
         uint32_t row = 0, term = 0;
         if constexpr (ROWS) {
-            state = (int)(node >> J.nodes_log2);
+            const int64_t number = J.node0 + node;
+            state = (int)(number >> J.nodes_log2);
             row = (uint32_t)(J.row0 + state);
             for (int b = 0; b < J.nodes_log2; b++)
-                if ((node >> b) & 1) term ^= (uint32_t)J.term[J.je + b];
+                if ((number >> b) & 1) term ^= (uint32_t)J.term[J.je + b];
             for (int b = 0; b < J.split; b++)
                 if ((part >> b) & 1) term ^= term_s[split0 + b];
         }

@@ -31,15 +31,16 @@ struct TreeDraw {
     int32_t k, pad;
 };
 
-// root nodes of `count` states: state i of the job is state first + i of draw
+// root nodes of `count` trees: tree i of the job is number first + i, 2^slice for each state of draw
 struct TreeRootJob {
     TreeDraw draw;
     int64_t first;
     const uint8_t* perm;  // position -> coordinate (t of them)
-    uint32_t* out;        // node planes, one node per state
+    const uint64_t* gen;  // the `slice` generators whose sum a tree's number chooses
+    uint32_t* out;        // node planes, one node per tree
     int64_t count, block0;
-    uint64_t x0;          // the roots' X
-    int32_t t, pad;
+    uint64_t x0;          // the X of a state's first root
+    int32_t t, slice;
 };
 
 // nodes of level jc from nodes of level jp = jc + sub (`count` of them, out, < 2^32)
@@ -64,11 +65,12 @@ struct TreeLeafJob {
     int32_t split, reps, group, shift;  // sums are scaled by 2^{shift / 2}
     uint16_t gen[16];     // generators of the levels below je, positions < m
     // exactProjector rows: state a is row row0 + a; only its terms j > row are summed, term
-    // j == row is written to diag + 4 a
+    // j == row is written to diag + 4 a.  The job's first node is number node0, 2^nodes_log2 for
+    // each state
     const uint64_t* term; // the generators' parts of the term index, all levels
     __int128* diag;
-    int64_t row0;
-    int32_t nodes_log2, pad;  // log2 of the nodes per state
+    int64_t row0, node0;
+    int32_t nodes_log2, pad;
 };
 
 constexpr int kTreeRootWarps = 4;      // states per root block

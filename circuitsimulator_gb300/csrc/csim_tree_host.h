@@ -39,30 +39,25 @@ inline bool tree_rows_ok(const csim::tree::Plan& p) { return p.r == p.k; }
 // ones give each thread several nodes, so its reduction at the end is shared.
 struct TreeLeafShape {
     int split = 0, reps = 1, group = 1;
-    int64_t threads_per_state = 1, parts_per_state = 1;
+    int64_t threads_per_tree = 1, parts_per_tree = 1, parts_per_state = 1;
 };
 inline TreeLeafShape tree_leaf_shape(const csim::tree::Plan& p, int64_t count) {
     TreeLeafShape s;
     const int je = p.level.back();
-    const int64_t nodes = (int64_t)1 << (p.r - je);
+    const int64_t nodes = (int64_t)1 << (p.level[0] - je);
+    count <<= p.slice;
     while (s.split < je && ((count * nodes) << s.split) < (1 << 17)) s.split++;
     const int64_t parts = nodes << s.split;
     while (s.reps < 8 && parts >= 2 * 128 * s.reps && count * parts / (2 * s.reps) >= (1 << 19)) s.reps *= 2;
-    s.threads_per_state = parts / s.reps;
-    s.group = (int)std::min<int64_t>(s.threads_per_state, csim::kTreeLeafThreads);
-    s.parts_per_state = std::max<int64_t>(1, s.threads_per_state / csim::kTreeLeafThreads);
+    s.threads_per_tree = parts / s.reps;
+    s.group = (int)std::min<int64_t>(s.threads_per_tree, csim::kTreeLeafThreads);
+    s.parts_per_tree = std::max<int64_t>(1, s.threads_per_tree / csim::kTreeLeafThreads);
+    s.parts_per_state = s.parts_per_tree << p.slice;
     return s;
 }
 
-// Bytes of node planes per state in the two scratch halves (written levels
-// alternate between them)
-inline void tree_scratch_per_state(const csim::tree::Plan& p, int64_t (&half)[2]) {
-    half[0] = half[1] = 0;
-    for (size_t i = 0; i < p.level.size(); i++) {
-        const int64_t b = ((int64_t)csim::tree::node_words(p.vert[i]) * 4) << (p.r - p.level[i]);
-        half[i & 1] = std::max(half[i & 1], b);
-    }
-}
+// Bytes of node planes per state (each of its trees, one after another) in the two scratch halves
+inline void tree_scratch_per_state(const csim::tree::Plan& p, int64_t (&half)[2]) { csim::tree::tree_planes(p, half); }
 
 // Scratch of a run's node planes: every chunk pays the latency of its draws and first stages,
 // about 0.2 ms at 40 to 64 qubits (256 states of 57 qubits, 2^18 terms: 5.36 ms with 1 GB, 5.05 with
@@ -75,7 +70,7 @@ constexpr int kTreeMaxRows = 30;
 class TreeRun {
   public:
     // Splits the groups into chunks whose node planes fit reserve()'s budget (one
-    // state at least).  Returns the scratch bytes needed.
+    // tree at least).  Returns the scratch bytes needed.
     size_t layout(const std::vector<TreeGroup>& groups) {
         const size_t budget = budget_;
         chunks_.clear();
@@ -86,9 +81,10 @@ class TreeRun {
             int64_t half[2];
             tree_scratch_per_state(*g.plan, half);
             const int64_t per = half[0] + half[1];
-            for (int64_t f = 0; f < g.count;) {
+            const int64_t trees = g.count << g.plan->slice;
+            for (int64_t f = 0; f < trees;) {
                 const int64_t room = (int64_t)((budget > used ? budget - used : 0)) / std::max<int64_t>(1, per);
-                int64_t c = std::min(g.count - f, room);
+                int64_t c = std::min(trees - f, room);
                 if (c <= 0) {
                     if (!cur.pieces.empty()) {
                         chunks_.push_back(cur);
@@ -100,9 +96,9 @@ class TreeRun {
                     c = 1;
                 }
                 // equal chunks of a large group
-                if (cur.pieces.empty() && c < g.count - f) {
-                    const int64_t n = (g.count - f + c - 1) / c;
-                    c = (g.count - f + n - 1) / n;
+                if (cur.pieces.empty() && c < trees - f) {
+                    const int64_t n = (trees - f + c - 1) / c;
+                    c = (trees - f + n - 1) / n;
                 }
                 Piece pc{g, f, c, {used, 0}};
                 used += align((size_t)(half[0] * c));
@@ -110,7 +106,7 @@ class TreeRun {
                 used += align((size_t)(half[1] * c));
                 cur.pieces.push_back(pc);
                 f += c;
-                if (f < g.count) {  // the group's next states start a chunk of their own
+                if (f < trees) {  // the group's next trees start a chunk of their own
                     chunks_.push_back(cur);
                     scratch_ = std::max(scratch_, used);
                     cur.pieces.clear();
@@ -151,6 +147,8 @@ class TreeRun {
                 r.draw = p.g.draw;
                 r.first = p.first;
                 r.perm = p.g.dplan + 2 * 64 * 8;
+                r.gen = (const uint64_t*)p.g.dplan + pl.level[0];
+                r.slice = pl.slice;
                 r.x0 = pl.x0;
                 r.out = (uint32_t*)(scratch + p.off[0]);
                 r.count = p.count;
@@ -163,9 +161,9 @@ class TreeRun {
                 csim::TreeLeafJob l{};
                 const int je = pl.level.back();
                 l.in = (const uint32_t*)(scratch + p.off[(pl.level.size() - 1) & 1]);
-                l.part = p.g.part + 4 * p.first * s.parts_per_state;
-                l.in_count = p.count << (pl.r - je);
-                l.threads = p.count * s.threads_per_state;
+                l.part = p.g.part + 4 * p.first * s.parts_per_tree;
+                l.in_count = p.count << (pl.level[0] - je);
+                l.threads = p.count * s.threads_per_tree;
                 const int wc = std::max(0, pl.tv - 5) + (p.g.rows ? 4 : 0) + (pl.pairs ? 8 : 0);
                 l.block0 = lb[wc];
                 l.m = pl.vert.back();
@@ -178,9 +176,10 @@ class TreeRun {
                 l.shift = pl.t - pl.tv + 2 * (pl.k - pl.r);  // each codeword 2^{k - r} times
                 for (int j = 0; j < je; j++) l.gen[j] = (uint16_t)pl.gen[j];
                 if (p.g.rows) {
-                    l.row0 = p.g.row0 + p.first;
+                    l.node0 = p.first << (pl.level[0] - je);
+                    l.row0 = p.g.row0;
                     l.term = (const uint64_t*)p.g.dplan + 64;
-                    l.diag = p.g.diag + 4 * p.first;
+                    l.diag = p.g.diag;
                     l.nodes_log2 = pl.r - je;
                 }
                 lb[wc] += (l.threads + csim::kTreeLeafThreads - 1) / csim::kTreeLeafThreads;
@@ -201,8 +200,8 @@ class TreeRun {
                         j.in = (const uint32_t*)(scratch + p.off[(d - 1) & 1]);
                         j.out = (uint32_t*)(scratch + p.off[d & 1]);
                         j.gen = (const uint64_t*)p.g.dplan + pl.level[d];
-                        j.in_count = p.count << (pl.r - pl.level[d - 1]);
-                        j.count = p.count << (pl.r - pl.level[d]);
+                        j.in_count = p.count << (pl.level[0] - pl.level[d - 1]);
+                        j.count = p.count << (pl.level[0] - pl.level[d]);
                         j.block0 = sb;
                         j.mp = pl.vert[d - 1];
                         j.mc = pl.vert[d];
@@ -241,7 +240,7 @@ class TreeRun {
   private:
     struct Piece {
         TreeGroup g;
-        int64_t first, count;
+        int64_t first, count;  // trees
         size_t off[2];
     };
     struct Chunk {

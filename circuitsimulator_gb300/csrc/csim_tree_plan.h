@@ -7,11 +7,14 @@
 #include <cstdint>
 #include <vector>
 
+#include "csim_tree.cuh"
+
 namespace csim {
 namespace tree {
 
 struct Plan {
     int t = 0, k = 0, r = 0;      // qubits, rows of L, its rank
+    int slice = 0;                // a state's sum is that of 2^slice trees, one for each sum of the last `slice` generators
     int m[65] = {0};              // m[j]: vertices of a node of level j (m[r] = t)
     uint8_t perm[64] = {0};       // position -> coordinate; C_j lives on positions < m[j]
     uint64_t gen[64] = {0};       // gen[j]: generator of C_{j+1} over C_j, in positions
@@ -19,7 +22,7 @@ struct Plan {
                                   // the index of a sum of generators is their sum's if r = k
     uint64_t x0 = 0;              // a root's X
     bool pairs = false;           // terms of |H^t>: products over vertex pairs (join_pairs) instead of codewords
-    // levels of the written nodes, root (r) first; the last one is the leaf kernel's
+    // levels of the written nodes, root (r - slice) first; the last one is the leaf kernel's
     // entry.  vert: their vertices
     std::vector<int> level, vert;
     int tj = 0, tv = 0;           // the table level, largest j with m[j] <= 8, and the table's vertices:
@@ -140,8 +143,8 @@ inline double stage_seconds(int vp, int vc, double nodes) {
     const double latency = 4e-6 + 2 * stage_steps(vp, vc) * (0.35e-6 + 0.012e-6 * vp);
     return latency + nodes * stage_ops(vp, vc) / kTreeOpsPerSecond;
 }
-inline void choose_levels(Plan& p, int64_t count) {
-    const int r = p.r;
+inline void choose_tree_levels(Plan& p, int64_t count) {
+    const int r = p.r - p.slice;
     // candidates: index 0 the root (r, t), then (j, m[j]) for j = r - 1 .. tj, with the table's
     // vertices alone at level tj
     std::vector<int> lv{r}, vt{p.t};
@@ -185,6 +188,30 @@ inline void choose_levels(Plan& p, int64_t count) {
     for (int i = end; i >= 0; i = from[(size_t)i]) {
         p.level.insert(p.level.begin(), lv[(size_t)i]);
         p.vert.insert(p.vert.begin(), vt[(size_t)i]);
+    }
+}
+
+// Bytes of a tree's node planes in the two scratch halves (written levels alternate
+// between them)
+inline void tree_planes(const Plan& p, int64_t (&half)[2]) {
+    half[0] = half[1] = 0;
+    for (size_t i = 0; i < p.level.size(); i++) {
+        const int64_t b = ((int64_t)node_words(p.vert[i]) * 4) << (p.level[0] - p.level[i]);
+        half[i & 1] = std::max(half[i & 1], b);
+    }
+}
+
+// The most that one tree's node planes may take.  They grow with the terms (64 qubits: 3.3 GB for
+// 2^26, 49 GB for 2^30), so a larger state is several trees, each from a root of its own.  Random
+// codes of up to 2^20 terms are one tree a state.
+constexpr int64_t kTreePlanes = 64 << 20;
+
+inline void choose_levels(Plan& p, int64_t count) {
+    for (p.slice = 0;; p.slice++) {
+        choose_tree_levels(p, count << p.slice);
+        int64_t half[2];
+        tree_planes(p, half);
+        if (half[0] + half[1] <= kTreePlanes || p.r - p.slice <= p.tj) return;
     }
 }
 

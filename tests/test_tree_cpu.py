@@ -185,3 +185,34 @@ def test_scratch_of_the_memory_there_is(t, k, count, room):
     assert used <= max(budget, per) + 1024 and first == min(count, max(1, -(-count // max(1, -(-count // max(1, budget // per))))))
     assert (status == 0) == (used <= room)
     assert status == 0 or budget == 64 << 20
+
+
+def _native(name, headers):
+    src, so = os.path.join(HERE, "native", name + ".cpp"), os.path.join(HERE, "native", "_build", "lib%s.so" % name)
+    os.makedirs(os.path.dirname(so), exist_ok=True)
+    deps = [src] + [os.path.join(CSRC, f) for f in headers]
+    if not os.path.exists(so) or os.path.getmtime(so) < max(os.path.getmtime(f) for f in deps):
+        subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", src, "-o", so])
+    return C.CDLL(so)
+
+
+@pytest.mark.parametrize("t,k,count", [(64, 30, 3), (64, 26, 5), (64, 22, 40), (57, 24, 7), (48, 30, 2), (60, -1, 2),
+                                       (40, 16, 4096), (24, 8, 60), (9, 3, 5), (64, 0, 3)])
+@pytest.mark.parametrize("room", [1 << 40, (1 << 30) + 4096, 65 << 20])
+@pytest.mark.parametrize("rows", [0, 1])
+def test_any_tree_fits_the_smallest_scratch(t, k, count, room, rows):
+    """Node planes of up to 2^30 terms: a state of many terms is several trees, so the
+    smallest scratch will do; every tree is made once, every partial sum written once,
+    no launch writes what another one still reads or beyond the scratch, and rows'
+    leaves know the number of their first node."""
+    lib = _native("tree_jobs_check", ("csim_tree.h", "csim_tree_host.h", "csim_tree.cuh", "csim_tree_plan.h"))
+    rs = np.random.RandomState(t + k)
+    L = np.array([int(rand_word(rs, t)) for _ in range(max(k, 1))], dtype=np.uint64)
+    out = np.zeros(7, dtype=np.int64)
+    lib.tree_jobs(C.c_void_p(L.ctypes.data if k >= 0 else None), max(k, 0), t, C.c_int64(count), C.c_int64(room), rows,
+                  C.c_void_p(out.ctypes.data))
+    status, used, jobs, violations, trees, written, parts = out.tolist()
+    assert status == 0 and used <= room
+    assert violations == 0 and written == parts
+    assert (trees > 1) == (k > 21 or k < 0)
+    assert jobs <= 12 * (1 + 2 * trees * count * (64 << 20) // min(room, 4 << 30))

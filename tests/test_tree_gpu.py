@@ -118,3 +118,31 @@ def test_inner_product_of_any_symmetric_or_asymmetric_form(gpu, oracle):
             want = oracle.inner_product(a[i:i + 1], b[i:i + 1])
             got = tuple(int(v[0]) for v in gpu.innerProductExact(a[i:i + 1], b[i:i + 1]))
             assert got == tuple(want), (n, i)
+
+
+@pytest.mark.parametrize("t,k,kind,count", [(64, 23, "random", 5), (57, 22, "random", 3), (48, 23, "low", 3),
+                                            (64, 24, "repeated", 3)])
+def test_tree_sampler_in_several_trees(gpu, t, k, kind, count):
+    """States of so many terms that each is several trees."""
+    rs = np.random.RandomState(t + k)
+    rows = random_projector_rows(rs, t, t // 2)
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    L = _code(kind, t, k, rs)
+    for rng in (backend.RNG_PHILOX, backend.RNG_LIBC):
+        a = _values(gpu, 0, P, L, False, count, rng, 19)
+        assert a.any()
+        assert (a == _values(gpu, 2, P, L, False, count, rng, 19)).all()
+
+
+def test_batched_queries_in_several_trees(gpu):
+    rs = np.random.RandomState(2)
+    qs = []
+    for i, (t, k, s) in enumerate([(64, 22, 3), (57, 23, 2), (24, 9, 200), (64, 22, 2)]):
+        g = random_projector_rows(rs, t, 4)
+        cfg = dict(quiet=1, verbose=0, noapprox=0, samples=s, bins=1, t=t, k=k, exact=0, fidbound=1e-5, fidelity=0,
+                   rank=0, forceL=0, forceSample=1)
+        qs.append({"cfg": cfg, "projs": [(*g, t), (g[0][1:], g[1][1:], g[2][1:], t)], "seed": 5 + i,
+                   "rng": backend.RNG_LIBC if i % 2 else backend.RNG_PHILOX})
+    for a, b in zip(gpu.run_queries(qs, batched=True), gpu.run_queries(qs, batched=False)):
+        assert a["status"] == 0
+        assert (a["numerator"], a["denominator"], a["pairs"]) == (b["numerator"], b["denominator"], b["pairs"])
