@@ -72,10 +72,7 @@ struct DevBuf {
         p = nullptr;
         cap = 0;
         const size_t c = align_up(bytes + bytes / 4);
-        if (cudaMalloc(&p, c) != cudaSuccess) {
-            p = nullptr;
-            return CSIM_ERR_NOMEM;
-        }
+        if (!(p = device_memory(c))) return CSIM_ERR_NOMEM;
         cap = c;
         return 0;
     }
@@ -96,10 +93,7 @@ struct HostBuf {
         p = nullptr;
         cap = 0;
         const size_t c = align_up(bytes + bytes / 4);
-        if (cudaMallocHost(&p, c) != cudaSuccess) {
-            p = nullptr;
-            return CSIM_ERR_NOMEM;
-        }
+        if (!(p = pinned_memory(c))) return CSIM_ERR_NOMEM;
         cap = c;
         return 0;
     }
@@ -429,10 +423,8 @@ int Engine::ensure_decomp(QueryRec* r, bool rows, bool* tree, bool force, Decomp
     }
     // device memory of this decomposition; what one call cannot make is made by the next
     auto grow = [&](void** p, size_t bytes) {
-        if (cudaMalloc(p, bytes) != cudaSuccess) {
-            *p = nullptr;
+        if (!(*p = device_memory(bytes)))
             return fail(ctx_, CSIM_ERR_NOMEM, "decomposition of 2^%d terms on t = %d", r->k, r->q.t);
-        }
         d->bytes += align_up(bytes);
         resident_ += (int64_t)align_up(bytes);
         return 0;
@@ -472,10 +464,8 @@ int Engine::ensure_decomp(QueryRec* r, bool rows, bool* tree, bool force, Decomp
             return fail(ctx_, CSIM_ERR_CUDA, "codeword launch failed");
     }
     if (want_phis && !d->phis) {
-        if (cudaMalloc(&d->phis, (size_t)chi * sizeof(csim_state)) != cudaSuccess) {
-            d->phis = nullptr;
+        if (!(d->phis = (csim_state*)device_memory((size_t)chi * sizeof(csim_state))))
             return fail(ctx_, CSIM_ERR_NOMEM, "term states of 2^%lld terms", (long long)chi);
-        }
         d->bytes += align_up((size_t)chi * sizeof(csim_state));
         resident_ += (int64_t)align_up((size_t)chi * sizeof(csim_state));
         if (d->exact) {

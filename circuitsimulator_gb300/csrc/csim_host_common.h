@@ -505,6 +505,21 @@ inline int fail(csim_ctx* ctx, int code, const char* fmt, ...) {
         if (r_ != 0) return r_; \
     } while (0)
 
+// Device and pinned memory, or nullptr.  The runtime keeps a failed allocation's error, which
+// the next launch would take for its own: it is cleared.
+inline void* device_memory(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, bytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+inline void* pinned_memory(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMallocHost(&p, bytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+
 inline int dbuf(csim_ctx* ctx, int id, size_t bytes, void** out) {
     if (bytes == 0) bytes = 16;
     if (ctx->cap[id] < bytes) {
@@ -515,10 +530,7 @@ inline int dbuf(csim_ctx* ctx, int id, size_t bytes, void** out) {
             ctx->cap[id] = 0;
         }
         size_t c = bytes + bytes / 4;
-        if (cudaMalloc(&ctx->buf[id], c) != cudaSuccess) {
-            ctx->buf[id] = nullptr;
-            return fail(ctx, CSIM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", c);
-        }
+        if (!(ctx->buf[id] = device_memory(c))) return fail(ctx, CSIM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", c);
         ctx->cap[id] = c;
     }
     *out = ctx->buf[id];
@@ -545,10 +557,8 @@ inline int staged_room(csim_ctx* ctx, int slot, size_t bytes, void** out) {
         ctx->pin[slot] = nullptr;
         ctx->pin_cap[slot] = 0;
         const size_t c = bytes + bytes / 4;
-        if (cudaMallocHost(&ctx->pin[slot], c) != cudaSuccess) {
-            ctx->pin[slot] = nullptr;
+        if (!(ctx->pin[slot] = pinned_memory(c)))
             return fail(ctx, CSIM_ERR_NOMEM, "cudaMallocHost of %zu bytes failed", c);
-        }
         ctx->pin_cap[slot] = c;
     }
     *out = ctx->pin[slot];
@@ -556,9 +566,8 @@ inline int staged_room(csim_ctx* ctx, int slot, size_t bytes, void** out) {
 }
 // a larger slot with the first `keep` bytes of the old one (no copy of it is in flight)
 inline int staged_grow(csim_ctx* ctx, int slot, size_t bytes, size_t keep, void** out) {
-    void* p;
-    if (cudaMallocHost(&p, bytes) != cudaSuccess)
-        return fail(ctx, CSIM_ERR_NOMEM, "cudaMallocHost of %zu bytes failed", bytes);
+    void* const p = pinned_memory(bytes);
+    if (!p) return fail(ctx, CSIM_ERR_NOMEM, "cudaMallocHost of %zu bytes failed", bytes);
     memcpy(p, ctx->pin[slot], keep);
     cudaFreeHost(ctx->pin[slot]);
     ctx->pin[slot] = *out = p;

@@ -127,7 +127,6 @@ class TreeRun {
         for (budget_ = kTreeScratchMax;; budget_ /= 4) {
             const int rc = alloc(layout(groups));
             if (rc == 0 || budget_ <= kTreeScratchMin) return rc;
-            cudaGetLastError();  // the failed allocation's
         }
     }
 
