@@ -225,7 +225,6 @@ class Engine {
         for (auto& kv : decomps_) kv.second->release();
         cum_.release();
         iota_.release();
-        tree_scratch_.release();
     }
 
     int init() {
@@ -291,7 +290,6 @@ class Engine {
     int next_set_ = 0;
     std::deque<RoundSet*> inflight_;
     DevBuf cum_, iota_;
-    DevBuf tree_scratch_;  // node planes; rounds on the stream take turns
     TreeRun tree_run_;
     int64_t iota_n_ = 0;
     int bucket_of_[CSIM_MAX_QUBITS + 1] = {0};
@@ -299,6 +297,11 @@ class Engine {
     int nbuckets_ = 0;
 
     csim::Launch launch_on(int* d_err) { return csim::Launch{ctx_->stream, d_err, &ctx_->launches, ctx_->num_sms}; }
+    // the node planes' part of the memory budget, and the rest
+    size_t tree_budget() const {
+        return std::min(kTreeScratchMax, std::max(kTreeScratchMin, (size_t)budget_ / 2));
+    }
+    int64_t decomp_budget() const { return budget_ - (int64_t)ctx_->cap[kBufTreeScratch]; }
     int ensure_decomp(QueryRec* r, bool rows, bool* tree, bool force, Decomp** out);
     void finish_eval(Eval* e);
     void finish_query(QueryRec* r);
@@ -396,20 +399,20 @@ int Engine::ensure_decomp(QueryRec* r, bool rows, bool* tree, bool force, Decomp
     if (want_cws && !(d && d->cws)) add += table;
     if (want_plan && !(d && d->dplan)) add += align_up(kTreePlanBytes);
     if (want_phis && !(d && d->phis)) add += align_up((size_t)chi * sizeof(csim_state));
-    if (add && resident_ + (int64_t)add > budget_) {  // evict unused decompositions, least recently used first
+    if (add && resident_ + (int64_t)add > decomp_budget()) {  // evict unused decompositions, least recently used first
         std::vector<std::pair<int64_t, std::vector<uint64_t>>> lru;
         for (auto& kv : decomps_)
             if (kv.second->refs == 0 && kv.second.get() != d) lru.push_back({kv.second->last_use, kv.first});
         std::sort(lru.begin(), lru.end());
         for (auto& e : lru) {
-            if (resident_ + (int64_t)add <= budget_) break;
+            if (resident_ + (int64_t)add <= decomp_budget()) break;
             auto jt = decomps_.find(e.second);
             cudaStreamSynchronize(ctx_->stream);
             resident_ -= (int64_t)jt->second->bytes;
             jt->second->release();
             decomps_.erase(jt);
         }
-        if (resident_ + (int64_t)add > budget_ && !force) return 0;
+        if (resident_ + (int64_t)add > decomp_budget() && !force) return 0;
     }
     if (!d) {
         auto nd = std::make_unique<Decomp>();
@@ -784,8 +787,9 @@ int Engine::launch_round() {
         v.diag0 = ndiags;
         if (g.rows) ndiags += sg.n;
     }
-    if (tree_run_.reserve(groups, [&](size_t bytes) { return tree_scratch_.ensure(bytes); }))
-        return fail(ctx_, CSIM_ERR_NOMEM, "tree sum buffers (%lld states)", (long long)ns);
+    void* scratch = nullptr;
+    CKR(tree_run_.reserve(groups, [&](size_t bytes) { return tree_scratch(ctx_, bytes, tree_budget(), &scratch); },
+                          tree_budget()));
     std::vector<unsigned char> tree_jobs;
     tree_run_.build(nullptr, tree_jobs);  // for its size
     // upload block: projectors | segments | tree jobs | words | word offsets | state descriptors | items | ranges
@@ -1003,7 +1007,7 @@ int Engine::launch_round() {
         }
     }
     tree_run_.layout(groups);
-    tree_run_.build((unsigned char*)tree_scratch_.p, tree_jobs);
+    tree_run_.build((unsigned char*)scratch, tree_jobs);
     if (!tree_jobs.empty()) memcpy(hb + o_tjobs, tree_jobs.data(), tree_jobs.size());
     int* derr = (int*)dd;
     const csim::Launch L = launch_on(derr);

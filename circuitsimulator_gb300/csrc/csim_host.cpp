@@ -777,7 +777,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             g.part = dpart;
             void* scratch;
             unsigned char* djobs;
-            CKR(run.reserve({g}, [&](size_t bytes) { return dbuf(ctx, kBufTreeScratch, bytes, &scratch); }));
+            CKR(run.reserve({g}, [&](size_t bytes) { return tree_scratch(ctx, bytes, kTreeScratchMax, &scratch); }));
             run.build((unsigned char*)scratch, jobs);
             if (!sent) {
                 CKR(send_inputs(ctx, in, jobs, &djobs));
@@ -1180,7 +1180,7 @@ int tree_rows(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, 
     std::vector<unsigned char> jobs;
     void* scratch;
     unsigned char* djobs;
-    CKR(run.reserve({g}, [&](size_t bytes) { return dbuf(ctx, kBufTreeScratch, bytes, &scratch); }));
+    CKR(run.reserve({g}, [&](size_t bytes) { return tree_scratch(ctx, bytes, kTreeScratchMax, &scratch); }));
     run.build((unsigned char*)scratch, jobs);
     CKR(send_inputs(ctx, in, jobs, &djobs));
     if (run.launch(launch_of(ctx), djobs, ctx->ev[1]))

@@ -520,7 +520,8 @@ inline void* pinned_memory(size_t bytes) {
     return nullptr;
 }
 
-inline int dbuf(csim_ctx* ctx, int id, size_t bytes, void** out) {
+// Buffer `id` with `bytes` of room or more (slack: bytes that a new one has in addition)
+inline int dbuf(csim_ctx* ctx, int id, size_t bytes, void** out, size_t slack = SIZE_MAX) {
     if (bytes == 0) bytes = 16;
     if (ctx->cap[id] < bytes) {
         if (ctx->buf[id]) {
@@ -529,12 +530,23 @@ inline int dbuf(csim_ctx* ctx, int id, size_t bytes, void** out) {
             ctx->buf[id] = nullptr;
             ctx->cap[id] = 0;
         }
-        size_t c = bytes + bytes / 4;
+        const size_t c = bytes + std::min(slack, bytes / 4);
         if (!(ctx->buf[id] = device_memory(c))) return fail(ctx, CSIM_ERR_NOMEM, "cudaMalloc of %zu bytes failed", c);
         ctx->cap[id] = c;
     }
     *out = ctx->buf[id];
     return 0;
+}
+
+// The tree sum's scratch: one for all estimators of a context (they take turns on its stream), of at
+// most `most` bytes unless more are asked for.  It is given up for a larger one only where the memory
+// for that seems to be there.
+inline int tree_scratch(csim_ctx* ctx, size_t bytes, size_t most, void** out) {
+    const size_t cap = ctx->cap[kBufTreeScratch];
+    size_t room, total;
+    if (cap < bytes && cudaMemGetInfo(&room, &total) == cudaSuccess && room + cap < bytes)
+        return fail(ctx, CSIM_ERR_NOMEM, "no %zu bytes for node planes", bytes);
+    return dbuf(ctx, kBufTreeScratch, bytes, out, most > bytes ? most - bytes : 0);
 }
 
 template <class T>

@@ -121,10 +121,10 @@ class TreeRun {
         return scratch_;
     }
 
-    // layout() for the largest budget whose scratch `alloc` (bytes -> 0 or an error) finds memory for
+    // layout() for the largest budget, `most` at most, whose scratch `alloc` (bytes -> 0 or an error) finds memory for
     template <class Alloc>
-    int reserve(const std::vector<TreeGroup>& groups, Alloc alloc) {
-        for (budget_ = kTreeScratchMax;; budget_ /= 4) {
+    int reserve(const std::vector<TreeGroup>& groups, Alloc alloc, size_t most = kTreeScratchMax) {
+        for (budget_ = most;; budget_ = std::max(budget_ / 4, kTreeScratchMin)) {
             const int rc = alloc(layout(groups));
             if (rc == 0 || budget_ <= kTreeScratchMin) return rc;
         }

@@ -307,7 +307,9 @@ typedef struct csim_server csim_server;
 typedef struct csim_server_config {
     int32_t device;
     int32_t per_thread;           /* terms per thread per work item (0: by t)  */
-    int64_t hbm_budget_bytes;     /* resident decompositions + round buffers   */
+    int64_t hbm_budget_bytes;     /* resident decompositions and node planes: the planes take half
+                                     of it at most (4 GB at most, 64 MB at least); the rounds'
+                                     states, words and sums come on top (0: 8 GB) */
     int64_t round_pairs;          /* inner products per round (0: 2^26)        */
     int64_t round_states;         /* states per round (0: 2^16)                */
 } csim_server_config;

@@ -48,3 +48,50 @@ def test_a_call_after_one_without_memory(rng):
         assert (again == small).all()
     finally:
         gpu.close()
+
+
+def _query(t, k, samples, seed=1):
+    rs = np.random.RandomState(t)
+    g = random_projector_rows(rs, t, 6)
+    cfg = dict(quiet=1, verbose=0, noapprox=0, samples=samples, bins=1, t=t, k=k, exact=0, fidbound=1e-5, fidelity=0,
+               rank=0, forceL=0, forceSample=1)
+    return {"cfg": cfg, "projs": [(*g, t), (g[0][1:], g[1][1:], g[2][1:], t)], "seed": seed, "rng": backend.RNG_PHILOX}
+
+
+def test_scratch_of_a_context():
+    """One scratch of 4 GB at most for the samplers and the query engine: 4096 states of
+    2^16 terms on 40 qubits take 5.3 GB of node planes at once."""
+    backend.Backend(0).close()
+    warm = backend.Backend(0)  # (the kernels' own memory)
+    warm.run_queries([_query(40, 16, 100)], batched=True)
+    warm.close()
+    before = _free()
+    gpu = backend.Backend(0)
+    try:
+        P, L = _problem(40, 16)
+        gpu.singleProjectorSample(P, L, False, 4096, backend.RNG_PHILOX, 5)
+        one = before - _free()
+        gpu.run_queries([_query(40, 16, 2048), _query(40, 15, 4096)], batched=True)
+        both = before - _free()
+        assert 4 << 30 > one > 2 << 30 and both < (4 << 30) + (200 << 20), (one, both)
+    finally:
+        gpu.close()
+
+
+@pytest.mark.parametrize("budget", [1 << 30, 16 << 20])
+def test_scratch_of_a_server(budget):
+    """Node planes take half of the memory budget at most, or 64 MB."""
+    gpu = backend.Backend(0)
+    q = _query(40, 16, 3000)
+    want = gpu.run_queries([q], batched=True)[0]
+    gpu.close()
+    before = _free()
+    srv = backend.Server(0, hbm_budget_bytes=budget, round_pairs=1 << 29)
+    try:
+        tickets = [srv.submit(q) for _ in range(3)]
+        got = [srv.wait(t) for t in tickets]
+        held = before - _free()
+    finally:
+        srv.close()
+    assert all((r["numerator"], r["denominator"]) == (want["numerator"], want["denominator"]) for r in got)
+    assert held < max(budget // 2, 64 << 20) + (150 << 20), held
