@@ -787,9 +787,19 @@ int Engine::launch_round() {
         v.diag0 = ndiags;
         if (g.rows) ndiags += sg.n;
     }
+    // without memory for the round its queries fail, the others go on
+    auto no_memory = [&] {
+        for (const Seg& sg : rs.segs) {
+            fail_query(sg.e->q, CSIM_ERR_NOMEM);
+            sg.e->q->inflight -= sg.n;
+        }
+        next_set_ ^= 1;  // this set is free, the other one may be in flight
+        return 0;
+    };
     void* scratch = nullptr;
-    CKR(tree_run_.reserve(groups, [&](size_t bytes) { return tree_scratch(ctx_, bytes, tree_budget(), &scratch); },
-                          tree_budget()));
+    if (tree_run_.reserve(groups, [&](size_t bytes) { return tree_scratch(ctx_, bytes, tree_budget(), &scratch); },
+                          tree_budget()))
+        return no_memory();
     std::vector<unsigned char> tree_jobs;
     tree_run_.build(nullptr, tree_jobs);  // for its size
     // upload block: projectors | segments | tree jobs | words | word offsets | state descriptors | items | ranges
@@ -835,9 +845,10 @@ int Engine::launch_round() {
     rs.off_chains = align_up(rs.off_val + (size_t)ns * 16);
     const size_t down_bytes = align_up(rs.off_chains + rs.draws.size() * sizeof(csim::DrawChain));
     if (rs.up.ensure(up_bytes) || rs.work.ensure(work_bytes) ||
-        rs.down.ensure(down_bytes) || rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes))
-        return fail(ctx_, CSIM_ERR_NOMEM, "round buffers (%lld states, %lld items)", (long long)ns,
-                    (long long)nitems);
+        rs.down.ensure(down_bytes) || rs.hup.ensure(up_bytes) || rs.hdown.ensure(down_bytes)) {
+        fail(ctx_, CSIM_ERR_NOMEM, "round buffers (%lld states, %lld items)", (long long)ns, (long long)nitems);
+        return no_memory();
+    }
     unsigned char* hb = (unsigned char*)rs.hup.p;
     unsigned char* db = (unsigned char*)rs.up.p;
     unsigned char* wb = (unsigned char*)rs.work.p;

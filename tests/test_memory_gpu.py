@@ -95,3 +95,29 @@ def test_scratch_of_a_server(budget):
         srv.close()
     assert all((r["numerator"], r["denominator"]) == (want["numerator"], want["denominator"]) for r in got)
     assert held < max(budget // 2, 64 << 20) + (150 << 20), held
+
+
+def _words_query(t, samples, rng):
+    q = _query(t, 4, samples, seed=3)
+    q["rng"] = rng
+    return q
+
+
+def test_a_round_without_memory_fails_its_queries_only():
+    """A query whose round finds no memory fails; the server and the queries behind it go on."""
+    small = _words_query(64, 700, backend.RNG_LIBC)
+    gpu = backend.Backend(0)
+    want = gpu.run_queries([small], batched=True)[0]
+    gpu.close()
+    srv = backend.Server(0)
+    try:
+        first = srv.wait(srv.submit(small))
+        with full_device(64 << 20):
+            big = srv.wait(srv.submit(_words_query(64, 20000, backend.RNG_LIBC)))
+            again = srv.wait(srv.submit(small))
+        after = srv.wait(srv.submit(_words_query(64, 20000, backend.RNG_LIBC)))
+        for r in (first, again):
+            assert (r["status"], r["numerator"], r["denominator"]) == (0, want["numerator"], want["denominator"])
+        assert big["status"] == -4 and after["status"] == 0
+    finally:
+        srv.close()
