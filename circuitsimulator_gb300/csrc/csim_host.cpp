@@ -653,10 +653,11 @@ int make_state_words(csim_ctx* ctx, int t, const double* cum, int64_t count, con
     return 0;
 }
 
-// Draws `count` states, projects them onto P, sums their terms on the GPU, and
-// returns singleProjectorSample's value for each (innerprod.c:88-144).
-int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, int exact, int64_t count,
-                  int rng, uint64_t seed, double* values) {
+// Draws `count` states, `batch` at a time, projects them onto P, sums their terms on the GPU, and
+// returns singleProjectorSample's value for each (innerprod.c:88-144).  *done: the states whose values
+// there are, also on an error (the streams stand behind them then).
+int sample_batches(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, int exact, int64_t count,
+                   int rng, uint64_t seed, int64_t batch, double* values, int64_t* done) {
     const int t = P->nqubits;
     CKR(check_code(ctx, t, exact, L, k));
     if (rng != CSIM_RNG_LIBC && rng != CSIM_RNG_PHILOX) return fail(ctx, CSIM_ERR_ARG, "unknown rng %d", rng);
@@ -678,7 +679,6 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
     const int P2 = 2 * t;
     const int64_t chunk = chunk_for(chi);
     const int pt = tn.per_thread;
-    const int64_t batch = 1 << 14;
     const int64_t shape_count = std::min(count, batch);
     if (tree) tree_plan_for(ctx, exact, L, k, t, shape_count);
     const int64_t nchunks = tree ? tree_leaf_shape(ctx->tree_plan, shape_count).parts_per_state
@@ -755,7 +755,6 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             if (!tree && csim::launch_random_states(launch_of(ctx), t, c, 0, ctx->philox_seed, ctx->philox_next,
                                                     nullptr, nullptr, in.cum, dth, nullptr))
                 return fail(ctx, CSIM_ERR_CUDA, "random state launch failed");
-            ctx->philox_next += c;
         }
         if (!tree && csim::launch_project(launch_of(ctx), nr, dth, c, P->nstabs, in.pm, in.pz, in.px, dcode))
             return fail(ctx, CSIM_ERR_CUDA, "projection launch failed");
@@ -867,10 +866,11 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             const int64_t live = *(const int64_t*)v;
             memcpy(values + o, (const unsigned char*)v + head, (size_t)c * 8);
             if (libc) ctx->lr.set_history(chain.history);
+            else ctx->philox_next += c;
             ctx->stats.states += c;
             ctx->stats.states_live += live;
             ctx->stats.pairs += live * chi;
-            o += c;
+            *done = o += c;
             ran_out = false;
             continue;
         }
@@ -894,6 +894,7 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
         }
         CKR(finish(ctx));
         if (libc) ctx->lr.set_history(chain.history);
+        else ctx->philox_next += c;
         CKR(stats_batch(ctx));
         const double scale = pow(2, t);
         ctx->stats.states += c;
@@ -910,10 +911,25 @@ int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int
             const double a = re * pf, b = im * pf;
             values[o + i] = scale * (a * a + b * b);
         }
-        o += c;
+        *done = o += c;
         ran_out = false;
     }
     return 0;
+}
+
+// sample_batches with batches that there is memory for
+int sample_values(csim_ctx* ctx, const csim_projector* P, const uint64_t* L, int k, int exact, int64_t count,
+                  int rng, uint64_t seed, double* values) {
+    int64_t o = 0;
+    for (int64_t batch = std::min<int64_t>(count, 1 << 14);; batch = std::max<int64_t>(64, batch / 4)) {
+        int64_t done = 0;
+        const int rc = sample_batches(ctx, P, L, k, exact, count - o, rng, o ? CSIM_SEED_CONTINUE : seed, batch, values + o,
+                                      &done);
+        o += done;
+        if (rc != CSIM_ERR_NOMEM || batch <= 64) return rc;
+        CK(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));  // (states whose words ran out)
+        CK(cudaStreamSynchronize(ctx->stream));
+    }
 }
 
 }  // namespace

@@ -39,12 +39,13 @@ def test_a_call_after_one_without_memory(rng):
     gpu = backend.Backend(0)
     try:
         P, L = _problem(64, 10)
-        small = gpu.singleProjectorSample(P, L, False, 600, rng, 5)  # (its kernels are loaded)
-        with full_device(128 << 20):
+        small = gpu.singleProjectorSample(P, L, False, 40, rng, 5)  # (its kernels are loaded)
+        large = _problem(64, 20)  # 50 MB of node planes for a state
+        with full_device(16 << 20):
             with pytest.raises(backend.CsimError) as e:
-                gpu.singleProjectorSample(P, L, False, 1 << 14, backend.RNG_LIBC, 5)
+                gpu.singleProjectorSample(*large, False, 64, backend.RNG_PHILOX, 5)
             assert e.value.code == -4, e.value  # CSIM_ERR_NOMEM
-            again = gpu.singleProjectorSample(P, L, False, 600, rng, 5)
+            again = gpu.singleProjectorSample(P, L, False, 40, rng, 5)
         assert (again == small).all()
     finally:
         gpu.close()
@@ -121,3 +122,25 @@ def test_a_round_without_memory_fails_its_queries_only():
         assert big["status"] == -4 and after["status"] == 0
     finally:
         srv.close()
+
+
+@pytest.mark.parametrize("t,k,count,rng,leave", [(64, 6, 20000, backend.RNG_LIBC, 100), (40, 16, 2000, backend.RNG_LIBC, 90),
+                                                 (57, 17, 300, backend.RNG_PHILOX, 90), (12, -1, 20000, backend.RNG_LIBC, 12)])
+def test_a_sampler_in_the_memory_there_is(t, k, count, rng, leave):
+    """Batches of fewer states where a batch of 2^14 finds no memory: the same values, and
+    the streams go on behind them."""
+    gpu = backend.Backend(0)
+    try:
+        P, L = _problem(t, max(k, 1))
+        L = None if k < 0 else L
+        want = gpu.singleProjectorSample(P, L, k < 0, count, rng, 5)
+        more = gpu.singleProjectorSample(P, L, k < 0, 100, rng)
+        gpu.close()
+        gpu = backend.Backend(0)
+        with full_device(leave << 20):
+            got = gpu.singleProjectorSample(P, L, k < 0, count, rng, 5)
+            assert gpu.last_stats().states == count
+            assert (gpu.singleProjectorSample(P, L, k < 0, 100, rng) == more).all()
+        assert (got == want).all()
+    finally:
+        gpu.close()
