@@ -146,3 +146,32 @@ def test_batched_queries_in_several_trees(gpu):
     for a, b in zip(gpu.run_queries(qs, batched=True), gpu.run_queries(qs, batched=False)):
         assert a["status"] == 0
         assert (a["numerator"], a["denominator"], a["pairs"]) == (b["numerator"], b["denominator"], b["pairs"])
+
+
+def test_tree_sampler_across_chunks(gpu):
+    """Node planes of 4200 states (40 qubits, 2^16 terms) are 4.9 GB, more than the scratch
+    takes at once: planes written again for later states, and partial sums from there on."""
+    rs = np.random.RandomState(3)
+    rows = random_projector_rows(rs, 40, 12)
+    P = backend.projector(rows[0], rows[1], rows[2], 40)
+    L = [rand_word(rs, 40) for _ in range(16)]
+    for rng in (backend.RNG_LIBC, backend.RNG_PHILOX):
+        assert (_values(gpu, 0, P, L, False, 4200, rng, 5) == _values(gpu, 5, P, L, False, 4200, rng, 5)).all()
+
+
+@pytest.mark.parametrize("t,lo", [(48, 0), (40, 1000)])
+def test_tree_rows_across_chunks(gpu, t, lo):
+    """The rows of 2^14 terms: 9 and 12 GB of node planes."""
+    rs = np.random.RandomState(3)
+    L = [rand_word(rs, t) for _ in range(14)]
+    rows = random_projector_rows(rs, t, 2)
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    out = []
+    try:
+        for kernel in (0, 1):
+            gpu.set_option(backend.OPT_PAIR_KERNEL, kernel)
+            out.append(gpu.exactProjectorRows(P, L, False, lo, 1 << 14))
+    finally:
+        gpu.set_option(backend.OPT_PAIR_KERNEL, 0)
+    assert out[0][0].any()
+    assert (out[0][0] == out[1][0]).all() and (out[0][1] == out[1][1]).all()
