@@ -175,3 +175,70 @@ def test_tree_rows_across_chunks(gpu, t, lo):
         gpu.set_option(backend.OPT_PAIR_KERNEL, 0)
     assert out[0][0].any()
     assert (out[0][0] == out[1][0]).all() and (out[0][1] == out[1][1]).all()
+
+
+@pytest.mark.parametrize("t,count", [(33, 5), (34, 4), (36, 3), (41, 3), (44, 2)])
+def test_tree_sampler_of_many_pairs(gpu, t, count):
+    """Terms of |H^t> with rows above 32 vertices, where the stages copy them past the registers."""
+    rs = np.random.RandomState(t)
+    rows = random_projector_rows(rs, t, 3)
+    P = backend.projector(rows[0], rows[1], rows[2], t)
+    for rng in (backend.RNG_PHILOX, backend.RNG_LIBC):
+        a = _values(gpu, 0, P, None, True, count, rng, 12)
+        assert a.any() and (a == _values(gpu, 1, P, None, True, count, rng, 12)).all()
+
+
+def _block(rs, n):
+    """n commuting independent Pauli rows (phases, x, z) of a random graph state with random
+    local Cliffords, and its state vector."""
+    while True:
+        adj = np.triu(rs.randint(2, size=(n, n)), 1)
+        adj = adj + adj.T
+        x, z = [1 << a for a in range(n)], [sum(1 << b for b in range(n) if adj[a][b]) for a in range(n)]
+        for q in range(n):
+            for _ in range(rs.randint(3)):  # X -> Z -> Y -> X
+                for a in range(n):
+                    xb, zb = (x[a] >> q) & 1, (z[a] >> q) & 1
+                    x[a] ^= (xb ^ (xb ^ zb)) << q
+                    z[a] ^= (zb ^ xb) << q
+        ph = [(bin(a & b).count("1") & 1) + 2 * int(rs.randint(2)) for a, b in zip(x, z)]
+        psi = rs.standard_normal(1 << n) + 1j * rs.standard_normal(1 << n)
+        y = np.arange(1 << n)
+        for p, a, b in zip(ph, x, z):
+            sign = 1.0 - 2.0 * (np.array([bin(v & b).count("1") for v in y]) & 1)
+            psi = 0.5 * (psi + 1j ** p * sign * psi[y ^ a])
+        if np.linalg.norm(psi) > 1e-6:
+            return (ph, x, z), psi / np.linalg.norm(psi)
+
+
+@pytest.mark.parametrize("t", [16, 33, 42, 49, 57, 60])
+def test_tree_sampler_of_pairs_in_closed_form(gpu, t):
+    """A projector onto one state, a product of states of six qubits: a sample is 0 or
+    2^t 2^-c |sum|^2, the sum over all 2^(t/2) terms of |H^t> a product of the blocks' sums.
+    Up to 2^30 terms and rows of 60 vertices, beyond what a pair kernel can check."""
+    rs = np.random.RandomState(t)
+    pair = 0.5 * np.array([1, 1, 1, -1]) + np.array([1, 0, 0, 1]) / np.sqrt(2)  # CZ|++> and (|00> + |11>) / sqrt2
+    one = np.array([1, 1]) / np.sqrt(2) + np.array([1, 0])                      # |+> and |0>
+    ph, xs, zs, amp, q = [], [], [], 1.0, 0
+    while q < t:
+        n = min(6, t - q)
+        terms = np.ones(1)
+        for i in range(0, n - 1, 2):
+            terms = np.kron(pair, terms)
+        if n % 2:
+            terms = np.kron(one, terms)
+        s = 0.0
+        while abs(s) < 1e-9:
+            rows, psi = _block(rs, n)
+            s = np.vdot(psi, terms)
+        amp *= abs(s) ** 2
+        ph += rows[0]
+        xs += [v << q for v in rows[1]]
+        zs += [v << q for v in rows[2]]
+        q += n
+    P = backend.projector(ph, xs, zs, t)
+    vals = gpu.singleProjectorSample(P, None, True, 12, backend.RNG_PHILOX, 1)
+    assert vals.any()
+    for v in vals[vals != 0]:
+        c = t - np.log2(v / amp)
+        assert abs(c - round(c)) < 1e-9 and 0 <= round(c) <= t, (v, amp, c)
