@@ -189,7 +189,7 @@ struct Seg {
 struct RoundSet {
     DevBuf up, work, down;
     HostBuf hup, hdown;
-    cudaEvent_t ev[4] = {};  // start, pair kernels start, pair kernels end, end
+    cudaEvent_t ev[4] = {};  // start, sums over terms start, end, end
     std::vector<Seg> segs;
     std::vector<std::pair<QueryRec*, int64_t>> draws;  // queries whose words the device makes, and their states
     int64_t pairs = 0;
@@ -1025,10 +1025,12 @@ int Engine::launch_round() {
     CK(cudaEventRecord(rs.ev[0], ctx_->stream));
     CK(cudaMemcpyAsync(db, hb, up_bytes, cudaMemcpyHostToDevice, ctx_->stream));
     CK(cudaMemsetAsync(derr, 0, 16, ctx_->stream));
+    if (!draws.empty() && csim::launch_draws(L, draws.data(), (int)draws.size()))
+        return fail(ctx_, CSIM_ERR_CUDA, "word launch failed");
     if (csim::launch_draw_project(L, (const csim::DrawDesc*)(db + o_desc), nother, (csim::GState*)(wb + w_states),
                                   dcode))
         return fail(ctx_, CSIM_ERR_CUDA, "draw/project launch failed");
-    CK(cudaEventRecord(rs.ev[1], ctx_->stream));
+    if (nother) CK(cudaEventRecord(rs.ev[1], ctx_->stream));  // without them it is recorded behind the first roots
     const csim::PairItem* ditems = (const csim::PairItem*)(db + o_items);
     unsigned long long* const queue = (unsigned long long*)(dd + kQueueOffset);
     // direct launches: the states in pivot form; those with more non-pivot
@@ -1068,10 +1070,9 @@ int Engine::launch_round() {
     }
     if (csim::launch_items_warp(L, ditems + nitp, niw, dstates, dcode, part + 4 * nitp, partd + 4 * nitp))
         return fail(ctx_, CSIM_ERR_CUDA, "pair launch failed");
-    if (!draws.empty() && csim::launch_draws(L, draws.data(), (int)draws.size()))
-        return fail(ctx_, CSIM_ERR_CUDA, "word launch failed");
     if (ndiags > nitems) CK(cudaMemsetAsync(partd + 4 * nitems, 0, (size_t)(ndiags - nitems) * 64, ctx_->stream));
-    if (!groups.empty() && tree_run_.launch(L, db + o_tjobs)) return fail(ctx_, CSIM_ERR_CUDA, "tree launch failed");
+    if (!groups.empty() && tree_run_.launch(L, db + o_tjobs, nother ? nullptr : rs.ev[1]))
+        return fail(ctx_, CSIM_ERR_CUDA, "tree launch failed");
     CK(cudaEventRecord(rs.ev[2], ctx_->stream));
     if (csim::launch_seg_values(L, (const csim::ValueSeg*)(db + o_vsegs), (int)nseg, ns, part, partd,
                                 (const int64_t*)(db + o_range), (const int64_t*)(db + o_range2),

@@ -104,7 +104,8 @@ int64_t csim_launch_count(const csim_ctx *ctx);
  * times come from CUDA events recorded on the context's stream. */
 typedef struct csim_stats {
     double device_ms;        /* first kernel start .. last kernel end, summed over batches */
-    double pair_kernel_ms;   /* the (theta, term) pair kernel alone                        */
+    double pair_kernel_ms;   /* of it the sums over terms: the pair kernels, or the tree from
+                                behind its first states' draws (those of later chunks included) */
     int64_t states;          /* random states drawn                                        */
     int64_t states_live;     /* states not annihilated by the projector                    */
     int64_t pairs;           /* inner products computed (live states x terms)              */

@@ -258,3 +258,15 @@ def test_server_wait_timeout_and_shutdown_with_work_queued():
     tickets = [srv.submit(q) for q in heavy]
     assert srv.wait(tickets[-1], timeout=0.0) is None
     srv.close()  # shuts down with work pending: must not hang
+
+
+@pytest.mark.parametrize("rng", [backend.RNG_PHILOX, backend.RNG_LIBC])
+def test_pair_kernel_time_leaves_the_draws_out(be, rng):
+    """Many states and two terms: most of the device's time is theirs, not the sums'."""
+    rs = np.random.RandomState(1)
+    g = random_projector_rows(rs, 64, 3)
+    q = {"cfg": _cfg(64, k=1, samples=8000), "projs": [(*g, 64), (g[0][1:], g[1][1:], g[2][1:], 64)], "seed": 1, "rng": rng}
+    be.run_queries([q], batched=True)
+    be.run_queries([q], batched=True)
+    st = be.last_stats()
+    assert 0 < st.pair_kernel_ms < 0.6 * st.device_ms, (st.pair_kernel_ms, st.device_ms)
