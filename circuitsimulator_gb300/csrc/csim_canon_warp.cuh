@@ -10,9 +10,6 @@
 
 namespace csim {
 
-__device__ __forceinline__ uint64_t ballot64(bool lo, bool hi) {
-    return (uint64_t)__ballot_sync(kFull, lo) | ((uint64_t)__ballot_sync(kFull, hi) << 32);
-}
 // coordinate-indexed mask of a variable-indexed one (variable a -> its pivot coordinate)
 template <class W>
 __device__ __forceinline__ W to_coords(W v, const unsigned char* piv) {

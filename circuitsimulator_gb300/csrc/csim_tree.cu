@@ -301,7 +301,7 @@ __device__ __forceinline__ void store_node(uint32_t* out, int64_t count, uint32_
 // moves on from one sibling to the other without a load: a stage from 28 to 15
 // vertices took 985 us for 14.3e6 nodes with a node per thread, 576 with a pair.
 // Up to 32 vertices ALU-bound (75 to 86% of the pipe), above it by the latency of few
-// resident warps: shared memory holds 7 to 18 (12 at 48 vertices).
+// resident warps: shared memory holds 6 to 18 (6 at 64 vertices, 12 at 48).
 // Nodes move as 16-byte vectors and several loads at a time: with a load per word and
 // no more than four in flight, rows of 64, 48 and 40 vertices took 39, 213 and 191 us
 // (300 states of 64 qubits, 2^14 terms), now 24, 98 and 85.
@@ -451,7 +451,9 @@ __global__ void __launch_bounds__(kTreeLeafThreads, 6) k_tree_leaf(const TreeLea
             for (int b = 0; b < J.split; b++)
                 if ((part >> b) & 1) term ^= term_s[split0 + b];
         }
-        int y[4] = {0, 0, 0, 0};  // this part's sum, relative to 2^{iso0 / 2}
+        // this part's sum, relative to 2^{iso0 / 2}: at most 2^16 leaves of at most 2^12.  iso0 / 2 is at
+        // most 24, a thread takes 8 parts and a sum 128 threads: z is at most 2^62
+        int y[4] = {0, 0, 0, 0};
         // table nodes two at a time, in Gray code order
         for (int s = 0; s < nsub; s += 2) {
             if (s) x ^= gen_s[tj + __ffs(s) - 1];
@@ -650,13 +652,11 @@ int launch_tree_stage(const Launch& L, const TreeStageJob* jobs, int njobs, int6
     if (njobs <= 0 || blocks <= 0) return 0;
     const auto kernel = pairs ? stage_kernel<true>(planes) : stage_kernel<false>(planes);
     if (blocks > 0x7fffffff || !kernel || mmax < 1 || row_planes(mmax) != planes) return -1;
-    // two copies of every lane's rows: at most 64 KB
+    // two copies of every lane's rows: 32 KB for rows of 64 vertices
+    static_assert(2 * 4 * (4 + 4) * 16 * kTreeStageThreads <= 48 * 1024, "shared memory of a stage's block");
     const int units = row_units(mmax);
     const int chunks = planes == 2 ? Rows<2>::chunks(units) : units;
     const size_t smem = (size_t)2 * 4 * (4 * chunks + row_tail(mmax) * units) * kTreeStageThreads;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess)
-        return -1;
     kernel<<<(unsigned)blocks, kTreeStageThreads, smem, L.stream>>>(jobs, njobs);
     (*L.launches)++;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;

@@ -53,7 +53,6 @@ __device__ __forceinline__ int popcount(uint32_t w) { return __popc(w); }
 __device__ __forceinline__ int popcount(uint64_t w) { return __popcll(w); }
 __device__ __forceinline__ int parity(uint32_t w) { return __popc(w) & 1; }
 __device__ __forceinline__ int parity(uint64_t w) { return __popc((uint32_t)w ^ (uint32_t)(w >> 32)) & 1; }
-__device__ __forceinline__ int par64(uint64_t w) { return parity(w); }
 // of a word that is not 0
 __device__ __forceinline__ int first_bit(uint32_t w) { return __ffs((int)w) - 1; }
 __device__ __forceinline__ int first_bit(uint64_t w) { return __ffsll((long long)w) - 1; }
@@ -626,7 +625,7 @@ __device__ void inner_product(WS<NR> st, const WS<NR>& s2, int k1, int& eps, int
     const bool trivial = (s2.Q == 0) && (s2.D1 == 0ull) && (s2.D2 == 0ull) && !any_row_nonzero<NR>(s2.J);
     WS<NR> t2 = s2;
     if (!trivial) {
-        // (a < s2.k: G_b lies in the space of s2)
+        // (a < s2.k: the shrinks left every G_b with an even overlap with the other Gbar_a, dual or not)
         const RW<NR> y = ballot_par<NR>(s2.B, st.h ^ s2.h);
         RW<NR> R[NR];
         RowPair<NR>* const rows = warp_rows<NR>();

@@ -122,8 +122,9 @@ int csim_last_stats(const csim_ctx *ctx, csim_stats *out);
 int csim_rng_position(csim_ctx *ctx, uint64_t seed, uint64_t first);
 
 /* Tuning options (no counterpart in the reference). */
-#define CSIM_OPT_PAIR_KERNEL 1 /* |L> terms: 0 = the samplers sum them as a tree of shared contractions, other calls
-                                  run one thread per pair, the tuner's kernel (default); 1 = one warp
+#define CSIM_OPT_PAIR_KERNEL 1 /* terms: 0 (default) = the samplers, the exactProjector and the query engine sum them as a
+                                  tree of shared contractions (up to 2^30 terms; exactProjector of codes with independent
+                                  rows), what is left runs one thread per pair, the tuner's kernel; 1 = one warp
                                   per pair; 2 = one thread per pair, block-shared top-bit shrinks; 3 = one thread per
                                   pair, per-thread runs of codewords with shared top-bit shrinks; 4 = as 2, one
                                   launch per occupancy class of the codewords' zero counts; 5 = one thread per
@@ -301,8 +302,8 @@ int csim_backend_serve(FILE *in, FILE *out, int device);
  * products, and runs them in shared launches while the host prepares the next
  * round.  Queries submitted while others are on the GPU join the next round
  * once their decomposition fits the device-memory budget; decompositions
- * (codeword tables, term states) stay resident and are shared by queries with
- * the same t and code.  Results are the same as csim_run_queries gives. */
+ * (tree plans; codeword tables and term states for the pair kernels) stay
+ * resident and are shared by queries with the same t and code.  Results are the same as csim_run_queries gives. */
 typedef struct csim_server csim_server;
 
 typedef struct csim_server_config {
