@@ -266,7 +266,8 @@ class Backend:
 
     def set_option(self, option, value):
         """CSIM_OPT_PAIR_KERNEL = 1 (0 tree sum, 1..5 pair kernels, csim.h), CSIM_OPT_PER_THREAD = 2,
-        CSIM_OPT_AUTOTUNE = 3 (1 tune on first use, 0 fixed rules)."""
+        CSIM_OPT_AUTOTUNE = 3 (1 tune on first use, 0 fixed rules), CSIM_OPT_DIRECT_SLOTS = 4,
+        CSIM_OPT_DRAW_WORDS = 5 (percent)."""
         self._check(self.lib.csim_set_option(self.ctx, int(option), int(value)))
 
     def autotune(self, t, P=None, L=None):
